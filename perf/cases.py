@@ -172,6 +172,17 @@ def tolerance(case):
 
 
 # ---- one case on the GPU ---------------------------------------------------------------------------------------------
+_context = None
+
+
+def _shared_context():
+    """The one context (device and stream) of this process: a serving program's steps follow one another on it."""
+    global _context
+    if _context is None:
+        _context = pkg.Context(0)
+    return _context
+
+
 class _Step:
     """Arena, page table, component and buffers of one case: what a serving program keeps between steps."""
 
@@ -194,7 +205,7 @@ class _Step:
         total = int(pages_of.sum()) * layers
         num_pages = total + total // 8 + 1
         page_bytes = 2 * hkv * page * d * esz
-        self.context = pkg.Context(0)
+        self.context = _shared_context()
         self.arena = normal(num_pages, page_bytes // esz)
         torch.cuda.synchronize()
         self.pages = pkg.PageArena(self.context, num_pages, page_bytes, device_ptr=self.arena)
@@ -299,11 +310,10 @@ class _Step:
     def __del__(self):
         if sys.is_finalizing():
             return
-        for name in ("graph", "gqa", "table", "pages", "context"):
+        torch.cuda.synchronize()
+        for name in ("graph", "gqa", "table", "pages"):
             held = getattr(self, name, None)
             if held is not None:
-                if name == "graph":
-                    self.context.sync()
                 held.close()
 
 
