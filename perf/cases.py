@@ -183,41 +183,66 @@ def _shared_context():
     return _context
 
 
-class _Step:
-    """Arena, page table, component and buffers of one case: what a serving program keeps between steps."""
+class _Inputs:
+    """What the seed draws for a case: requests in their order, the arena's values, which pages each row owns, and the
+    step's tensors.  Needs no object of the package, so that ``exact`` starts from the same numbers."""
 
     def __init__(self, case, seed):
-        self.case = case
-        code, dtype, esz = _DTYPES[case["dtype"]]
+        dtype, esz = _DTYPES[case["dtype"]][1:]
         hq, hkv, d, page, layers = (case[k] for k in ("q_heads", "kv_heads", "head_dim", "page", "layers"))
-        front = self.front = case["front"]
+        front = case["front"]
         rng = np.random.default_rng(seed)
         gen = torch.Generator(device="cuda").manual_seed(int(seed))
         order = rng.permutation(case["requests"])
-        ctx, run = (x[order] for x in _lengths(case))
-        n, tokens = len(ctx), int(run.sum())
+        self.ctx, self.run = ctx, run = [x[order] for x in _lengths(case)]
+        n, self.tokens = len(ctx), int(run.sum())
 
         def normal(*shape):
             return torch.empty(shape, dtype=dtype, device="cuda").normal_(generator=gen)
 
         held = ctx if front == "draft" else ctx + run
-        pages_of = -(-held // page)
-        total = int(pages_of.sum()) * layers
-        num_pages = total + total // 8 + 1
-        page_bytes = 2 * hkv * page * d * esz
-        self.context = _shared_context()
-        self.arena = normal(num_pages, page_bytes // esz)
-        torch.cuda.synchronize()
-        self.pages = pkg.PageArena(self.context, num_pages, page_bytes, device_ptr=self.arena)
-        ids = case["ids_per_block"]
-        layout = pkg.GQAPageTableLayout(n, layers, -(-int(pages_of.max()) // ids), ids)
-        self.table = pkg.GQARequestPageTable(self.context, layout)
-        pool, at = rng.permutation(num_pages).astype(np.uint32), 0
+        self.pages_of = -(-held // page)
+        total = int(self.pages_of.sum()) * layers
+        self.num_pages = total + total // 8 + 1
+        self.page_bytes = 2 * hkv * page * d * esz
+        self.arena = normal(self.num_pages, self.page_bytes // esz)
+        pool, at = rng.permutation(self.num_pages).astype(np.uint32), 0
+        self.rows = {}
         for slot in range(n):
             for layer in range(layers):
-                self.table.write_row(slot, layer, pool[at:at + int(pages_of[slot])])
-                at += int(pages_of[slot])
-        self.gqa = pkg.GQA(self.context, pkg.GQAConfig(hq, hkv, d, 1.0 / math.sqrt(d), page_bytes, code, layout, tokens))
+                self.rows[slot, layer] = pool[at:at + int(self.pages_of[slot])]
+                at += int(self.pages_of[slot])
+        self.shape_q, self.shape_kv = (layers, self.tokens, hq, d), (layers, self.tokens, hkv, d)
+        if front == "gated":
+            self.projection = normal(layers, self.tokens, (2 * hq + 2 * hkv) * d)
+        else:
+            self.q, self.k, self.v = normal(*self.shape_q), normal(*self.shape_kv), normal(*self.shape_kv)
+        if front in ("norm", "gated"):
+            # the 256-wide profiles rotate a quarter of the head, the others all of it
+            self.rope_dim, self.eps, self.theta = 64 if d == 256 else d, 1e-6, 1e6
+            self.weights = [(1.0 + 0.1 * torch.from_numpy(rng.standard_normal(d))).to(torch.bfloat16) for _ in range(2)]
+
+
+class _Step:
+    """Arena, page table, component and buffers of one case: what a serving program keeps between steps."""
+
+    def __init__(self, case, seed):
+        self.case = case
+        code, dtype = _DTYPES[case["dtype"]][:2]
+        hq, hkv, d, layers = (case[k] for k in ("q_heads", "kv_heads", "head_dim", "layers"))
+        front = self.front = case["front"]
+        given = _Inputs(case, seed)
+        ctx, run, n, tokens = given.ctx, given.run, len(given.ctx), given.tokens
+        self.context = _shared_context()
+        self.arena = given.arena
+        torch.cuda.synchronize()
+        self.pages = pkg.PageArena(self.context, given.num_pages, given.page_bytes, device_ptr=self.arena)
+        ids = case["ids_per_block"]
+        layout = pkg.GQAPageTableLayout(n, layers, -(-int(given.pages_of.max()) // ids), ids)
+        self.table = pkg.GQARequestPageTable(self.context, layout)
+        for (slot, layer), row in given.rows.items():
+            self.table.write_row(slot, layer, row)
+        self.gqa = pkg.GQA(self.context, pkg.GQAConfig(hq, hkv, d, 1.0 / math.sqrt(d), given.page_bytes, code, layout, tokens))
 
         slots = np.arange(n, dtype=np.uint32)
         if front == "draft":  # every draft token is a row of its own at the last history position
@@ -227,21 +252,20 @@ class _Step:
         else:
             self.batch = (slots, ctx.astype(np.uint32), np.concatenate([[0], np.cumsum(run)]).astype(np.uint32))
         self.tokens = tokens
-        shape_q, shape_kv = (layers, tokens, hq, d), (layers, tokens, hkv, d)
+        shape_q = given.shape_q
         zeros = lambda shape, kind=dtype: torch.zeros(shape, dtype=kind, device="cuda")  # noqa: E731
         self.out = zeros(shape_q)
         self.answer = {"out": self.out}
-        self.per_layer = []
         if front == "host":
-            self.q, self.k, self.v = (normal(*s[1:]).cpu().pin_memory() for s in (shape_q, shape_kv, shape_kv))
+            self.q, self.k, self.v = (x[0].cpu().pin_memory() for x in (given.q, given.k, given.v))
             self.out = torch.zeros(shape_q[1:], dtype=dtype).pin_memory()
             self.answer = {"out": self.out}
         elif front == "gated":
-            self.projection = normal(layers, tokens, (2 * hq + 2 * hkv) * d)
+            self.projection = given.projection
             self.q, self.gates = zeros(shape_q), zeros(shape_q)
             self.answer.update(q=self.q, gates=self.gates)
         else:
-            self.q_in, self.k, self.v = normal(*shape_q), normal(*shape_kv), normal(*shape_kv)
+            self.q_in, self.k, self.v = given.q, given.k, given.v
             self.q = self.q_in
             if front == "norm":
                 self.q = zeros(shape_q)
@@ -252,11 +276,8 @@ class _Step:
         if front not in ("draft",):
             self.answer["pages"] = self.arena
         if front in ("norm", "gated"):
-            # the 256-wide profiles rotate a quarter of the head, the others all of it
-            rope = pkg.NormRopeConfig(64 if d == 256 else d, 1e-6, 1e6, 0, 1.0, 1.0, 32.0, 1.0, 1, 0)
-            weights = [(1.0 + 0.1 * torch.from_numpy(rng.standard_normal(d))).to(torch.bfloat16).view(torch.int16)
-                       .numpy().view(np.uint16) for _ in range(2)]
-            self.gqa.set_norm_rope(rope, *weights)
+            rope = pkg.NormRopeConfig(given.rope_dim, given.eps, given.theta, 0, 1.0, 1.0, 32.0, 1.0, 1, 0)
+            self.gqa.set_norm_rope(rope, *(w.view(torch.int16).numpy().view(np.uint16) for w in given.weights))
         self.layers = list(range(layers))
         torch.cuda.synchronize()
         self.graph = None
@@ -323,3 +344,86 @@ def prepare(case, seed):
 
 def run(state):
     return state.step()
+
+
+# ---- the same step in 64 bits ----------------------------------------------------------------------------------------
+def _norm_rope(x, weight, positions, given):
+    """RMSNorm over the head and RoPE of its first ``rope_dim`` dims, x [tokens][heads][D] in float64."""
+    x = x * torch.rsqrt((x * x).mean(-1, keepdim=True) + given.eps) * weight
+    half = given.rope_dim // 2
+    inverse = given.theta ** (-torch.arange(half, dtype=torch.float64, device=x.device) / half)
+    angle = (positions[:, None] * inverse)[:, None]
+    a, b = x[..., :half], x[..., half:2 * half]
+    return torch.cat([a * angle.cos() - b * angle.sin(), a * angle.sin() + b * angle.cos(), x[..., 2 * half:]], -1)
+
+
+def _softmax_values(q, k, v, group, scale, first=None):
+    """(o, m, l) of q [rows][Hq][D] over k, v [keys][Hkv][D]; with `first`, row i sees keys [0, first + i]."""
+    parts = []
+    for head in range(q.shape[1]):
+        s = q[:, head] @ k[:, head // group].T * scale
+        if first is not None:
+            keys = torch.arange(k.shape[0], device=q.device)
+            s.masked_fill_(keys[None] > first + torch.arange(q.shape[0], device=q.device)[:, None], -math.inf)
+        m = s.max(-1).values
+        w = torch.exp(s - m[:, None])
+        parts.append(((w @ v[:, head // group]) / w.sum(-1, keepdim=True), m, w.sum(-1)))
+    return [torch.stack(x, 1) for x in zip(*parts)]
+
+
+def exact(case, seed):
+    """What ``run`` returns for these inputs, by plain torch in float64.  The arena comes back where the step computes
+    rows of it (norm and RoPE) and it is small; elsewhere its rows are copies."""
+    if work(case)["flops"] > 4e11:
+        return None
+    given = _Inputs(case, seed)
+    hq, hkv, d, page, front = (case[k] for k in ("q_heads", "kv_heads", "head_dim", "page", "front"))
+    group, scale = hq // hkv, 1.0 / math.sqrt(d)
+    tokens, layers = given.tokens, case["layers"]
+    starts = np.concatenate([[0], np.cumsum(given.run)])
+    positions = torch.from_numpy(np.concatenate([c + np.arange(r) for c, r in zip(given.ctx, given.run)])).to("cuda", torch.float64)
+    arena = given.arena.view(-1, 2, hkv, page, d)
+    computed = front in ("norm", "gated")
+    full = arena.double() if computed and arena.numel() <= 1 << 27 else None
+    names = ["out"] + (["q"] if computed else []) + (["gates"] if front == "gated" else [])
+    answer = {name: torch.zeros(given.shape_q, dtype=torch.float64, device="cuda") for name in names}
+    parts = [[torch.zeros(s, dtype=torch.float64, device="cuda") for s in (given.shape_q, given.shape_q[:3], given.shape_q[:3])]
+             for _ in range(2)]
+    for layer in range(layers):
+        if front == "gated":
+            pair, k, v = given.projection[layer].double().split([2 * hq * d, hkv * d, hkv * d], -1)
+            q, gates = pair.view(tokens, hq, 2, d).unbind(2)
+            k, v = k.view(tokens, hkv, d), v.view(tokens, hkv, d)
+            answer["gates"][layer] = gates
+        else:
+            q, k, v = (x[layer].double() for x in (given.q, given.k, given.v))
+        if computed:
+            q, k = (_norm_rope(x, w.to("cuda", torch.float64), positions, given) for x, w in zip((q, k), given.weights))
+            answer["q"][layer] = q
+        for slot in range(len(given.ctx)):
+            ctx, run = int(given.ctx[slot]), int(given.run[slot])
+            at = slice(int(starts[slot]), int(starts[slot]) + run)
+            ids = torch.from_numpy(given.rows[slot, layer].astype(np.int64)).cuda()
+            old = arena[ids[:-(-ctx // page)]].permute(1, 0, 3, 2, 4).reshape(2, -1, hkv, d)[:, :ctx].double()
+            if front == "draft":
+                both = [_softmax_values(q[at], old[0], old[1], group, scale), _softmax_values(q[at], k[at], v[at], group, scale)]
+                for part, found in zip(parts, both):
+                    for whole, x in zip(part, found):
+                        whole[layer, at] = x
+                top = torch.maximum(both[0][1], both[1][1])
+                mass = [x[2] * torch.exp(x[1] - top) for x in both]
+                answer["out"][layer, at] = sum(x[0] * w[..., None] for x, w in zip(both, mass)) / sum(mass)[..., None]
+                continue
+            out = _softmax_values(q[at], torch.cat([old[0], k[at]]), torch.cat([old[1], v[at]]), group, scale, ctx)[0]
+            answer["out"][layer, at] = out * torch.sigmoid(gates[at]) if front == "gated" else out
+            if full is not None:
+                place = torch.arange(ctx, ctx + run, device="cuda")
+                full[ids[place // page], 0, :, place % page] = k[at]
+                full[ids[place // page], 1, :, place % page] = v[at]
+    if front == "host":
+        answer["out"] = answer["out"][0]
+    if front == "draft":
+        answer["history"], answer["local"] = parts
+    else:
+        answer["pages"] = None if full is None else full.view(given.arena.shape)
+    return answer
