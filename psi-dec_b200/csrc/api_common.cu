@@ -71,7 +71,6 @@ AttendParams attend_params(psi_gqa* g, const psi_pages* pages, const psi_table* 
     p.unit_counters = static_cast<uint32_t*>(g->unit_counters.ptr);
     p.scalars = block_words(g, 0);
     p.num_q_heads = g->cfg.num_q_heads;
-    p.tokens_per_tile = g->geo.tokens_per_tile;
     p.dtype = g->cfg.dtype;
     p.scale_log2 = g->cfg.scale * 1.4426950408889634f;
     p.tma_feed = g->cfg.kernel_mode == PSI_KERNEL_MMA_TMA ? 1u : 0u;
@@ -260,13 +259,14 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             g->plan = build_balanced_plan(g->geo, req_slots, token_indices, cu_tokens, decode_reqs, g->grid_cap,
                                           min_tiles, g->item_start_cost);
             // K/V the long runs touch: below a third of the L2 the order of the work cannot cost HBM traffic, and exactly
-            // equal shares beat stream order
+            // equal balance beats stream order
             uint64_t chunk_kv_bytes = 0;
             for (uint32_t r : chunk_reqs)
                 chunk_kv_bytes += uint64_t(token_indices[r] + (cu_tokens[r + 1] - cu_tokens[r])) * (uint64_t(g->cfg.page_bytes) / g->tokens_per_page);
             g->chunk = build_chunk_plan(g->geo, req_slots, token_indices, cu_tokens, chunk_reqs, g->grid_cap,
                                         g->plan.num_partial_slots, static_cast<uint32_t>(g->plan.reduces.size()),
-                                        chunk_kv_bytes <= (40ull << 20));
+                                        chunk_kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident : ChunkOrder::kStream,
+                                        kChunkUnitCostTiles);
         }
         const WorkPlan& plan = g->plan;
         const ChunkPlan& chunk = g->chunk;

@@ -62,17 +62,14 @@ __global__ void __launch_bounds__(kThreads, 1) attend_chunk_kernel(AttendParams 
         const ItemView v = view_item(p, index);
         __syncthreads();  // the previous item is done with the ring
 
-        const uint32_t tokens_per_warp = p.tokens_per_tile;  // query tokens the plan packs into one 16-row tile
-        const uint32_t token_off = min(v.num_tokens, warp * tokens_per_warp);
-        const uint32_t my_tokens = min(tokens_per_warp, v.num_tokens - token_off);
-        const uint32_t my_rows = my_tokens * v.num_heads;
-        const uint32_t my_first_pos = v.first_pos + token_off;
-        // keys my rows may see: row r -> [0, my_first_pos + r / heads]; nothing at or beyond my_end counts for me
-        const uint32_t my_end = min(v.kv_end, my_first_pos + my_tokens);
-        const uint32_t my_min_limit = min(v.kv_end, my_first_pos + 1);
-        const uint32_t limit0 = frag.quad_row < my_rows ? min(v.kv_end, my_first_pos + frag.quad_row / v.num_heads + 1) : v.kv_end;
-        const uint32_t limit1 =
-            frag.quad_row + 8 < my_rows ? min(v.kv_end, my_first_pos + (frag.quad_row + 8) / v.num_heads + 1) : v.kv_end;
+        // this warp's rows: 16 of the item's rows (token, head), which are packed without gaps
+        const uint32_t row0 = min(v.rows, warp * kMaxRows);
+        const uint32_t my_rows = min(kMaxRows, v.rows - row0);
+        // keys row r may see: [0, item_row_limit(r)); nothing at or beyond my_end counts for this warp
+        const uint32_t my_end = my_rows > 0 ? item_row_limit(v, row0 + my_rows - 1) : 0u;
+        const uint32_t my_min_limit = item_row_limit(v, row0);
+        const uint32_t limit0 = frag.quad_row < my_rows ? item_row_limit(v, row0 + frag.quad_row) : v.kv_end;
+        const uint32_t limit1 = frag.quad_row + 8 < my_rows ? item_row_limit(v, row0 + frag.quad_row + 8) : v.kv_end;
         const uint32_t paged_end = fused ? min(v.kv_end, v.new_begin) : v.kv_end;
 
         const uint32_t first_tile = v.kv_begin / kTile;
@@ -132,8 +129,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_chunk_kernel(AttendParams 
             const uint32_t r = i / kChunks, c = i % kChunks;
             uint4 value = make_uint4(0, 0, 0, 0);
             if (r < my_rows) {
-                const uint64_t row = static_cast<uint64_t>(v.flat_begin + token_off + r / v.num_heads) * p.num_q_heads +
-                                     v.head0 + r % v.num_heads;
+                const uint64_t row = item_row_index(p, v, row0 + r);
                 value = *reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + row * D + c * 8);
             }
             *reinterpret_cast<uint4*>(smem + warp * L::kTileBytes + swizzled(r, c, L::kRowBytes)) = value;
@@ -186,9 +182,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_chunk_kernel(AttendParams 
         const float inv0 = st.l0 > 0.0f ? 1.0f / st.l0 : 0.0f, inv1 = st.l1 > 0.0f ? 1.0f / st.l1 : 0.0f;
         const uint32_t r0 = frag.quad_row, r1 = frag.quad_row + 8;
         const bool is_partial = v.partial_slot != kU32Max;
-        auto out_row = [&](uint32_t r) {
-            return static_cast<uint64_t>(v.flat_begin + token_off + r / v.num_heads) * p.num_q_heads + v.head0 + r % v.num_heads;
-        };
+        auto out_row = [&](uint32_t r) { return item_row_index(p, v, row0 + r); };
         if (is_partial) {
             const uint64_t base = static_cast<uint64_t>(v.partial_slot + warp) * kMaxRows;
 #pragma unroll
@@ -273,12 +267,12 @@ __global__ void __launch_bounds__(kThreads, 1) attend_chunk_kernel(AttendParams 
                 }
             }
         } else {
-            const uint64_t row0 = r0 < my_rows ? out_row(r0) : 0, row1 = r1 < my_rows ? out_row(r1) : 0;
+            const uint64_t out0 = r0 < my_rows ? out_row(r0) : 0, out1 = r1 < my_rows ? out_row(r1) : 0;
 #pragma unroll
             for (int j = 0; j < D / 8; ++j) {
                 const uint32_t col = 8 * j + 2 * frag.quad_col;
-                if (r0 < my_rows) store_out2<T>(p, row0 * D + col, st.o[j][0] * inv0, st.o[j][1] * inv0);
-                if (r1 < my_rows) store_out2<T>(p, row1 * D + col, st.o[j][2] * inv1, st.o[j][3] * inv1);
+                if (r0 < my_rows) store_out2<T>(p, out0 * D + col, st.o[j][0] * inv0, st.o[j][1] * inv0);
+                if (r1 < my_rows) store_out2<T>(p, out1 * D + col, st.o[j][2] * inv1, st.o[j][3] * inv1);
             }
         }
     }

@@ -325,12 +325,14 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
         // ================================ one accumulator row per thread ===============================================
         const uint32_t lane_base = (warp * 32u) << 16;  // this warp's TMEM lanes
         const uint32_t tmem_o = tmem + kColO;
-        // Row of this thread in an item: 16-row tile w = tid / 16, row rr inside it -> (token, head) of the super-tile.
+        const bool wide_out = (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
+        // Row of this thread in an item: row tid = (token tid / heads, head tid % heads) of the super-tile, packed without
+        // gaps; w and rr are its 16-row tile and its row inside it, the unit of partial slots and arrival counters.
         const uint32_t w = tid >> 4, rr = tid & 15;
         auto row_of = [&](const ItemView& v, bool& valid) {
-            const uint32_t token_off = w * p.tokens_per_tile + rr / v.num_heads;
-            valid = rr < p.tokens_per_tile * v.num_heads && token_off < v.num_tokens;
-            return static_cast<uint64_t>(v.flat_begin + (valid ? token_off : 0)) * p.num_q_heads + v.head0 + rr % v.num_heads;
+            valid = tid < v.rows;
+            return static_cast<uint64_t>(v.flat_begin + (valid ? tid / v.num_heads : 0)) * p.num_q_heads + v.head0 +
+                   (valid ? tid % v.num_heads : 0);
         };
         // This thread's query row of an item into its TMEM lane (zero for rows the super-tile does not have).  Called
         // when every Q K^T of the previous item has completed; 16 loads in flight at a time.
@@ -363,8 +365,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
             const ItemView v = view_item(p, index);
             bool row_valid;
             const uint64_t out_row = row_of(v, row_valid);
-            const uint32_t token_off = w * p.tokens_per_tile + rr / v.num_heads;
-            const uint32_t limit = row_valid ? min(v.kv_end, v.first_pos + token_off + 1) : v.kv_end;
+            const uint32_t limit = row_valid ? item_row_limit(v, tid) : v.kv_end;
             const uint32_t min_limit = min(v.kv_end, v.first_pos + 1);
             const uint32_t first_tile = v.kv_begin / kUmmaN;
             const uint32_t num_tiles = (v.kv_end + kUmmaN - 1) / kUmmaN - first_tile;
@@ -454,6 +455,20 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 mbar_arrive(bar(kBarP + buf));
                 if (i > 0 && !rescale) wait(kBarO + ((tile - 1) & 1), (tile - 1) >> 1);
             }
+            const bool is_partial = v.partial_slot != kU32Max;
+            // The output gates of this row, 32 columns at a time and one pass ahead of their use: the first ones travel
+            // under the last P V, each later pass's under the pass before it.
+            const bool gated = p.gates != nullptr && row_valid && !is_partial && p.ext_o == nullptr;
+            const uint2* gate_row = reinterpret_cast<const uint2*>(static_cast<const T*>(p.gates) + out_row * D);  // 8-byte aligned
+            uint2 gate_next[8];
+            if (gated) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) gate_next[j] = gate_row[j];
+            }
+            // The next item's query rows go to TMEM under this item's last P V (S of its last tile has been read, so all
+            // its Q K^T are complete), and the first Q K^T products of that item run under the epilogue (O is not
+            // touched before P of that item's first tile exists).
+            if (index + 1 < item_end) load_q(view_item(p, index + 1));
             if (num_tiles > 0) {
                 const uint32_t last = tile_base + num_tiles - 1;
                 wait(kBarO + (last & 1), last >> 1);
@@ -461,15 +476,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 tc_fence_after();
             }
             tile_base += num_tiles;
-            // The next item's query rows go to TMEM before this item's output is written: its first Q K^T products then
-            // run under the epilogue (O is not touched before P of that item's first tile exists).
-            if (index + 1 < item_end) load_q(view_item(p, index + 1));
 
             // ---- epilogue: every thread finishes its own row ---------------------------------------------------------------
             // back to the true max as the reference: l' = l * 2^(ref - max); O / l is unchanged by the shift
             const float inv = row_sum > 0.0f ? 1.0f / row_sum : 0.0f;
             const float sum_at_max = row_max == -INFINITY ? row_sum : row_sum * fast_exp2(row_ref - row_max);
-            const bool is_partial = v.partial_slot != kU32Max;
             const uint64_t prow = is_partial ? static_cast<uint64_t>(v.partial_slot + w) * kMaxRows + rr : 0;
 #pragma unroll 1
             for (uint32_t c = 0; c < uint32_t(D); c += 32) {
@@ -483,6 +494,21 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 if (row_valid) {
 #pragma unroll
                     for (int e = 0; e < 32; ++e) o[e] *= inv;
+                    if (gated) {
+                        uint2 gate_raw[8];
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) gate_raw[j] = gate_next[j];
+                        if (c + 32 < uint32_t(D)) {
+#pragma unroll
+                            for (int j = 0; j < 8; ++j) gate_next[j] = gate_row[c / 4 + 8 + j];
+                        }
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            const T* gate = reinterpret_cast<const T*>(&gate_raw[j]);
+#pragma unroll
+                            for (int e = 0; e < 4; ++e) o[4 * j + e] *= gate_sigmoid_approx(static_cast<float>(gate[e]));
+                        }
+                    }
                     if (is_partial) {
                         // a partial slot of this kernel is stored column-major in float4 units, [D / 4][16 rows]: the
                         // 16 rows of a tile are 16 consecutive lanes here, so every store instruction writes whole
@@ -499,7 +525,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                             *reinterpret_cast<float4*>(dst + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
                     } else {
 #pragma unroll
-                        for (int e = 0; e < 32; e += 8) store_out8<T>(p, out_row * D + c + e, o + e);
+                        for (int e = 0; e < 32; e += 8) store_plain8<T>(p.out, out_row * D + c + e, o + e, wide_out);
                     }
                 }
                 __syncwarp();  // the TMEM load of the next pass is warp-collective
@@ -520,7 +546,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 __threadfence();
                 row_threads_sync();
                 if (tid < 8) {
-                    const bool has_rows = tid * p.tokens_per_tile < v.num_tokens;
+                    const bool has_rows = tid * kMaxRows < v.rows;
                     last_s[tid] = has_rows && atomicAdd(p.unit_counters + v.reduce_unit + tid, 1u) == v.unit_num_items - 1;
                     __threadfence();  // the other pieces' partials are read (from L2) only after their arrivals were seen
                 }
@@ -529,8 +555,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                     if (!last_s[tile]) continue;
                     // 16 rows x D / 4 float4 outputs per tile: a thread takes row tid % 16 and the float4 columns
                     // tid / 16 + 8 j (16 consecutive lanes read 256 consecutive bytes of the column-major slots)
-                    const uint32_t tile_tokens = min(p.tokens_per_tile, v.num_tokens - tile * p.tokens_per_tile);
-                    const uint32_t tile_rows = tile_tokens * v.num_heads;
+                    const uint32_t tile_rows = min(kMaxRows, v.rows - tile * kMaxRows);
                     constexpr uint32_t kPerThread = kMaxRows * (D / 4) / kRowThreads;
                     constexpr uint32_t kColumnStep = kRowThreads / kMaxRows;  // float4 columns between a thread's outputs
                     // a row beyond the tile's last one is computed on the last row and dropped at the end: the loops
@@ -582,9 +607,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                     }
                     if (row_present) {
                         const float scale = sum_all > 0.0f ? 1.0f / sum_all : 0.0f;
-                        const uint64_t row =
-                            static_cast<uint64_t>(v.flat_begin + tile * p.tokens_per_tile + r / v.num_heads) * p.num_q_heads +
-                            v.head0 + r % v.num_heads;
+                        const uint64_t row = item_row_index(p, v, tile * kMaxRows + r);
 #pragma unroll
                         for (uint32_t j = 0; j < kPerThread; ++j) {
                             const uint32_t c4 = c4_0 + j * kColumnStep;

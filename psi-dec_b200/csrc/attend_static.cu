@@ -210,7 +210,6 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         p.unit_counters = reinterpret_cast<uint32_t*>(scratch + kOffCounters);
         p.scalars = reinterpret_cast<const uint32_t*>(scratch + kOffScalars);
         p.num_q_heads = c.num_q_heads;
-        p.tokens_per_tile = geo.tokens_per_tile;
         p.dtype = c.dtype;
         p.scale_log2 = c.scale * 1.4426950408889634f;
         if (mma) {

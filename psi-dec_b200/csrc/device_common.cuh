@@ -151,6 +151,13 @@ __device__ __forceinline__ float gate_sigmoid(float x) {
     return x < 0.0f ? 1.0f - y : y;
 }
 
+// The same with the division as a reciprocal of the special-function unit (the divisor lies in [1, 2]): for kernels
+// that write 16-bit outputs and work the gate out on few threads.
+__device__ __forceinline__ float gate_sigmoid_approx(float x) {
+    const float y = __fdividef(1.0f, 1.0f + __expf(-fabsf(x)));
+    return x < 0.0f ? 1.0f - y : y;
+}
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
     for (int offset = 16; offset > 0; offset >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, offset);

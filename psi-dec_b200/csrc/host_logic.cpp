@@ -414,7 +414,7 @@ WorkPlan build_reference_plan(const PlanGeometry& geo, const ReferenceMetadata& 
 
 ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
                            const uint32_t* cu_tokens, const std::vector<uint32_t>& requests, uint32_t max_ctas,
-                           uint32_t slot_base, uint32_t counter_base, bool equal_shares) {
+                           uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost) {
     ChunkPlan plan;
     // Units in stream order: all super-tiles of one (request, KV head) follow one another, so that CTAs working on
     // neighbouring units at the same time read the same K/V pages (once from HBM, then from L2).
@@ -422,9 +422,10 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
         uint32_t req, flat_begin, flat_end, ctx_end, head;
     };
     std::vector<Unit> units;
-    const uint32_t tokens_per_item = geo.tokens_per_tile * kChunkTilesPerItem;
+    // the rows of an item are packed (token, head) pairs: as many whole tokens as its 128 rows hold
+    const uint32_t tokens_per_item = kMaxRows * kChunkTilesPerItem / geo.heads_per_tile;
     const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
-    uint64_t total = 0;
+    uint64_t total = 0, longest = 0;
     // longest requests first: the work dealt last, which decides how far the last CTA trails, is the cheapest
     std::vector<uint32_t> by_length(requests);
     std::stable_sort(by_length.begin(), by_length.end(), [&](uint32_t a, uint32_t b) {
@@ -436,6 +437,7 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
                 const uint32_t end = std::min(cu_tokens[r + 1], begin + tokens_per_item);
                 units.push_back({r, begin, end, token_indices[r] + (end - cu_tokens[r]), h});
                 total += div_ceil(units.back().ctx_end, kKvTile);
+                longest = std::max(longest, div_ceil(units.back().ctx_end, kKvTile));
                 begin = end;
             }
         }
@@ -476,18 +478,45 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
         plan.num_partial_slots += n * kChunkTilesPerItem;
         plan.num_counters += kChunkTilesPerItem;
     };
-    if (equal_shares) {
-        // A working set that stays in L2 whatever the order: contiguous shares of exactly equal size, units cut where a
-        // share ends (two or three pieces per cut unit instead of many), slivers below a quarter of the minimum piece
-        // folded into their neighbour.
+    const bool l2_resident = order == ChunkOrder::kL2Resident;
+    const uint64_t fair_share = (total + uint64_t(unit_start_cost) * units.size()) / num_ctas;
+    if (l2_resident && longest <= std::max<uint64_t>(fair_share / 2, 2 * kChunkMinPieceTiles)) {
+        // Whole units, longest first, each to the CTA with the least work so far.  Nothing is cut: a cut saves half a
+        // unit's tiles on one CTA and costs two partial writes, a fence and a merge, about kChunkMinPieceTiles of them,
+        // so it pays only for units of more than twice that which are also long against a CTA's share.
+        std::stable_sort(units.begin(), units.end(), [](const Unit& a, const Unit& b) { return a.ctx_end > b.ctx_end; });
+        std::priority_queue<std::pair<uint64_t, uint32_t>, std::vector<std::pair<uint64_t, uint32_t>>, std::greater<>> free_first;
+        for (uint32_t c = 0; c < num_ctas; ++c) free_first.push({0, c});
+        std::vector<std::vector<DeviceItem>> per_cta(num_ctas);
+        for (const Unit& u : units) {
+            auto [load, c] = free_first.top();
+            free_first.pop();
+            const uint64_t tiles = div_ceil(u.ctx_end, kKvTile);
+            per_cta[c].push_back(make_item(u, 0, tiles));
+            free_first.push({load + tiles + unit_start_cost, c});
+        }
+        plan.cta_item_begin.assign(1, 0);
+        for (const auto& list : per_cta) {
+            plan.items.insert(plan.items.end(), list.begin(), list.end());
+            plan.cta_item_begin.push_back(static_cast<uint32_t>(plan.items.size()));
+        }
+        return plan;
+    }
+    if (l2_resident || order == ChunkOrder::kEqualShares) {
+        // A working set that stays in L2 whatever the order: contiguous shares of equal cost, units cut where a share
+        // ends (two or three pieces per cut unit instead of many), slivers below a quarter of the minimum piece folded
+        // into their neighbour.  A unit costs its KV tiles plus `unit_start_cost`, so that a share of many
+        // short units (the first tokens of a prompt) is not longer than one of a few long ones.
         const uint64_t sliver = kChunkMinPieceTiles / 4;
         plan.items.reserve(units.size() + num_ctas);
         std::vector<uint32_t> owner;  // CTA of every item, in item order
         uint64_t cursor = 0;
         uint32_t cta = 0;
-        auto share_end = [&](uint64_t c) { return total * (c + 1) / num_ctas; };
+        const uint64_t span = total + uint64_t(unit_start_cost) * units.size();
+        auto share_end = [&](uint64_t c) { return span * (c + 1) / num_ctas; };
         std::vector<std::pair<size_t, size_t>> unit_items;  // [first, last) item of every unit
         for (const Unit& u : units) {
+            cursor += unit_start_cost;
             const uint64_t unit_tiles = div_ceil(u.ctx_end, kKvTile);
             const size_t first = plan.items.size();
             uint64_t done = 0;
@@ -532,24 +561,10 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
     for (const Unit& u : units) {
         const uint64_t unit_tiles = div_ceil(u.ctx_end, kKvTile);
         const uint32_t n = static_cast<uint32_t>(div_ceil(unit_tiles, piece_cap));
-        const uint32_t head_tile = u.head % geo.head_tiles;
         const uint32_t first_slot = slot_base + plan.num_partial_slots;
         for (uint32_t k = 0; k < n; ++k) {
             const uint64_t tile_begin = unit_tiles * k / n, tile_end = unit_tiles * (k + 1) / n;
-            DeviceItem d{};
-            d.kv_begin = static_cast<uint32_t>(tile_begin * kKvTile);
-            d.kv_end = static_cast<uint32_t>(std::min<uint64_t>(tile_end * kKvTile, u.ctx_end));
-            d.partial_slot = kU32Max;
-            d.flat_begin = u.flat_begin;
-            d.num_tokens = u.flat_end - u.flat_begin;
-            d.req_slot = req_slots[u.req];
-            d.kv_head = u.head / geo.head_tiles;
-            d.head0 = d.kv_head * geo.group + head_tile * geo.heads_per_tile;
-            d.num_heads = std::min(geo.heads_per_tile, geo.group - head_tile * geo.heads_per_tile);
-            d.first_pos = token_indices[u.req] + (u.flat_begin - cu_tokens[u.req]);
-            d.new_begin = token_indices[u.req];
-            d.flat_req_begin = cu_tokens[u.req];
-            d.writes_kv = head_tile == 0 ? 1u : 0u;
+            DeviceItem d = make_item(u, tile_begin, tile_end);
             if (n > 1) {  // the unit is shared between CTAs: partial slots 8 apart, eight arrival counters
                 d.partial_slot = first_slot + k * kChunkTilesPerItem;
                 d.reduce_unit = counter_base + plan.num_counters;

@@ -176,13 +176,21 @@ struct ChunkPlan {
 };
 constexpr uint32_t kChunkTilesPerItem = 8;  // one query tile per warp
 constexpr uint32_t kChunkMinPieceTiles = 64;   // a KV piece of a cut unit is at least this many 16-token tiles
-constexpr uint32_t kChunkStartCostTiles = 8;   // fixed cost of a work item (query load, epilogue) in KV tiles
+constexpr uint32_t kChunkStartCostTiles = 8;   // fixed cost of a work item (query load, epilogue) in KV tiles, stream order
+constexpr uint32_t kChunkUnitCostTiles = 16;   // the same in the other orders
 
-// `equal_shares`: contiguous shares of exactly equal size (for working sets that stay in L2 in any order); otherwise
-// units are dealt whole, in stream order, to the CTA that is free first, and only long units are cut.
+// How the units of a chunk plan are dealt to CTAs.
+enum class ChunkOrder {
+    kStream,       // in stream order to the CTA that is free first; only long units are cut
+    kEqualShares,  // contiguous shares of equal size, units cut where a share ends
+    kL2Resident    // any order will do, the K/V stays in L2: whole units, longest first, where no unit is long against a
+                   // CTA's share; else equal shares
+};
+
+// Outside stream order a unit counts as its KV tiles plus `unit_start_cost`.
 ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
                            const uint32_t* cu_tokens, const std::vector<uint32_t>& requests, uint32_t max_ctas,
-                           uint32_t slot_base, uint32_t counter_base, bool equal_shares = false);
+                           uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost = 0);
 
 // Device form of a finished plan.
 std::vector<DeviceItem> flatten_plan(const WorkPlan& plan, const PlanGeometry& geo);

@@ -120,7 +120,6 @@ struct AttendParams {
     uint32_t* unit_counters;      // [reduce units], zero between launches: arrivals of a unit's items (mma kernel)
     const uint32_t* scalars;
     uint32_t num_q_heads;
-    uint32_t tokens_per_tile;     // query tokens of one 16-row tile (plan geometry)
     uint32_t dtype;
     float scale_log2;             // scale * log2(e)
     uint32_t* status;             // nullptr, or the word a bounded device-side wait writes PSI_ERR_TIMEOUT to
