@@ -10,6 +10,7 @@
 // de-interleave of the fused projection output (metal/gqa_qgkv_split.metal:14-42 with gates,
 // metal/gqa_qkv_split.metal:13-36 without).  Its q, g, k and v rows are read where the projection left them; only the
 // gate rows, which the attention epilogue wants contiguous, are copied out.
+#include <cstdlib>
 #include "device_common.cuh"
 
 namespace psi {
@@ -106,12 +107,216 @@ __global__ void __launch_bounds__(kPrepWarps * 32) norm_rope_append_kernel(PrepP
     }
 }
 
+// Eight consecutive elements as a lane holds them.
+template <uint32_t DTYPE>
+struct Eight {
+    static constexpr int kWords = DTYPE == PSI_DTYPE_F32 ? 8 : 4;
+    uint4 raw[kWords / 4];
+    __device__ __forceinline__ uint32_t* words() { return reinterpret_cast<uint32_t*>(raw); }
+    __device__ __forceinline__ const uint32_t* words() const { return reinterpret_cast<const uint32_t*>(raw); }
+    __device__ __forceinline__ void load(const void* base, uint64_t index) {
+        const uint4* src = reinterpret_cast<const uint4*>(static_cast<const unsigned char*>(base) + index * (kWords / 2));
+#pragma unroll
+        for (int i = 0; i < kWords / 4; ++i) raw[i] = src[i];
+    }
+    __device__ __forceinline__ void store(void* base, uint64_t index) const {
+        uint4* dst = reinterpret_cast<uint4*>(static_cast<unsigned char*>(base) + index * (kWords / 2));
+#pragma unroll
+        for (int i = 0; i < kWords / 4; ++i) dst[i] = raw[i];
+    }
+    __device__ __forceinline__ void widen(float (&v)[8]) const {
+#pragma unroll
+        for (int j = 0; j < kWords; ++j) {
+            if constexpr (DTYPE == PSI_DTYPE_F32) {
+                v[j] = __uint_as_float(words()[j]);
+            } else {
+                const uint32_t w = words()[j];
+                const float2 pair = DTYPE == PSI_DTYPE_BF16 ? __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w))
+                                                            : __half22float2(*reinterpret_cast<const __half2*>(&w));
+                v[2 * j] = pair.x;
+                v[2 * j + 1] = pair.y;
+            }
+        }
+    }
+    __device__ __forceinline__ void narrow(const float (&v)[8]) {
+#pragma unroll
+        for (int j = 0; j < kWords; ++j) {
+            if constexpr (DTYPE == PSI_DTYPE_F32) {
+                words()[j] = __float_as_uint(v[j]);
+            } else if constexpr (DTYPE == PSI_DTYPE_BF16) {
+                const __nv_bfloat162 pair = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+                words()[j] = *reinterpret_cast<const uint32_t*>(&pair);
+            } else {
+                const __half2 pair = __floats2half2_rn(v[2 * j], v[2 * j + 1]);
+                words()[j] = *reinterpret_cast<const uint32_t*>(&pair);
+            }
+        }
+    }
+    // T(weight) * T(x * inv_rms), rounded to T.  In the 16-bit types the product of two such values is exact in f32, so
+    // the packed multiplication, which rounds once, gives the same bits as an f32 product rounded to T.
+    __device__ __forceinline__ void normalise(const float (&x)[8], float inv_rms, const Eight& weight) {
+        float v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = x[j] * inv_rms;
+        narrow(v);
+#pragma unroll
+        for (int j = 0; j < kWords; ++j) {
+            if constexpr (DTYPE == PSI_DTYPE_F32) {
+                words()[j] = __float_as_uint(__uint_as_float(weight.words()[j]) * v[j]);
+            } else if constexpr (DTYPE == PSI_DTYPE_BF16) {
+                const __nv_bfloat162 pair = __hmul2(*reinterpret_cast<const __nv_bfloat162*>(weight.words() + j),
+                                                    *reinterpret_cast<const __nv_bfloat162*>(words() + j));
+                words()[j] = *reinterpret_cast<const uint32_t*>(&pair);
+            } else {
+                const __half2 pair = __hmul2(*reinterpret_cast<const __half2*>(weight.words() + j),
+                                             *reinterpret_cast<const __half2*>(words() + j));
+                words()[j] = *reinterpret_cast<const uint32_t*>(&pair);
+            }
+        }
+    }
+};
+
+// The same stage for head sizes whose row is a power-of-two number of lanes of eight elements (LPR lanes, 32 / LPR rows
+// per warp) and 16-byte aligned buffers.  Bound by HBM on prompts and by latency on decode steps.  A CTA works on rows
+// of one token (blockIdx.x): the token's sines and cosines are worked out once into shared memory instead of once per
+// row, its page is looked up once, every lane moves 16 bytes at a time, and a warp has kHeld rows in flight.  blockIdx.y
+// deals the token's rows (q, k, v, gates) to CTAs.
+constexpr int kHeld = 4;
+constexpr uint64_t kRowsResidentCtas = 148 * 4;
+
+template <uint32_t DTYPE, int LPR>
+__global__ void __launch_bounds__(kPrepWarps * 32, 4) norm_rope_rows_kernel(PrepParams p) {
+    constexpr uint32_t D = LPR * 8, kRows = 32 / LPR;
+    __shared__ float2 turn_s[D / 2];  // (cosine, sine) of the token's position at every frequency
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t group = lane / LPR, sub = lane % LPR, d0 = sub * 8;
+    const uint32_t token = blockIdx.x;
+    if (token >= min(p.scalars[kScalarNumActiveTokens], p.num_total_tokens)) return;
+    const uint32_t hq = p.num_q_heads, hkv = p.geo.num_kv_heads;
+    const uint32_t num_rows = hq + 2 * hkv + (p.g_in != nullptr ? hq : 0);  // q | k | v | gates
+    const uint32_t stride = gridDim.y * kPrepWarps * kRows;
+    const uint32_t first = (blockIdx.y * kPrepWarps + warp) * kRows + group;
+    const uint32_t pos = p.flat_token_indices[token], slot = p.req_slots[token];
+
+    auto fetch = [&](uint32_t row, Eight<DTYPE>& x) {
+        const uint64_t q_row = token * p.q_token_stride + d0, kv_row = token * p.kv_token_stride + d0;
+        if (row < hq) x.load(p.q_in, q_row + row * p.q_head_stride);
+        else if (row < hq + hkv) x.load(p.k_in, kv_row + static_cast<uint64_t>(row - hq) * D);
+        else if (row < hq + 2 * hkv) x.load(p.v_in, kv_row + static_cast<uint64_t>(row - hq - hkv) * D);
+        else if (row < num_rows) x.load(p.g_in, q_row + (row - hq - 2 * hkv) * p.q_head_stride);
+    };
+    Eight<DTYPE> held[kHeld];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) fetch(first + i * stride, held[i]);
+
+    Eight<DTYPE> q_weight, k_weight;  // the bf16 weights in T
+    {
+        Eight<PSI_DTYPE_BF16> w;
+        float v[8];
+        w.load(p.q_weight, d0);
+        w.widen(v);
+        q_weight.narrow(v);
+        w.load(p.k_weight, d0);
+        w.widen(v);
+        k_weight.narrow(v);
+    }
+    uint32_t page_id;
+    const bool page_ok = checked_page_id(p.geo, table_row(p.geo, slot), pos / p.geo.tokens_per_page, page_id);
+    const uint64_t page_row = kv_row_offset(p.geo, page_id, 0, pos % p.geo.tokens_per_page) + d0;
+    const uint32_t rope_half = p.rope_dim / 2, half_lanes = rope_half / 8;
+    for (uint32_t i = tid; i < rope_half; i += kPrepWarps * 32) {
+        float s, c;
+        sincosf(static_cast<float>(pos) * p.inverse_frequencies[i], &s, &c);
+        turn_s[i] = make_float2(c, s);
+    }
+    __syncthreads();
+    const bool in_rope = sub < 2 * half_lanes, low = sub < half_lanes;
+    const uint32_t partner = in_rope ? (low ? lane + half_lanes : lane - half_lanes) : lane;
+    const float2* turns = turn_s + (low ? d0 : d0 - rope_half);
+
+    for (uint32_t base = first - group; base < num_rows; base += kHeld * stride) {
+#pragma unroll
+        for (int i = 0; i < kHeld; ++i) {
+            if (base + i * stride >= num_rows) break;  // warp-uniform
+            const uint32_t row = base + i * stride + group;
+            const bool is_q = row < hq, is_k = !is_q && row < hq + hkv;
+            Eight<DTYPE> x = held[i];
+            fetch(row + kHeld * stride, held[i]);  // the row this place holds next, under the arithmetic of this one
+            if (base + i * stride < hq + hkv) {  // warp-uniform: some row of this pass is normalised
+                float v[8], acc = 0.0f;
+                x.widen(v);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc += v[j] * v[j];
+#pragma unroll
+                for (int offset = LPR / 2; offset > 0; offset >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, offset);
+                const float inv_rms = 1.0f / sqrtf(acc / static_cast<float>(D) + p.eps);
+                Eight<DTYPE> n, other;
+                n.normalise(v, inv_rms, is_q ? q_weight : k_weight);
+#pragma unroll
+                for (int j = 0; j < Eight<DTYPE>::kWords; ++j)
+                    other.words()[j] = __shfl_sync(0xFFFFFFFFu, n.words()[j], partner);
+                if (in_rope) {
+                    float mine[8], theirs[8];
+                    n.widen(mine);
+                    other.widen(theirs);
+#pragma unroll
+                    for (int j = 0; j < 8; j += 2) {
+                        const float4 turn = *reinterpret_cast<const float4*>(turns + j);  // two frequencies
+                        mine[j] = p.attention_factor * (low ? mine[j] * turn.x - theirs[j] * turn.y : theirs[j] * turn.y + mine[j] * turn.x);
+                        mine[j + 1] = p.attention_factor * (low ? mine[j + 1] * turn.z - theirs[j + 1] * turn.w
+                                                                : theirs[j + 1] * turn.w + mine[j + 1] * turn.z);
+                    }
+                    n.narrow(mine);
+                }
+                if (is_q || is_k) x = n;
+            }
+            if (is_q) {
+                x.store(p.q_out, (static_cast<uint64_t>(token) * hq + row) * D + d0);
+            } else if (row < hq + 2 * hkv) {
+                const uint64_t head_row = static_cast<uint64_t>(row - hq - (is_k ? 0 : hkv)) * p.geo.tokens_per_page * D;
+                if (page_ok) x.store(const_cast<void*>(p.geo.pages), page_row + head_row + (is_k ? 0 : v_region_offset(p.geo)));
+            } else if (row < num_rows) {
+                x.store(p.g_out, (static_cast<uint64_t>(token) * hq + (row - hq - 2 * hkv)) * D + d0);
+            }
+        }
+    }
+}
+
+bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
+
+template <uint32_t DTYPE>
+bool launch_rows(const PrepParams& p, cudaStream_t stream) {
+    const uint32_t d = p.geo.head_dim;
+    if ((d != 64 && d != 128 && d != 256) || p.rope_dim % 16 != 0 || !aligned16(p.q_in) || !aligned16(p.k_in) || !aligned16(p.v_in) ||
+        !aligned16(p.g_in) || !aligned16(p.q_out) || !aligned16(p.g_out) || !aligned16(p.geo.pages) || !aligned16(p.q_weight) ||
+        !aligned16(p.k_weight)) {
+        return false;
+    }
+    // Rows per warp: one while the device has room for every warp at once (a decode step: nothing but latency), more
+    // when the step is long (a prompt: the per-CTA work is spread over more rows).
+    const uint32_t rows = p.num_q_heads * (p.g_in != nullptr ? 2 : 1) + 2 * p.geo.num_kv_heads;
+    const uint32_t rows_per_cta = kPrepWarps * (256 / d);
+    const uint64_t ctas = static_cast<uint64_t>(p.num_total_tokens) * ((rows + rows_per_cta - 1) / rows_per_cta);
+    const uint32_t per_warp = static_cast<uint32_t>(ctas <= kRowsResidentCtas ? 1 : (getenv("PSI_UC") ? atoi(getenv("PSI_UC")) : 4));
+    const uint32_t split = (rows + rows_per_cta * per_warp - 1) / (rows_per_cta * per_warp);
+    if (split > 65535) return false;
+    const dim3 grid(p.num_total_tokens, split);
+    if (d == 64) norm_rope_rows_kernel<DTYPE, 8><<<grid, kPrepWarps * 32, 0, stream>>>(p);
+    else if (d == 128) norm_rope_rows_kernel<DTYPE, 16><<<grid, kPrepWarps * 32, 0, stream>>>(p);
+    else norm_rope_rows_kernel<DTYPE, 32><<<grid, kPrepWarps * 32, 0, stream>>>(p);
+    return true;
+}
+
 }  // namespace
 
 cudaError_t launch_norm_rope_append(const PrepParams& p, cudaStream_t stream) {
     const uint64_t rows = static_cast<uint64_t>(p.num_total_tokens) *
                           ((p.g_in != nullptr ? 2ull : 1ull) * p.num_q_heads + 2ull * p.geo.num_kv_heads);
     if (rows == 0) return cudaSuccess;
+    if (p.dtype == PSI_DTYPE_F32 ? launch_rows<PSI_DTYPE_F32>(p, stream)
+                                 : (p.dtype == PSI_DTYPE_BF16 ? launch_rows<PSI_DTYPE_BF16>(p, stream) : launch_rows<PSI_DTYPE_F16>(p, stream))) {
+        return cudaGetLastError();
+    }
     const unsigned blocks = static_cast<unsigned>((rows + kPrepWarps - 1) / kPrepWarps);
     switch (p.dtype) {
         case PSI_DTYPE_F32: norm_rope_append_kernel<PSI_DTYPE_F32><<<blocks, kPrepWarps * 32, 0, stream>>>(p); break;
