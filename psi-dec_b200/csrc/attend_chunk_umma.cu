@@ -15,6 +15,10 @@
 //   warps 5 and 6: bring the K and the V tiles from their pages by TMA, one 5-D box per page segment that lands in
 //       exactly the order the MMA descriptors read ([8-row group][64-element block][8 rows][64 elements], 128-byte
 //       swizzle); an item's last, ragged tile is copied with zero-filling 16-byte cp.async instead.
+// An item costs about 10 us beside its tiles (0.9 us each at head_dim 256): query rows, the fill of the pipeline, the
+// epilogue of one row per thread.  Prompts have many short items, so the query rows and the first gates travel under the
+// last P V, the gates one pass ahead of their use, rows are packed (a group of six fills 126 of 128 rows, not 96), and
+// the plan deals whole units: three prompts of 611 to 2,500 tokens (24/4 heads x 256, gated) 186 us a layer, 1,066 before.
 // All hand-offs are mbarriers (TMA byte counts, tcgen05.commit, thread arrivals); every wait is bounded and reports
 // PSI_ERR_TIMEOUT through the status word instead of hanging, and the kernel frees its TMEM on every path.  The kernel
 // reads pages only: a step that appends and attends runs the append launch first.

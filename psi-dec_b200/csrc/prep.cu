@@ -10,7 +10,6 @@
 // de-interleave of the fused projection output (metal/gqa_qgkv_split.metal:14-42 with gates,
 // metal/gqa_qkv_split.metal:13-36 without).  Its q, g, k and v rows are read where the projection left them; only the
 // gate rows, which the attention epilogue wants contiguous, are copied out.
-#include <cstdlib>
 #include "device_common.cuh"
 
 namespace psi {
@@ -177,15 +176,17 @@ struct Eight {
 };
 
 // The same stage for head sizes whose row is a power-of-two number of lanes of eight elements (LPR lanes, 32 / LPR rows
-// per warp) and 16-byte aligned buffers.  Bound by HBM on prompts and by latency on decode steps.  A CTA works on rows
-// of one token (blockIdx.x): the token's sines and cosines are worked out once into shared memory instead of once per
-// row, its page is looked up once, every lane moves 16 bytes at a time, and a warp has kHeld rows in flight.  blockIdx.y
-// deals the token's rows (q, k, v, gates) to CTAs.
+// per warp) and 16-byte aligned buffers.  A CTA works on rows of one token (blockIdx.x): the token's sines and cosines
+// are worked out once into shared memory instead of once per row, its page is looked up once, every lane moves 16 bytes
+// at a time, the 16-bit types are rounded and multiplied in pairs, and a warp has kHeld rows in flight.  blockIdx.y deals
+// the token's rows (q, k, v, gates) to CTAs.  Bound by issue slots on prompts (72 % of them) and by latency on decode
+// steps.  Measured: 4,667 prompt tokens of 24/4 heads x 256 with gates (267 MB) 71 us = 3.8 TB/s, against 133 us with a
+// warp per row and one element per lane; a decode step of 32 tokens 5.2 us against 7.5 us.
 constexpr int kHeld = 4;
 constexpr uint64_t kRowsResidentCtas = 148 * 4;
 
 template <uint32_t DTYPE, int LPR>
-__global__ void __launch_bounds__(kPrepWarps * 32, 4) norm_rope_rows_kernel(PrepParams p) {
+__global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 4) norm_rope_rows_kernel(PrepParams p) {
     constexpr uint32_t D = LPR * 8, kRows = 32 / LPR;
     __shared__ float2 turn_s[D / 2];  // (cosine, sine) of the token's position at every frequency
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -292,12 +293,13 @@ bool launch_rows(const PrepParams& p, cudaStream_t stream) {
         !aligned16(p.k_weight)) {
         return false;
     }
-    // Rows per warp: one while the device has room for every warp at once (a decode step: nothing but latency), more
-    // when the step is long (a prompt: the per-CTA work is spread over more rows).
+    // Rows per warp: one while the device has room for every CTA at once (a decode step: nothing but latency), eight
+    // when the step is long: the per-CTA part is then spread over more rows (a prompt step of 4,667 tokens and two
+    // layers measured 675 us with one, 551 with four, 538 with eight).
     const uint32_t rows = p.num_q_heads * (p.g_in != nullptr ? 2 : 1) + 2 * p.geo.num_kv_heads;
     const uint32_t rows_per_cta = kPrepWarps * (256 / d);
     const uint64_t ctas = static_cast<uint64_t>(p.num_total_tokens) * ((rows + rows_per_cta - 1) / rows_per_cta);
-    const uint32_t per_warp = static_cast<uint32_t>(ctas <= kRowsResidentCtas ? 1 : (getenv("PSI_UC") ? atoi(getenv("PSI_UC")) : 4));
+    const uint32_t per_warp = static_cast<uint32_t>(ctas <= kRowsResidentCtas ? 1 : 8);
     const uint32_t split = (rows + rows_per_cta * per_warp - 1) / (rows_per_cta * per_warp);
     if (split > 65535) return false;
     const dim3 grid(p.num_total_tokens, split);
