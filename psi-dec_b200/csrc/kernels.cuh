@@ -181,6 +181,9 @@ uint32_t attend_staged_ctas_per_sm(uint32_t dtype);
 // The staged CUDA-core map kernel (attend_staged.cu): taken by launch_attend_generic when the launch qualifies.
 bool attend_staged_supported(const AttendParams& p);
 cudaError_t launch_attend_staged(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
+// The ring-fed f32 map kernel (attend_f32.cu): taken before the staged one when the launch qualifies.
+bool attend_f32_supported(const AttendParams& p);
+cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 cudaError_t launch_attend_mma(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 // Long query runs: one CTA = up to eight query tiles of one request sharing one pass over the KV range.
