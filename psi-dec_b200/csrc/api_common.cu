@@ -143,6 +143,27 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     }
 }
 
+void split_requests(const psi_gqa* g, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs,
+                    std::vector<uint32_t>& decode_reqs, std::vector<uint32_t>& chunk_reqs) {
+    const uint32_t per_tile = g->geo.tokens_per_tile;
+    uint32_t min_tiles = kU32Max;
+    if (g->chunk_supported) {
+        uint64_t units = 0, longest = 0;
+        for (uint32_t r = 0; r < num_reqs; ++r) {
+            const uint32_t run = cu_tokens[r + 1] - cu_tokens[r];
+            if (run <= per_tile) continue;
+            units += uint64_t(g->geo.num_kv_heads) * g->geo.head_tiles;
+            longest = std::max<uint64_t>(longest, uint64_t(token_indices[r]) + run);
+        }
+        const bool short_runs = units * kChunkMaxPieces >= g->grid_cap || longest <= kChunkWholeTokens;
+        min_tiles = short_runs ? 2u : kChunkMinTiles;
+    }
+    for (uint32_t r = 0; r < num_reqs; ++r) {
+        const uint32_t tiles = (cu_tokens[r + 1] - cu_tokens[r] + per_tile - 1) / per_tile;
+        if (tiles > 0) (tiles >= min_tiles ? chunk_reqs : decode_reqs).push_back(r);
+    }
+}
+
 void run_append(psi_gqa* g, psi_pages* pages, psi_table* table, uint32_t layer, const void* k, const void* v) {
     require(g->prepared, "GQA batch metadata must be updated before recording");
     require(k != nullptr && v != nullptr, "k and v must not be null");
@@ -250,22 +271,22 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             // Requests with a long run of query tokens go to the chunk kernel (one pass over their KV for eight query
             // tiles at a time); the rest are decode rows.
             std::vector<uint32_t> decode_reqs, chunk_reqs;
-            for (uint32_t r = 0; r < num_reqs; ++r) {
-                const uint32_t tiles = (cu_tokens[r + 1] - cu_tokens[r] + g->geo.tokens_per_tile - 1) / g->geo.tokens_per_tile;
-                if (tiles == 0) continue;
-                (g->chunk_supported && tiles >= kChunkMinTiles ? chunk_reqs : decode_reqs).push_back(r);
-            }
+            split_requests(g, token_indices, cu_tokens, num_reqs, decode_reqs, chunk_reqs);
             const uint32_t min_tiles = g->kernel == PSI_KERNEL_MMA ? 16u : 4u;
             g->plan = build_balanced_plan(g->geo, req_slots, token_indices, cu_tokens, decode_reqs, g->grid_cap,
                                           min_tiles, g->item_start_cost);
             // K/V the long runs touch: below a third of the L2 the order of the work cannot cost HBM traffic, and exactly
             // equal balance beats stream order
             uint64_t chunk_kv_bytes = 0;
-            for (uint32_t r : chunk_reqs)
+            bool one_pass = true;  // every long run fits one super-tile: nothing is read twice in whatever order
+            for (uint32_t r : chunk_reqs) {
+                one_pass = one_pass && (cu_tokens[r + 1] - cu_tokens[r]) * g->geo.heads_per_tile <= kMaxRows * kChunkTilesPerItem;
                 chunk_kv_bytes += uint64_t(token_indices[r] + (cu_tokens[r + 1] - cu_tokens[r])) * (uint64_t(g->cfg.page_bytes) / g->tokens_per_page);
+            }
             g->chunk = build_chunk_plan(g->geo, req_slots, token_indices, cu_tokens, chunk_reqs, g->grid_cap,
                                         g->plan.num_partial_slots, static_cast<uint32_t>(g->plan.reduces.size()),
-                                        chunk_kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident : ChunkOrder::kStream,
+                                        chunk_kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident
+                                                                     : (one_pass ? ChunkOrder::kEqualShares : ChunkOrder::kStream),
                                         kChunkUnitCostTiles);
         }
         const WorkPlan& plan = g->plan;

@@ -191,10 +191,9 @@ int32_t psi_gqa_step_host(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
         // their kernel takes q and the appended rows through device memory.
         bool direct = q_bytes + 2 * kv_bytes >= kDirectHostBytes && !g->replay_reserved;
         if (direct && g->chunk_supported) {
-            for (uint32_t r = 0; r < num_reqs && direct; ++r) {
-                const uint32_t tiles = (cu_tokens[r + 1] - cu_tokens[r] + g->geo.tokens_per_tile - 1) / g->geo.tokens_per_tile;
-                if (tiles >= kChunkMinTiles) direct = false;
-            }
+            std::vector<uint32_t> decode_reqs, chunk_reqs;
+            split_requests(g, token_indices, cu_tokens, num_reqs, decode_reqs, chunk_reqs);
+            direct = chunk_reqs.empty();
         }
         if (!direct && q_bytes + 2 * kv_bytes >= kPipelineHostBytes && num_reqs >= 2 && !g->replay_reserved &&
             g->cfg.plan_mode == PSI_PLAN_BALANCED) {

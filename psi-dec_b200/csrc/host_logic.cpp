@@ -444,7 +444,8 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
     }
     plan.total_kv_tiles = total;
     if (total == 0) return plan;
-    const uint64_t num_ctas = std::min<uint64_t>(std::max(1u, max_ctas), std::max<uint64_t>(1, total / 4));
+    uint64_t num_ctas = std::min<uint64_t>(std::max(1u, max_ctas), std::max<uint64_t>(1, total / 4));
+    if (order != ChunkOrder::kStream) num_ctas = std::min<uint64_t>(num_ctas, uint64_t(kChunkMaxPieces) * units.size());
     auto make_item = [&](const Unit& u, uint64_t tile_begin, uint64_t tile_end) {
         const uint32_t head_tile = u.head % geo.head_tiles;
         DeviceItem d{};
@@ -480,7 +481,7 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
     };
     const bool l2_resident = order == ChunkOrder::kL2Resident;
     const uint64_t fair_share = (total + uint64_t(unit_start_cost) * units.size()) / num_ctas;
-    if (l2_resident && longest <= std::max<uint64_t>(fair_share / 2, 2 * kChunkMinPieceTiles)) {
+    if (l2_resident && longest <= std::max<uint64_t>(fair_share / 2, kChunkWholeTokens / kKvTile)) {
         // Whole units, longest first, each to the CTA with the least work so far.  Nothing is cut: a cut saves half a
         // unit's tiles on one CTA and costs two partial writes, a fence and a merge, about kChunkMinPieceTiles of them,
         // so it pays only for units of more than twice that which are also long against a CTA's share.

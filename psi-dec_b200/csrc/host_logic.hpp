@@ -176,6 +176,8 @@ struct ChunkPlan {
 };
 constexpr uint32_t kChunkTilesPerItem = 8;  // one query tile per warp
 constexpr uint32_t kChunkMinPieceTiles = 64;   // a KV piece of a cut unit is at least this many 16-token tiles
+constexpr uint32_t kChunkMaxPieces = 16;      // equal shares: a unit is cut into about this many pieces at most
+constexpr uint32_t kChunkWholeTokens = 2 * kChunkMinPieceTiles * 16;  // units of at most this many keys are not worth a cut
 constexpr uint32_t kChunkStartCostTiles = 8;   // fixed cost of a work item (query load, epilogue) in KV tiles, stream order
 constexpr uint32_t kChunkUnitCostTiles = 16;  // the same in the other orders (0 to 64 measured the same on whole units)
 
