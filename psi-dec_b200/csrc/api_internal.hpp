@@ -177,6 +177,7 @@ struct psi_gqa {
     psi_gqa_config cfg{};
     uint32_t tokens_per_page = 0;
     uint32_t kernel = PSI_KERNEL_GENERIC;  // resolved kernel
+    bool any_mma = false;                  // the generic path runs on the tensor cores (attend_mma_any.cu)
     uint32_t grid_cap = 1;
     uint32_t item_start_cost = 0;  // KV tiles one item switch is worth when shares are balanced
     psi::PlanGeometry geo{};

@@ -123,6 +123,7 @@ struct AttendParams {
     uint32_t dtype;
     float scale_log2;             // scale * log2(e)
     uint32_t* status;             // nullptr, or the word a bounded device-side wait writes PSI_ERR_TIMEOUT to
+    uint32_t tensor_cores;        // generic launches: 16-bit profiles may take attend_mma_any (not PSI_KERNEL_GENERIC)
     uint32_t tma_feed;            // decode kernel: whole K/V tiles by TMA boxes instead of cp.async (PSI_KERNEL_MMA_TMA)
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none
 };
@@ -181,6 +182,11 @@ uint32_t attend_staged_ctas_per_sm(uint32_t dtype);
 // The staged CUDA-core map kernel (attend_staged.cu): taken by launch_attend_generic when the launch qualifies.
 bool attend_staged_supported(const AttendParams& p);
 cudaError_t launch_attend_staged(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
+// The tensor-core map kernel for 16-bit profiles outside attend_mma_supported (attend_mma_any.cu): `profile` says whether a
+// component plans for it, `supported` whether a launch's buffers qualify.
+bool attend_mma_any_profile(uint32_t dtype, uint32_t head_dim);
+bool attend_mma_any_supported(const AttendParams& p);
+cudaError_t launch_attend_mma_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 // The ring-fed f32 map kernel (attend_f32.cu): taken before the staged one when the launch qualifies.
 bool attend_f32_supported(const AttendParams& p);
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
