@@ -55,21 +55,26 @@ const uint32_t* block_words(const psi_gqa* g, uint64_t offset) {
 }
 
 
+// Points a launch at one of the block's plans.
+static void use_plan(const psi_gqa* g, const PlanOffsets& off, AttendParams& p) {
+    p.scalars = block_words(g, off.scalars);
+    p.items = reinterpret_cast<const DeviceItem*>(block_words(g, off.items));
+    p.cta_item_begin = block_words(g, off.cta);
+    if (g->kernel == PSI_KERNEL_MMA) p.cta_first_items = reinterpret_cast<const DeviceItem*>(block_words(g, off.first_items));
+    p.reduces = reinterpret_cast<const ReduceUnit*>(block_words(g, off.reduces));
+}
+
 AttendParams attend_params(psi_gqa* g, const psi_pages* pages, const psi_table* table, uint32_t layer, const void* q) {
     require(g->prepared, "GQA batch metadata must be updated before recording");
     require(q != nullptr, "q must not be null");
     AttendParams p{};
     p.geo = page_geometry(g, pages, table, layer);
     p.q = q;
-    p.items = reinterpret_cast<const DeviceItem*>(block_words(g, g->off_items));
-    p.cta_item_begin = block_words(g, g->off_cta);
-    if (g->kernel == PSI_KERNEL_MMA) p.cta_first_items = reinterpret_cast<const DeviceItem*>(block_words(g, g->off_first_items));
-    p.reduces = reinterpret_cast<const ReduceUnit*>(block_words(g, g->off_reduces));
+    use_plan(g, g->off, p);
     p.partial_o = static_cast<float*>(g->partial_o.ptr);
     p.partial_m = static_cast<float*>(g->partial_ml.ptr);
     p.partial_l = p.partial_m == nullptr ? nullptr : p.partial_m + g->partial_slots_cap * kMaxRows;
     p.unit_counters = static_cast<uint32_t*>(g->unit_counters.ptr);
-    p.scalars = block_words(g, 0);
     p.num_q_heads = g->cfg.num_q_heads;
     p.dtype = g->cfg.dtype;
     p.scale_log2 = g->cfg.scale * 1.4426950408889634f;
@@ -86,7 +91,12 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     // launches (append, map, chunk, reduce where the kernel needs one), each at its capacity grid, each reading its
     // active counts from the device block.
     const bool fixed = g->replay_reserved;
-    if (p.new_k != nullptr && (fixed || g->chunk.num_ctas() > 0)) {
+    const bool merged = g->has_merged && p.new_k == nullptr && p.xchg.flag == nullptr;
+    const WorkPlan& plan = merged ? g->merged_plan : g->plan;
+    const ChunkPlan& chunk = merged ? g->merged_chunk : g->chunk;
+    const PlanOffsets& off = merged ? g->merged_off : g->off;
+    if (merged) use_plan(g, off, p);
+    if (p.new_k != nullptr && (fixed || chunk.num_ctas() > 0)) {
         // A fused step that carries long query runs: their K/V tiles are fetched page-wise by TMA, so the step's rows
         // go to their pages first (one more launch, against milliseconds of attention) and both kernels read pages only.
         AppendParams a{};
@@ -104,7 +114,7 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
         p.new_k = nullptr;
         p.new_v = nullptr;
     }
-    const uint32_t num_ctas = fixed ? g->grid_cap : g->plan.num_ctas();
+    const uint32_t num_ctas = fixed ? g->grid_cap : plan.num_ctas();
     if (num_ctas > 0) {
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_MAP);
         if (g->kernel == PSI_KERNEL_MMA) {
@@ -113,11 +123,11 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
             cuda_check(launch_attend_generic(p, num_ctas, ctx->stream), "attend (generic) launch");
         }
     }
-    const uint32_t chunk_ctas = fixed ? (g->chunk_supported ? g->grid_cap : 0u) : g->chunk.num_ctas();
+    const uint32_t chunk_ctas = fixed ? (g->chunk_supported ? g->grid_cap : 0u) : chunk.num_ctas();
     if (chunk_ctas > 0) {
         AttendParams c = p;
-        c.items = reinterpret_cast<const DeviceItem*>(block_words(g, g->off_chunk_items));
-        c.cta_item_begin = block_words(g, g->off_chunk_cta);
+        c.items = reinterpret_cast<const DeviceItem*>(block_words(g, off.chunk_items));
+        c.cta_item_begin = block_words(g, off.chunk_cta);
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_CHUNK);
         cudaError_t launched = cudaErrorNotSupported;
         if (g->chunk_umma) {
@@ -137,30 +147,29 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     // separate reduce pass.
     const uint32_t num_reduces = g->kernel == PSI_KERNEL_MMA
                                      ? 0u
-                                     : static_cast<uint32_t>(fixed ? g->cap_reduces : g->plan.reduces.size());
+                                     : static_cast<uint32_t>(fixed ? g->cap_reduces : plan.reduces.size());
     if (num_reduces > 0) {
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_REDUCE);
         cuda_check(launch_attend_reduce(p, num_reduces, ctx->stream), "attend reduce launch");
     }
 }
 
-void split_requests(const psi_gqa* g, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs,
-                    std::vector<uint32_t>& decode_reqs, std::vector<uint32_t>& chunk_reqs) {
+void split_requests(const psi_gqa* g, const RequestRuns& runs, std::vector<uint32_t>& decode_reqs,
+                    std::vector<uint32_t>& chunk_reqs) {
     const uint32_t per_tile = g->geo.tokens_per_tile;
     uint32_t min_tiles = kU32Max;
     if (g->chunk_supported) {
         uint64_t units = 0, longest = 0;
-        for (uint32_t r = 0; r < num_reqs; ++r) {
-            const uint32_t run = cu_tokens[r + 1] - cu_tokens[r];
-            if (run <= per_tile) continue;
+        for (uint32_t r = 0; r < runs.size(); ++r) {
+            if (runs.run(r) <= per_tile) continue;
             units += uint64_t(g->geo.num_kv_heads) * g->geo.head_tiles;
-            longest = std::max<uint64_t>(longest, uint64_t(token_indices[r]) + run);
+            longest = std::max<uint64_t>(longest, runs.context(r, runs.cu_tokens[r + 1]));
         }
         const bool short_runs = units * kChunkMaxPieces >= g->grid_cap || longest <= kChunkWholeTokens;
         min_tiles = short_runs ? 2u : kChunkMinTiles;
     }
-    for (uint32_t r = 0; r < num_reqs; ++r) {
-        const uint32_t tiles = (cu_tokens[r + 1] - cu_tokens[r] + per_tile - 1) / per_tile;
+    for (uint32_t r = 0; r < runs.size(); ++r) {
+        const uint32_t tiles = (runs.run(r) + per_tile - 1) / per_tile;
         if (tiles > 0) (tiles >= min_tiles ? chunk_reqs : decode_reqs).push_back(r);
     }
 }
@@ -213,6 +222,67 @@ void run_staged_host_step(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
     cuda_check(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
 }
 
+
+// This library's plan of a step: requests with a long run of query tokens go to the chunk kernel (one pass over their KV
+// for eight query tiles at a time); the rest are decode rows.
+static void plan_runs(const psi_gqa* g, const RequestRuns& runs, WorkPlan& plan, ChunkPlan& chunk) {
+    std::vector<uint32_t> decode_reqs, chunk_reqs;
+    split_requests(g, runs, decode_reqs, chunk_reqs);
+    const uint32_t min_tiles = g->kernel == PSI_KERNEL_MMA ? 16u : 4u;
+    plan = build_balanced_plan(g->geo, runs, decode_reqs, g->grid_cap, min_tiles, g->item_start_cost);
+    // K/V the long runs touch: below a third of the L2 the order of the work cannot cost HBM traffic, and balance beats
+    // stream order; so does it where every long run fits one super-tile and nothing is read twice in whatever order
+    uint64_t chunk_kv_bytes = 0;
+    bool one_pass = true;
+    for (uint32_t r : chunk_reqs) {
+        one_pass = one_pass && runs.run(r) * g->geo.heads_per_tile <= kMaxRows * kChunkTilesPerItem;
+        chunk_kv_bytes += uint64_t(runs.context(r, runs.cu_tokens[r + 1])) * (uint64_t(g->cfg.page_bytes) / g->tokens_per_page);
+    }
+    const ChunkOrder order = chunk_kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident
+                                                             : (one_pass ? ChunkOrder::kEqualShares : ChunkOrder::kStream);
+    chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots,
+                             static_cast<uint32_t>(plan.reduces.size()), order, kChunkUnitCostTiles);
+}
+
+// Places the arrays of one plan behind `cursor` words of the block.
+static void place_plan(PlanOffsets& off, uint64_t& cursor, const WorkPlan& plan, const ChunkPlan& chunk, uint64_t num_items) {
+    constexpr uint64_t kItemWords = sizeof(DeviceItem) / sizeof(uint32_t);
+    off.cta = cursor;
+    cursor += pad_words(plan.cta_item_begin.size());
+    off.reduces = cursor;
+    cursor += pad_words(plan.reduces.size() * 2);
+    off.items = cursor;
+    cursor += pad_words(num_items * kItemWords);
+    off.first_items = cursor;
+    cursor += pad_words(static_cast<uint64_t>(plan.num_ctas()) * kItemWords);
+    off.chunk_cta = cursor;
+    cursor += pad_words(chunk.cta_item_begin.size());
+    off.chunk_items = cursor;
+    cursor += pad_words(chunk.items.size() * kItemWords);
+}
+
+// Writes one plan into the staging block.
+static void pack_plan(uint32_t* s, const PlanOffsets& off, const WorkPlan& plan, const ChunkPlan& chunk,
+                      const std::vector<DeviceItem>& items, uint32_t num_tokens) {
+    constexpr uint64_t kItemWords = sizeof(DeviceItem) / sizeof(uint32_t);
+    std::fill(s + off.scalars, s + off.scalars + kScalarCount, 0u);
+    s[off.scalars + kScalarNumActiveTokens] = num_tokens;
+    s[off.scalars + kScalarNumCtas] = plan.num_ctas();
+    s[off.scalars + kScalarNumReduces] = static_cast<uint32_t>(plan.reduces.size());
+    s[off.scalars + kScalarNumChunkCtas] = chunk.num_ctas();
+    std::copy(plan.cta_item_begin.begin(), plan.cta_item_begin.end(), s + off.cta);
+    if (!plan.reduces.empty()) std::memcpy(s + off.reduces, plan.reduces.data(), plan.reduces.size() * sizeof(ReduceUnit));
+    if (!items.empty()) std::memcpy(s + off.items, items.data(), items.size() * sizeof(DeviceItem));
+    // a copy of every CTA's first item at a place the CTA can read without knowing its range (zeros for a CTA
+    // without items, which its empty range tells it not to use)
+    for (uint32_t c = 0; c < plan.num_ctas(); ++c) {
+        DeviceItem first{};
+        if (plan.cta_item_begin[c] < plan.cta_item_begin[c + 1]) first = items[plan.cta_item_begin[c]];
+        std::memcpy(s + off.first_items + c * kItemWords, &first, sizeof(DeviceItem));
+    }
+    std::copy(chunk.cta_item_begin.begin(), chunk.cta_item_begin.end(), s + off.chunk_cta);
+    if (!chunk.items.empty()) std::memcpy(s + off.chunk_items, chunk.items.data(), chunk.items.size() * sizeof(DeviceItem));
+}
 
 // GQAMetadataBuffers::update plus this library's plan.  With `defer_upload` the packed block stays in the pinned
 // staging buffer and its size comes back in *deferred_words: the caller brings it to the device itself.
@@ -268,33 +338,21 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             g->plan = build_reference_plan(g->geo, *g->md, shape, variant.tiled_q != 0, token_indices, cu_tokens,
                                            num_reqs);
             g->chunk = ChunkPlan{};
+            g->has_merged = false;
         } else {
-            // Requests with a long run of query tokens go to the chunk kernel (one pass over their KV for eight query
-            // tiles at a time); the rest are decode rows.
-            std::vector<uint32_t> decode_reqs, chunk_reqs;
-            split_requests(g, token_indices, cu_tokens, num_reqs, decode_reqs, chunk_reqs);
-            const uint32_t min_tiles = g->kernel == PSI_KERNEL_MMA ? 16u : 4u;
-            g->plan = build_balanced_plan(g->geo, req_slots, token_indices, cu_tokens, decode_reqs, g->grid_cap,
-                                          min_tiles, g->item_start_cost);
-            // K/V the long runs touch: below a third of the L2 the order of the work cannot cost HBM traffic, and exactly
-            // equal balance beats stream order
-            uint64_t chunk_kv_bytes = 0;
-            bool one_pass = true;  // every long run fits one super-tile: nothing is read twice in whatever order
-            for (uint32_t r : chunk_reqs) {
-                one_pass = one_pass && (cu_tokens[r + 1] - cu_tokens[r]) * g->geo.heads_per_tile <= kMaxRows * kChunkTilesPerItem;
-                chunk_kv_bytes += uint64_t(token_indices[r] + (cu_tokens[r + 1] - cu_tokens[r])) * (uint64_t(g->cfg.page_bytes) / g->tokens_per_page);
-            }
-            g->chunk = build_chunk_plan(g->geo, req_slots, token_indices, cu_tokens, chunk_reqs, g->grid_cap,
-                                        g->plan.num_partial_slots, static_cast<uint32_t>(g->plan.reduces.size()),
-                                        chunk_kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident
-                                                                     : (one_pass ? ChunkOrder::kEqualShares : ChunkOrder::kStream),
-                                        kChunkUnitCostTiles);
+            const RequestRuns runs = plain_runs(req_slots, token_indices, cu_tokens, num_reqs);
+            RequestRuns merged;
+            const bool can_merge = merge_one_position_runs(runs, merged);
+            plan_runs(g, can_merge && g->replay_reserved ? merged : runs, g->plan, g->chunk);
+            g->has_merged = can_merge && !g->replay_reserved;
+            if (g->has_merged) plan_runs(g, merged, g->merged_plan, g->merged_chunk);
         }
         const WorkPlan& plan = g->plan;
         const ChunkPlan& chunk = g->chunk;
         const std::vector<DeviceItem> device_items = flatten_plan(plan, g->geo);
-        const uint32_t total_slots = plan.num_partial_slots + chunk.num_partial_slots;
-        const uint32_t total_counters = static_cast<uint32_t>(plan.reduces.size()) + chunk.num_counters;
+        const std::vector<DeviceItem> merged_items = g->has_merged ? flatten_plan(g->merged_plan, g->geo) : std::vector<DeviceItem>{};
+        uint32_t total_slots = plan.num_partial_slots + chunk.num_partial_slots;
+        if (g->has_merged) total_slots = std::max(total_slots, g->merged_plan.num_partial_slots + g->merged_chunk.num_partial_slots);
 
         // Pack the device block: scalars | req_slots | flat_token_indices | cta ranges | reduces | items.
         uint64_t words = 0;
@@ -305,9 +363,9 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
                         plan.reduces.size() <= g->cap_reduces && total_slots <= g->partial_slots_cap &&
                         plan.num_ctas() <= g->grid_cap && chunk.num_ctas() <= g->grid_cap,
                     "the step exceeds the reserved replay capacity");
-            words = g->off_items + device_items.size() * kItemWords;
-            if (!chunk.items.empty()) words = g->off_chunk_items + chunk.items.size() * kItemWords;
-            if (!plan.reduces.empty()) words = g->off_reduces + plan.reduces.size() * 2;
+            words = g->off.items + device_items.size() * kItemWords;
+            if (!chunk.items.empty()) words = g->off.chunk_items + chunk.items.size() * kItemWords;
+            if (!plan.reduces.empty()) words = g->off.reduces + plan.reduces.size() * 2;
             cuda_check(cudaEventSynchronize(g->upload_done), "cudaEventSynchronize");  // previous upload left staging
         } else {
             uint64_t cursor = pad_words(kScalarCount);
@@ -315,18 +373,12 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             cursor += pad_words(num_tokens);
             g->off_token_indices = cursor;
             cursor += pad_words(num_tokens);
-            g->off_cta = cursor;
-            cursor += pad_words(plan.cta_item_begin.size());
-            g->off_reduces = cursor;
-            cursor += pad_words(plan.reduces.size() * 2);
-            g->off_items = cursor;
-            cursor += pad_words(device_items.size() * (sizeof(DeviceItem) / sizeof(uint32_t)));
-            g->off_first_items = cursor;
-            cursor += pad_words(static_cast<uint64_t>(plan.num_ctas()) * (sizeof(DeviceItem) / sizeof(uint32_t)));
-            g->off_chunk_cta = cursor;
-            cursor += pad_words(chunk.cta_item_begin.size());
-            g->off_chunk_items = cursor;
-            cursor += pad_words(chunk.items.size() * (sizeof(DeviceItem) / sizeof(uint32_t)));
+            place_plan(g->off, cursor, plan, chunk, device_items.size());
+            if (g->has_merged) {
+                g->merged_off.scalars = cursor;
+                cursor += pad_words(kScalarCount);
+                place_plan(g->merged_off, cursor, g->merged_plan, g->merged_chunk, merged_items.size());
+            }
             words = cursor;
 
             if (g->staging_words < words) {
@@ -351,44 +403,25 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             g->partial_slots_cap = slots;
         }
         // Arrival counters start at zero (cleared when allocated) and every launch returns them to zero itself.
-        (void)total_counters;
 
         uint32_t* s = g->staging;
-        std::fill(s, s + kScalarCount, 0u);
-        s[kScalarNumActiveTokens] = num_tokens;
-        s[kScalarNumCtas] = plan.num_ctas();
-        s[kScalarNumReduces] = static_cast<uint32_t>(plan.reduces.size());
-        s[kScalarNumChunkCtas] = chunk.num_ctas();
+        pack_plan(s, g->off, plan, chunk, device_items, num_tokens);
+        if (g->has_merged) pack_plan(s, g->merged_off, g->merged_plan, g->merged_chunk, merged_items, num_tokens);
         std::copy(g->md->req_slots.begin(), g->md->req_slots.begin() + num_tokens, s + g->off_req_slots);
         std::copy(g->md->flat_token_indices.begin(), g->md->flat_token_indices.begin() + num_tokens,
                   s + g->off_token_indices);
-        std::copy(plan.cta_item_begin.begin(), plan.cta_item_begin.end(), s + g->off_cta);
         if (g->replay_reserved) {
             // launches run at the capacity grid: CTAs beyond the plan's find an empty range and a zero first item
             constexpr uint64_t kItemWords = sizeof(DeviceItem) / sizeof(uint32_t);
             const uint32_t items_end = static_cast<uint32_t>(device_items.size());
-            for (uint64_t c = plan.cta_item_begin.size(); c < g->grid_cap + 2ull; ++c) s[g->off_cta + c] = items_end;
-            if (plan.cta_item_begin.empty()) s[g->off_cta] = 0;
-            std::fill(s + g->off_first_items, s + g->off_first_items + uint64_t(g->grid_cap) * kItemWords, 0u);
+            for (uint64_t c = plan.cta_item_begin.size(); c < g->grid_cap + 2ull; ++c) s[g->off.cta + c] = items_end;
+            if (plan.cta_item_begin.empty()) s[g->off.cta] = 0;
+            std::fill(s + g->off.first_items + uint64_t(plan.num_ctas()) * kItemWords,
+                      s + g->off.first_items + uint64_t(g->grid_cap) * kItemWords, 0u);
             const uint32_t chunk_end = static_cast<uint32_t>(chunk.items.size());
-            for (uint64_t c = chunk.cta_item_begin.size(); c < g->grid_cap + 2ull; ++c) s[g->off_chunk_cta + c] = chunk_end;
-            if (chunk.cta_item_begin.empty()) s[g->off_chunk_cta] = 0;
+            for (uint64_t c = chunk.cta_item_begin.size(); c < g->grid_cap + 2ull; ++c) s[g->off.chunk_cta + c] = chunk_end;
+            if (chunk.cta_item_begin.empty()) s[g->off.chunk_cta] = 0;
         }
-        if (!plan.reduces.empty())
-            std::memcpy(s + g->off_reduces, plan.reduces.data(), plan.reduces.size() * sizeof(ReduceUnit));
-        if (!device_items.empty())
-            std::memcpy(s + g->off_items, device_items.data(), device_items.size() * sizeof(DeviceItem));
-        // a copy of every CTA's first item at a place the CTA can read without knowing its range (zeros for a CTA
-        // without items, which its empty range tells it not to use)
-        for (uint32_t c = 0; c < plan.num_ctas(); ++c) {
-            DeviceItem first{};
-            if (plan.cta_item_begin[c] < plan.cta_item_begin[c + 1]) first = device_items[plan.cta_item_begin[c]];
-            std::memcpy(s + g->off_first_items + static_cast<uint64_t>(c) * (sizeof(DeviceItem) / sizeof(uint32_t)), &first,
-                        sizeof(DeviceItem));
-        }
-        std::copy(chunk.cta_item_begin.begin(), chunk.cta_item_begin.end(), s + g->off_chunk_cta);
-        if (!chunk.items.empty())
-            std::memcpy(s + g->off_chunk_items, chunk.items.data(), chunk.items.size() * sizeof(DeviceItem));
         if (defer_upload) {
             *deferred_words = words;
         } else {

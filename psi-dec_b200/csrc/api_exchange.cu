@@ -26,17 +26,37 @@ static int32_t combine_impl(psi_gqa* g, const float* const* o, const float* cons
     if (g == nullptr) return PSI_ERR_INVALID_ARGUMENT;
     return guarded(g->ctx, [&] {
         require(o != nullptr && m != nullptr && l != nullptr && out != nullptr, "combine arguments must not be null");
-        require(n > 0 && n <= 64, "combine takes between 1 and 64 partials");
+        require(n > 0 && n <= kCombineMaxPartials, "combine takes between 1 and 64 partials");
         require(num_tokens > 0 && num_tokens <= g->cfg.max_tokens, "combine token count out of range");
         psi_ctx* ctx = g->ctx;
         ctx->bind();
-        g->combine_ptrs.ensure(ctx, 3 * 64 * sizeof(void*), false);
-        std::vector<const float*> host(3 * 64, nullptr);
+        // the pointer table is reserved whichever kernel runs: whether a capture needs it does not depend on the call
+        g->combine_ptrs.ensure(ctx, 3 * kCombineMaxPartials * sizeof(void*), false);
+        std::vector<const float*> host(3 * kCombineMaxPartials, nullptr);
+        CombineRowsParams r{};
+        bool rows = flags == nullptr && n <= kCombineRowsPartials && g->cfg.head_dim % 4 == 0 &&
+                    uint64_t(num_tokens) * g->cfg.num_q_heads * g->cfg.head_dim / 4 < (1ull << 31);
         for (uint32_t i = 0; i < n; ++i) {
             require(o[i] != nullptr && m[i] != nullptr && l[i] != nullptr, "combine partial pointers must not be null");
             host[i] = o[i];
-            host[64 + i] = m[i];
-            host[128 + i] = l[i];
+            host[kCombineMaxPartials + i] = m[i];
+            host[2 * kCombineMaxPartials + i] = l[i];
+            rows = rows && (reinterpret_cast<uintptr_t>(o[i]) & 15u) == 0;
+            if (i < kCombineRowsPartials) {
+                r.o[i] = o[i];
+                r.m[i] = m[i];
+                r.l[i] = l[i];
+            }
+        }
+        if (rows) {
+            r.n = n;
+            r.num_rows = num_tokens * g->cfg.num_q_heads;
+            r.head_dim = g->cfg.head_dim;
+            r.dtype = g->cfg.dtype;
+            r.out = out;
+            LaunchScope scope(ctx, PSI_KERNEL_CLASS_COMBINE);
+            cuda_check(launch_combine_rows(r, ctx->stream), "combine launch");
+            return;
         }
         // Pageable source: the runtime stages the bytes before the call returns, so `host` may go out of scope.
         cuda_check(cudaMemcpyAsync(g->combine_ptrs.ptr, host.data(), host.size() * sizeof(void*),
@@ -45,8 +65,8 @@ static int32_t combine_impl(psi_gqa* g, const float* const* o, const float* cons
         CombineParams p{};
         auto* base = static_cast<const float* const*>(g->combine_ptrs.ptr);
         p.o = base;
-        p.m = base + 64;
-        p.l = base + 128;
+        p.m = base + kCombineMaxPartials;
+        p.l = base + 2 * kCombineMaxPartials;
         p.n = n;
         p.num_rows = num_tokens * g->cfg.num_q_heads;
         p.head_dim = g->cfg.head_dim;

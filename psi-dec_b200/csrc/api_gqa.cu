@@ -104,17 +104,17 @@ static void reserved_layout(psi_gqa* g) {
     cursor += pad_words(t);
     g->off_token_indices = cursor;
     cursor += pad_words(t);
-    g->off_cta = cursor;
+    g->off.cta = cursor;
     cursor += pad_words(g->grid_cap + 2);
-    g->off_first_items = cursor;
+    g->off.first_items = cursor;
     cursor += pad_words(uint64_t(g->grid_cap) * kItemWords);
-    g->off_chunk_cta = cursor;
+    g->off.chunk_cta = cursor;
     cursor += pad_words(g->grid_cap + 2);
-    g->off_items = cursor;
+    g->off.items = cursor;
     cursor += pad_words(g->cap_items * kItemWords);
-    g->off_chunk_items = cursor;
+    g->off.chunk_items = cursor;
     cursor += pad_words(g->cap_chunk_items * kItemWords);
-    g->off_reduces = cursor;
+    g->off.reduces = cursor;
     cursor += pad_words(g->cap_reduces * 2);
     g->staging_words = cursor;
 }

@@ -172,6 +172,15 @@ struct psi_id_allocator {
     explicit psi_id_allocator(uint64_t capacity) : impl(capacity) {}
 };
 
+namespace psi {
+// Where the arrays of one plan lie in the device block (in words).
+struct PlanOffsets {
+    uint64_t scalars = 0, cta = 0, reduces = 0, items = 0;
+    uint64_t first_items = 0;  // copies of every CTA's first item (mma kernel)
+    uint64_t chunk_cta = 0, chunk_items = 0;
+};
+}  // namespace psi
+
 struct psi_gqa {
     psi_ctx* ctx = nullptr;
     psi_gqa_config cfg{};
@@ -196,9 +205,15 @@ struct psi_gqa {
     uint64_t staging_words = 0;
     cudaEvent_t upload_done = nullptr;
     // section offsets (in words) of the block uploaded by the last prepare
-    uint64_t off_req_slots = 0, off_token_indices = 0, off_cta = 0, off_reduces = 0, off_items = 0;
-    uint64_t off_chunk_cta = 0, off_chunk_items = 0;
-    uint64_t off_first_items = 0;  // copies of every CTA's first item (mma kernel)
+    uint64_t off_req_slots = 0, off_token_indices = 0;
+    psi::PlanOffsets off;
+    // The plan with adjacent requests of one position merged (merge_one_position_runs), for launches that read this step's
+    // K/V from their pages; beside the plan above, which fused launches take.  Under a replay reservation every launch
+    // reads pages, so the merged plan is the only one.
+    bool has_merged = false;
+    psi::WorkPlan merged_plan;
+    psi::ChunkPlan merged_chunk;
+    psi::PlanOffsets merged_off;
     // Replay reservation: every array of the device block at a fixed offset sized for max_tokens, every scratch buffer
     // at its largest, every launch at its capacity grid, so that a captured graph stays valid from step to step.
     bool replay_reserved = false;
@@ -281,8 +296,8 @@ constexpr uint32_t kPipelineMaxGroups = 8;
 AttendParams attend_params(psi_gqa* g, const psi_pages* pages, const psi_table* table, uint32_t layer, const void* q);
 void run_attend(psi_gqa* g, const AttendParams& params);
 // Deals a step's requests to the decode kernel and the chunk kernels.
-void split_requests(const psi_gqa* g, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs,
-                    std::vector<uint32_t>& decode_reqs, std::vector<uint32_t>& chunk_reqs);
+void split_requests(const psi_gqa* g, const RequestRuns& runs, std::vector<uint32_t>& decode_reqs,
+                    std::vector<uint32_t>& chunk_reqs);
 void run_append(psi_gqa* g, psi_pages* pages, psi_table* table, uint32_t layer, const void* k, const void* v);
 // Device-side address of a pinned, device-mapped host buffer (16-byte aligned), or nullptr for any other memory.
 void* mapped_device_pointer(const void* host);

@@ -119,8 +119,8 @@ int32_t psi_chunk_plan_preview(uint32_t num_q_heads, uint32_t num_kv_heads, cons
             slots[r] = r;
             requests[r] = r;
         }
-        const ChunkPlan plan = build_chunk_plan(plan_geometry(num_q_heads, num_kv_heads), slots.data(), token_indices,
-                                                cu_tokens, requests, max_ctas, 0, 0,
+        const ChunkPlan plan = build_chunk_plan(plan_geometry(num_q_heads, num_kv_heads),
+                                                plain_runs(slots.data(), token_indices, cu_tokens, num_reqs), requests, max_ctas, 0, 0,
                                                 equal_shares != 0 ? ChunkOrder::kEqualShares : ChunkOrder::kStream);
         out_counts[0] = static_cast<uint32_t>(plan.items.size());
         out_counts[1] = plan.num_ctas();

@@ -134,7 +134,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_chunk_kernel(AttendParams 
             }
             *reinterpret_cast<uint4*>(smem + warp * L::kTileBytes + swizzled(r, c, L::kRowBytes)) = value;
         }
-        if (fused && v.writes_kv) {
+        if (fused && (v.flags & kItemWritesKv)) {
             for (uint32_t i = tid; i < v.num_tokens * 2 * kChunks; i += kThreads) {
                 const uint32_t c = i % kChunks, which = (i / kChunks) & 1, j = i / (2 * kChunks);
                 const uint32_t pos = v.first_pos + j;

@@ -8,6 +8,7 @@
 // crates/inference-backend-metal/src/components/metal/gqa_split_kv_single_q_map.metal:85-252 (visibility through
 // kv_end only) extended with the per-row causal limit of metal/gqa_split_kv_tiled_q.metal:233-244.
 #include <cmath>
+#include <type_traits>
 
 #include "device_common.cuh"
 #include "exchange.cuh"
@@ -257,6 +258,140 @@ __global__ void __launch_bounds__(kBlockPartialWarps * 32) block_partial_kernel(
     }
 }
 
+// The same for head dims of 32 VEC (64, 128, 256) in the 16-bit types and aligned buffers: a lane holds VEC consecutive
+// elements, the K (and then the V) rows of eight block tokens are loaded together and their dot products reduced side by
+// side.  Bound by latency: one row after the other put a load and a five-step reduction in a chain for every block token.
+// Measured: 84 draft tokens of 40/8 heads x 128 in blocks of seven 5.5 us against 12.5 us.
+template <typename T, int VEC>
+__global__ void __launch_bounds__(kBlockPartialWarps * 32) block_partial_rows_kernel(BlockPartialParams p) {
+    constexpr uint32_t D = 32 * VEC, kStep = 8;
+    using Raw = typename std::conditional<VEC == 8, uint4, typename std::conditional<VEC == 4, uint2, uint32_t>::type>::type;
+    __shared__ float weights_s[kBlockPartialWarps][kBlockPartialMaxBlock];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint64_t pair = static_cast<uint64_t>(blockIdx.x) * kBlockPartialWarps + warp;
+    if (pair >= static_cast<uint64_t>(p.num_tokens) * p.num_q_heads) return;
+    const uint32_t token = static_cast<uint32_t>(pair / p.num_q_heads), head = static_cast<uint32_t>(pair % p.num_q_heads);
+    const uint32_t kv_head = head / (p.num_q_heads / p.num_kv_heads);
+    const uint32_t begin = token / p.block_size * p.block_size;
+    float* weights = weights_s[warp];
+    auto widen = [](const Raw& raw, float (&v)[VEC]) {
+        const T* e = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) v[i] = static_cast<float>(e[i]);
+    };
+    // rows j0 .. j0 + 7 of the block (the last row again beyond its end)
+    auto load_rows = [&](const void* base, uint32_t j0, Raw (&raw)[kStep]) {
+#pragma unroll
+        for (uint32_t i = 0; i < kStep; ++i) {
+            const uint64_t row = static_cast<uint64_t>(begin + min(j0 + i, p.block_size - 1)) * p.num_kv_heads + kv_head;
+            raw[i] = reinterpret_cast<const Raw*>(static_cast<const T*>(base) + row * D)[lane];
+        }
+    };
+    float q[VEC];
+    widen(reinterpret_cast<const Raw*>(static_cast<const T*>(p.q) + pair * D)[lane], q);
+
+    Raw raw[kStep], v_raw[kStep];
+    load_rows(p.local_k, 0, raw);
+    load_rows(p.local_v, 0, v_raw);
+    float block_max = -INFINITY;
+    for (uint32_t j0 = 0; j0 < p.block_size; j0 += kStep) {
+        if (j0 > 0) load_rows(p.local_k, j0, raw);
+        float s[kStep];
+#pragma unroll
+        for (uint32_t i = 0; i < kStep; ++i) {
+            float k[VEC];
+            widen(raw[i], k);
+            s[i] = 0.0f;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) s[i] += q[e] * k[e];
+        }
+#pragma unroll
+        for (int offset = 16; offset > 0; offset >>= 1)
+#pragma unroll
+            for (uint32_t i = 0; i < kStep; ++i) s[i] += __shfl_xor_sync(0xFFFFFFFFu, s[i], offset);
+#pragma unroll
+        for (uint32_t i = 0; i < kStep; ++i) {
+            if (j0 + i >= p.block_size) break;
+            const float score = s[i] * p.scale;
+            if (lane == 0) weights[j0 + i] = score;
+            block_max = fmaxf(block_max, score);
+        }
+    }
+    __syncwarp();
+    float exp_sum = 0.0f;
+    for (uint32_t j = lane; j < p.block_size; j += 32) {
+        const float w = expf(weights[j] - block_max);
+        weights[j] = w;
+        exp_sum += w;
+    }
+    exp_sum = warp_sum(exp_sum);
+    __syncwarp();
+    float acc[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) acc[e] = 0.0f;
+    for (uint32_t j0 = 0; j0 < p.block_size; j0 += kStep) {
+        if (j0 > 0) load_rows(p.local_v, j0, v_raw);
+#pragma unroll
+        for (uint32_t i = 0; i < kStep; ++i) {
+            if (j0 + i >= p.block_size) break;
+            const float w = weights[j0 + i];
+            float v[VEC];
+            widen(v_raw[i], v);
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) acc[e] += w * v[e];
+        }
+    }
+    const uint64_t slot = p.slot_indices != nullptr ? p.slot_indices[token] : token;
+    const uint64_t out_row = slot * p.num_q_heads + head;
+    if (lane == 0) {
+        p.m[out_row] = block_max;
+        p.l[out_row] = exp_sum;
+    }
+    float* out = p.o + out_row * D + lane * VEC;
+#pragma unroll
+    for (int e = 0; e < VEC; e += 2)
+        *reinterpret_cast<float2*>(out + e) = make_float2(exp_sum > 0.0f ? acc[e] / exp_sum : 0.0f, exp_sum > 0.0f ? acc[e + 1] / exp_sum : 0.0f);
+}
+
+// Merge of up to four partials whose rows are whole float4 columns: a thread owns four columns of a row, and the row's
+// statistics and its columns of every partial go out together.  Measured
+// (84 draft rows of 40 heads x 128, two partials): 4.0 us against 9.7 us with an element per thread and a pointer table.
+__global__ void __launch_bounds__(kReduceThreads) combine_rows_kernel(const __grid_constant__ CombineRowsParams p) {
+    const uint32_t c4 = p.head_dim / 4;
+    const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kReduceThreads + threadIdx.x;
+    if (i >= static_cast<uint64_t>(p.num_rows) * c4) return;
+    const uint64_t row = i / c4;
+    float pm[kCombineRowsPartials], pl[kCombineRowsPartials];
+    float4 po[kCombineRowsPartials];
+#pragma unroll
+    for (uint32_t s = 0; s < kCombineRowsPartials; ++s) {
+        pm[s] = -INFINITY;
+        if (s < p.n) {
+            pm[s] = __ldcg(p.m[s] + row);
+            pl[s] = __ldcg(p.l[s] + row);
+            po[s] = __ldcg(reinterpret_cast<const float4*>(p.o[s]) + i);
+        }
+    }
+    float global_max = -INFINITY;
+#pragma unroll
+    for (uint32_t s = 0; s < kCombineRowsPartials; ++s) global_max = fmaxf(global_max, pm[s]);
+    float sum = 0.0f;
+    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (uint32_t s = 0; s < kCombineRowsPartials; ++s) {
+        if (s >= p.n) break;
+        const float w = isfinite(pm[s]) ? expf(pm[s] - global_max) * pl[s] : 0.0f;
+        sum += w;
+        acc.x += w * po[s].x;
+        acc.y += w * po[s].y;
+        acc.z += w * po[s].z;
+        acc.w += w * po[s].w;
+    }
+    const float v[4] = {acc.x, acc.y, acc.z, acc.w};
+#pragma unroll
+    for (int e = 0; e < 4; ++e) store_from_float(p.out, 4 * i + e, p.dtype, sum > 0.0f ? v[e] / sum : 0.0f);
+}
+
 // Cross-device merge of per-device partials in the natural-log domain (same algebra as above).
 __global__ void __launch_bounds__(kReduceThreads) combine_kernel(CombineParams p) {
     bool ready = true;
@@ -347,7 +482,27 @@ cudaError_t launch_block_partial(const BlockPartialParams& p, cudaStream_t strea
     if (pairs == 0) return cudaSuccess;
     if (p.block_size == 0 || p.block_size > kBlockPartialMaxBlock) return cudaErrorInvalidValue;
     const uint64_t blocks = (pairs + kBlockPartialWarps - 1) / kBlockPartialWarps;
+    const uint32_t d = p.head_dim;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.local_k) |
+                           reinterpret_cast<uintptr_t>(p.local_v) | reinterpret_cast<uintptr_t>(p.o)) & 15u) == 0;
+    if (p.dtype != PSI_DTYPE_F32 && (d == 64 || d == 128 || d == 256) && aligned) {
+        auto launch = [&](auto kernel) {
+            kernel<<<static_cast<uint32_t>(blocks), kBlockPartialWarps * 32, 0, stream>>>(p);
+            return cudaGetLastError();
+        };
+        const bool bf16 = p.dtype == PSI_DTYPE_BF16;
+        if (d == 64) return launch(bf16 ? block_partial_rows_kernel<__nv_bfloat16, 2> : block_partial_rows_kernel<__half, 2>);
+        if (d == 128) return launch(bf16 ? block_partial_rows_kernel<__nv_bfloat16, 4> : block_partial_rows_kernel<__half, 4>);
+        return launch(bf16 ? block_partial_rows_kernel<__nv_bfloat16, 8> : block_partial_rows_kernel<__half, 8>);
+    }
     block_partial_kernel<<<static_cast<uint32_t>(blocks), kBlockPartialWarps * 32, 0, stream>>>(p);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_combine_rows(const CombineRowsParams& p, cudaStream_t stream) {
+    const uint64_t columns = static_cast<uint64_t>(p.num_rows) * p.head_dim / 4;
+    if (columns == 0) return cudaSuccess;
+    combine_rows_kernel<<<static_cast<unsigned>((columns + kReduceThreads - 1) / kReduceThreads), kReduceThreads, 0, stream>>>(p);
     return cudaGetLastError();
 }
 

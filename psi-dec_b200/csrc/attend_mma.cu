@@ -226,7 +226,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
         // ---- with the first tiles in flight: the per-row causal limits, and in the fused step this item's share of the
         // step's K/V rows into their pages -------------------------------------------------------------------------------
         if (tid < kTile) limit_s[tid] = tid < v.rows ? item_row_limit(v, tid) : v.kv_end;
-        if (fused && v.writes_kv) {
+        if (fused && (v.flags & kItemWritesKv)) {
             for (uint32_t i = tid; i < v.num_tokens * 2 * kChunks; i += kThreads) {
                 const uint32_t c = i % kChunks, which = (i / kChunks) & 1, j = i / (2 * kChunks);
                 const uint32_t pos = v.first_pos + j;

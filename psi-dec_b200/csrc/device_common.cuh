@@ -207,9 +207,9 @@ __device__ __forceinline__ uint64_t item_row_index(const AttendParams& p, const 
     return static_cast<uint64_t>(v.flat_begin + r / v.num_heads) * p.num_q_heads + v.head0 + r % v.num_heads;
 }
 
-// Keys row r may see: [0, first_pos + token(r)] clipped to the item's range end.
+// Keys row r may see: [0, first_pos + token(r)] clipped to the item's range end ([0, first_pos] in a run at one position).
 __device__ __forceinline__ uint32_t item_row_limit(const ItemView& v, uint32_t r) {
-    return min(v.kv_end, v.first_pos + r / v.num_heads + 1);
+    return min(v.kv_end, v.first_pos + ((v.flags & kItemOnePosition) ? 0u : r / v.num_heads) + 1);
 }
 
 constexpr float kLn2 = 0.6931471805599453f;

@@ -268,6 +268,38 @@ PlanGeometry plan_geometry(uint32_t num_q_heads, uint32_t num_kv_heads) {
     return g;
 }
 
+RequestRuns plain_runs(const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs) {
+    RequestRuns runs;
+    runs.req_slots.assign(req_slots, req_slots + num_reqs);
+    runs.token_indices.assign(token_indices, token_indices + num_reqs);
+    runs.cu_tokens.assign(cu_tokens, cu_tokens + num_reqs + 1);
+    runs.one_position.assign(num_reqs, 0);
+    return runs;
+}
+
+bool merge_one_position_runs(const RequestRuns& runs, RequestRuns& merged) {
+    auto same = [&](uint32_t a, uint32_t b) {
+        return runs.run(a) == 1 && runs.run(b) == 1 && runs.req_slots[a] == runs.req_slots[b] &&
+               runs.token_indices[a] == runs.token_indices[b];
+    };
+    const uint32_t n = runs.size();
+    bool any = false;
+    for (uint32_t r = 1; r < n && !any; ++r) any = same(r - 1, r);
+    if (!any) return false;
+    merged = RequestRuns{};
+    merged.cu_tokens.push_back(0);
+    for (uint32_t r = 0; r < n;) {
+        uint32_t end = r + 1;
+        while (end < n && same(r, end)) ++end;
+        merged.req_slots.push_back(runs.req_slots[r]);
+        merged.token_indices.push_back(runs.token_indices[r]);
+        merged.cu_tokens.push_back(runs.cu_tokens[end]);
+        merged.one_position.push_back(end - r > 1 ? 1 : 0);
+        r = end;
+    }
+    return true;
+}
+
 namespace {
 
 // Closes the plan: assigns partial slots to every item whose (tile, head_sel) unit is shared with another item and
@@ -306,21 +338,20 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots,
                              uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
     std::vector<uint32_t> all(num_reqs);
     for (uint32_t r = 0; r < num_reqs; ++r) all[r] = r;
-    return build_balanced_plan(geo, req_slots, token_indices, cu_tokens, all, max_ctas, min_kv_tiles_per_cta,
-                               item_start_cost);
+    return build_balanced_plan(geo, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), all, max_ctas,
+                               min_kv_tiles_per_cta, item_start_cost);
 }
 
-WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
-                             const uint32_t* cu_tokens, const std::vector<uint32_t>& requests, uint32_t max_ctas,
-                             uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
+                             uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
     WorkPlan plan;
     std::vector<uint32_t> tile_ctx;
     for (uint32_t r : requests) {
-        for (uint32_t begin = cu_tokens[r]; begin < cu_tokens[r + 1];) {
-            uint32_t end = std::min(cu_tokens[r + 1], begin + geo.tokens_per_tile);
-            plan.tiles.push_back({begin, end, req_slots[r], token_indices[r] + (begin - cu_tokens[r]),
-                                  token_indices[r], cu_tokens[r]});
-            tile_ctx.push_back(token_indices[r] + (end - cu_tokens[r]));
+        for (uint32_t begin = runs.cu_tokens[r]; begin < runs.cu_tokens[r + 1];) {
+            uint32_t end = std::min(runs.cu_tokens[r + 1], begin + geo.tokens_per_tile);
+            plan.tiles.push_back({begin, end, runs.req_slots[r], runs.position(r, begin), runs.token_indices[r],
+                                  runs.cu_tokens[r], runs.one_position[r] != 0});
+            tile_ctx.push_back(runs.context(r, end));
             begin = end;
         }
     }
@@ -387,7 +418,7 @@ WorkPlan build_reference_plan(const PlanGeometry& geo, const ReferenceMetadata& 
             const uint32_t tile = static_cast<uint32_t>(plan.tiles.size());
             while (req + 1 < num_reqs && begin >= cu_tokens[req + 1]) ++req;
             plan.tiles.push_back({begin, end, md.req_slots[begin], md.flat_token_indices[begin], token_indices[req],
-                                  cu_tokens[req]});
+                                  cu_tokens[req], false});
             const uint32_t ctx = md.flat_token_indices[end - 1] + 1;  // keys the sub-tile's last token sees
             for (uint32_t h = 0; h < heads; ++h) {
                 for (uint32_t s = s_begin; s < s_end; ++s) {
@@ -412,8 +443,7 @@ WorkPlan build_reference_plan(const PlanGeometry& geo, const ReferenceMetadata& 
     return plan;
 }
 
-ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
-                           const uint32_t* cu_tokens, const std::vector<uint32_t>& requests, uint32_t max_ctas,
+ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint32_t max_ctas,
                            uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost) {
     ChunkPlan plan;
     // Units in stream order: all super-tiles of one (request, KV head) follow one another, so that CTAs working on
@@ -429,13 +459,13 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
     // longest requests first: the work dealt last, which decides how far the last CTA trails, is the cheapest
     std::vector<uint32_t> by_length(requests);
     std::stable_sort(by_length.begin(), by_length.end(), [&](uint32_t a, uint32_t b) {
-        return token_indices[a] + (cu_tokens[a + 1] - cu_tokens[a]) > token_indices[b] + (cu_tokens[b + 1] - cu_tokens[b]);
+        return runs.context(a, runs.cu_tokens[a + 1]) > runs.context(b, runs.cu_tokens[b + 1]);
     });
     for (uint32_t r : by_length) {
         for (uint32_t h = 0; h < heads; ++h) {
-            for (uint32_t begin = cu_tokens[r]; begin < cu_tokens[r + 1];) {
-                const uint32_t end = std::min(cu_tokens[r + 1], begin + tokens_per_item);
-                units.push_back({r, begin, end, token_indices[r] + (end - cu_tokens[r]), h});
+            for (uint32_t begin = runs.cu_tokens[r]; begin < runs.cu_tokens[r + 1];) {
+                const uint32_t end = std::min(runs.cu_tokens[r + 1], begin + tokens_per_item);
+                units.push_back({r, begin, end, runs.context(r, end), h});
                 total += div_ceil(units.back().ctx_end, kKvTile);
                 longest = std::max(longest, div_ceil(units.back().ctx_end, kKvTile));
                 begin = end;
@@ -454,14 +484,14 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, c
         d.partial_slot = kU32Max;
         d.flat_begin = u.flat_begin;
         d.num_tokens = u.flat_end - u.flat_begin;
-        d.req_slot = req_slots[u.req];
+        d.req_slot = runs.req_slots[u.req];
         d.kv_head = u.head / geo.head_tiles;
         d.head0 = d.kv_head * geo.group + head_tile * geo.heads_per_tile;
         d.num_heads = std::min(geo.heads_per_tile, geo.group - head_tile * geo.heads_per_tile);
-        d.first_pos = token_indices[u.req] + (u.flat_begin - cu_tokens[u.req]);
-        d.new_begin = token_indices[u.req];
-        d.flat_req_begin = cu_tokens[u.req];
-        d.writes_kv = head_tile == 0 ? 1u : 0u;
+        d.first_pos = runs.position(u.req, u.flat_begin);
+        d.new_begin = runs.token_indices[u.req];
+        d.flat_req_begin = runs.cu_tokens[u.req];
+        d.flags = (head_tile == 0 ? kItemWritesKv : 0u) | (runs.one_position[u.req] ? kItemOnePosition : 0u);
         return d;
     };
     // `n` consecutive items starting at `first` are the pieces of one unit cut across CTAs: partial slots 8 apart,
@@ -613,7 +643,7 @@ std::vector<DeviceItem> flatten_plan(const WorkPlan& plan, const PlanGeometry& g
         d.first_pos = tile.first_pos;
         d.new_begin = tile.new_begin;
         d.flat_req_begin = tile.flat_req_begin;
-        d.writes_kv = head_tile == 0 ? 1u : 0u;
+        d.flags = (head_tile == 0 ? kItemWritesKv : 0u) | (tile.one_position ? kItemOnePosition : 0u);
     }
     return out;
 }

@@ -85,6 +85,7 @@ struct ExecTile {
     uint32_t first_pos;       // request-absolute position of the tile's first token
     uint32_t new_begin;       // request-absolute position of the request's first token of this step
     uint32_t flat_req_begin;  // flat index of that token
+    bool one_position;        // every token of the tile stands at first_pos (RequestRuns::one_position)
 };
 
 // One unit of map work while the plan is being built: the rows of (tile, head_sel) against KV tokens
@@ -117,8 +118,10 @@ struct DeviceItem {
     uint32_t first_pos;       // position of the tile's first token: token j sees keys [0, first_pos + j]
     uint32_t new_begin;       // positions at or beyond this belong to this step's appended tokens
     uint32_t flat_req_begin;  // flat index of the token at position new_begin
-    uint32_t writes_kv;       // 1: the item appends its tile's K/V rows that fall into its KV range (fused step)
+    uint32_t flags;           // kItemWritesKv, kItemOnePosition
 };
+constexpr uint32_t kItemWritesKv = 1u;     // the item appends its tile's K/V rows that fall into its KV range (fused step)
+constexpr uint32_t kItemOnePosition = 2u;  // every token of the item sees keys [0, first_pos]
 static_assert(sizeof(DeviceItem) == 64, "DeviceItem is read as four 16-byte words");
 
 struct ReduceUnit {
@@ -135,6 +138,22 @@ struct PlanGeometry {
 };
 
 PlanGeometry plan_geometry(uint32_t num_q_heads, uint32_t num_kv_heads);
+
+// The step's requests as the planners see them: a run of consecutive query tokens of one slot each.
+struct RequestRuns {
+    std::vector<uint32_t> req_slots, token_indices, cu_tokens;
+    std::vector<uint8_t> one_position;  // the run's tokens all stand at token_indices[r] instead of following one another
+    uint32_t size() const { return static_cast<uint32_t>(req_slots.size()); }
+    uint32_t run(uint32_t r) const { return cu_tokens[r + 1] - cu_tokens[r]; }
+    // position of flat token `t` of request r, and the keys its run sees up to and with the token before `end`
+    uint32_t position(uint32_t r, uint32_t t) const { return token_indices[r] + (one_position[r] ? 0 : t - cu_tokens[r]); }
+    uint32_t context(uint32_t r, uint32_t end) const { return token_indices[r] + (one_position[r] ? 1 : end - cu_tokens[r]); }
+};
+RequestRuns plain_runs(const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs);
+// Adjacent one-token requests of one slot at one position (the rows of a draft block, which all see the same history)
+// become one run, so that the history is read once for all of them; false when there are none.  Not for launches that
+// take this step's K/V rows from the caller's buffers: there every request reads its own row at that position.
+bool merge_one_position_runs(const RequestRuns& runs, RequestRuns& merged);
 
 struct WorkPlan {
     std::vector<ExecTile> tiles;
@@ -153,9 +172,8 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots,
                              const uint32_t* cu_tokens, uint32_t num_reqs, uint32_t max_ctas,
                              uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost = 0);
 // The same over a subset of the batch's requests (indices into the request arrays, ascending).
-WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
-                             const uint32_t* cu_tokens, const std::vector<uint32_t>& requests, uint32_t max_ctas,
-                             uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost = 0);
+WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
+                             uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost = 0);
 
 // One CTA per (reference KV split, head_sel); reference q tiles wider than tokens_per_tile are cut into sub-tiles
 // that share the split boundaries.
@@ -190,8 +208,7 @@ enum class ChunkOrder {
 };
 
 // Outside stream order a unit counts as its KV tiles plus `unit_start_cost`.
-ChunkPlan build_chunk_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
-                           const uint32_t* cu_tokens, const std::vector<uint32_t>& requests, uint32_t max_ctas,
+ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint32_t max_ctas,
                            uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost = 0);
 
 // Device form of a finished plan.

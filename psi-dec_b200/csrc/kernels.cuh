@@ -128,6 +128,22 @@ struct AttendParams {
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none
 };
 
+constexpr uint32_t kCombineMaxPartials = 64;
+constexpr uint32_t kCombineRowsPartials = 4;
+
+// Merge of up to four partials without flags: the pointers travel with the launch, so that it waits for no upload.
+struct CombineRowsParams {
+    const float* o[kCombineRowsPartials];
+    const float* m[kCombineRowsPartials];
+    const float* l[kCombineRowsPartials];
+    uint32_t n;
+    uint32_t num_rows;            // num_tokens * Hq
+    uint32_t head_dim;            // a multiple of four; o 16-byte aligned
+    uint32_t dtype;
+    void* out;
+};
+cudaError_t launch_combine_rows(const CombineRowsParams& p, cudaStream_t stream);
+
 struct CombineParams {
     const float* const* o;        // device array of n pointers
     const float* const* m;
