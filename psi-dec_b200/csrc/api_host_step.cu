@@ -230,6 +230,7 @@ int32_t psi_gqa_step_host(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
         p.out = dout;
         p.new_k = direct ? dk : g->step_k.ptr;
         p.new_v = direct ? dv : g->step_v.ptr;
+        p.plan_ready = 0;  // the pull launch brings it
         run_attend(g, p);
         cuda_check(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
     });

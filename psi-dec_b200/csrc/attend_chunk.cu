@@ -38,6 +38,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_chunk_kernel(AttendParams 
     constexpr uint32_t kRowsPerPass = kThreads / kChunks;
 
     const uint32_t cta = blockIdx.x;
+    await_previous_kernel();
     if (cta >= p.scalars[kScalarNumChunkCtas]) return;
 
     extern __shared__ __align__(1024) unsigned char smem[];
@@ -291,8 +292,7 @@ cudaError_t launch_one(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
     static std::atomic<uint64_t> configured{0};  // per instantiation, one bit per device
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(L::kTotal), configured);
     if (err != cudaSuccess) return err;
-    kernel<<<num_ctas, kThreads, L::kTotal, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, num_ctas, kThreads, L::kTotal, stream, p);
 }
 
 template <typename T>

@@ -158,7 +158,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                        kBarQ = kBarP + 2, kNumBarriers = kBarQ + 1;
 
     const uint32_t cta = blockIdx.x;
-    if (cta >= p.scalars[kScalarNumChunkCtas]) return;
+    const bool early = p.plan_ready != 0;  // the set-up below runs before the wait for the inputs
+    if (!early) await_previous_kernel();
+    if (cta >= p.scalars[kScalarNumChunkCtas]) {
+        if (early) await_previous_kernel();
+        return;
+    }
 
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t bars[kNumBarriers];
@@ -186,6 +191,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base_s;
+    if (early) await_previous_kernel();
 
     const uint32_t page_mask = p.geo.tokens_per_page - 1;
     const uint32_t page_shift = 31 - __clz(p.geo.tokens_per_page);
@@ -651,8 +657,7 @@ cudaError_t launch_one(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
     static std::atomic<uint64_t> configured{0};  // per instantiation, one bit per device
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(kSmem), configured);
     if (err != cudaSuccess) return err;
-    kernel<<<num_ctas, kUmmaThreads, kSmem, stream>>>(p, map, box_rows);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, num_ctas, kUmmaThreads, kSmem, stream, p, map, box_rows);
 }
 
 template <typename T>

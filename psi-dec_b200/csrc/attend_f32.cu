@@ -280,6 +280,7 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
 template <int DG, int NSLOT>
 __global__ void __launch_bounds__(kF32Threads, 1) attend_f32_kernel(AttendParams p) {
     const uint32_t cta = blockIdx.x;
+    await_previous_kernel();
     if (cta >= p.scalars[kScalarNumCtas]) return;
     extern __shared__ __align__(128) unsigned char f32_smem[];
     __shared__ F32Shared shared;
@@ -357,8 +358,7 @@ cudaError_t launch_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
     // the largest head_dim sets the limit once; smaller ones fit under it
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(f32_smem_bytes(128 * DG, NSLOT)), configured);
     if (err != cudaSuccess) return err;
-    kernel<<<num_ctas, kF32Threads, f32_smem_bytes(p.geo.head_dim, NSLOT), stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, num_ctas, kF32Threads, f32_smem_bytes(p.geo.head_dim, NSLOT), stream, p);
 }
 
 }  // namespace

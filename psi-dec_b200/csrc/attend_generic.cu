@@ -12,6 +12,7 @@
 
 #include "device_common.cuh"
 #include "exchange.cuh"
+#include "launch_util.hpp"
 
 namespace psi {
 
@@ -22,6 +23,7 @@ constexpr int kGenericThreads = 32;
 template <int DPL>
 __global__ void __launch_bounds__(kGenericThreads) attend_generic_kernel(AttendParams p) {
     const uint32_t cta = blockIdx.x;
+    await_previous_kernel();
     if (cta >= p.scalars[kScalarNumCtas]) return;
     const uint32_t lane = threadIdx.x;
     const uint32_t D = p.geo.head_dim;
@@ -136,6 +138,7 @@ __device__ __forceinline__ float reduce_warp_max(float v) {
 
 __global__ void __launch_bounds__(kReduceThreads) attend_reduce_kernel(AttendParams p) {
     const uint32_t unit = blockIdx.x, r = blockIdx.y;
+    await_previous_kernel();
     if (unit >= p.scalars[kScalarNumReduces]) return;
     const ReduceUnit ru = p.reduces[unit];
     const ItemView v = view_item(p, ru.first_item);
@@ -213,6 +216,7 @@ constexpr uint32_t kBlockPartialWarps = 4;
 constexpr uint32_t kBlockPartialMaxBlock = 256;
 
 __global__ void __launch_bounds__(kBlockPartialWarps * 32) block_partial_kernel(BlockPartialParams p) {
+    await_previous_kernel();
     __shared__ float weights_s[kBlockPartialWarps][kBlockPartialMaxBlock];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t pair = static_cast<uint64_t>(blockIdx.x) * kBlockPartialWarps + warp;
@@ -266,6 +270,7 @@ template <typename T, int VEC>
 __global__ void __launch_bounds__(kBlockPartialWarps * 32) block_partial_rows_kernel(BlockPartialParams p) {
     constexpr uint32_t D = 32 * VEC, kStep = 8;
     using Raw = typename std::conditional<VEC == 8, uint4, typename std::conditional<VEC == 4, uint2, uint32_t>::type>::type;
+    await_previous_kernel();
     __shared__ float weights_s[kBlockPartialWarps][kBlockPartialMaxBlock];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint64_t pair = static_cast<uint64_t>(blockIdx.x) * kBlockPartialWarps + warp;
@@ -357,6 +362,7 @@ __global__ void __launch_bounds__(kBlockPartialWarps * 32) block_partial_rows_ke
 // statistics and its columns of every partial go out together.  Measured
 // (84 draft rows of 40 heads x 128, two partials): 4.0 us against 9.7 us with an element per thread and a pointer table.
 __global__ void __launch_bounds__(kReduceThreads) combine_rows_kernel(const __grid_constant__ CombineRowsParams p) {
+    await_previous_kernel();
     const uint32_t c4 = p.head_dim / 4;
     const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kReduceThreads + threadIdx.x;
     if (i >= static_cast<uint64_t>(p.num_rows) * c4) return;
@@ -457,24 +463,15 @@ cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cuda
     if (attend_f32_supported(p)) return launch_attend_f32(p, num_ctas, stream);
     if (attend_staged_supported(p)) return launch_attend_staged(p, num_ctas, stream);
     const uint32_t dpl = (p.geo.head_dim + 31) / 32;
-    if (dpl <= 1) {
-        attend_generic_kernel<1><<<num_ctas, kGenericThreads, 0, stream>>>(p);
-    } else if (dpl <= 2) {
-        attend_generic_kernel<2><<<num_ctas, kGenericThreads, 0, stream>>>(p);
-    } else if (dpl <= 4) {
-        attend_generic_kernel<4><<<num_ctas, kGenericThreads, 0, stream>>>(p);
-    } else if (dpl <= 8) {
-        attend_generic_kernel<8><<<num_ctas, kGenericThreads, 0, stream>>>(p);
-    } else {
-        return cudaErrorInvalidValue;
-    }
-    return cudaGetLastError();
+    if (dpl > 8) return cudaErrorInvalidValue;
+    auto kernel = dpl <= 1 ? attend_generic_kernel<1>
+                           : (dpl <= 2 ? attend_generic_kernel<2> : (dpl <= 4 ? attend_generic_kernel<4> : attend_generic_kernel<8>));
+    return launch_overlapped(kernel, num_ctas, kGenericThreads, 0, stream, p);
 }
 
 cudaError_t launch_attend_reduce(const AttendParams& p, uint32_t num_reduces, cudaStream_t stream) {
     if (num_reduces == 0) return cudaSuccess;
-    attend_reduce_kernel<<<dim3(num_reduces, kMaxRows), kReduceThreads, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(attend_reduce_kernel, dim3(num_reduces, kMaxRows), kReduceThreads, 0, stream, p);
 }
 
 cudaError_t launch_block_partial(const BlockPartialParams& p, cudaStream_t stream) {
@@ -487,23 +484,21 @@ cudaError_t launch_block_partial(const BlockPartialParams& p, cudaStream_t strea
                            reinterpret_cast<uintptr_t>(p.local_v) | reinterpret_cast<uintptr_t>(p.o)) & 15u) == 0;
     if (p.dtype != PSI_DTYPE_F32 && (d == 64 || d == 128 || d == 256) && aligned) {
         auto launch = [&](auto kernel) {
-            kernel<<<static_cast<uint32_t>(blocks), kBlockPartialWarps * 32, 0, stream>>>(p);
-            return cudaGetLastError();
+            return launch_overlapped(kernel, static_cast<uint32_t>(blocks), kBlockPartialWarps * 32, 0, stream, p);
         };
         const bool bf16 = p.dtype == PSI_DTYPE_BF16;
         if (d == 64) return launch(bf16 ? block_partial_rows_kernel<__nv_bfloat16, 2> : block_partial_rows_kernel<__half, 2>);
         if (d == 128) return launch(bf16 ? block_partial_rows_kernel<__nv_bfloat16, 4> : block_partial_rows_kernel<__half, 4>);
         return launch(bf16 ? block_partial_rows_kernel<__nv_bfloat16, 8> : block_partial_rows_kernel<__half, 8>);
     }
-    block_partial_kernel<<<static_cast<uint32_t>(blocks), kBlockPartialWarps * 32, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(block_partial_kernel, static_cast<uint32_t>(blocks), kBlockPartialWarps * 32, 0, stream, p);
 }
 
 cudaError_t launch_combine_rows(const CombineRowsParams& p, cudaStream_t stream) {
     const uint64_t columns = static_cast<uint64_t>(p.num_rows) * p.head_dim / 4;
     if (columns == 0) return cudaSuccess;
-    combine_rows_kernel<<<static_cast<unsigned>((columns + kReduceThreads - 1) / kReduceThreads), kReduceThreads, 0, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(combine_rows_kernel, static_cast<unsigned>((columns + kReduceThreads - 1) / kReduceThreads),
+                             kReduceThreads, 0, stream, p);
 }
 
 cudaError_t launch_combine(const CombineParams& p, cudaStream_t stream) {

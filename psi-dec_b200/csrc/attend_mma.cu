@@ -57,6 +57,8 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
     // The plan and the page table are read again by the next launch of the step (one launch per layer) while hundreds
     // of megabytes of K/V pass through the L2 in between: their lines are loaded to be evicted last.
     const uint64_t keep = l2_evict_last_policy();
+    const bool early = !kExchange && p.plan_ready != 0;  // plan and page table are read before the wait for the inputs
+    if (!early) await_previous_kernel();
     // One round trip for everything the first tile copies depend on: the CTA count, this CTA's item range and a copy
     // of its first item all go out before the first of them is needed.
     const uint32_t num_ctas = ld_u32_hinted(p.scalars + kScalarNumCtas, keep);
@@ -64,7 +66,10 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
     const uint32_t item_end = ld_u32_hinted(p.cta_item_begin + cta + 1, keep);
     const bool have_first = p.cta_first_items != nullptr;
     const ItemView first_item = view_item_hinted(have_first ? p.cta_first_items + cta : p.items, keep);
-    if (cta >= num_ctas) return;
+    if (cta >= num_ctas || item_begin >= item_end) {
+        if (early) await_previous_kernel();
+        if (!kExchange || cta >= num_ctas) return;
+    }
 
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ uint32_t limit_s[kTile];
@@ -196,6 +201,12 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
         RowState<D> st;
         st.clear();
 
+        // ids of the tile whose halves are issued next, and of the tile after it
+        uint32_t cur_lo = 0, cur_hi = 0, next_lo = 0, next_hi = 0;
+        if (my_tiles > 0) lookup(0, cur_lo, cur_hi);
+        if (my_tiles > 1) lookup(1, next_lo, next_hi);
+        if (early && index == item_begin) await_previous_kernel();
+
         // The query rows go straight into shared memory (zero rows beyond the item's) as the item's oldest copy group:
         // they need nothing but the item, so they are under way before the first page id is known.
         for (uint32_t i = tid; i < kTile * kChunks; i += kThreads) {
@@ -206,10 +217,6 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
         }
         cp_async_commit();
 
-        // ids of the tile whose halves are issued next, and of the tile after it
-        uint32_t cur_lo = 0, cur_hi = 0, next_lo = 0, next_hi = 0;
-        if (my_tiles > 0) lookup(0, cur_lo, cur_hi);
-        if (my_tiles > 1) lookup(1, next_lo, next_hi);
 #pragma unroll
         for (uint32_t h = 0; h < NSLOT - 1; ++h) {
             if (h < my_halves) {
@@ -480,6 +487,7 @@ cudaError_t launch_one(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
     static std::atomic<uint64_t> configured{0};  // per instantiation, one bit per device
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(L::kTotal), configured);
     if (err != cudaSuccess) return err;
+    if (!kExchange) return launch_overlapped(kernel, num_ctas, kThreads, L::kTotal, stream, p, map, box_rows);
     kernel<<<num_ctas, kThreads, L::kTotal, stream>>>(p, map, box_rows);
     return cudaGetLastError();
 }

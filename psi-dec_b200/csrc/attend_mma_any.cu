@@ -8,8 +8,8 @@
 // item and a ring of its own (K tile, V tile, K tile, ...) fed by 16-byte cp.async, the next tile's page looked up one
 // tile ahead.  Rows are padded to DP elements plus one 16-byte chunk: an odd number of chunks per row keeps ldmatrix free
 // of bank conflicts without a swizzle, and the chunks beyond head_dim hold zeros.
-// Measured: 24 requests of 300 to 6,000 tokens, 24/8 heads x 96, pages of 12 (233 MB): 73 us = 3.2 TB/s (five-eighths of
-// the items are short), the whole step with append and reduce 78 us, against 472 us on the staged kernel.
+// Measured: 24 requests of 300 to 6,000 tokens, 24/8 heads x 96, pages of 12 (233 MB): 73 us = 3.2 TB/s, the
+// whole step with append and reduce 78 us, against 472 us on the staged kernel.
 #include <atomic>
 
 #include "launch_util.hpp"
@@ -53,6 +53,7 @@ template <typename T, int DP, int NSLOT>
 __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParams p) {
     using L = AnySmem<DP, NSLOT>;
     const uint32_t cta = blockIdx.x;
+    await_previous_kernel();
     if (cta >= p.scalars[kScalarNumCtas]) return;
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t limit_s[kTile];
@@ -299,8 +300,7 @@ cudaError_t launch_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
     static std::atomic<uint64_t> configured{0};
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kBytes, configured);
     if (err != cudaSuccess) return err;
-    kernel<<<num_ctas, kThreads, kBytes, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, num_ctas, kThreads, kBytes, stream, p);
 }
 
 template <typename T>

@@ -84,6 +84,7 @@ __global__ void __launch_bounds__(kStagedThreads, sizeof(T) == 4 ? 1 : 2) attend
     constexpr bool kAsync = sizeof(T) == 4;
     constexpr uint32_t kStages = kAsync ? 2 : 1;
     const uint32_t cta = blockIdx.x;
+    await_previous_kernel();
     if (cta >= p.scalars[kScalarNumCtas]) return;
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t D = p.geo.head_dim, C4 = D / 4, k_stride = D + 4;
@@ -333,8 +334,7 @@ cudaError_t launch_staged(const AttendParams& p, uint32_t num_ctas, cudaStream_t
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel),
                                           static_cast<int>(staged_smem_floats(256, stages) * sizeof(float)), configured);
     if (err != cudaSuccess) return err;
-    kernel<<<num_ctas, kStagedThreads, bytes, stream>>>(p);
-    return cudaGetLastError();
+    return launch_overlapped(kernel, num_ctas, kStagedThreads, bytes, stream, p);
 }
 
 }  // namespace

@@ -8,6 +8,16 @@
 
 namespace psi {
 
+// For kernels launched with launch_overlapped: returns once every earlier kernel of the stream has completed and its
+// writes are visible, then lets the next kernel's CTAs become resident.  Because a kernel lets its successor start only
+// after this point, a kernel that has started knows that the one before its predecessor has completed.  Nothing that an
+// earlier kernel writes is touched before this call; the step's plan, the page table and the front stage's weights are
+// written by copies, which order kernels around them fully, and may be read before it.  Every CTA makes the call, also
+// one without work: a kernel that completed before its predecessor would let its successor run too early.
+__device__ __forceinline__ void await_previous_kernel() {
+    asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
+}
+
 __device__ __forceinline__ float load_as_float(const void* base, uint64_t index, uint32_t dtype) {
     if (dtype == PSI_DTYPE_F32) return static_cast<const float*>(base)[index];
     if (dtype == PSI_DTYPE_BF16) return __bfloat162float(static_cast<const __nv_bfloat16*>(base)[index]);

@@ -123,6 +123,7 @@ struct AttendParams {
     uint32_t dtype;
     float scale_log2;             // scale * log2(e)
     uint32_t* status;             // nullptr, or the word a bounded device-side wait writes PSI_ERR_TIMEOUT to
+    uint32_t plan_ready;          // the plan was in place before the stream's previous kernel started (no kernel copies it)
     uint32_t tensor_cores;        // generic launches: 16-bit profiles may take attend_mma_any (not PSI_KERNEL_GENERIC)
     uint32_t tma_feed;            // decode kernel: whole K/V tiles by TMA boxes instead of cp.async (PSI_KERNEL_MMA_TMA)
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none

@@ -7,6 +7,7 @@
 #include <algorithm>
 
 #include "device_common.cuh"
+#include "launch_util.hpp"
 
 namespace psi {
 
@@ -14,6 +15,7 @@ namespace {
 
 template <typename Unit>
 __global__ void kv_append_kernel(AppendParams p, uint32_t units_per_row) {
+    await_previous_kernel();
     const uint32_t num_active = min(p.scalars[kScalarNumActiveTokens], p.num_total_tokens);
     const uint64_t rows = static_cast<uint64_t>(num_active) * p.geo.num_kv_heads;
     const uint64_t total = rows * units_per_row;
@@ -100,14 +102,8 @@ cudaError_t launch_kv_append(const AppendParams& p, cudaStream_t stream) {
     const bool wide = row_bytes % 16 == 0 && aligned16(p.flat_k) && aligned16(p.flat_v) && aligned16(p.geo.pages);
     const uint32_t units = wide ? row_bytes / 16 : p.geo.head_dim;
     const uint64_t blocks = (rows * units + kCopyThreads - 1) / kCopyThreads;
-    if (wide) {
-        kv_append_kernel<uint4><<<static_cast<unsigned>(blocks), kCopyThreads, 0, stream>>>(p, units);
-    } else if (p.geo.elem_bytes == 4) {
-        kv_append_kernel<uint32_t><<<static_cast<unsigned>(blocks), kCopyThreads, 0, stream>>>(p, units);
-    } else {
-        kv_append_kernel<uint16_t><<<static_cast<unsigned>(blocks), kCopyThreads, 0, stream>>>(p, units);
-    }
-    return cudaGetLastError();
+    auto kernel = wide ? kv_append_kernel<uint4> : (p.geo.elem_bytes == 4 ? kv_append_kernel<uint32_t> : kv_append_kernel<uint16_t>);
+    return launch_overlapped(kernel, static_cast<unsigned>(blocks), kCopyThreads, 0, stream, p, units);
 }
 
 cudaError_t launch_page_gather(const GatherParams& p, cudaStream_t stream) {

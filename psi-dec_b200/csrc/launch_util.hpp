@@ -23,4 +23,21 @@ inline cudaError_t ensure_dynamic_smem(const void* kernel, int bytes, std::atomi
     return cudaSuccess;
 }
 
+// Launches `kernel` so that its CTAs may become resident while the previous kernel of the stream still runs (programmatic
+// dependent launch).  Every kernel launched this way passes await_previous_kernel() (device_common.cuh) in every CTA.
+template <typename... Params, typename... Args>
+cudaError_t launch_overlapped(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
+    cudaLaunchAttribute attribute{};
+    attribute.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attribute.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = grid;
+    config.blockDim = block;
+    config.dynamicSmemBytes = smem;
+    config.stream = stream;
+    config.attrs = &attribute;
+    config.numAttrs = 1;
+    return cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
 }  // namespace psi

@@ -11,6 +11,7 @@
 // metal/gqa_qkv_split.metal:13-36 without).  Its q, g, k and v rows are read where the projection left them; only the
 // gate rows, which the attention epilogue wants contiguous, are copied out.
 #include "device_common.cuh"
+#include "launch_util.hpp"
 
 namespace psi {
 
@@ -37,6 +38,7 @@ __device__ __forceinline__ void copy_element(void* dst, uint64_t dst_index, cons
 
 template <uint32_t DTYPE>
 __global__ void __launch_bounds__(kPrepWarps * 32) norm_rope_append_kernel(PrepParams p) {
+    await_previous_kernel();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t num_active = min(p.scalars[kScalarNumActiveTokens], p.num_total_tokens);
     const uint32_t hq = p.num_q_heads, hkv = p.geo.num_kv_heads, D = p.geo.head_dim;
@@ -192,7 +194,10 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t group = lane / LPR, sub = lane % LPR, d0 = sub * 8;
     const uint32_t token = blockIdx.x;
-    if (token >= min(p.scalars[kScalarNumActiveTokens], p.num_total_tokens)) return;
+    if (token >= min(p.scalars[kScalarNumActiveTokens], p.num_total_tokens)) {
+        await_previous_kernel();
+        return;
+    }
     const uint32_t hq = p.num_q_heads, hkv = p.geo.num_kv_heads;
     const uint32_t num_rows = hq + 2 * hkv + (p.g_in != nullptr ? hq : 0);  // q | k | v | gates
     const uint32_t stride = gridDim.y * kPrepWarps * kRows;
@@ -206,10 +211,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
         else if (row < hq + 2 * hkv) x.load(p.v_in, kv_row + static_cast<uint64_t>(row - hq - hkv) * D);
         else if (row < num_rows) x.load(p.g_in, q_row + (row - hq - 2 * hkv) * p.q_head_stride);
     };
-    Eight<DTYPE> held[kHeld];
-#pragma unroll
-    for (int i = 0; i < kHeld; ++i) fetch(first + i * stride, held[i]);
-
+    // everything that needs only the plan, the table and the weights comes before the wait for the inputs
     Eight<DTYPE> q_weight, k_weight;  // the bf16 weights in T
     {
         Eight<PSI_DTYPE_BF16> w;
@@ -230,6 +232,10 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
         sincosf(static_cast<float>(pos) * p.inverse_frequencies[i], &s, &c);
         turn_s[i] = make_float2(c, s);
     }
+    await_previous_kernel();
+    Eight<DTYPE> held[kHeld];
+#pragma unroll
+    for (int i = 0; i < kHeld; ++i) fetch(first + i * stride, held[i]);
     __syncthreads();
     const bool in_rope = sub < 2 * half_lanes, low = sub < half_lanes;
     const uint32_t partner = in_rope ? (low ? lane + half_lanes : lane - half_lanes) : lane;
@@ -286,7 +292,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
 bool aligned16(const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; }
 
 template <uint32_t DTYPE>
-bool launch_rows(const PrepParams& p, cudaStream_t stream) {
+bool launch_rows(const PrepParams& p, cudaStream_t stream, cudaError_t& status) {
     const uint32_t d = p.geo.head_dim;
     if ((d != 64 && d != 128 && d != 256) || p.rope_dim % 16 != 0 || !aligned16(p.q_in) || !aligned16(p.k_in) || !aligned16(p.v_in) ||
         !aligned16(p.g_in) || !aligned16(p.q_out) || !aligned16(p.g_out) || !aligned16(p.geo.pages) || !aligned16(p.q_weight) ||
@@ -303,9 +309,8 @@ bool launch_rows(const PrepParams& p, cudaStream_t stream) {
     const uint32_t split = (rows + rows_per_cta * per_warp - 1) / (rows_per_cta * per_warp);
     if (split > 65535) return false;
     const dim3 grid(p.num_total_tokens, split);
-    if (d == 64) norm_rope_rows_kernel<DTYPE, 8><<<grid, kPrepWarps * 32, 0, stream>>>(p);
-    else if (d == 128) norm_rope_rows_kernel<DTYPE, 16><<<grid, kPrepWarps * 32, 0, stream>>>(p);
-    else norm_rope_rows_kernel<DTYPE, 32><<<grid, kPrepWarps * 32, 0, stream>>>(p);
+    auto kernel = d == 64 ? norm_rope_rows_kernel<DTYPE, 8> : (d == 128 ? norm_rope_rows_kernel<DTYPE, 16> : norm_rope_rows_kernel<DTYPE, 32>);
+    status = launch_overlapped(kernel, grid, kPrepWarps * 32, 0, stream, p);
     return true;
 }
 
@@ -315,17 +320,16 @@ cudaError_t launch_norm_rope_append(const PrepParams& p, cudaStream_t stream) {
     const uint64_t rows = static_cast<uint64_t>(p.num_total_tokens) *
                           ((p.g_in != nullptr ? 2ull : 1ull) * p.num_q_heads + 2ull * p.geo.num_kv_heads);
     if (rows == 0) return cudaSuccess;
-    if (p.dtype == PSI_DTYPE_F32 ? launch_rows<PSI_DTYPE_F32>(p, stream)
-                                 : (p.dtype == PSI_DTYPE_BF16 ? launch_rows<PSI_DTYPE_BF16>(p, stream) : launch_rows<PSI_DTYPE_F16>(p, stream))) {
-        return cudaGetLastError();
+    cudaError_t status = cudaSuccess;
+    if (p.dtype == PSI_DTYPE_F32 ? launch_rows<PSI_DTYPE_F32>(p, stream, status)
+                                 : (p.dtype == PSI_DTYPE_BF16 ? launch_rows<PSI_DTYPE_BF16>(p, stream, status)
+                                                              : launch_rows<PSI_DTYPE_F16>(p, stream, status))) {
+        return status;
     }
     const unsigned blocks = static_cast<unsigned>((rows + kPrepWarps - 1) / kPrepWarps);
-    switch (p.dtype) {
-        case PSI_DTYPE_F32: norm_rope_append_kernel<PSI_DTYPE_F32><<<blocks, kPrepWarps * 32, 0, stream>>>(p); break;
-        case PSI_DTYPE_BF16: norm_rope_append_kernel<PSI_DTYPE_BF16><<<blocks, kPrepWarps * 32, 0, stream>>>(p); break;
-        default: norm_rope_append_kernel<PSI_DTYPE_F16><<<blocks, kPrepWarps * 32, 0, stream>>>(p); break;
-    }
-    return cudaGetLastError();
+    auto kernel = p.dtype == PSI_DTYPE_F32 ? norm_rope_append_kernel<PSI_DTYPE_F32>
+                                           : (p.dtype == PSI_DTYPE_BF16 ? norm_rope_append_kernel<PSI_DTYPE_BF16> : norm_rope_append_kernel<PSI_DTYPE_F16>);
+    return launch_overlapped(kernel, blocks, kPrepWarps * 32, 0, stream, p);
 }
 
 }  // namespace psi
