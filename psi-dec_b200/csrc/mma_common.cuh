@@ -91,6 +91,9 @@ __device__ __forceinline__ void cp_async_16_hinted(uint32_t dst, const void* src
                  : "memory");
 }
 
+// Requests the 128-byte line at `ptr` into the L2.
+__device__ __forceinline__ void prefetch_l2(const void* ptr) { asm volatile("prefetch.global.L2 [%0];\n" ::"l"(ptr)); }
+
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 
 template <int N>
