@@ -15,10 +15,12 @@
 //   warps 5 and 6: bring the K and the V tiles from their pages by TMA, one 5-D box per page segment that lands in
 //       exactly the order the MMA descriptors read ([8-row group][64-element block][8 rows][64 elements], 128-byte
 //       swizzle); an item's last, ragged tile is copied with zero-filling 16-byte cp.async instead.
-// An item costs about 10 us beside its tiles (0.9 us each at head_dim 256): query rows, the fill of the pipeline, the
-// epilogue of one row per thread.  Prompts have many short items, so the query rows and the first gates travel under the
-// last P V, the gates one pass ahead of their use, rows are packed (a group of six fills 126 of 128 rows, not 96), and
-// the plan deals whole units: three prompts of 611 to 2,500 tokens (24/4 heads x 256, gated) 186 us a layer, 1,066 before.
+// Beside its tiles (0.96 us each at head_dim 256, 0.82 at 128) an item costs query rows, the fill of the pipeline and the
+// epilogue of one row per thread: 13 us at head_dim 256 with gates when every thread reads and writes global memory for
+// its own row (32 lines an access), hence the staging areas and, paying for them, six ring slots instead of seven at
+// head_dim 256.  Prompts have many short items, so the next query rows are staged under the tiles and loaded under the
+// last P V, rows are packed (a group of six fills 126 of 128 rows, not 96), and the plan deals whole units.  Three prompts
+// of 611 to 2,500 tokens, 24/4 heads x 256, gated, two layers: 461 us a step, 501 without the staging, 2,414 at first.
 // All hand-offs are mbarriers (TMA byte counts, tcgen05.commit, thread arrivals); every wait is bounded and reports
 // PSI_ERR_TIMEOUT through the status word instead of hanging, and the kernel frees its TMEM on every path.  The kernel
 // reads pages only: a step that appends and attends runs the append launch first.
@@ -137,9 +139,26 @@ __device__ __forceinline__ float fast_exp2(float x) {
 // (log2 domain): P then stays below 2^8, well inside bf16/f16, and O is rescaled only on a real jump.
 template <int D>
 struct Ring {
-    static constexpr uint32_t kSlots = D == 256 ? 7u : 12u;
+    static constexpr uint32_t kSlots = D == 256 ? 6u : 12u;
 };
 constexpr float kRescaleThreshold = 8.0f;
+static_assert(offsetof(DeviceItem, flat_begin) == 24 && offsetof(DeviceItem, num_tokens) == 28 && offsetof(DeviceItem, head0) == 40 &&
+                  offsetof(DeviceItem, num_heads) == 44,
+              "the row threads read these fields of the next item as the ends of two 16-byte words");
+constexpr uint32_t kUmmaStageColumns = 128;  // columns of the row warps' staging areas
+
+// 8-byte global->shared copy; src_bytes == 0 zero-fills.
+__device__ __forceinline__ void cp_async_8(uint32_t dst, const void* src, uint32_t src_bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
+}
+__device__ __forceinline__ uint4 ld_shared_16(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared_16(uint32_t addr, uint4 v) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
 
 template <typename T, int D>
 __global__ void __launch_bounds__(kUmmaThreads, 1)
@@ -153,6 +172,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
     // overwritten by P (again two elements per column), O
     constexpr uint32_t kColQ = 0, kColS = D / 2, kColO = D / 2 + 2 * kUmmaN;
     static_assert(kColO + D <= kTmemColumns, "Q, S and O share one TMEM allocation");
+    constexpr uint32_t kStageColumns = kUmmaStageColumns, kStageBytes = 32 * kStageColumns * 2;  // staging area of a row warp
     // barriers
     constexpr uint32_t kBarFull = 0, kBarEmpty = kSlots, kBarS = 2 * kSlots, kBarO = kBarS + 2, kBarP = kBarO + 2,
                        kBarQ = kBarP + 2, kNumBarriers = kBarQ + 1;
@@ -335,6 +355,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
         // ================================ one accumulator row per thread ===============================================
         const uint32_t lane_base = (warp * 32u) << 16;  // this warp's TMEM lanes
         const uint32_t tmem_o = tmem + kColO;
+        const bool wide_gates = (reinterpret_cast<uintptr_t>(p.gates) & 15u) == 0;
         const bool wide_out = (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0;
         // Row of this thread in an item: row tid = (token tid / heads, head tid % heads) of the super-tile, packed without
         // gaps; w and rr are its 16-row tile and its row inside it, the unit of partial slots and arrival counters.
@@ -344,35 +365,67 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
             return static_cast<uint64_t>(v.flat_begin + (valid ? tid / v.num_heads : 0)) * p.num_q_heads + v.head0 +
                    (valid ? tid % v.num_heads : 0);
         };
-        // This thread's query row of an item into its TMEM lane (zero for rows the super-tile does not have).  Called
-        // when every Q K^T of the previous item has completed; 16 loads in flight at a time.
-        auto load_q = [&](const ItemView& v) {
-            bool valid;
-            const uint64_t row = row_of(v, valid);
-            const uint4* q_row = reinterpret_cast<const uint4*>(static_cast<const T*>(p.q) + row * D);
+        // Rows of q, the gates and the output pass through a staging area of this warp, 32 rows x 128 columns: one thread per
+        // row would touch 32 lines with every access, so global memory is read and written two whole rows at a time and
+        // every thread reads or writes its own row in shared memory (16-byte chunks XOR-ed with the row: no bank conflicts).
+        const uint32_t stage = smem_base + kSlots * kTileBytes + warp * kStageBytes;
+        auto stage_at = [&](uint32_t row, uint32_t chunk) { return stage + row * (kStageColumns * 2) + ((chunk ^ (row & 7u)) << 4); };
+        // Starts the copy of columns [c0, c0 + 128) of this warp's rows; `row` is this thread's row of `base`, and rows at
+        // and beyond `rows` become zero.
+        auto stage_in = [&](const void* base, uint32_t row, uint32_t rows, uint32_t c0, bool wide) {
+#pragma unroll 4
+            for (uint32_t i = 0; i < 32; i += 2) {
+                const uint32_t r = i + (lane >> 4), chunk = lane & 15u;
+                const bool valid = warp * 32 + r < rows;
+                const T* src = static_cast<const T*>(base) + static_cast<uint64_t>(__shfl_sync(0xFFFFFFFFu, row, r)) * D + c0 + chunk * 8;
+                if (wide) {
+                    cp_async_16(stage_at(r, chunk), src, valid ? 16u : 0u);
+                } else {
+                    cp_async_8(stage_at(r, chunk), src, valid ? 8u : 0u);
+                    cp_async_8(stage_at(r, chunk) + 8, src + 4, valid ? 8u : 0u);
+                }
+            }
+            cp_async_commit();
+        };
+        // This thread's query row of an item into its TMEM lane (zero for rows the super-tile does not have); its first 128
+        // columns have been requested into the staging area.  Called when every Q K^T of the previous item has completed.
+        auto load_q = [&](uint32_t row, uint32_t rows) {
 #pragma unroll 1
-            for (uint32_t c = 0; c < uint32_t(D) / 2; c += 64) {
+            for (uint32_t c0 = 0; c0 < uint32_t(D); c0 += kStageColumns) {
+                if (c0 > 0) stage_in(p.q, row, rows, c0, true);
+                cp_async_wait<0>();
+                __syncwarp();
                 uint32_t regs[2][32];
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
-                    const uint4 value = valid ? q_row[c / 4 + j] : make_uint4(0, 0, 0, 0);
+                    const uint4 value = ld_shared_16(stage_at(lane, j));
                     regs[j / 8][4 * (j % 8)] = value.x;
                     regs[j / 8][4 * (j % 8) + 1] = value.y;
                     regs[j / 8][4 * (j % 8) + 2] = value.z;
                     regs[j / 8][4 * (j % 8) + 3] = value.w;
                 }
                 __syncwarp();
-                tmem_store32_bits(tmem + kColQ + lane_base + c, regs[0]);
-                tmem_store32_bits(tmem + kColQ + lane_base + c + 32, regs[1]);
+                tmem_store32_bits(tmem + kColQ + lane_base + c0 / 2, regs[0]);
+                tmem_store32_bits(tmem + kColQ + lane_base + c0 / 2 + 32, regs[1]);
             }
             tmem_store_wait();
             tc_fence_before();
             mbar_arrive(bar(kBarQ));
         };
 
-        if (item_begin < item_end) load_q(view_item(p, item_begin));
+        if (item_begin < item_end) {
+            const ItemView first = view_item(p, item_begin);
+            bool valid;
+            const uint32_t row = static_cast<uint32_t>(row_of(first, valid));
+            stage_in(p.q, row, first.rows, 0, true);
+            load_q(row, first.rows);
+        }
         for (uint32_t index = item_begin; index < item_end; ++index, ++item_count) {
             const ItemView v = view_item(p, index);
+            // the next item, requested here and looked at after this item's first tile
+            const DeviceItem* next_item = p.items + min(index + 1, item_end - 1);
+            const uint4 next_rows_of = reinterpret_cast<const uint4*>(next_item)[1];   // flat_begin and num_tokens (.z, .w)
+            const uint4 next_heads_of = reinterpret_cast<const uint4*>(next_item)[2];  // head0 and num_heads (.z, .w)
             bool row_valid;
             const uint64_t out_row = row_of(v, row_valid);
             const uint32_t limit = row_valid ? item_row_limit(v, tid) : v.kv_end;
@@ -383,6 +436,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
             // softmax state in the log2 domain: `row_ref` is the reference the exponentials are taken against (it
             // trails the true running max `row_max` by at most kRescaleThreshold), `row_sum` is relative to it
             float row_ref = -INFINITY, row_max = -INFINITY, row_sum = 0.0f;
+            uint32_t next_row = 0, next_rows = 0;  // this thread's row of the next item
             for (uint32_t i = 0; i < num_tiles; ++i) {
                 const uint32_t tile = tile_base + i, buf = tile & 1;
                 const uint32_t token0 = (first_tile + i) * kUmmaN;
@@ -463,22 +517,21 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 tmem_store_wait();
                 tc_fence_before();
                 mbar_arrive(bar(kBarP + buf));
+                if (i == 0 && index + 1 < item_end) {  // the next item's query rows travel under this item's tiles
+                    next_rows = next_rows_of.w * next_heads_of.w;
+                    const uint32_t r = tid < next_rows ? tid : 0;
+                    next_row = (next_rows_of.z + r / next_heads_of.w) * p.num_q_heads + next_heads_of.z + r % next_heads_of.w;
+                    stage_in(p.q, next_row, next_rows, 0, true);
+                }
                 if (i > 0 && !rescale) wait(kBarO + ((tile - 1) & 1), (tile - 1) >> 1);
             }
             const bool is_partial = v.partial_slot != kU32Max;
-            // The output gates of this row, 32 columns at a time and one pass ahead of their use: the first ones travel
-            // under the last P V, each later pass's under the pass before it.
-            const bool gated = p.gates != nullptr && row_valid && !is_partial && p.ext_o == nullptr;
-            const uint2* gate_row = reinterpret_cast<const uint2*>(static_cast<const T*>(p.gates) + out_row * D);  // 8-byte aligned
-            uint2 gate_next[8];
-            if (gated) {
-#pragma unroll
-                for (int j = 0; j < 8; ++j) gate_next[j] = gate_row[j];
-            }
             // The next item's query rows go to TMEM under this item's last P V (S of its last tile has been read, so all
             // its Q K^T are complete), and the first Q K^T products of that item run under the epilogue (O is not
             // touched before P of that item's first tile exists).
-            if (index + 1 < item_end) load_q(view_item(p, index + 1));
+            if (index + 1 < item_end) load_q(next_row, next_rows);
+            const bool staged_out = !is_partial && p.ext_o == nullptr, gated = staged_out && p.gates != nullptr;
+            if (gated) stage_in(p.gates, static_cast<uint32_t>(out_row), v.rows, 0, wide_gates);
             if (num_tiles > 0) {
                 const uint32_t last = tile_base + num_tiles - 1;
                 wait(kBarO + (last & 1), last >> 1);
@@ -504,21 +557,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 if (row_valid) {
 #pragma unroll
                     for (int e = 0; e < 32; ++e) o[e] *= inv;
-                    if (gated) {
-                        uint2 gate_raw[8];
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) gate_raw[j] = gate_next[j];
-                        if (c + 32 < uint32_t(D)) {
-#pragma unroll
-                            for (int j = 0; j < 8; ++j) gate_next[j] = gate_row[c / 4 + 8 + j];
-                        }
-#pragma unroll
-                        for (int j = 0; j < 8; ++j) {
-                            const T* gate = reinterpret_cast<const T*>(&gate_raw[j]);
-#pragma unroll
-                            for (int e = 0; e < 4; ++e) o[4 * j + e] *= gate_sigmoid_approx(static_cast<float>(gate[e]));
-                        }
-                    }
                     if (is_partial) {
                         // a partial slot of this kernel is stored column-major in float4 units, [D / 4][16 rows]: the
                         // 16 rows of a tile are 16 consecutive lanes here, so every store instruction writes whole
@@ -533,12 +571,46 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
 #pragma unroll
                         for (int e = 0; e < 32; e += 4)
                             *reinterpret_cast<float4*>(dst + e) = make_float4(o[e], o[e + 1], o[e + 2], o[e + 3]);
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 32; e += 8) store_plain8<T>(p.out, out_row * D + c + e, o + e, wide_out);
                     }
                 }
-                __syncwarp();  // the TMEM load of the next pass is warp-collective
+                if (staged_out) {
+                    const uint32_t in_stage = c % kStageColumns;
+                    if (gated && in_stage == 0) {
+                        if (c > 0) stage_in(p.gates, static_cast<uint32_t>(out_row), v.rows, c, wide_gates);
+                        cp_async_wait<0>();
+                        __syncwarp();
+                    }
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const uint32_t at = stage_at(lane, in_stage / 8 + j);
+                        if (gated) {
+                            const uint4 raw = ld_shared_16(at);
+                            const T* gate = reinterpret_cast<const T*>(&raw);
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) o[8 * j + e] *= gate_sigmoid_approx(static_cast<float>(gate[e]));
+                        }
+                        const float* x = o + 8 * j;
+                        st_shared_16(at, make_uint4(Mma<T>::pack(x[0], x[1]), Mma<T>::pack(x[2], x[3]), Mma<T>::pack(x[4], x[5]), Mma<T>::pack(x[6], x[7])));
+                    }
+                    if (in_stage + 32 == kStageColumns) {  // the staged columns go out, two rows per access
+                        __syncwarp();
+#pragma unroll 4
+                        for (uint32_t i = 0; i < 32; i += 2) {
+                            const uint32_t r = i + (lane >> 4), chunk = lane & 15u;
+                            const uint32_t row = __shfl_sync(0xFFFFFFFFu, static_cast<uint32_t>(out_row), r);
+                            const uint4 value = ld_shared_16(stage_at(r, chunk));
+                            T* dst = static_cast<T*>(p.out) + static_cast<uint64_t>(row) * D + (c + 32 - kStageColumns) + chunk * 8;
+                            if (warp * 32 + r >= v.rows) continue;
+                            if (wide_out) {
+                                *reinterpret_cast<uint4*>(dst) = value;
+                            } else {
+                                reinterpret_cast<uint2*>(dst)[0] = make_uint2(value.x, value.y);
+                                reinterpret_cast<uint2*>(dst)[1] = make_uint2(value.z, value.w);
+                            }
+                        }
+                    }
+                }
+                __syncwarp();  // the TMEM load of the next pass is warp-collective; the staging area is free again
             }
             if (row_valid) {
                 if (is_partial) {
@@ -649,7 +721,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
 
 template <typename T, int D>
 cudaError_t launch_one(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
-    constexpr uint32_t kSmem = Ring<D>::kSlots * (D * 2 * kUmmaN) + 1024;
+    constexpr uint32_t kSmem = Ring<D>::kSlots * (D * 2 * kUmmaN) + kRowThreads * kUmmaStageColumns * 2 + 1024;
     const uint32_t box_rows = p.geo.tokens_per_page < kUmmaN ? p.geo.tokens_per_page : kUmmaN;
     CUtensorMap map;
     if (!make_kv_map(p, box_rows, &map)) return cudaErrorNotSupported;

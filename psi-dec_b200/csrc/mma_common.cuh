@@ -121,20 +121,6 @@ __device__ __forceinline__ void store_out4(const AttendParams& p, uint64_t index
     Mma<T>::store4(static_cast<T*>(p.out) + index, v);
 }
 
-// Eight consecutive outputs, already gated, as one 16-byte store (two of 8 bytes where `out` is aligned to no more).
-template <typename T>
-__device__ __forceinline__ void store_plain8(void* out, uint64_t index, const float* v, bool wide) {
-    const uint4 packed = make_uint4(Mma<T>::pack(v[0], v[1]), Mma<T>::pack(v[2], v[3]), Mma<T>::pack(v[4], v[5]),
-                                    Mma<T>::pack(v[6], v[7]));
-    T* dst = static_cast<T*>(out) + index;
-    if (wide) {
-        *reinterpret_cast<uint4*>(dst) = packed;
-    } else {
-        reinterpret_cast<uint2*>(dst)[0] = make_uint2(packed.x, packed.y);
-        reinterpret_cast<uint2*>(dst)[1] = make_uint2(packed.z, packed.w);
-    }
-}
-
 template <typename T>
 __device__ __forceinline__ void store_out2(const AttendParams& p, uint64_t index, float a, float b) {
     if (p.gates != nullptr) {
