@@ -20,7 +20,7 @@
 // its own row (32 lines an access), hence the staging areas and, paying for them, six ring slots instead of seven at
 // head_dim 256.  Prompts have many short items, so the next query rows are staged under the tiles and loaded under the
 // last P V, rows are packed (a group of six fills 126 of 128 rows, not 96), and the plan deals whole units.  Three prompts
-// of 611 to 2,500 tokens, 24/4 heads x 256, gated, two layers: 461 us a step, 501 without the staging, 2,414 at first.
+// of 611 to 2,500 tokens, 24/4 heads x 256, gated, two layers: 448 us a step, 501 without the staging, 2,414 at first.
 // All hand-offs are mbarriers (TMA byte counts, tcgen05.commit, thread arrivals); every wait is bounded and reports
 // PSI_ERR_TIMEOUT through the status word instead of hanging, and the kernel frees its TMEM on every path.  The kernel
 // reads pages only: a step that appends and attends runs the append launch first.
@@ -420,12 +420,18 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
             stage_in(p.q, row, first.rows, 0, true);
             load_q(row, first.rows);
         }
+        // flat_begin, num_tokens (.z, .w) and head0, num_heads (.z, .w) of the item behind the current one.  They are
+        // requested an item ahead and the rows staged before the tile loop: a load in flight across the loop, or the staging
+        // inside it, cost 9 % of a long run (1,247 TFLOP/s against 1,378 on 512-token chunks of long prompts).
+        uint4 next_rows_of = make_uint4(0, 0, 0, 0), next_heads_of = make_uint4(0, 0, 0, 1);
+        auto look_ahead = [&](uint32_t index) {
+            const uint4* item = reinterpret_cast<const uint4*>(p.items + min(index, item_end - 1));
+            next_rows_of = item[1];
+            next_heads_of = item[2];
+        };
+        if (item_begin < item_end) look_ahead(item_begin + 1);
         for (uint32_t index = item_begin; index < item_end; ++index, ++item_count) {
             const ItemView v = view_item(p, index);
-            // the next item, requested here and looked at after this item's first tile
-            const DeviceItem* next_item = p.items + min(index + 1, item_end - 1);
-            const uint4 next_rows_of = reinterpret_cast<const uint4*>(next_item)[1];   // flat_begin and num_tokens (.z, .w)
-            const uint4 next_heads_of = reinterpret_cast<const uint4*>(next_item)[2];  // head0 and num_heads (.z, .w)
             bool row_valid;
             const uint64_t out_row = row_of(v, row_valid);
             const uint32_t limit = row_valid ? item_row_limit(v, tid) : v.kv_end;
@@ -437,6 +443,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
             // trails the true running max `row_max` by at most kRescaleThreshold), `row_sum` is relative to it
             float row_ref = -INFINITY, row_max = -INFINITY, row_sum = 0.0f;
             uint32_t next_row = 0, next_rows = 0;  // this thread's row of the next item
+                if (index + 1 < item_end) {  // the next item's query rows travel under this item's tiles
+                    next_rows = next_rows_of.w * next_heads_of.w;
+                    const uint32_t r = tid < next_rows ? tid : 0;
+                    next_row = (next_rows_of.z + r / next_heads_of.w) * p.num_q_heads + next_heads_of.z + r % next_heads_of.w;
+                    stage_in(p.q, next_row, next_rows, 0, true);
+                }
             for (uint32_t i = 0; i < num_tiles; ++i) {
                 const uint32_t tile = tile_base + i, buf = tile & 1;
                 const uint32_t token0 = (first_tile + i) * kUmmaN;
@@ -517,12 +529,6 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 tmem_store_wait();
                 tc_fence_before();
                 mbar_arrive(bar(kBarP + buf));
-                if (i == 0 && index + 1 < item_end) {  // the next item's query rows travel under this item's tiles
-                    next_rows = next_rows_of.w * next_heads_of.w;
-                    const uint32_t r = tid < next_rows ? tid : 0;
-                    next_row = (next_rows_of.z + r / next_heads_of.w) * p.num_q_heads + next_heads_of.z + r % next_heads_of.w;
-                    stage_in(p.q, next_row, next_rows, 0, true);
-                }
                 if (i > 0 && !rescale) wait(kBarO + ((tile - 1) & 1), (tile - 1) >> 1);
             }
             const bool is_partial = v.partial_slot != kU32Max;
@@ -539,6 +545,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 tc_fence_after();
             }
             tile_base += num_tiles;
+            look_ahead(index + 2);  // used by the next item, under whose tiles that item's query rows travel
 
             // ---- epilogue: every thread finishes its own row ---------------------------------------------------------------
             // back to the true max as the reference: l' = l * 2^(ref - max); O / l is unchanged by the shift
