@@ -129,6 +129,7 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
         AttendParams c = p;
         c.items = reinterpret_cast<const DeviceItem*>(block_words(g, off.chunk_items));
         c.cta_item_begin = block_words(g, off.chunk_cta);
+        c.chunk_weights = fixed ? kChunkWeightsByPlan : (chunk.fine ? kChunkWeightsFine : kChunkWeightsPlain);
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_CHUNK);
         cudaError_t launched = cudaErrorNotSupported;
         if (g->chunk_umma) {
@@ -155,24 +156,20 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     }
 }
 
-void split_requests(const psi_gqa* g, const RequestRuns& runs, std::vector<uint32_t>& decode_reqs,
+ChunkRule chunk_rule(const psi_gqa* g) {
+    ChunkRule rule;
+    rule.max_ctas = g->grid_cap;
+    rule.token_bytes = g->cfg.page_bytes / g->tokens_per_page;
+    rule.short_runs = g->chunk_umma;
+    return rule;
+}
+
+bool split_requests(const psi_gqa* g, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                     std::vector<uint32_t>& chunk_reqs) {
-    const uint32_t per_tile = g->geo.tokens_per_tile;
-    uint32_t min_tiles = kU32Max;
-    if (g->chunk_supported) {
-        uint64_t units = 0, longest = 0;
-        for (uint32_t r = 0; r < runs.size(); ++r) {
-            if (runs.run(r) <= per_tile) continue;
-            units += uint64_t(g->geo.num_kv_heads) * g->geo.head_tiles;
-            longest = std::max<uint64_t>(longest, runs.context(r, runs.cu_tokens[r + 1]));
-        }
-        const bool short_runs = units * kChunkMaxPieces >= g->grid_cap || longest <= kChunkWholeTokens;
-        min_tiles = short_runs ? 2u : kChunkMinTiles;
-    }
-    for (uint32_t r = 0; r < runs.size(); ++r) {
-        const uint32_t tiles = (runs.run(r) + per_tile - 1) / per_tile;
-        if (tiles > 0) (tiles >= min_tiles ? chunk_reqs : decode_reqs).push_back(r);
-    }
+    if (g->chunk_supported) return split_runs(g->geo, runs, rule, decode_reqs, chunk_reqs);
+    for (uint32_t r = 0; r < runs.size(); ++r)
+        if (runs.run(r) > 0) decode_reqs.push_back(r);
+    return false;
 }
 
 void run_append(psi_gqa* g, psi_pages* pages, psi_table* table, uint32_t layer, const void* k, const void* v) {
@@ -228,21 +225,13 @@ void run_staged_host_step(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
 // for eight query tiles at a time); the rest are decode rows.
 static void plan_runs(const psi_gqa* g, const RequestRuns& runs, WorkPlan& plan, ChunkPlan& chunk) {
     std::vector<uint32_t> decode_reqs, chunk_reqs;
-    split_requests(g, runs, decode_reqs, chunk_reqs);
+    const ChunkRule rule = chunk_rule(g);
+    const bool fine = split_requests(g, runs, rule, decode_reqs, chunk_reqs);
     const uint32_t min_tiles = g->kernel == PSI_KERNEL_MMA ? 16u : 4u;
     plan = build_balanced_plan(g->geo, runs, decode_reqs, g->grid_cap, min_tiles, g->item_start_cost);
-    // K/V the long runs touch: below a third of the L2 the order of the work cannot cost HBM traffic, and balance beats
-    // stream order; so does it where every long run fits one super-tile and nothing is read twice in whatever order
-    uint64_t chunk_kv_bytes = 0;
-    bool one_pass = true;
-    for (uint32_t r : chunk_reqs) {
-        one_pass = one_pass && runs.run(r) * g->geo.heads_per_tile <= kMaxRows * kChunkTilesPerItem;
-        chunk_kv_bytes += uint64_t(runs.context(r, runs.cu_tokens[r + 1])) * (uint64_t(g->cfg.page_bytes) / g->tokens_per_page);
-    }
-    const ChunkOrder order = chunk_kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident
-                                                             : (one_pass ? ChunkOrder::kEqualShares : ChunkOrder::kStream);
-    chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots,
-                             static_cast<uint32_t>(plan.reduces.size()), order, kChunkUnitCostTiles);
+    chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots, static_cast<uint32_t>(plan.reduces.size()),
+                             chunk_order(g->geo, runs, chunk_reqs, rule.token_bytes), kChunkUnitCostTiles);
+    chunk.fine = fine;
 }
 
 // Places the arrays of one plan behind `cursor` words of the block.
@@ -271,6 +260,7 @@ static void pack_plan(uint32_t* s, const PlanOffsets& off, const WorkPlan& plan,
     s[off.scalars + kScalarNumCtas] = plan.num_ctas();
     s[off.scalars + kScalarNumReduces] = static_cast<uint32_t>(plan.reduces.size());
     s[off.scalars + kScalarNumChunkCtas] = chunk.num_ctas();
+    s[off.scalars + kScalarFineChunks] = chunk.fine ? 1u : 0u;
     std::copy(plan.cta_item_begin.begin(), plan.cta_item_begin.end(), s + off.cta);
     if (!plan.reduces.empty()) std::memcpy(s + off.reduces, plan.reduces.data(), plan.reduces.size() * sizeof(ReduceUnit));
     if (!items.empty()) std::memcpy(s + off.items, items.data(), items.size() * sizeof(DeviceItem));

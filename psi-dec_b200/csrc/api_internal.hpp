@@ -278,13 +278,6 @@ void validate_layout(const psi_page_table_layout& l);
 PageGeometry page_geometry(const psi_gqa* g, const psi_pages* pages, const psi_table* table, uint32_t layer);
 const uint32_t* block_words(const psi_gqa* g, uint64_t offset);
 
-// Requests whose query run spans at least this many query tiles always go to the chunk kernels, which read a request's
-// K/V once for all of its query rows; the decode kernel reads it once per query tile.
-constexpr uint32_t kChunkMinTiles = 5;
-// Runs of two tiles and more go there as well when their units (request, KV head) are enough to give every unit of a full
-// grid at most kChunkMaxPieces pieces, or short enough not to be cut at all: a cut unit is merged by one CTA, which costs
-// about a microsecond a piece.  Eight tokens per request, 24/4 heads x 256, two layers: 64 requests of 1,500 to 3,000
-// tokens 252 us against 695 on the decode kernel, 8 of up to 30,000 290 against 813, 1 of 3,000 123 against 59.
 // psi_gqa_step_host: from this many bytes of q + k + v the attention launch reads pinned host buffers in place.
 constexpr uint64_t kDirectHostBytes = 1ull << 20;
 // psi_gqa_step_host: from this many bytes of q + k + v in pinned buffers a step with long query runs is cut into groups
@@ -295,9 +288,10 @@ constexpr uint32_t kPipelineMaxGroups = 8;
 
 AttendParams attend_params(psi_gqa* g, const psi_pages* pages, const psi_table* table, uint32_t layer, const void* q);
 void run_attend(psi_gqa* g, const AttendParams& params);
-// Deals a step's requests to the decode kernel and the chunk kernels.
-void split_requests(const psi_gqa* g, const RequestRuns& runs, std::vector<uint32_t>& decode_reqs,
+// Deals a step's requests to the decode kernel and the chunk kernels (split_runs).
+bool split_requests(const psi_gqa* g, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                     std::vector<uint32_t>& chunk_reqs);
+ChunkRule chunk_rule(const psi_gqa* g);
 void run_append(psi_gqa* g, psi_pages* pages, psi_table* table, uint32_t layer, const void* k, const void* v);
 // Device-side address of a pinned, device-mapped host buffer (16-byte aligned), or nullptr for any other memory.
 void* mapped_device_pointer(const void* host);

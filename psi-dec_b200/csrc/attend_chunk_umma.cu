@@ -142,6 +142,16 @@ struct Ring {
     static constexpr uint32_t kSlots = D == 256 ? 6u : 12u;
 };
 constexpr float kRescaleThreshold = 8.0f;
+// Launches over short query runs and rows at one position (kFine) carry the weights as two 16-bit parts, each with a P V of
+// its own, over the two halves of the S buffer: the decode kernel, the other one that takes these rows, keeps a maximum per
+// warp and rounds less than one part would.  Against 64 bits, seven draft rows a request over a history of 512 to 12,288
+// tokens, 40/8 heads x 128: 1.6e-3 with one part, 1.3e-3 on the decode kernel, 8e-6 with two.  The high part is rounded down
+// and the low part holds the rest plus 2^-10 of the weight, so that both are positive wherever the weight is (an infinity in
+// V stays one instead of meeting 0 x Inf); every weight is then 1 + 2^-10 times itself, which the end of the item divides out.
+// Costs 5 to 12 % of such a step (16 requests of 512 to 16,384 tokens, eight rows each, 40/8 heads x 128, two layers: 164 us
+// with one part, 184 with two, 275 on the decode kernel).  Long runs keep one part, in code of their own: a branch on the
+// kind inside the MMA warp's loop alone cost them 3 %.
+constexpr float kFineScale = 1.0009765625f;
 static_assert(offsetof(DeviceItem, flat_begin) == 24 && offsetof(DeviceItem, num_tokens) == 28 && offsetof(DeviceItem, head0) == 40 &&
                   offsetof(DeviceItem, num_heads) == 44,
               "the row threads read these fields of the next item as the ends of two 16-byte words");
@@ -160,9 +170,21 @@ __device__ __forceinline__ void st_shared_16(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kUmmaThreads, 1)
-    attend_chunk_umma_kernel(const AttendParams p, const __grid_constant__ CUtensorMap kv_map, const uint32_t box_rows) {
+// What the rounding down of two weights left (see kFineScale).
+template <typename T>
+__device__ __forceinline__ uint32_t low_part(float a, float b, uint32_t high) {
+    const float2 h = Mma<T>::unpack(high);
+    return Mma<T>::pack(fmaf(a, kFineScale, -h.x), fmaf(b, kFineScale, -h.y));
+}
+
+struct UmmaShared {
+    uint64_t bars[2 * 12 + 7];
+    uint32_t tmem_base, abort, last[8];
+};
+
+template <typename T, int D, bool kFine>
+__device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const CUtensorMap& kv_map, const uint32_t box_rows,
+                                                  const bool early, UmmaShared& shared) {
     constexpr uint32_t kChunks = D / 8;               // 16-byte chunks per row of K / V
     constexpr uint32_t kBlocks = D / 64;              // 64-element (128-byte) blocks per row
     constexpr uint32_t kTileBytes = D * 2 * kUmmaN;   // one K or V tile: [D/64][64][64]
@@ -177,22 +199,18 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
     constexpr uint32_t kBarFull = 0, kBarEmpty = kSlots, kBarS = 2 * kSlots, kBarO = kBarS + 2, kBarP = kBarO + 2,
                        kBarQ = kBarP + 2, kNumBarriers = kBarQ + 1;
 
-    const uint32_t cta = blockIdx.x;
-    const bool early = p.plan_ready != 0;  // the set-up below runs before the wait for the inputs
-    if (!early) await_previous_kernel();
-    if (cta >= p.scalars[kScalarNumChunkCtas]) {
-        if (early) await_previous_kernel();
-        return;
-    }
+    static_assert(kNumBarriers <= sizeof(UmmaShared::bars) / sizeof(uint64_t), "every barrier has a word");
 
+    const uint32_t cta = blockIdx.x;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    __shared__ __align__(8) uint64_t bars[kNumBarriers];
-    __shared__ uint32_t tmem_base_s, abort_s, last_s[8];
+    uint32_t& tmem_base_s = shared.tmem_base;
+    uint32_t& abort_s = shared.abort;
+    uint32_t (&last_s)[8] = shared.last;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     // the swizzled operand layouts repeat every 1024 bytes: place them on that boundary whatever the toolchain did
     const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-    const uint32_t bar0 = smem_u32(bars);
+    const uint32_t bar0 = smem_u32(shared.bars);
     auto bar = [&](uint32_t which) { return bar0 + which * 8; };
 
     if (warp == 0) {
@@ -345,6 +363,11 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                     for (uint32_t ks = 0; ks < kUmmaN / 16; ++ks)
                         umma_issue_ts(tmem + kColO, p_tmem + ks * 8, v_desc + ks * 2 * (kBlocks * 1024) / 16, idesc_pv,
                                       (i > 0 || ks > 0) ? 1u : 0u);
+                    if constexpr (kFine) {  // the low parts of P, over the second half of the S buffer
+#pragma unroll
+                        for (uint32_t ks = 0; ks < kUmmaN / 16; ++ks)
+                            umma_issue_ts(tmem + kColO, p_tmem + kUmmaN / 2 + ks * 8, v_desc + ks * 2 * (kBlocks * 1024) / 16, idesc_pv, 1u);
+                    }
                     umma_commit(bar(kBarO + (tile & 1)));
                     umma_commit(bar(kBarEmpty + slot));
                 }
@@ -493,6 +516,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 const float base = row_ref == -INFINITY ? 0.0f : row_ref;
                 float sum4[4] = {0.f, 0.f, 0.f, 0.f};
                 uint32_t packed[kUmmaN / 2];
+                [[maybe_unused]] uint32_t low[kUmmaN / 2];
 #pragma unroll
                 for (int c = 0; c < int(kUmmaN); c += 4) {
                     const float e0 = fast_exp2(fmaf(s[c], p.scale_log2, -base));
@@ -503,8 +527,15 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                     sum4[1] += e1;
                     sum4[2] += e2;
                     sum4[3] += e3;
-                    packed[c / 2] = Mma<T>::pack(e0, e1);
-                    packed[c / 2 + 1] = Mma<T>::pack(e2, e3);
+                    if constexpr (kFine) {
+                        packed[c / 2] = Mma<T>::pack_down(e0, e1);
+                        packed[c / 2 + 1] = Mma<T>::pack_down(e2, e3);
+                        low[c / 2] = low_part<T>(e0, e1, packed[c / 2]);
+                        low[c / 2 + 1] = low_part<T>(e2, e3, packed[c / 2 + 1]);
+                    } else {
+                        packed[c / 2] = Mma<T>::pack(e0, e1);
+                        packed[c / 2 + 1] = Mma<T>::pack(e2, e3);
+                    }
                 }
                 row_sum = row_sum * corr + ((sum4[0] + sum4[1]) + (sum4[2] + sum4[3]));
 
@@ -526,6 +557,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
                 }
                 __syncwarp();
                 tmem_store32_bits(tmem_s, packed);  // P over the first 32 columns of this S buffer
+                if constexpr (kFine) tmem_store32_bits(tmem_s + kUmmaN / 2, low);  // and its low part over the other 32
                 tmem_store_wait();
                 tc_fence_before();
                 mbar_arrive(bar(kBarP + buf));
@@ -549,7 +581,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
 
             // ---- epilogue: every thread finishes its own row ---------------------------------------------------------------
             // back to the true max as the reference: l' = l * 2^(ref - max); O / l is unchanged by the shift
-            const float inv = row_sum > 0.0f ? 1.0f / row_sum : 0.0f;
+            const float inv = row_sum > 0.0f ? 1.0f / (kFine ? row_sum * kFineScale : row_sum) : 0.0f;
             const float sum_at_max = row_max == -INFINITY ? row_sum : row_sum * fast_exp2(row_ref - row_max);
             const uint64_t prow = is_partial ? static_cast<uint64_t>(v.partial_slot + w) * kMaxRows + rr : 0;
 #pragma unroll 1
@@ -726,24 +758,52 @@ __global__ void __launch_bounds__(kUmmaThreads, 1)
     }
 }
 
-template <typename T, int D>
+// kWeights: one of ChunkWeights.
+template <typename T, int D, uint32_t kWeights>
+__global__ void __launch_bounds__(kUmmaThreads, 1)
+    attend_chunk_umma_kernel(const AttendParams p, const __grid_constant__ CUtensorMap kv_map, const uint32_t box_rows) {
+    __shared__ UmmaShared shared;
+    const bool early = p.plan_ready != 0;  // the set-up runs before the wait for the inputs
+    if (!early) await_previous_kernel();
+    if (blockIdx.x >= p.scalars[kScalarNumChunkCtas]) {
+        if (early) await_previous_kernel();
+        return;
+    }
+    if constexpr (kWeights == kChunkWeightsByPlan) {
+        if (p.scalars[kScalarFineChunks] != 0) attend_chunk_umma<T, D, true>(p, kv_map, box_rows, early, shared);
+        else attend_chunk_umma<T, D, false>(p, kv_map, box_rows, early, shared);
+    } else {
+        attend_chunk_umma<T, D, kWeights == kChunkWeightsFine>(p, kv_map, box_rows, early, shared);
+    }
+}
+
+template <typename T, int D, uint32_t kWeights>
 cudaError_t launch_one(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     constexpr uint32_t kSmem = Ring<D>::kSlots * (D * 2 * kUmmaN) + kRowThreads * kUmmaStageColumns * 2 + 1024;
     const uint32_t box_rows = p.geo.tokens_per_page < kUmmaN ? p.geo.tokens_per_page : kUmmaN;
     CUtensorMap map;
     if (!make_kv_map(p, box_rows, &map)) return cudaErrorNotSupported;
-    auto kernel = attend_chunk_umma_kernel<T, D>;
+    auto kernel = attend_chunk_umma_kernel<T, D, kWeights>;
     static std::atomic<uint64_t> configured{0};  // per instantiation, one bit per device
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(kSmem), configured);
     if (err != cudaSuccess) return err;
     return launch_overlapped(kernel, num_ctas, kUmmaThreads, kSmem, stream, p, map, box_rows);
 }
 
+template <typename T, int D>
+cudaError_t launch_for_weights(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
+    switch (p.chunk_weights) {
+        case kChunkWeightsPlain: return launch_one<T, D, kChunkWeightsPlain>(p, num_ctas, stream);
+        case kChunkWeightsFine: return launch_one<T, D, kChunkWeightsFine>(p, num_ctas, stream);
+        default: return launch_one<T, D, kChunkWeightsByPlan>(p, num_ctas, stream);
+    }
+}
+
 template <typename T>
 cudaError_t launch_for_dim(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     switch (p.geo.head_dim) {
-        case 128: return launch_one<T, 128>(p, num_ctas, stream);
-        case 256: return launch_one<T, 256>(p, num_ctas, stream);
+        case 128: return launch_for_weights<T, 128>(p, num_ctas, stream);
+        case 256: return launch_for_weights<T, 256>(p, num_ctas, stream);
         default: return cudaErrorInvalidValue;
     }
 }

@@ -30,22 +30,15 @@ struct AnySmem {
     static constexpr uint32_t kTotal = kRingOffset + (kRingBytes > kMergeBytes ? kRingBytes : kMergeBytes);
 };
 
-template <typename T>
-__device__ __forceinline__ float2 unpack2(uint32_t v);
-template <>
-__device__ __forceinline__ float2 unpack2<__nv_bfloat16>(uint32_t v) { return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v)); }
-template <>
-__device__ __forceinline__ float2 unpack2<__half>(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
-
 // Two f32 weights as three packed 16-bit parts, each the rounded rest of the ones before it.
 template <typename T>
 __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
     hi = Mma<T>::pack(a, b);
-    const float2 h = unpack2<T>(hi);
+    const float2 h = Mma<T>::unpack(hi);
     a -= h.x;
     b -= h.y;
     mid = Mma<T>::pack(a, b);
-    const float2 m = unpack2<T>(mid);
+    const float2 m = Mma<T>::unpack(mid);
     lo = Mma<T>::pack(a - m.x, b - m.y);
 }
 

@@ -443,6 +443,58 @@ WorkPlan build_reference_plan(const PlanGeometry& geo, const ReferenceMetadata& 
     return plan;
 }
 
+namespace {
+
+// Query rows of one chunk item are packed (token, head) pairs: as many whole tokens as its rows hold.
+uint32_t tokens_per_chunk_item(const PlanGeometry& geo) { return kMaxRows * kChunkTilesPerItem / geo.heads_per_tile; }
+
+// Whole units, longest first, where none is long against a CTA's share or worth a cut.
+bool whole_units(uint64_t longest, uint64_t fair_share) {
+    return longest <= std::max<uint64_t>(fair_share / 2, kChunkWholeTokens / kKvTile);
+}
+
+}  // namespace
+
+ChunkOrder chunk_order(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint64_t token_bytes) {
+    // K/V the runs touch: below a third of the L2 the order of the work cannot cost HBM traffic, and balance beats stream
+    // order; so does it where every run fits one super-tile and nothing is read twice in whatever order
+    uint64_t kv_bytes = 0;
+    bool one_pass = true;
+    for (uint32_t r : requests) {
+        one_pass = one_pass && runs.run(r) * geo.heads_per_tile <= kMaxRows * kChunkTilesPerItem;
+        kv_bytes += uint64_t(runs.context(r, runs.cu_tokens[r + 1])) * token_bytes;
+    }
+    return kv_bytes <= (40ull << 20) ? ChunkOrder::kL2Resident : (one_pass ? ChunkOrder::kEqualShares : ChunkOrder::kStream);
+}
+
+bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
+                std::vector<uint32_t>& chunk_reqs) {
+    const uint64_t heads = uint64_t(geo.num_kv_heads) * geo.head_tiles;
+    auto tiles_of = [&](uint32_t r) { return static_cast<uint32_t>(div_ceil(runs.run(r), geo.tokens_per_tile)); };
+    bool any_long = false;
+    uint64_t units = 0, longest = 0;  // of the runs of several tiles
+    for (uint32_t r = 0; r < runs.size(); ++r) {
+        const uint64_t tiles = tiles_of(r);
+        any_long = any_long || (tiles >= kChunkMinTiles && !runs.one_position[r]);
+        if (tiles < 2) continue;
+        const uint64_t keys = div_ceil(runs.context(r, runs.cu_tokens[r + 1]), kKvTile);
+        const uint64_t passes = div_ceil(runs.run(r), tokens_per_chunk_item(geo));
+        units += passes * heads;
+        longest = std::max(longest, keys);
+    }
+    bool take = false;
+    if (rule.short_runs && !any_long && units > 0) {
+        take = units * kChunkMaxPieces >= rule.max_ctas || longest * kKvTile <= kChunkWholeTokens;
+    }
+    for (uint32_t r = 0; r < runs.size(); ++r) {
+        const uint32_t tiles = tiles_of(r);
+        if (tiles == 0) continue;
+        const bool chunk = take ? tiles >= 2 : (tiles >= kChunkMinTiles && !runs.one_position[r]);
+        (chunk ? chunk_reqs : decode_reqs).push_back(r);
+    }
+    return take;
+}
+
 ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint32_t max_ctas,
                            uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost) {
     ChunkPlan plan;
@@ -452,8 +504,7 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, con
         uint32_t req, flat_begin, flat_end, ctx_end, head;
     };
     std::vector<Unit> units;
-    // the rows of an item are packed (token, head) pairs: as many whole tokens as its 128 rows hold
-    const uint32_t tokens_per_item = kMaxRows * kChunkTilesPerItem / geo.heads_per_tile;
+    const uint32_t tokens_per_item = tokens_per_chunk_item(geo);
     const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
     uint64_t total = 0, longest = 0;
     // longest requests first: the work dealt last, which decides how far the last CTA trails, is the cheapest
@@ -511,7 +562,7 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, con
     };
     const bool l2_resident = order == ChunkOrder::kL2Resident;
     const uint64_t fair_share = (total + uint64_t(unit_start_cost) * units.size()) / num_ctas;
-    if (l2_resident && longest <= std::max<uint64_t>(fair_share / 2, kChunkWholeTokens / kKvTile)) {
+    if (l2_resident && whole_units(longest, fair_share)) {
         // Whole units, longest first, each to the CTA with the least work so far.  Nothing is cut: a cut saves half a
         // unit's tiles on one CTA and costs two partial writes, a fence and a merge, about kChunkMinPieceTiles of them,
         // so it pays only for units of more than twice that which are also long against a CTA's share.

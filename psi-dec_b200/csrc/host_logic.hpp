@@ -190,9 +190,13 @@ struct ChunkPlan {
     uint32_t num_partial_slots = 0;   // slots used beyond slot_base
     uint32_t num_counters = 0;        // counters used beyond counter_base
     uint64_t total_kv_tiles = 0;
+    bool fine = false;                // short runs: the kernel holds the softmax weights in two parts
     uint32_t num_ctas() const { return cta_item_begin.empty() ? 0u : static_cast<uint32_t>(cta_item_begin.size() - 1); }
 };
 constexpr uint32_t kChunkTilesPerItem = 8;  // one query tile per warp
+// Requests whose query run spans at least this many query tiles always go to the chunk kernels, which read a request's
+// K/V once for all of its query rows; the decode kernel reads it once per query tile.
+constexpr uint32_t kChunkMinTiles = 5;
 constexpr uint32_t kChunkMinPieceTiles = 64;   // a KV piece of a cut unit is at least this many 16-token tiles
 constexpr uint32_t kChunkMaxPieces = 16;      // equal shares: a unit is cut into about this many pieces at most
 constexpr uint32_t kChunkWholeTokens = 2 * kChunkMinPieceTiles * 16;  // units of at most this many keys are not worth a cut
@@ -206,6 +210,21 @@ enum class ChunkOrder {
     kL2Resident    // any order will do, the K/V stays in L2: whole units, longest first, where no unit is long against a
                    // CTA's share; else equal shares
 };
+
+// What decides between the decode kernel and the chunk kernels.
+struct ChunkRule {
+    uint32_t max_ctas = 1;
+    uint64_t token_bytes = 0;   // K and V of one token in one layer
+    bool short_runs = false;    // the tcgen05 kernel runs: it may take short runs as well
+};
+// Deals a step's requests.  Runs of kChunkMinTiles query tiles always go to the chunk kernels.  In a step without any, the
+// runs of two tiles and more (and rows at one position) go there together, with weights in two parts (the result: true),
+// when their units (request, KV head) are enough to give every unit of a full grid at most kChunkMaxPieces pieces, or short
+// enough not to be cut at all: a cut unit is merged by one CTA, which costs about a microsecond a piece.
+bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
+                std::vector<uint32_t>& chunk_reqs);
+// The order for the requests `split_runs` left to the chunk kernels.
+ChunkOrder chunk_order(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint64_t token_bytes);
 
 // Outside stream order a unit counts as its KV tiles plus `unit_start_cost`.
 ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint32_t max_ctas,

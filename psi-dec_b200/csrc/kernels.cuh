@@ -15,6 +15,7 @@ enum ScalarSlot : uint32_t {
     kScalarNumCtas = 1,
     kScalarNumReduces = 2,
     kScalarNumChunkCtas = 3,
+    kScalarFineChunks = 4,        // the chunk plan's items want their weights in two parts (tcgen05 kernel)
     kScalarCount = 8
 };
 
@@ -98,6 +99,10 @@ struct ExchangeParams {
     uint32_t num_rows;            // query tokens * q heads
 };
 
+// How the tcgen05 kernel holds its softmax weights for P V: in one 16-bit part, in two, or as the plan says (launches that
+// are captured before the plan is known).
+enum ChunkWeights : uint32_t { kChunkWeightsPlain = 0, kChunkWeightsFine = 1, kChunkWeightsByPlan = 2 };
+
 enum SyncWord : uint32_t { kSyncLaunchArrivals = 0, kSyncMergeArrivals = 1, kSyncVerdict = 2, kSyncWordCount = 4 };
 
 struct AttendParams {
@@ -125,6 +130,7 @@ struct AttendParams {
     uint32_t* status;             // nullptr, or the word a bounded device-side wait writes PSI_ERR_TIMEOUT to
     uint32_t plan_ready;          // the plan was in place before the stream's previous kernel started (no kernel copies it)
     uint32_t tensor_cores;        // generic launches: 16-bit profiles may take attend_mma_any (not PSI_KERNEL_GENERIC)
+    uint32_t chunk_weights;       // ChunkWeights of a long-run launch (tcgen05 kernel)
     uint32_t tma_feed;            // decode kernel: whole K/V tiles by TMA boxes instead of cp.async (PSI_KERNEL_MMA_TMA)
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none
 };

@@ -28,6 +28,11 @@ struct Mma<__nv_bfloat16> {
         __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
         return *reinterpret_cast<uint32_t*>(&v);
     }
+    // the same towards zero
+    __device__ static __forceinline__ uint32_t pack_down(float lo, float hi) {
+        return __byte_perm(__float_as_uint(lo), __float_as_uint(hi), 0x7632);
+    }
+    __device__ static __forceinline__ float2 unpack(uint32_t v) { return make_float2(__uint_as_float(v << 16), __uint_as_float(v & 0xFFFF0000u)); }
     __device__ static __forceinline__ void store4(void* dst, float4 v) {
         uint2 packed = make_uint2(pack(v.x, v.y), pack(v.z, v.w));
         *reinterpret_cast<uint2*>(dst) = packed;
@@ -46,6 +51,13 @@ struct Mma<__half> {
         __half2 v = __floats2half2_rn(lo, hi);
         return *reinterpret_cast<uint32_t*>(&v);
     }
+    // the same towards zero
+    __device__ static __forceinline__ uint32_t pack_down(float lo, float hi) {
+        uint32_t v;
+        asm("cvt.rz.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+        return v;
+    }
+    __device__ static __forceinline__ float2 unpack(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
     __device__ static __forceinline__ void store4(void* dst, float4 v) {
         uint2 packed = make_uint2(pack(v.x, v.y), pack(v.z, v.w));
         *reinterpret_cast<uint2*>(dst) = packed;
