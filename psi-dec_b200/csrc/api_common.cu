@@ -156,11 +156,13 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     }
 }
 
-ChunkRule chunk_rule(const psi_gqa* g) {
+ChunkRule chunk_rule(const psi_gqa* g, uint64_t handicap) {
     ChunkRule rule;
     rule.max_ctas = g->grid_cap;
+    rule.head_dim = g->cfg.head_dim;
     rule.token_bytes = g->cfg.page_bytes / g->tokens_per_page;
     rule.short_runs = g->chunk_umma;
+    rule.handicap = handicap;
     return rule;
 }
 
@@ -223,9 +225,9 @@ void run_staged_host_step(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
 
 // This library's plan of a step: requests with a long run of query tokens go to the chunk kernel (one pass over their KV
 // for eight query tiles at a time); the rest are decode rows.
-static void plan_runs(const psi_gqa* g, const RequestRuns& runs, WorkPlan& plan, ChunkPlan& chunk) {
+static void plan_runs(const psi_gqa* g, const RequestRuns& runs, uint64_t handicap, WorkPlan& plan, ChunkPlan& chunk) {
     std::vector<uint32_t> decode_reqs, chunk_reqs;
-    const ChunkRule rule = chunk_rule(g);
+    const ChunkRule rule = chunk_rule(g, handicap);
     const bool fine = split_requests(g, runs, rule, decode_reqs, chunk_reqs);
     const uint32_t min_tiles = g->kernel == PSI_KERNEL_MMA ? 16u : 4u;
     plan = build_balanced_plan(g->geo, runs, decode_reqs, g->grid_cap, min_tiles, g->item_start_cost);
@@ -334,9 +336,9 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             const RequestRuns runs = plain_runs(req_slots, token_indices, cu_tokens, num_reqs);
             RequestRuns merged;
             const bool can_merge = merge_one_position_runs(runs, merged);
-            plan_runs(g, can_merge && g->replay_reserved ? merged : runs, g->plan, g->chunk);
+            plan_runs(g, can_merge && g->replay_reserved ? merged : runs, 0, g->plan, g->chunk);
             g->has_merged = can_merge && !g->replay_reserved;
-            if (g->has_merged) plan_runs(g, merged, g->merged_plan, g->merged_chunk);
+            if (g->has_merged) plan_runs(g, merged, 0, g->merged_plan, g->merged_chunk);
         }
         const WorkPlan& plan = g->plan;
         const ChunkPlan& chunk = g->chunk;

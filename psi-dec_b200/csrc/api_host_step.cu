@@ -192,7 +192,7 @@ int32_t psi_gqa_step_host(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
         bool direct = q_bytes + 2 * kv_bytes >= kDirectHostBytes && !g->replay_reserved;
         if (direct && g->chunk_supported) {
             std::vector<uint32_t> decode_reqs, chunk_reqs;
-            split_requests(g, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), chunk_rule(g), decode_reqs, chunk_reqs);
+            split_requests(g, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), chunk_rule(g, 0), decode_reqs, chunk_reqs);
             direct = chunk_reqs.empty();
         }
         if (!direct && q_bytes + 2 * kv_bytes >= kPipelineHostBytes && num_reqs >= 2 && !g->replay_reserved &&

@@ -291,7 +291,7 @@ void run_attend(psi_gqa* g, const AttendParams& params);
 // Deals a step's requests to the decode kernel and the chunk kernels (split_runs).
 bool split_requests(const psi_gqa* g, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                     std::vector<uint32_t>& chunk_reqs);
-ChunkRule chunk_rule(const psi_gqa* g);
+ChunkRule chunk_rule(const psi_gqa* g, uint64_t handicap);
 void run_append(psi_gqa* g, psi_pages* pages, psi_table* table, uint32_t layer, const void* k, const void* v);
 // Device-side address of a pinned, device-mapped host buffer (16-byte aligned), or nullptr for any other memory.
 void* mapped_device_pointer(const void* host);

@@ -472,19 +472,35 @@ bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRul
     const uint64_t heads = uint64_t(geo.num_kv_heads) * geo.head_tiles;
     auto tiles_of = [&](uint32_t r) { return static_cast<uint32_t>(div_ceil(runs.run(r), geo.tokens_per_tile)); };
     bool any_long = false;
-    uint64_t units = 0, longest = 0;  // of the runs of several tiles
+    std::vector<uint32_t> several;                             // runs of several tiles, none of them a long one
+    uint64_t once = 0, per_tile = 0, units = 0, longest = 0;   // KV tiles of `several`: read once, read per query tile
     for (uint32_t r = 0; r < runs.size(); ++r) {
         const uint64_t tiles = tiles_of(r);
         any_long = any_long || (tiles >= kChunkMinTiles && !runs.one_position[r]);
         if (tiles < 2) continue;
         const uint64_t keys = div_ceil(runs.context(r, runs.cu_tokens[r + 1]), kKvTile);
         const uint64_t passes = div_ceil(runs.run(r), tokens_per_chunk_item(geo));
+        several.push_back(r);
+        once += keys * passes * heads;
+        per_tile += keys * tiles * heads;
         units += passes * heads;
         longest = std::max(longest, keys);
     }
     bool take = false;
     if (rule.short_runs && !any_long && units > 0) {
-        take = units * kChunkMaxPieces >= rule.max_ctas || longest * kKvTile <= kChunkWholeTokens;
+        // KV tiles a CTA works off on either kernel, and the pieces of a cut unit.  Measured with 2 to 9 rows a request, 1 to
+        // 64 requests of 100 to 30,000 tokens, 40/8, 32/8 and 4/1 heads x 128, 16/2 and 24/4 x 256, fused and after the front
+        // stage: a tile saved is worth 0.11 us at head_dim 128 and 0.2 at 256, a piece costs 1.2 us and the kernel itself 5.
+        // Of 800 such steps none is slower by more than 0.1 us than on the decode kernel, and 96 % of what taking
+        // every step at its best would gain is left.  (Four tokens on 2,000 keys, 40/8 x 128: 20 us a layer against 42;
+        // 64 requests of 1,500 to 3,000 tokens, eight rows, 24/4 x 256: 350 us against 124.)
+        const uint64_t ctas = std::max<uint64_t>(1, std::min<uint64_t>({rule.max_ctas, kChunkMaxPieces * units, once / 4}));
+        const bool whole = chunk_order(geo, runs, several, rule.token_bytes) == ChunkOrder::kL2Resident &&
+                           whole_units(longest, (once + kChunkUnitCostTiles * units) / ctas);
+        const double share = whole ? std::max<double>(longest, double(once) / rule.max_ctas) : double(once) / ctas;
+        const double pieces = whole ? 0.0 : double(ctas) / units;
+        const double saved = (double(per_tile) / rule.max_ctas - share) * (rule.head_dim / 128.0) * 0.9;
+        take = saved > 45.0 + 11.0 * pieces + double(rule.handicap);
     }
     for (uint32_t r = 0; r < runs.size(); ++r) {
         const uint32_t tiles = tiles_of(r);

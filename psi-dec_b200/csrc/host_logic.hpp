@@ -214,13 +214,15 @@ enum class ChunkOrder {
 // What decides between the decode kernel and the chunk kernels.
 struct ChunkRule {
     uint32_t max_ctas = 1;
+    uint32_t head_dim = 0;
     uint64_t token_bytes = 0;   // K and V of one token in one layer
     bool short_runs = false;    // the tcgen05 kernel runs: it may take short runs as well
+    uint64_t handicap = 0;      // what taking short runs costs beside the attention, in KV tiles per CTA at head_dim 128
 };
 // Deals a step's requests.  Runs of kChunkMinTiles query tiles always go to the chunk kernels.  In a step without any, the
 // runs of two tiles and more (and rows at one position) go there together, with weights in two parts (the result: true),
-// when their units (request, KV head) are enough to give every unit of a full grid at most kChunkMaxPieces pieces, or short
-// enough not to be cut at all: a cut unit is merged by one CTA, which costs about a microsecond a piece.
+// when that pays: the decode kernel reads a request's K/V once per query tile, the tcgen05 kernel once, but a unit
+// (request, KV head) that is cut is merged by one CTA, and one that is not occupies one CTA.
 bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                 std::vector<uint32_t>& chunk_reqs);
 // The order for the requests `split_runs` left to the chunk kernels.

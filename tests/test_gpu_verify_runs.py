@@ -9,11 +9,12 @@ import gpuharness as G
 pkg = G.pkg
 pytestmark = pytest.mark.gpu
 
-# (heads, head_dim, contexts, runs, long-run kernel expected): two tiles and more go there once their units give a full
-# grid at most sixteen pieces each, or are short
-CASES = [((40, 8), 128, [300], [4], True), ((40, 8), 128, [5000], [4], False), ((16, 2), 256, [3000] * 5, [3] * 5, True),
+# (heads, head_dim, contexts, runs, long-run kernel expected): two tiles and more go there once reading the K/V once instead
+# of once per tile saves more than cutting the units costs
+CASES = [((40, 8), 128, [300], [4], False), ((40, 8), 128, [5000], [4], False), ((16, 2), 256, [3000] * 5, [3] * 5, False),
          ((16, 2), 256, [3000] * 4, [3] * 4, False), ((24, 4), 256, [700, 9000, 64, 4000], [8, 9, 2, 43], True),
-         ((24, 4), 256, [9000] * 8, [2] * 8, False), ((18, 2), 128, [900, 40], [2, 1], True), ((12, 2), 128, [4000], [11], True)]
+         ((24, 4), 256, [9000] * 8, [2] * 8, False), ((18, 2), 128, [900, 40], [2, 1], False), ((12, 2), 128, [4000], [11], True),
+         ((40, 8), 128, [900] * 40, [4] * 40, True), ((16, 2), 256, [2500] * 24, [8, 3] * 12, True), ((24, 4), 256, [9000] * 8, [3] * 8, True)]
 
 
 @pytest.mark.parametrize("heads,head_dim,contexts,runs,long_run", CASES)
