@@ -265,7 +265,9 @@ PSI_API int32_t psi_table_read(psi_table* table, uint32_t req_slot, uint32_t lay
                                uint32_t n);
 /* reset_req_slots: zero every row of the listed slots. */
 PSI_API int32_t psi_table_reset_slots(psi_table* table, const uint32_t* req_slots, uint32_t n);
-/* page_ids_buffer */
+/* page_ids_buffer.  The caller's own kernels may fill the table through this address in the order of the context's
+ * stream; from the first call on, launches with this table read it only after all earlier work of the stream.  Take the
+ * address before a stream capture whose graphs the caller's kernels will write the table between. */
 PSI_API int32_t psi_table_device_ptr(psi_table* table, void** out);
 /* Bulk load of whole (slot, layer) rows from host memory: ids holds num_blocks*num_page_ids_per_block entries. */
 PSI_API int32_t psi_table_write_row(psi_table* table, uint32_t req_slot, uint32_t layer, const uint32_t* ids,

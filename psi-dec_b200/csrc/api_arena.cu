@@ -269,6 +269,7 @@ int32_t psi_table_reset_slots(psi_table* table, const uint32_t* req_slots, uint3
 
 int32_t psi_table_device_ptr(psi_table* table, void** out) {
     if (table == nullptr || out == nullptr) return PSI_ERR_INVALID_ARGUMENT;
+    table->exposed = true;
     *out = table->dev;
     return PSI_OK;
 }

@@ -37,6 +37,7 @@ PageGeometry page_geometry(const psi_gqa* g, const psi_pages* pages, const psi_t
     PageGeometry geo{};
     geo.pages = pages->ptr;
     geo.page_ids = table->dev;
+    geo.table_settled = table->exposed ? 0u : 1u;
     geo.elem_bytes = dtype_bytes(g->cfg.dtype);
     geo.page_elems = g->cfg.page_bytes / geo.elem_bytes;
     geo.num_pages = pages->num_pages;

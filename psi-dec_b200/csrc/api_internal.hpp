@@ -137,6 +137,7 @@ struct psi_table {
     uint32_t* dev = nullptr;
     std::vector<uint32_t> host;
     uint64_t page_bound = 0;  // 0: none declared; else every stored page ID must be below it
+    bool exposed = false;     // the device address was handed out: the caller's kernels may write the table
     void check_ids(const uint32_t* ids, uint64_t n) const {
         if (page_bound == 0) return;
         for (uint64_t i = 0; i < n; ++i) {

@@ -61,7 +61,8 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
     // The plan and the page table are read again by the next launch of the step (one launch per layer) while hundreds
     // of megabytes of K/V pass through the L2 in between: their lines are loaded to be evicted last.
     const uint64_t keep = l2_evict_last_policy();
-    const bool early = !kExchange && p.plan_ready != 0;  // plan and page table are read before the wait for the inputs
+    // plan and page table are read before the wait for the inputs
+    const bool early = !kExchange && p.plan_ready != 0 && p.geo.table_settled != 0;
     if (!early) await_previous_kernel();
     // One round trip for everything the first tile copies depend on: the CTA count, this CTA's item range and a copy
     // of its first item all go out before the first of them is needed.

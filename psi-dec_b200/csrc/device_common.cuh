@@ -11,9 +11,10 @@ namespace psi {
 // For kernels launched with launch_overlapped: returns once every earlier kernel of the stream has completed and its
 // writes are visible, then lets the next kernel's CTAs become resident.  Because a kernel lets its successor start only
 // after this point, a kernel that has started knows that the one before its predecessor has completed.  Nothing that an
-// earlier kernel writes is touched before this call; the step's plan, the page table and the front stage's weights are
-// written by copies, which order kernels around them fully, and may be read before it.  Every CTA makes the call, also
-// one without work: a kernel that completed before its predecessor would let its successor run too early.
+// earlier kernel writes is touched before this call.  What only copies write, which order kernels around them fully, may be
+// read before it: the step's plan, the front stage's weights and the page table, this one as long as its address has not
+// been handed out (PageGeometry::table_settled), since a kernel of the caller's may write it after that.  Every CTA makes
+// the call, also one without work: a kernel that completed before its predecessor would let its successor run too early.
 __device__ __forceinline__ void await_previous_kernel() {
     asm volatile("griddepcontrol.wait;\n\tgriddepcontrol.launch_dependents;" ::: "memory");
 }

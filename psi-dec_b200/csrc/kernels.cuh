@@ -32,6 +32,7 @@ struct PageGeometry {
     uint32_t head_dim;
     uint32_t elem_bytes;
     uint32_t* fault;              // nullptr, or the status word a failed bounds check writes PSI_ERR_PAGE_ID to
+    uint32_t table_settled;       // only copies write the table: it may be read before await_previous_kernel()
 };
 
 struct AppendParams {

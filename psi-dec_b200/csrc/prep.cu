@@ -223,9 +223,10 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
         w.widen(v);
         k_weight.narrow(v);
     }
-    uint32_t page_id;
-    const bool page_ok = checked_page_id(p.geo, table_row(p.geo, slot), pos / p.geo.tokens_per_page, page_id);
-    const uint64_t page_row = kv_row_offset(p.geo, page_id, 0, pos % p.geo.tokens_per_page) + d0;
+    uint32_t page_id = 0;
+    bool page_ok = false;
+    auto find_page = [&] { page_ok = checked_page_id(p.geo, table_row(p.geo, slot), pos / p.geo.tokens_per_page, page_id); };
+    if (p.geo.table_settled != 0) find_page();
     const uint32_t rope_half = p.rope_dim / 2, half_lanes = rope_half / 8;
     for (uint32_t i = tid; i < rope_half; i += kPrepWarps * 32) {
         float s, c;
@@ -233,6 +234,8 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
         turn_s[i] = make_float2(c, s);
     }
     await_previous_kernel();
+    if (p.geo.table_settled == 0) find_page();
+    const uint64_t page_row = kv_row_offset(p.geo, page_id, 0, pos % p.geo.tokens_per_page) + d0;
     Eight<DTYPE> held[kHeld];
 #pragma unroll
     for (int i = 0; i < kHeld; ++i) fetch(first + i * stride, held[i]);
