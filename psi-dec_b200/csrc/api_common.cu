@@ -98,6 +98,8 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     const ChunkPlan& chunk = merged ? g->merged_chunk : g->chunk;
     const PlanOffsets& off = merged ? g->merged_off : g->off;
     if (merged) use_plan(g, off, p);
+    // The tensor-core kernels move 16 bytes at a time; refused here, before anything of the step is launched.
+    if (g->kernel == PSI_KERNEL_MMA && !attend_mma_aligned(p)) cuda_check(cudaErrorMisalignedAddress, "attend (mma) launch");
     if (p.new_k != nullptr && (fixed || chunk.num_ctas() > 0)) {
         // A fused step that carries long query runs: their K/V tiles are fetched page-wise by TMA, so the step's rows
         // go to their pages first (one more launch, against milliseconds of attention) and both kernels read pages only.

@@ -552,13 +552,14 @@ bool attend_mma_supported(uint32_t dtype, uint32_t head_dim, uint32_t tokens_per
 
 uint32_t attend_mma_ctas_per_sm(uint32_t /*head_dim*/) { return 1; }
 
+bool attend_mma_aligned(const AttendParams& p) {
+    auto aligned = [](const void* ptr, uintptr_t to) { return (reinterpret_cast<uintptr_t>(ptr) & (to - 1)) == 0; };
+    return aligned(p.q, 16) && aligned(p.geo.pages, 16) && aligned(p.out, 8);
+}
 
 cudaError_t launch_attend_mma(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     if (num_ctas == 0) return cudaSuccess;
-    if ((reinterpret_cast<uintptr_t>(p.q) & 15u) != 0 || (reinterpret_cast<uintptr_t>(p.geo.pages) & 15u) != 0 ||
-        (p.out != nullptr && (reinterpret_cast<uintptr_t>(p.out) & 7u) != 0)) {
-        return cudaErrorMisalignedAddress;
-    }
+    if (!attend_mma_aligned(p)) return cudaErrorMisalignedAddress;
     if (p.xchg.flag != nullptr) {
         if (p.ext_o == nullptr || p.xchg.sync_words == nullptr || p.xchg.consumed == nullptr) return cudaErrorInvalidValue;
         return p.dtype == PSI_DTYPE_BF16 ? launch_for_dim<__nv_bfloat16, true>(p, num_ctas, stream)

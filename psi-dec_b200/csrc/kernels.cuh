@@ -215,6 +215,8 @@ cudaError_t launch_attend_mma_any(const AttendParams& p, uint32_t num_ctas, cuda
 bool attend_f32_supported(const AttendParams& p);
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
+// q and the arena on 16-byte boundaries, out on an 8-byte one: what the decode and the chunk kernels need.
+bool attend_mma_aligned(const AttendParams& p);
 cudaError_t launch_attend_mma(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 // Long query runs: one CTA = up to eight query tiles of one request sharing one pass over the KV range.
 bool attend_chunk_supported(uint32_t dtype, uint32_t head_dim, uint32_t tokens_per_page);

@@ -45,3 +45,42 @@ def test_partials_of_short_runs_are_as_close_as_the_decode_kernel(dtype, heads, 
 def _rows_of(s, request):
     cu = np.concatenate([[0], np.cumsum(s.spec.q_len)])
     return np.arange(cu[request], cu[request + 1])
+
+
+@pytest.mark.parametrize("engine", [pkg.KERNEL_AUTO, pkg.KERNEL_MMA_SYNC, pkg.KERNEL_MMA_TMA])
+@pytest.mark.parametrize("runs,contexts", [([1] * 3, [70, 9, 300]), ([8] * 40, [900] * 40), ([300, 1], [20, 400])])
+def test_unaligned_buffers_are_refused_before_anything_is_launched(engine, runs, contexts):
+    # host side only: no kernel sees one of these pointers
+    import torch
+    s = W.Session(W.Spec("shift", pkg.BF16, 40, 8, 128, 16, contexts, runs, seed=53), kernel_mode=engine)
+    s.append()
+    s.attend()
+    s.ctx.sync()
+    good = checks.to_numpy_bits(s.out).copy()
+
+    def shifted(elements):
+        x = torch.zeros(s.q.numel() + elements, dtype=s.tdtype, device=s.device)[elements:].view(s.q.shape)
+        x.copy_(s.q)
+        return x
+
+    o, m, l = (torch.zeros(x, device=s.device) for x in (s.q.shape, s.q.shape[:2], s.q.shape[:2]))
+    torch.cuda.synchronize()
+    for q, out in ((shifted(4), s.out), (shifted(1), s.out), (s.q, shifted(2))):
+        before = s.ctx.launch_count
+        with pytest.raises(pkg.PsiError, match="cudaErrorMisalignedAddress"):
+            s.gqa.attend(s.pages, s.table, 0, q, out)
+        with pytest.raises(pkg.PsiError, match="cudaErrorMisalignedAddress"):
+            s.gqa.append_attend(s.pages, s.table, 0, s.k, s.v, q, out)
+        if q is not s.q:
+            with pytest.raises(pkg.PsiError, match="cudaErrorMisalignedAddress"):
+                s.gqa.attend_partial(s.pages, s.table, 0, q, o, m, l)
+        assert s.ctx.launch_count == before
+    off = pkg.PageArena(s.ctx, s.spec.num_pages - 1, s.spec.page_bytes, device_ptr=s.arena.view(-1)[4:])
+    with pytest.raises(pkg.PsiError, match="cudaErrorMisalignedAddress"):
+        s.gqa.attend(off, s.table, 0, s.q, s.out)
+    off.close()
+    s.out.zero_()
+    s.attend()
+    s.ctx.sync()
+    assert np.array_equal(checks.to_numpy_bits(s.out), good)
+    s.close()
