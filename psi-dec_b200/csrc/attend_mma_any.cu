@@ -2,9 +2,11 @@
 // that are no multiple of 64 (any multiple of eight up to 256) and any page size.
 //
 // Same work items, partial slots and reduce pass as the CUDA-core kernels (attend_generic.cu), whose arithmetic it keeps:
-// the weights stay f32.  Each is split into three 16-bit parts that add up to it exactly (bf16: 3 x 8 bits), and O += P V
-// runs once per part; K, V and q are 16-bit values already and all accumulators are f32.  Bound by HBM; the tensor pipe
-// has room for the two extra products.  One CTA of eight warps per SM, every warp owning every eighth 16-token tile of the
+// the weights stay f32.  Each is split into three 16-bit parts, and O += P V runs once per part; K, V and q are 16-bit values
+// already and all accumulators are f32.  In bf16, which has f32's exponents, the parts add up to the weight exactly.  f16
+// ends at steps of 2^-24, so there the weights are taken 2^15 times as large (kWeightShift): exact down to 2^-16 of the
+// heaviest key of the warp, and within 2^-40 of it below that, where f32 sums over an item do not see it.  Bound by HBM; the
+// tensor pipe has room for the two extra products.  One CTA of eight warps per SM, every warp owning every eighth 16-token tile of the
 // item and a ring of its own (K tile, V tile, K tile, ...) fed by 16-byte cp.async, the next tile's page looked up one
 // tile ahead.  Rows are padded to DP elements plus one 16-byte chunk: an odd number of chunks per row keeps ldmatrix free
 // of bank conflicts without a swizzle, and the chunks beyond head_dim hold zeros.
@@ -41,6 +43,13 @@ __device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t&
     const float2 m = Mma<T>::unpack(mid);
     lo = Mma<T>::pack(a - m.x, b - m.y);
 }
+
+// Exponent by which the weights (at most 1, the running maximum) are raised: 2^15 is the largest power of two in f16.  The
+// row sum is of the raised weights too and is brought back when the item's warps meet; O / l does not change.
+template <typename T>
+constexpr float kWeightShift = 0.0f;
+template <>
+constexpr float kWeightShift<__half> = 15.0f;
 
 template <typename T, int DP, int NSLOT>
 __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParams p) {
@@ -197,7 +206,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
                     st.m0 = new0;
                     st.m1 = new1;
                 }
-                const float base0 = st.m0 == -INFINITY ? 0.0f : st.m0, base1 = st.m1 == -INFINITY ? 0.0f : st.m1;
+                const float base0 = (st.m0 == -INFINITY ? 0.0f : st.m0) - kWeightShift<T>, base1 = (st.m1 == -INFINITY ? 0.0f : st.m1) - kWeightShift<T>;
                 float w[2][4];
 #pragma unroll
                 for (int n = 0; n < 2; ++n)
@@ -229,6 +238,9 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
         st.l0 += __shfl_xor_sync(0xFFFFFFFFu, st.l0, 2);
         st.l1 += __shfl_xor_sync(0xFFFFFFFFu, st.l1, 1);
         st.l1 += __shfl_xor_sync(0xFFFFFFFFu, st.l1, 2);
+        constexpr float kBack = 1.0f / static_cast<float>(1u << static_cast<uint32_t>(kWeightShift<T>));
+        st.l0 *= kBack;
+        st.l1 *= kBack;
         if (quad_col == 0) {
             merge_m[warp][quad_row] = st.m0;
             merge_m[warp][quad_row + 8] = st.m1;
@@ -238,8 +250,8 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
         float* mine = merge_o + warp * kTile * L::kMergeStride + 2 * quad_col;
 #pragma unroll
         for (int j = 0; j < DP / 8; ++j) {
-            *reinterpret_cast<float2*>(mine + quad_row * L::kMergeStride + 8 * j) = make_float2(st.o[j][0], st.o[j][1]);
-            *reinterpret_cast<float2*>(mine + (quad_row + 8) * L::kMergeStride + 8 * j) = make_float2(st.o[j][2], st.o[j][3]);
+            *reinterpret_cast<float2*>(mine + quad_row * L::kMergeStride + 8 * j) = make_float2(st.o[j][0] * kBack, st.o[j][1] * kBack);
+            *reinterpret_cast<float2*>(mine + (quad_row + 8) * L::kMergeStride + 8 * j) = make_float2(st.o[j][2] * kBack, st.o[j][3] * kBack);
         }
         __syncthreads();
         const uint32_t c4_count = D / 4;

@@ -1,0 +1,49 @@
+"""The tensor-core kernel of the odd 16-bit profiles where its split weights could show: a dominant key over a long flat tail
+in f16, infinities in V, buffers on 2-byte boundaries; the f32 kernel against the staged one; the static entry point."""
+import numpy as np
+import pytest
+
+import checks
+import workloads as W
+import gpuharness as G
+from oracle import psi_oracle as O
+
+pkg = G.pkg
+pytestmark = pytest.mark.gpu
+
+
+def _partial(s):
+    import torch
+    out = [torch.zeros(x, device=s.device) for x in (s.q.shape, s.q.shape[:2], s.q.shape[:2])]
+    s.gqa.attend_partial(s.pages, s.table, 0, s.q, *out)
+    s.ctx.sync()
+    return [x.cpu().numpy().astype(np.float64) for x in out]
+
+
+@pytest.mark.parametrize("dtype", [pkg.F16, pkg.BF16])
+@pytest.mark.parametrize("head_dim", [96, 200])
+@pytest.mark.parametrize("below", [17.5, 21.0, 26.0])   # log2 of the dominant key's weight over a tail key's
+def test_a_long_tail_under_a_dominant_key_keeps_its_weights(dtype, head_dim, below):
+    # Scores are set through one element of q and K: the tail's all are 0, one key's is `below` in log2.  V is 0 for that key
+    # and about 1 for the tail, so that the partial is the tail's share, n 2^-below of the whole.
+    import torch
+    n = 6000
+    answers = {}
+    for mode in (pkg.KERNEL_AUTO, pkg.KERNEL_GENERIC):
+        s = W.Session(W.Spec("tail", dtype, 4, 2, head_dim, 12, [n], [1], seed=71), kernel_mode=mode)
+        pages = s.arena.view(s.arena.shape[0], 2, 2, 12, head_dim)
+        ids = s.spec.block_tables[0]
+        pages[:, 0] = 0
+        pages[:, 1] = (1.0 + 0.25 * torch.randn(pages[:, 1].shape, generator=torch.Generator("cuda").manual_seed(3), device="cuda")).to(s.tdtype)
+        s.q.zero_()
+        s.q[..., 0] = 8.0
+        key = 64  # in the first warp's share of the first item
+        pages[int(ids[key // 12]), 0, :, key % 12, 0] = below * np.log(2.0) / (8.0 * s.spec.scale)
+        pages[int(ids[key // 12]), 1, :, key % 12] = 0
+        o, m, l = _partial(s)
+        expected, rows = checks.oracle_attention(s)
+        answers[mode] = np.linalg.norm(o[rows] - expected) / np.linalg.norm(expected)
+        score = float(pages[int(ids[key // 12]), 0, 0, key % 12, 0]) * 8.0 * s.spec.scale
+        assert np.allclose(m, score, rtol=1e-6) and np.allclose(l, 1.0 + n * np.exp(-score), rtol=1e-5)
+        s.close()
+    assert answers[pkg.KERNEL_AUTO] <= max(2e-6, 2 * answers[pkg.KERNEL_GENERIC]), answers
