@@ -51,6 +51,23 @@ constexpr float kWeightShift = 0.0f;
 template <>
 constexpr float kWeightShift<__half> = 15.0f;
 
+// Stores those of four consecutive results that are infinite.
+template <typename T>
+__device__ __forceinline__ void write_infinities(const AttendParams& p, const ItemView& v, uint32_t r, uint32_t d, float4 value) {
+    const float x[4] = {value.x, value.y, value.z, value.w};
+#pragma unroll
+    for (uint32_t e = 0; e < 4; ++e) {
+        if (!isinf(x[e])) continue;
+        if (v.partial_slot != kU32Max) {
+            p.partial_o[(static_cast<uint64_t>(v.partial_slot) * kMaxRows + r) * p.geo.head_dim + d + e] = x[e];
+            continue;
+        }
+        const uint64_t at = item_row_index(p, v, r) * p.geo.head_dim + d + e;
+        if (p.ext_o != nullptr) p.ext_o[at] = x[e];
+        else store_from_float(p.out, at, p.dtype, x[e] * gate_factor(p, at));
+    }
+}
+
 template <typename T, int DP, int NSLOT>
 __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParams p) {
     using L = AnySmem<DP, NSLOT>;
@@ -79,9 +96,15 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
     constexpr uint32_t kRowsPerCopy = DP <= 128 ? 2 : 1;
     const uint32_t copy_row = kRowsPerCopy == 2 ? lane >> 4 : 0, copy_chunk = kRowsPerCopy == 2 ? lane & 15 : lane;
 
-    for (uint32_t index = p.cta_item_begin[cta]; index < p.cta_item_begin[cta + 1]; ++index) {
+    // An infinity in V meets parts that are zero or negative, and 0 x Inf or Inf - Inf is no number where the weight itself
+    // would have kept the infinity.  An item that ends in anything but finite values is therefore done once more with the
+    // high parts alone, which have the weight's sign, and its infinities are written over what the first pass left.
+    bool again = false;
+    const uint32_t item_end = p.cta_item_begin[cta + 1];
+    for (uint32_t index = p.cta_item_begin[cta]; index < item_end;) {
         const ItemView v = view_item(p, index);
-        __syncthreads();  // the previous item's merge is done with the ring, q and limit_s
+        // (the previous item's merge is done with the ring, q and limit_s: the barrier at the end of this loop)
+        bool not_finite = false;
         const uint32_t* row_ids = table_row(p.geo, v.req_slot);
         const uint32_t first_tile = v.kv_begin / kTile;
         const uint32_t item_tiles = (v.kv_end + kTile - 1) / kTile - first_tile;
@@ -217,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
 #pragma unroll
                 for (int i = 0; i < 4; ++i)
                     split3<T>(w[i >> 1][2 * (i & 1)], w[i >> 1][2 * (i & 1) + 1], pa[0][i], pa[1][i], pa[2][i]);
-            } else {
+            } else if (!again) {
 #pragma unroll
                 for (int j = 0; j < DP / 16; ++j) {
                     uint32_t b[4];
@@ -227,6 +250,14 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
                         Mma<T>::run(st.o[2 * j], pa[part], b[0], b[1]);
                         Mma<T>::run(st.o[2 * j + 1], pa[part], b[2], b[3]);
                     }
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < DP / 16; ++j) {
+                    uint32_t b[4];
+                    ldmatrix_x4_trans(b, tile + v_lane + 32 * j);
+                    Mma<T>::run(st.o[2 * j], pa[0], b[0], b[1]);
+                    Mma<T>::run(st.o[2 * j + 1], pa[0], b[2], b[3]);
                 }
             }
         }
@@ -274,6 +305,11 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
             }
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
             const float4 value = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
+            not_finite = not_finite || !(isfinite(acc.x) && isfinite(acc.y) && isfinite(acc.z) && isfinite(acc.w));
+            if (again) {
+                write_infinities<T>(p, v, r, d, value);
+                continue;
+            }
             if (v.partial_slot != kU32Max) {
                 const uint64_t prow = static_cast<uint64_t>(v.partial_slot) * kMaxRows + r;
                 *reinterpret_cast<float4*>(p.partial_o + prow * D + d) = value;
@@ -294,6 +330,8 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
                 store_out4<T>(p, row * D + d, value);
             }
         }
+        again = __syncthreads_or(not_finite && !again);
+        if (!again) ++index;
     }
 }
 

@@ -47,3 +47,32 @@ def test_a_long_tail_under_a_dominant_key_keeps_its_weights(dtype, head_dim, bel
         assert np.allclose(m, score, rtol=1e-6) and np.allclose(l, 1.0 + n * np.exp(-score), rtol=1e-5)
         s.close()
     assert answers[pkg.KERNEL_AUTO] <= max(2e-6, 2 * answers[pkg.KERNEL_GENERIC]), answers
+
+
+@pytest.mark.parametrize("dtype", [pkg.F16, pkg.BF16])
+@pytest.mark.parametrize("entry", ["partial", "gated"])
+def test_infinities_stay_infinities(dtype, entry):
+    import torch
+    s = W.Session(W.Spec("inf", dtype, 12, 4, 96, 12, [5000, 30], [1, 2], seed=72))
+    s.append()
+    gates = torch.randn(s.q.shape, generator=torch.Generator("cuda").manual_seed(5), device="cuda").to(s.tdtype)
+
+    def run():
+        if entry == "partial":
+            return _partial(s)[0]
+        s.gqa.attend_gated(s.pages, s.table, 0, s.q, gates, s.out)
+        s.ctx.sync()
+        return s.out.float().cpu().numpy()
+
+    clean = run()
+    pages = s.arena.view(s.arena.shape[0], 2, 4, 12, 96)
+    expected = clean.copy()
+    for request, position, head, column, value in ((0, 700, 0, 1, np.inf), (0, 4100, 1, 95, -np.inf), (0, 33, 2, 40, np.nan), (1, 4, 3, 7, np.inf),
+                                                   (0, 100, 3, 0, np.inf), (0, 3000, 3, 0, -np.inf)):
+        pages[int(s.spec.block_tables[request][position // 12]), 1, head, position % 12, column] = value
+        rows = slice(0, 1) if request == 0 else slice(1, 3)
+        at = expected[rows, 3 * head:3 * head + 3, column]
+        expected[rows, 3 * head:3 * head + 3, column] = np.nan if np.isinf(at).all() else value   # Inf - Inf
+    dirty = run()
+    assert np.array_equal(dirty, expected, equal_nan=True)
+    s.close()
