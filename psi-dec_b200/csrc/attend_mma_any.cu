@@ -68,7 +68,25 @@ __device__ __forceinline__ void write_infinities(const AttendParams& p, const It
     }
 }
 
-template <typename T, int DP, int NSLOT>
+__device__ __forceinline__ void st_shared_zero_16(uint32_t dst) {
+    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(dst), "r"(0u) : "memory");
+}
+
+// 16 bytes from a source on a 2-byte boundary into shared memory.
+__device__ __forceinline__ void copy_16_by_elements(uint32_t dst, const void* src, bool present) {
+    uint32_t w[4] = {0, 0, 0, 0};
+    if (present) {
+        const uint16_t* e = static_cast<const uint16_t*>(src);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) w[i] = e[2 * i] | static_cast<uint32_t>(e[2 * i + 1]) << 16;
+    }
+    asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]) : "memory");
+}
+
+// kAligned: the arena lies on a 16-byte boundary.  Off it, and for a q off it, elements are copied one by one: slower than
+// cp.async, but the plan is one CTA per SM for this kernel whatever the buffers of a launch, and the CUDA-core kernels
+// on such a plan took 1,037 us with an odd q for the step above (541 on a plan of their own; 85 here).
+template <typename T, int DP, int NSLOT, bool kAligned>
 __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParams p) {
     using L = AnySmem<DP, NSLOT>;
     const uint32_t cta = blockIdx.x;
@@ -100,6 +118,7 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
     // would have kept the infinity.  An item that ends in anything but finite values is therefore done once more with the
     // high parts alone, which have the weight's sign, and its infinities are written over what the first pass left.
     bool again = false;
+    const bool wide_q = (reinterpret_cast<uintptr_t>(p.q) & 15u) == 0, wide_out = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
     const uint32_t item_end = p.cta_item_begin[cta + 1];
     for (uint32_t index = p.cta_item_begin[cta]; index < item_end;) {
         const ItemView v = view_item(p, index);
@@ -124,8 +143,10 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
 #pragma unroll
             for (uint32_t r = 0; r < uint32_t(kTile); r += kRowsPerCopy) {
                 const unsigned char* src = arena + __shfl_sync(0xFFFFFFFFu, offset, r + copy_row) + copy_chunk * 16;
-                if (copy_chunk < chunks)  // rows beyond the item are zero
-                    cp_async_16_hinted(dst + r * L::kStride, src, r + copy_row < in_range ? 16u : 0u, stream_policy);
+                if (copy_chunk < chunks) {  // rows beyond the item are zero
+                    if constexpr (kAligned) cp_async_16_hinted(dst + r * L::kStride, src, r + copy_row < in_range ? 16u : 0u, stream_policy);
+                    else copy_16_by_elements(dst + r * L::kStride, src, r + copy_row < in_range);
+                }
             }
         };
 
@@ -135,12 +156,13 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
             const uint32_t r = i / (DP / 8), c = i % (DP / 8);
             const bool present = r < v.rows && c < chunks;
             const T* src = static_cast<const T*>(p.q) + (present ? item_row_index(p, v, r) * D + c * 8 : 0);
-            cp_async_16(q_base + r * L::kStride + c * 16, src, present ? 16u : 0u);
+            if (wide_q) cp_async_16(q_base + r * L::kStride + c * 16, src, present ? 16u : 0u);
+            else copy_16_by_elements(q_base + r * L::kStride + c * 16, src, present);
         }
         if (chunks < DP / 8) {
             const uint32_t pad = DP / 8 - chunks;
             for (uint32_t i = lane; i < NSLOT * kTile * pad; i += 32)
-                cp_async_16(ring_base + (i / pad) * L::kStride + (chunks + i % pad) * 16, p.q, 0u);
+                st_shared_zero_16(ring_base + (i / pad) * L::kStride + (chunks + i % pad) * 16);
         }
         if (tid < kTile) limit_s[tid] = tid < v.rows ? item_row_limit(v, tid) : v.kv_end;
         cp_async_commit();
@@ -326,8 +348,12 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
                     p.ext_m[row] = top * kLn2;
                     p.ext_l[row] = sum;
                 }
-            } else {
+            } else if (wide_out) {
                 store_out4<T>(p, row * D + d, value);
+            } else {
+                const float x[4] = {value.x, value.y, value.z, value.w};
+#pragma unroll
+                for (uint32_t e = 0; e < 4; ++e) store_from_float(p.out, row * D + d + e, p.dtype, x[e] * gate_factor(p, row * D + d + e));
             }
         }
         again = __syncthreads_or(not_finite && !again);
@@ -335,9 +361,9 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
     }
 }
 
-template <typename T, int DP, int NSLOT>
+template <typename T, int DP, int NSLOT, bool kAligned>
 cudaError_t launch_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
-    auto kernel = attend_mma_any_kernel<T, DP, NSLOT>;
+    auto kernel = attend_mma_any_kernel<T, DP, NSLOT, kAligned>;
     constexpr int kBytes = AnySmem<DP, NSLOT>::kTotal;
     static_assert(kBytes <= 220 * 1024, "query tile and ring share one CTA's shared memory");
     static std::atomic<uint64_t> configured{0};
@@ -346,14 +372,20 @@ cudaError_t launch_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
     return launch_overlapped(kernel, num_ctas, kThreads, kBytes, stream, p);
 }
 
-template <typename T>
+template <typename T, bool kAligned>
 cudaError_t launch_for_dim(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     const uint32_t d = p.geo.head_dim;
-    if (d <= 64) return launch_any<T, 64, 8>(p, num_ctas, stream);
-    if (d <= 96) return launch_any<T, 96, 8>(p, num_ctas, stream);
-    if (d <= 128) return launch_any<T, 128, 6>(p, num_ctas, stream);
-    if (d <= 192) return launch_any<T, 192, 4>(p, num_ctas, stream);
-    return launch_any<T, 256, 3>(p, num_ctas, stream);
+    if (d <= 64) return launch_any<T, 64, 8, kAligned>(p, num_ctas, stream);
+    if (d <= 96) return launch_any<T, 96, 8, kAligned>(p, num_ctas, stream);
+    if (d <= 128) return launch_any<T, 128, 6, kAligned>(p, num_ctas, stream);
+    if (d <= 192) return launch_any<T, 192, 4, kAligned>(p, num_ctas, stream);
+    return launch_any<T, 256, 3, kAligned>(p, num_ctas, stream);
+}
+
+template <typename T>
+cudaError_t launch_for_arena(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
+    return (reinterpret_cast<uintptr_t>(p.geo.pages) & 15u) == 0 ? launch_for_dim<T, true>(p, num_ctas, stream)
+                                                                 : launch_for_dim<T, false>(p, num_ctas, stream);
 }
 
 }  // namespace
@@ -362,17 +394,12 @@ bool attend_mma_any_profile(uint32_t dtype, uint32_t head_dim) {
     return (dtype == PSI_DTYPE_BF16 || dtype == PSI_DTYPE_F16) && head_dim >= 8 && head_dim <= 256 && head_dim % 8 == 0;
 }
 
-// Arena and q on 16-byte boundaries (16-byte copies), out and gates on 8-byte ones; other buffers stay on the staged
-// kernel.
-bool attend_mma_any_supported(const AttendParams& p) {
-    auto aligned = [](const void* ptr, uintptr_t to) { return (reinterpret_cast<uintptr_t>(ptr) & (to - 1)) == 0; };
-    return attend_mma_any_profile(p.dtype, p.geo.head_dim) && aligned(p.geo.pages, 16) && aligned(p.q, 16) && aligned(p.out, 8) &&
-           aligned(p.gates, 8) && aligned(p.ext_o, 16) && aligned(p.partial_o, 16);
-}
+// (The entry points ask for gates on an 8-byte boundary and partial outputs on a 16-byte one.)
+bool attend_mma_any_supported(const AttendParams& p) { return attend_mma_any_profile(p.dtype, p.geo.head_dim); }
 
 cudaError_t launch_attend_mma_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
-    return p.dtype == PSI_DTYPE_BF16 ? launch_for_dim<__nv_bfloat16>(p, num_ctas, stream)
-                                     : launch_for_dim<__half>(p, num_ctas, stream);
+    return p.dtype == PSI_DTYPE_BF16 ? launch_for_arena<__nv_bfloat16>(p, num_ctas, stream)
+                                     : launch_for_arena<__half>(p, num_ctas, stream);
 }
 
 }  // namespace psi

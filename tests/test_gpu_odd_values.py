@@ -76,3 +76,39 @@ def test_infinities_stay_infinities(dtype, entry):
     dirty = run()
     assert np.array_equal(dirty, expected, equal_nan=True)
     s.close()
+
+
+@pytest.mark.parametrize("dtype", [pkg.F16, pkg.BF16])
+@pytest.mark.parametrize("head_dim,page", [(96, 12), (200, 8), (8, 16)])
+@pytest.mark.parametrize("where", ["q", "out", "arena", "gated"])
+def test_buffers_on_two_byte_boundaries_give_the_same_bits(dtype, head_dim, page, where):
+    import torch
+    s = W.Session(W.Spec("shift", dtype, 6, 2, head_dim, page, [500, 70, 2300], [1, 2, 9], seed=73))
+    s.append()
+
+    def shifted(x):
+        y = torch.zeros(x.numel() + 1, dtype=s.tdtype, device=s.device)[1:].view(x.shape)
+        y.copy_(x)
+        return y
+
+    q, out, pages = s.q, torch.zeros_like(s.q), s.pages
+    gates = torch.randn(s.q.shape, device="cuda").to(s.tdtype) if where == "gated" else None
+    call = (lambda p, a, b: s.gqa.attend_gated(p, s.table, 0, a, gates, b)) if gates is not None else (lambda p, a, b: s.gqa.attend(p, s.table, 0, a, b))
+    call(pages, q, out)
+    s.ctx.sync()
+    wanted = checks.to_numpy_bits(out).copy()
+    held = None
+    if where in ("q", "gated"):
+        q = shifted(s.q)
+    if where in ("out", "gated"):
+        out = shifted(torch.zeros_like(out))
+    if where == "arena":
+        held = shifted(s.arena)
+        pages = pkg.PageArena(s.ctx, s.spec.num_pages, s.spec.page_bytes, device_ptr=held)
+    torch.cuda.synchronize()
+    call(pages, q, out)
+    s.ctx.sync()
+    assert np.array_equal(checks.to_numpy_bits(out), wanted)
+    if held is not None:
+        pages.close()
+    s.close()
