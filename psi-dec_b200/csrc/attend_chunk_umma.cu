@@ -180,7 +180,15 @@ __device__ __forceinline__ uint32_t low_part(float a, float b, uint32_t high) {
 struct UmmaShared {
     uint64_t bars[2 * 12 + 7];
     uint32_t tmem_base, abort, last[8];
+    uint32_t cleaned[2];  // by item parity: the item (its index + 1) in whose V tiles values were replaced
 };
+
+// Whether one of two packed 16-bit values is infinite or no number.
+template <typename T>
+__device__ __forceinline__ bool any_not_finite(uint32_t two) {
+    constexpr uint32_t kExponent = std::is_same<T, __half>::value ? 0x7C00u : 0x7F80u;
+    return (two & kExponent) == kExponent || (two >> 16 & kExponent) == kExponent;
+}
 
 template <typename T, int D, bool kFine>
 __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const CUtensorMap& kv_map, const uint32_t box_rows,
@@ -224,6 +232,7 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
         for (uint32_t b = kBarP; b < kNumBarriers; ++b) mbar_init(bar(b), kRowThreads);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         abort_s = 0;
+        shared.cleaned[0] = shared.cleaned[1] = 0;
     }
     tc_fence_before();
     __syncthreads();
@@ -465,6 +474,36 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
             // softmax state in the log2 domain: `row_ref` is the reference the exponentials are taken against (it
             // trails the true running max `row_max` by at most kRescaleThreshold), `row_sum` is relative to it
             float row_ref = -INFINITY, row_max = -INFINITY, row_sum = 0.0f;
+            // A weight of zero does not hide an infinity: 0 x Inf is no number, and an item of a short run holds up to 128
+            // rows, of which those of one query token see one of the step's own keys more than those of the one before.
+            // Values that are not finite in V rows that some row of the item must not see are therefore set to zero in the
+            // tile, by the row threads while S is at hand, and come back at the end of the item in the rows that see them
+            // (the decode kernel's items, tiles of 16 rows, keep such a value to themselves); so are those of the keys before
+            // the piece's first, which share its first tile.
+            [[maybe_unused]] auto clean_values = [&](uint32_t tile, uint32_t token0) {
+                const uint32_t before = max(token0, v.kv_begin) - token0, end = min(token0 + kUmmaN, v.kv_end) - token0;
+                const uint32_t first = min(max(token0, min_limit) - token0, end);  // rows [0, before) and [first, end)
+                const uint32_t fill = 2 * tile + 1, slot = fill % kSlots;
+                wait(kBarFull + slot, fill / kSlots);
+                bool cleaned = false;
+                for (uint32_t i = tid; i < (before + end - first) * kChunks; i += kRowThreads) {
+                    const uint32_t row = i / kChunks < before ? i / kChunks : first - before + i / kChunks;
+                    const uint32_t at = smem_base + slot * kTileBytes + operand_offset(kBlocks, row, i % kChunks);
+                    uint4 value = ld_shared_16(at);
+                    if (!any_not_finite<T>(value.x) && !any_not_finite<T>(value.y) && !any_not_finite<T>(value.z) && !any_not_finite<T>(value.w)) continue;
+                    uint32_t* two = &value.x;
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        if (any_not_finite<T>(two[k] & 0xFFFFu)) two[k] &= 0xFFFF0000u;
+                        if (any_not_finite<T>(two[k] >> 16)) two[k] &= 0xFFFFu;
+                    }
+                    st_shared_16(at, value);
+                    cleaned = true;
+                }
+                if (!cleaned) return;
+                fence_async_smem();
+                *reinterpret_cast<volatile uint32_t*>(&shared.cleaned[index & 1]) = index + 1;
+            };
             uint32_t next_row = 0, next_rows = 0;  // this thread's row of the next item
                 if (index + 1 < item_end) {  // the next item's query rows travel under this item's tiles
                     next_rows = next_rows_of.w * next_heads_of.w;
@@ -496,6 +535,7 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                         const uint32_t token = token0 + c;
                         if (token >= limit || token < v.kv_begin) s[c] = -INFINITY;
                     }
+                    if constexpr (kFine) clean_values(tile, token0);
                 }
                 float m4[4] = {s[0], s[1], s[2], s[3]};
 #pragma unroll
@@ -592,6 +632,21 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                 } else {
 #pragma unroll
                     for (int e = 0; e < 32; ++e) o[e] = 0.0f;
+                }
+                if constexpr (kFine) {
+                    if (row_valid && *reinterpret_cast<volatile uint32_t*>(&shared.cleaned[index & 1]) == index + 1) {
+                        const uint32_t* row_ids = table_row(p.geo, v.req_slot);
+                        for (uint32_t token = max(min_limit, v.kv_begin); token < limit; ++token) {
+                            const uint64_t page = page_id_or_zero(p.geo, row_ids, token >> page_shift);
+                            const T* src = reinterpret_cast<const T*>(pages + page * page_bytes + v_region_bytes) +
+                                           (static_cast<uint64_t>(v.kv_head) * p.geo.tokens_per_page + (token & page_mask)) * D + c;
+#pragma unroll
+                            for (int e = 0; e < 32; ++e) {
+                                const float value = static_cast<float>(src[e]);
+                                if (!isfinite(value)) o[e] += value;
+                            }
+                        }
+                    }
                 }
                 if (row_valid) {
 #pragma unroll

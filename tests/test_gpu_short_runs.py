@@ -47,6 +47,33 @@ def _rows_of(s, request):
     return np.arange(cu[request], cu[request + 1])
 
 
+@pytest.mark.parametrize("dtype", [pkg.BF16, pkg.F16])
+@pytest.mark.parametrize("heads,head_dim,context,count", [((40, 8), 128, 897, 40), ((16, 2), 256, 2500, 24), ((24, 4), 256, 8130, 4)])
+@pytest.mark.parametrize("bad", [float("inf"), float("-inf"), float("nan")])
+def test_a_value_that_is_not_finite_stays_in_the_rows_that_see_it(dtype, heads, head_dim, context, count, bad):
+    import torch
+    run, hit = 8, 5   # value column 3 of KV head 1 of the sixth token of request 1; column 70 of a key of its history
+    s = W.Session(W.Spec("inf", dtype, *heads, head_dim, 16, [context] * count, [run] * count, seed=52))
+    s.append()
+    assert s.gqa.plan_stats()["chunk_ctas"] > 0
+    clean = _partial(s).cpu().numpy()
+    rows, group = _rows_of(s, 1), heads[0] // heads[1]
+    pages = s.arena.view(s.arena.shape[0], 2, heads[1], 16, head_dim)
+    for position, column in ((context + hit, 3), (context // 2, 60)):
+        page = int(s.spec.block_tables[1][position // 16])
+        pages[page, 1, 1, position % 16, column] = bad
+    dirty = _partial(s).cpu().numpy()
+    expected = clean.copy()
+    expected[rows[hit:], group:2 * group, 3] = bad
+    expected[rows, group:2 * group, 60] = bad
+    same = np.isfinite(expected)
+    assert np.array_equal(np.isfinite(dirty), same)
+    assert np.array_equal(dirty[same], clean[same])
+    assert np.array_equal(dirty[~same], expected[~same], equal_nan=True)
+    assert s.gqa.device_status() == 0
+    s.close()
+
+
 @pytest.mark.parametrize("engine", [pkg.KERNEL_AUTO, pkg.KERNEL_MMA_SYNC, pkg.KERNEL_MMA_TMA])
 @pytest.mark.parametrize("runs,contexts", [([1] * 3, [70, 9, 300]), ([8] * 40, [900] * 40), ([300, 1], [20, 400])])
 def test_unaligned_buffers_are_refused_before_anything_is_launched(engine, runs, contexts):
