@@ -190,7 +190,7 @@ constexpr uint64_t kRowsResidentCtas = 148 * 4;
 template <uint32_t DTYPE, int LPR>
 __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 4) norm_rope_rows_kernel(PrepParams p) {
     constexpr uint32_t D = LPR * 8, kRows = 32 / LPR;
-    __shared__ float2 turn_s[D / 2];  // (cosine, sine) of the token's position at every frequency
+    __shared__ __align__(16) float2 turn_s[D / 2];  // (cosine, sine) of the position at every frequency, read two at a time
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t group = lane / LPR, sub = lane % LPR, d0 = sub * 8;
     const uint32_t token = blockIdx.x;
