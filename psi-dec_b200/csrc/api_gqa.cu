@@ -41,8 +41,7 @@ int32_t psi_gqa_create(psi_ctx* ctx, const psi_gqa_config* config, psi_gqa** out
             g->kernel == PSI_KERNEL_MMA ? attend_mma_ctas_per_sm(c.head_dim)
                                         : (g->any_mma ? 1u : attend_generic_ctas_per_sm(c.head_dim, c.dtype));
         g->grid_cap = c.max_ctas > 0 ? c.max_ctas : static_cast<uint32_t>(ctx->sm_count) * per_sm;
-        // (24 requests of 300 to 6,000 tokens at head_dim 96: 91 us a step with 0, 77 with 16, 87 with 64; f32 is best with 0)
-        g->item_start_cost = g->kernel == PSI_KERNEL_MMA ? 32u : (g->any_mma ? 16u : 0u);
+        g->item_start_cost = g->kernel == PSI_KERNEL_MMA ? kMmaItemStartCost : (g->any_mma ? kMmaAnyItemStartCost : 0u);
         // (a component whose batches cannot hold a run of two query tiles never launches the long-run kernel, which under a
         // replay reservation would otherwise be part of every step)
         g->chunk_supported = g->kernel == PSI_KERNEL_MMA && c.plan_mode == PSI_PLAN_BALANCED && c.max_tokens > g->geo.tokens_per_tile &&

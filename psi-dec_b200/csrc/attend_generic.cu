@@ -459,8 +459,10 @@ uint32_t attend_generic_ctas_per_sm(uint32_t head_dim, uint32_t dtype) {
 
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     if (num_ctas == 0) return cudaSuccess;
-    if (p.tensor_cores != 0 && attend_mma_any_supported(p)) return launch_attend_mma_any(p, num_ctas, stream);
-    if (attend_f32_supported(p)) return launch_attend_f32(p, num_ctas, stream);
+    if (p.generic_only == 0) {
+        if (attend_mma_any_supported(p)) return launch_attend_mma_any(p, num_ctas, stream);
+        if (attend_f32_supported(p)) return launch_attend_f32(p, num_ctas, stream);
+    }
     if (attend_staged_supported(p)) return launch_attend_staged(p, num_ctas, stream);
     const uint32_t dpl = (p.geo.head_dim + 31) / 32;
     if (dpl > 8) return cudaErrorInvalidValue;

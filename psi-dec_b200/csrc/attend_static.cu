@@ -151,11 +151,13 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         const PlanGeometry geo = plan_geometry(c.num_q_heads, c.num_kv_heads);
         const bool mma = c.kernel_mode != PSI_KERNEL_GENERIC && attend_mma_supported(c.dtype, c.head_dim, tokens_per_page);
         require(mma || c.kernel_mode < PSI_KERNEL_MMA, "the mma kernel does not support this profile");
-        const uint32_t per_sm = mma ? attend_mma_ctas_per_sm(c.head_dim) : attend_generic_ctas_per_sm(c.head_dim, c.dtype);
+        const bool any_mma = !mma && c.kernel_mode != PSI_KERNEL_GENERIC && attend_mma_any_profile(c.dtype, c.head_dim);
+        const uint32_t per_sm = mma ? attend_mma_ctas_per_sm(c.head_dim)
+                                    : (any_mma ? 1u : attend_generic_ctas_per_sm(c.head_dim, c.dtype));
         uint32_t max_ctas = std::min<uint32_t>(kStaticMaxCtas, static_cast<uint32_t>(sm_count) * per_sm);
         if (c.max_ctas > 0) max_ctas = std::min(max_ctas, c.max_ctas);
         const WorkPlan plan = build_balanced_plan(geo, req_slots, token_indices, cu_tokens, num_reqs, max_ctas,
-                                                  mma ? 16u : 4u, mma ? 32u : 0u);
+                                                  mma ? 16u : 4u, mma ? kMmaItemStartCost : (any_mma ? kMmaAnyItemStartCost : 0u));
         if (plan.items.size() > kStaticMaxItems) {
             return fail(PSI_ERR_INVALID_ARGUMENT,
                         "the step needs " + std::to_string(plan.items.size()) + " work items; the static scratch holds " +
@@ -212,6 +214,7 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         p.num_q_heads = c.num_q_heads;
         p.dtype = c.dtype;
         p.scale_log2 = c.scale * 1.4426950408889634f;
+        p.generic_only = c.kernel_mode == PSI_KERNEL_GENERIC ? 1u : 0u;
         if (mma) {
             err = launch_attend_mma(p, plan.num_ctas(), stream);
         } else {

@@ -112,3 +112,36 @@ def test_buffers_on_two_byte_boundaries_give_the_same_bits(dtype, head_dim, page
     if held is not None:
         pages.close()
     s.close()
+
+
+@pytest.mark.parametrize("heads,head_dim", [((8, 2), 128), ((16, 2), 256), ((3, 1), 32)])
+def test_f32_kernels_agree_on_partials(heads, head_dim):
+    import torch
+    found = []
+    for mode in (pkg.KERNEL_AUTO, pkg.KERNEL_GENERIC):
+        s = W.Session(W.Spec("f32", pkg.F32, *heads, head_dim, 16, [4000, 33, 900], [1, 3, 2], seed=74), kernel_mode=mode)
+        s.append()
+        found.append(_partial(s))
+        s.close()
+    # other sums in another order, and so other last bits: two kernels and not one
+    assert not np.array_equal(found[0][0], found[1][0])
+    for a, b in zip(*found):
+        assert np.abs(a - b).max() <= 2e-5 * max(1.0, np.abs(b).max())
+
+
+@pytest.mark.parametrize("dtype,heads,head_dim,page,mode", [(pkg.BF16, (24, 8), 96, 12, pkg.KERNEL_AUTO), (pkg.F16, (16, 2), 200, 8, pkg.KERNEL_AUTO),
+                                                            (pkg.F32, (8, 2), 128, 16, pkg.KERNEL_AUTO), (pkg.BF16, (24, 8), 96, 12, pkg.KERNEL_GENERIC),
+                                                            (pkg.F32, (8, 2), 128, 16, pkg.KERNEL_GENERIC)])
+def test_the_static_entry_point_takes_the_same_kernel(dtype, heads, head_dim, page, mode):
+    # the same plan, kernel and reduce pass: the same bits (the static scratch holds plans of up to PSI_STATIC_MAX_CTAS)
+    import torch
+    s = W.Session(W.Spec("static", dtype, *heads, head_dim, page, [2600, 70, 900], [1, 2, 1], seed=75), kernel_mode=mode, max_ctas=64)
+    s.append()
+    s.attend()
+    out = torch.zeros_like(s.out)
+    config = pkg.GQAConfig(*heads, head_dim, s.spec.scale, s.spec.page_bytes, dtype, s.layout, s.spec.num_tokens, pkg.PLAN_BALANCED, mode, 64)
+    pkg.attend_static(0, s.stream.cuda_stream, config, s.arena, s.table.page_ids_buffer(), *s.spec.batch(), s.spec.layer, s.q, out)
+    s.ctx.sync()
+    torch.cuda.synchronize()
+    assert np.array_equal(checks.to_numpy_bits(out), checks.to_numpy_bits(s.out))
+    s.close()
