@@ -337,11 +337,11 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             g->has_merged = false;
         } else {
             const RequestRuns runs = plain_runs(req_slots, token_indices, cu_tokens, num_reqs);
-            RequestRuns merged;
+            MergedRuns merged;
             const bool can_merge = merge_one_position_runs(runs, merged);
-            plan_runs(g, can_merge && g->replay_reserved ? merged : runs, 0, g->plan, g->chunk);
+            plan_runs(g, can_merge && g->replay_reserved ? merged.view() : runs, 0, g->plan, g->chunk);
             g->has_merged = can_merge && !g->replay_reserved;
-            if (g->has_merged) plan_runs(g, merged, 0, g->merged_plan, g->merged_chunk);
+            if (g->has_merged) plan_runs(g, merged.view(), 0, g->merged_plan, g->merged_chunk);
         }
         const WorkPlan& plan = g->plan;
         const ChunkPlan& chunk = g->chunk;

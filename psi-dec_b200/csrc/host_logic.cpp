@@ -268,16 +268,7 @@ PlanGeometry plan_geometry(uint32_t num_q_heads, uint32_t num_kv_heads) {
     return g;
 }
 
-RequestRuns plain_runs(const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs) {
-    RequestRuns runs;
-    runs.req_slots.assign(req_slots, req_slots + num_reqs);
-    runs.token_indices.assign(token_indices, token_indices + num_reqs);
-    runs.cu_tokens.assign(cu_tokens, cu_tokens + num_reqs + 1);
-    runs.one_position.assign(num_reqs, 0);
-    return runs;
-}
-
-bool merge_one_position_runs(const RequestRuns& runs, RequestRuns& merged) {
+bool merge_one_position_runs(const RequestRuns& runs, MergedRuns& merged) {
     auto same = [&](uint32_t a, uint32_t b) {
         return runs.run(a) == 1 && runs.run(b) == 1 && runs.req_slots[a] == runs.req_slots[b] &&
                runs.token_indices[a] == runs.token_indices[b];
@@ -286,7 +277,7 @@ bool merge_one_position_runs(const RequestRuns& runs, RequestRuns& merged) {
     bool any = false;
     for (uint32_t r = 1; r < n && !any; ++r) any = same(r - 1, r);
     if (!any) return false;
-    merged = RequestRuns{};
+    merged = MergedRuns{};
     merged.cu_tokens.push_back(0);
     for (uint32_t r = 0; r < n;) {
         uint32_t end = r + 1;
@@ -350,7 +341,7 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, c
         for (uint32_t begin = runs.cu_tokens[r]; begin < runs.cu_tokens[r + 1];) {
             uint32_t end = std::min(runs.cu_tokens[r + 1], begin + geo.tokens_per_tile);
             plan.tiles.push_back({begin, end, runs.req_slots[r], runs.position(r, begin), runs.token_indices[r],
-                                  runs.cu_tokens[r], runs.one_position[r] != 0});
+                                  runs.cu_tokens[r], runs.one_position(r)});
             tile_ctx.push_back(runs.context(r, end));
             begin = end;
         }
@@ -470,13 +461,17 @@ ChunkOrder chunk_order(const PlanGeometry& geo, const RequestRuns& runs, const s
 bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                 std::vector<uint32_t>& chunk_reqs) {
     const uint64_t heads = uint64_t(geo.num_kv_heads) * geo.head_tiles;
-    auto tiles_of = [&](uint32_t r) { return static_cast<uint32_t>(div_ceil(runs.run(r), geo.tokens_per_tile)); };
+    // (most runs of most steps are one tile: no division for those)
+    auto tiles_of = [&](uint32_t r) {
+        const uint32_t run = runs.run(r);
+        return run <= geo.tokens_per_tile ? std::min(run, 1u) : (run + geo.tokens_per_tile - 1) / geo.tokens_per_tile;
+    };
     bool any_long = false;
     std::vector<uint32_t> several;                             // runs of several tiles, none of them a long one
     uint64_t once = 0, per_tile = 0, units = 0, longest = 0;   // KV tiles of `several`: read once, read per query tile
     for (uint32_t r = 0; r < runs.size(); ++r) {
         const uint64_t tiles = tiles_of(r);
-        any_long = any_long || (tiles >= kChunkMinTiles && !runs.one_position[r]);
+        any_long = any_long || (tiles >= kChunkMinTiles && !runs.one_position(r));
         if (tiles < 2) continue;
         const uint64_t keys = div_ceil(runs.context(r, runs.cu_tokens[r + 1]), kKvTile);
         const uint64_t passes = div_ceil(runs.run(r), tokens_per_chunk_item(geo));
@@ -505,7 +500,7 @@ bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRul
     for (uint32_t r = 0; r < runs.size(); ++r) {
         const uint32_t tiles = tiles_of(r);
         if (tiles == 0) continue;
-        const bool chunk = take ? tiles >= 2 : (tiles >= kChunkMinTiles && !runs.one_position[r]);
+        const bool chunk = take ? tiles >= 2 : (tiles >= kChunkMinTiles && !runs.one_position(r));
         (chunk ? chunk_reqs : decode_reqs).push_back(r);
     }
     return take;
@@ -558,7 +553,7 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, con
         d.first_pos = runs.position(u.req, u.flat_begin);
         d.new_begin = runs.token_indices[u.req];
         d.flat_req_begin = runs.cu_tokens[u.req];
-        d.flags = (head_tile == 0 ? kItemWritesKv : 0u) | (runs.one_position[u.req] ? kItemOnePosition : 0u);
+        d.flags = (head_tile == 0 ? kItemWritesKv : 0u) | (runs.one_position(u.req) ? kItemOnePosition : 0u);
         return d;
     };
     // `n` consecutive items starting at `first` are the pieces of one unit cut across CTAs: partial slots 8 apart,

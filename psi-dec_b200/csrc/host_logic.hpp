@@ -139,21 +139,36 @@ struct PlanGeometry {
 
 PlanGeometry plan_geometry(uint32_t num_q_heads, uint32_t num_kv_heads);
 
-// The step's requests as the planners see them: a run of consecutive query tokens of one slot each.
+// The step's requests as the planners see them: a run of consecutive query tokens of one slot each.  A view of the
+// caller's arrays (a step is planned in microseconds; copies of them are a part of that).
 struct RequestRuns {
-    std::vector<uint32_t> req_slots, token_indices, cu_tokens;
-    std::vector<uint8_t> one_position;  // the run's tokens all stand at token_indices[r] instead of following one another
-    uint32_t size() const { return static_cast<uint32_t>(req_slots.size()); }
+    const uint32_t* req_slots = nullptr;
+    const uint32_t* token_indices = nullptr;
+    const uint32_t* cu_tokens = nullptr;
+    uint32_t num_reqs = 0;
+    const uint8_t* one_position_runs = nullptr;  // nullptr: none
+    uint32_t size() const { return num_reqs; }
+    // the run's tokens all stand at token_indices[r] instead of following one another
+    bool one_position(uint32_t r) const { return one_position_runs != nullptr && one_position_runs[r] != 0; }
     uint32_t run(uint32_t r) const { return cu_tokens[r + 1] - cu_tokens[r]; }
     // position of flat token `t` of request r, and the keys its run sees up to and with the token before `end`
-    uint32_t position(uint32_t r, uint32_t t) const { return token_indices[r] + (one_position[r] ? 0 : t - cu_tokens[r]); }
-    uint32_t context(uint32_t r, uint32_t end) const { return token_indices[r] + (one_position[r] ? 1 : end - cu_tokens[r]); }
+    uint32_t position(uint32_t r, uint32_t t) const { return token_indices[r] + (one_position(r) ? 0 : t - cu_tokens[r]); }
+    uint32_t context(uint32_t r, uint32_t end) const { return token_indices[r] + (one_position(r) ? 1 : end - cu_tokens[r]); }
 };
-RequestRuns plain_runs(const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs);
+inline RequestRuns plain_runs(const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens, uint32_t num_reqs) {
+    return {req_slots, token_indices, cu_tokens, num_reqs, nullptr};
+}
+struct MergedRuns {
+    std::vector<uint32_t> req_slots, token_indices, cu_tokens;
+    std::vector<uint8_t> one_position;
+    RequestRuns view() const {
+        return {req_slots.data(), token_indices.data(), cu_tokens.data(), static_cast<uint32_t>(req_slots.size()), one_position.data()};
+    }
+};
 // Adjacent one-token requests of one slot at one position (the rows of a draft block, which all see the same history)
 // become one run, so that the history is read once for all of them; false when there are none.  Not for launches that
 // take this step's K/V rows from the caller's buffers: there every request reads its own row at that position.
-bool merge_one_position_runs(const RequestRuns& runs, RequestRuns& merged);
+bool merge_one_position_runs(const RequestRuns& runs, MergedRuns& merged);
 
 struct WorkPlan {
     std::vector<ExecTile> tiles;
