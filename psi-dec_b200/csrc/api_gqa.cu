@@ -127,25 +127,16 @@ int32_t psi_gqa_reserve_replay(psi_gqa* g) {
         psi_ctx* ctx = g->ctx;
         require(!ctx->capturing, "replay capacity cannot be reserved during stream capture");
         ctx->bind();
-        // worst cases for max_tokens: every token a query tile of its own, every unit cut at every CTA boundary
-        const uint64_t heads = uint64_t(g->geo.num_kv_heads) * g->geo.head_tiles;
-        const uint64_t units = uint64_t(g->cfg.max_tokens) * heads;
-        const uint64_t cap_items = units + g->grid_cap;
-        // (a run of two query tiles is at least two tokens long); of the chunk items only pieces of cut units take partial
-        // slots: in equal shares a CTA holds at most two, in stream order
-        // they number at most two per CTA and one per unit, and at most four per CTA
-        const uint64_t chunk_units = g->chunk_supported ? units / 2 + heads : 0;
-        const uint64_t cap_chunk_items = g->chunk_supported ? chunk_units + 4ull * g->grid_cap + 8 : 0;
-        const uint64_t chunk_pieces = g->chunk_supported ? std::min<uint64_t>(chunk_units + 2ull * g->grid_cap, 4ull * g->grid_cap) + 8 : 0;
-        const uint64_t slots = cap_items + chunk_pieces * kChunkTilesPerItem;
+        const ReplayCapacity cap = replay_capacity(g->geo, g->cfg.max_tokens, g->grid_cap, g->chunk_supported);
+        const uint64_t slots = cap.slots;
         const uint64_t partial_bytes = slots * kMaxRows * g->cfg.head_dim * sizeof(float);
         require(partial_bytes <= (2ull << 30),
                 "replay reservation needs more than 2 GiB of partial-output scratch for this max_tokens: create the "
                 "component with the largest batch the replayed steps carry");
         cuda_check(cudaStreamSynchronize(ctx->stream), "cudaStreamSynchronize");
-        g->cap_items = cap_items;
-        g->cap_chunk_items = cap_chunk_items;
-        g->cap_reduces = units;
+        g->cap_items = cap.items;
+        g->cap_chunk_items = cap.chunk_items;
+        g->cap_reduces = cap.reduces;
         if (g->staging != nullptr) {
             cuda_check(cudaFreeHost(g->staging), "cudaFreeHost");
             g->staging = nullptr;

@@ -683,6 +683,20 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, con
     return plan;
 }
 
+ReplayCapacity replay_capacity(const PlanGeometry& geo, uint32_t max_tokens, uint32_t max_ctas, bool chunks) {
+    const uint64_t heads = uint64_t(geo.num_kv_heads) * geo.head_tiles, units = max_tokens * heads;
+    ReplayCapacity cap;
+    cap.items = units + max_ctas;
+    cap.reduces = units;
+    cap.slots = cap.items;
+    if (chunks) {
+        const uint64_t chunk_units = units / 2 + heads;
+        cap.chunk_items = chunk_units + 4ull * max_ctas + 8;
+        cap.slots += (std::min<uint64_t>(chunk_units + 2ull * max_ctas, 4ull * max_ctas) + 8) * kChunkTilesPerItem;
+    }
+    return cap;
+}
+
 std::vector<DeviceItem> flatten_plan(const WorkPlan& plan, const PlanGeometry& geo) {
     std::vector<DeviceItem> out(plan.items.size());
     for (size_t i = 0; i < plan.items.size(); ++i) {

@@ -247,6 +247,16 @@ ChunkOrder chunk_order(const PlanGeometry& geo, const RequestRuns& runs, const s
 ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint32_t max_ctas,
                            uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost = 0);
 
+// What a replay reservation for steps of up to `max_tokens` query tokens sets aside: every token a query tile of its own,
+// every unit cut at every CTA boundary; a run of the chunk kernels is at least two tokens long.  Of the chunk items only
+// pieces of cut units take partial slots, eight a piece.  In equal shares a CTA holds at most two such pieces.  In stream
+// order a unit is cut where it is longer than half a CTA's share, so its pieces are at least a quarter of a share each: at
+// most four a CTA, and at most two a CTA and one a unit.
+struct ReplayCapacity {
+    uint64_t items = 0, reduces = 0, chunk_items = 0, slots = 0;
+};
+ReplayCapacity replay_capacity(const PlanGeometry& geo, uint32_t max_tokens, uint32_t max_ctas, bool chunks);
+
 // Device form of a finished plan.
 std::vector<DeviceItem> flatten_plan(const WorkPlan& plan, const PlanGeometry& geo);
 
