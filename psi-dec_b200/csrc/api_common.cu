@@ -165,7 +165,7 @@ ChunkRule chunk_rule(const psi_gqa* g, uint64_t handicap) {
     rule.head_dim = g->cfg.head_dim;
     rule.token_bytes = g->cfg.page_bytes / g->tokens_per_page;
     rule.short_runs = g->chunk_umma;
-    rule.handicap = handicap;
+    rule.handicap = handicap + (g->exchanges ? kExchangeHandicap : 0u);
     return rule;
 }
 
@@ -284,7 +284,7 @@ static void pack_plan(uint32_t* s, const PlanOffsets& off, const WorkPlan& plan,
 // staging buffer and its size comes back in *deferred_words: the caller brings it to the device itself.
 void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens,
                   uint32_t num_reqs, uint32_t capacity_mode, uint32_t caller_num_total_tokens,
-                  psi_replay_shape* out_shape, bool defer_upload, uint64_t* deferred_words, bool plan_only) {
+                  psi_replay_shape* out_shape, bool defer_upload, uint64_t* deferred_words, bool plan_only, uint64_t handicap) {
     {
         require(!plan_only || g->cfg.plan_mode == PSI_PLAN_BALANCED, "a plan-only prepare needs the balanced plan mode");
         require(req_slots != nullptr && token_indices != nullptr && cu_tokens != nullptr, "metadata inputs must not be null");
@@ -339,9 +339,9 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
             const RequestRuns runs = plain_runs(req_slots, token_indices, cu_tokens, num_reqs);
             MergedRuns merged;
             const bool can_merge = merge_one_position_runs(runs, merged);
-            plan_runs(g, can_merge && g->replay_reserved ? merged.view() : runs, 0, g->plan, g->chunk);
+            plan_runs(g, can_merge && g->replay_reserved ? merged.view() : runs, handicap, g->plan, g->chunk);
             g->has_merged = can_merge && !g->replay_reserved;
-            if (g->has_merged) plan_runs(g, merged.view(), 0, g->merged_plan, g->merged_chunk);
+            if (g->has_merged) plan_runs(g, merged.view(), handicap, g->merged_plan, g->merged_chunk);
         }
         const WorkPlan& plan = g->plan;
         const ChunkPlan& chunk = g->chunk;

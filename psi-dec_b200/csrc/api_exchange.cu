@@ -155,6 +155,7 @@ int32_t psi_gqa_attend_exchange(psi_gqa* g, psi_pages* pages, psi_table* table, 
         require(!ctx->capturing, "the exchange carries a step counter and stays outside captured graphs");
         ctx->bind();
         AttendParams p = attend_params(g, pages, table, layer, q);
+        g->exchanges = true;  // from the next prepare on
         const uint64_t rows = uint64_t(g->shape.num_tokens) * g->cfg.num_q_heads;
         const uint64_t floats = rows * (uint64_t(g->cfg.head_dim) + 2);
         require(e.slot_floats >= floats && e.slot_floats % 4 == 0,

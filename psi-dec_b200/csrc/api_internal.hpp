@@ -189,6 +189,7 @@ struct psi_gqa {
     uint32_t kernel = PSI_KERNEL_GENERIC;  // resolved kernel
     bool any_mma = false;                  // the generic path runs on the tensor cores (attend_mma_any.cu)
     uint32_t grid_cap = 1;
+    bool exchanges = false;      // attend_exchange has been called: short runs leave its single launch only where that pays more
     uint32_t item_start_cost = 0;  // KV tiles one item switch is worth when shares are balanced
     psi::PlanGeometry geo{};
     std::unique_ptr<psi::SplitKvSelector> selector;  // null when the profile is outside the reference selector's domain
@@ -289,6 +290,10 @@ constexpr uint32_t kPipelineMaxGroups = 8;
 
 AttendParams attend_params(psi_gqa* g, const psi_pages* pages, const psi_table* table, uint32_t layer, const void* q);
 void run_attend(psi_gqa* g, const AttendParams& params);
+// ChunkRule::handicap of a component that exchanges: beside short runs on the long-run kernel an exchange is an append, a push
+// and a merge launch of their own, ten to twenty microseconds (4 requests of 15,000 to 30,000 tokens, eight rows, 16/2 x 256:
+// 111 us a step in one launch, 124 in several).
+constexpr uint64_t kExchangeHandicap = 200;
 // Deals a step's requests to the decode kernel and the chunk kernels (split_runs).
 bool split_requests(const psi_gqa* g, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                     std::vector<uint32_t>& chunk_reqs);
@@ -306,6 +311,7 @@ void run_staged_host_step(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
 // library's plan; the replay shape then names the token count alone.
 void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_indices, const uint32_t* cu_tokens,
                   uint32_t num_reqs, uint32_t capacity_mode, uint32_t caller_num_total_tokens,
-                  psi_replay_shape* out_shape, bool defer_upload, uint64_t* deferred_words, bool plan_only = false);
+                  psi_replay_shape* out_shape, bool defer_upload, uint64_t* deferred_words, bool plan_only = false,
+                  uint64_t handicap = 0);
 
 }  // namespace psi
