@@ -517,10 +517,11 @@ PSI_API int32_t psi_gqa_decode_step_host(psi_gqa* gqa, psi_pages* pages, psi_tab
  * metadata and buffers together (the executor's update-then-submit pair of
  * crates/inference-executor-metal/src/attn/gqa/batch_metadata.rs:128-317 and backend.rs:493-612): with pinned buffers
  * one launch pulls the packed plan and q/k/v over the host link (no copy-engine transfer) and the attention launch
- * stores out straight into the host buffer; from 1 MiB of q + k + v on (and no long query runs in the step) the attention launch reads the pinned
- * buffers in place, so that the transfer runs under the K/V stream instead of in front of it.  Same result as the two
- * calls.  A step with long query runs and 64 MiB or more of q + k + v in pinned buffers (balanced plan mode, no replay
- * reservation) runs as up to eight groups of consecutive requests instead: group i's inputs travel on a copy stream
+ * stores out straight into the host buffer; from 1 MiB of q + k + v on (and no long query runs in the step) the
+ * attention launch reads the pinned buffers in place, so that the transfer runs under the K/V stream instead of in front
+ * of it.  Same result as the two calls; runs of a few query tokens may then take another kernel than psi_gqa_prepare,
+ * which does not know where q, k and v lie, chooses for them, and agree within rounding.  A step with long query runs
+ * and 64 MiB or more of q + k + v in pinned buffers (balanced plan mode, no replay reservation) runs as up to eight groups of consecutive requests instead: group i's inputs travel on a copy stream
  * while group i-1 is planned and launched and group i-2's output travels back on a second copy stream, so the step
  * takes about as long as the slowest of transfer in, compute and transfer out rather than their sum.  Every group gets a
  * plan of its own (its KV splits differ from the whole step's: results agree within the tolerance of any other split),

@@ -183,19 +183,23 @@ int32_t psi_gqa_step_host(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
             run_staged_host_step(g, pages, table, layer, k_host, v_host, q_host, out_host, kv_bytes, q_bytes, q_cap);
             return;
         }
-        // Small steps pull q/k/v into device staging.  From
-        // kDirectHostBytes on, that pull would sit in front of the attention for longer than the attention loses by
-        // fetching each item's query rows and the step's K/V rows over the host link itself, so the launch reads the
-        // host buffers in place and the transfer hides under the K/V stream (256 verify tokens of 24/4 heads, 5.2 MB:
-        // 853 -> 778 us per step; 32 decode tokens, 0.33 MB: no difference).  Long query runs keep the staged path:
-        // their kernel takes q and the appended rows through device memory.
-        bool direct = q_bytes + 2 * kv_bytes >= kDirectHostBytes && !g->replay_reserved;
+        // Small steps pull q/k/v into device staging.  From kDirectHostBytes on, that pull would sit in front of the
+        // attention for longer than the attention loses by fetching each item's query rows and the step's K/V rows over
+        // the host link itself, so the launch reads the host buffers in place and the transfer hides under the K/V stream
+        // (256 verify tokens, two a request, 24/4 heads, 5.2 MB: 853 -> 778 us per step; 32 decode tokens, 0.33 MB: no
+        // difference).  Steps with runs on the long-run kernel keep the staged path: that kernel takes the appended rows
+        // through their pages, and q read in place by each piece of a unit cost more than the pull where units are cut
+        // (16 requests of eight rows on 512 to 16,384 tokens, 16/2 heads x 256: 240 us against 148).  Short runs therefore
+        // go there only where the kernel also saves the pull (kHostPullTiles).
+        const uint64_t io_bytes = q_bytes + 2 * kv_bytes;
+        bool direct = io_bytes >= kDirectHostBytes && !g->replay_reserved;
+        const uint64_t handicap = direct ? io_bytes * kHostPullTiles >> 20 : 0;
         if (direct && g->chunk_supported) {
             std::vector<uint32_t> decode_reqs, chunk_reqs;
-            split_requests(g, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), chunk_rule(g, 0), decode_reqs, chunk_reqs);
+            split_requests(g, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), chunk_rule(g, handicap), decode_reqs, chunk_reqs);
             direct = chunk_reqs.empty();
         }
-        if (!direct && q_bytes + 2 * kv_bytes >= kPipelineHostBytes && num_reqs >= 2 && !g->replay_reserved &&
+        if (!direct && io_bytes >= kPipelineHostBytes && num_reqs >= 2 && !g->replay_reserved &&
             g->cfg.plan_mode == PSI_PLAN_BALANCED) {
             run_pipelined_host_step(g, pages, table, layer, req_slots, token_indices, cu_tokens, num_reqs, k_host, v_host,
                                     q_host, out_host);
@@ -205,7 +209,7 @@ int32_t psi_gqa_step_host(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
         // q/k/v (or the plan alone when q/k/v are read in place), and the attention launch stores `out` straight into
         // the host buffer.
         uint64_t words = 0;
-        prepare_impl(g, req_slots, token_indices, cu_tokens, num_reqs, PSI_CAPACITY_EXACT, 0, nullptr, true, &words);
+        prepare_impl(g, req_slots, token_indices, cu_tokens, num_reqs, PSI_CAPACITY_EXACT, 0, nullptr, true, &words, false, handicap);
         const uint64_t padded_words = (words + 3) / 4 * 4;
         void* staging_dev = nullptr;
         const bool plan_mapped = padded_words <= g->staging_words &&

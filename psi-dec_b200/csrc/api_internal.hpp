@@ -294,6 +294,12 @@ void run_attend(psi_gqa* g, const AttendParams& params);
 // and a merge launch of their own, ten to twenty microseconds (4 requests of 15,000 to 30,000 tokens, eight rows, 16/2 x 256:
 // 111 us a step in one launch, 124 in several).
 constexpr uint64_t kExchangeHandicap = 200;
+// The same per MiB of q + k + v for psi_gqa_step_host where it could read them in place: 18 us, the pull over the host link.
+// Of 25 such steps (8 to 128 requests of four to eight rows, 300 to 30,000 tokens, 40/8 and 32/8 heads x 128, 24/4 and 16/2
+// x 256, 1 to 8 MiB), timed on both, each takes the faster side or one within 5 us of it: 64 requests of eight rows on 1,500
+// to 3,000 tokens, 32/8 x 128, 360 us staged on the long-run kernel and 291 in place on the decode kernel; 32 on 1,024 to
+// 8,192, 24/4 x 256, 270 and 354.
+constexpr uint64_t kHostPullTiles = 165;
 // Deals a step's requests to the decode kernel and the chunk kernels (split_runs).
 bool split_requests(const psi_gqa* g, const RequestRuns& runs, const ChunkRule& rule, std::vector<uint32_t>& decode_reqs,
                     std::vector<uint32_t>& chunk_reqs);

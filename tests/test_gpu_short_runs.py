@@ -111,3 +111,21 @@ def test_unaligned_buffers_are_refused_before_anything_is_launched(engine, runs,
     s.ctx.sync()
     assert np.array_equal(checks.to_numpy_bits(s.out), good)
     s.close()
+
+
+# (first: the decode kernel in place beats the long-run kernel behind a pull of 6 MiB; second: the pull of 1.2 MiB is worth it)
+@pytest.mark.parametrize("heads,head_dim,contexts,long_run", [((32, 8), 128, [1500 + 23 * i for i in range(64)], False),
+                                                               ((16, 2), 256, [512 + 1050 * i for i in range(16)], True)])
+def test_host_steps_with_short_runs_take_the_long_run_kernel_where_it_saves_the_pull(heads, head_dim, contexts, long_run):
+    import torch
+    s = W.Session(W.Spec("host", pkg.BF16, *heads, head_dim, 16, contexts, [8] * len(contexts), seed=54))
+    assert s.gqa.plan_stats()["chunk_ctas"] > 0
+    host = [x.cpu().pin_memory() for x in (s.k, s.v, s.q)]
+    out = torch.zeros_like(host[2]).pin_memory()
+    before = checks.to_numpy_bits(s.arena)
+    s.gqa.step_host(s.pages, s.table, 0, *s.spec.batch(), *host, out)
+    assert (s.gqa.plan_stats()["chunk_ctas"] > 0) == long_run
+    assert np.array_equal(checks.to_numpy_bits(s.arena).reshape(-1), checks.expected_arena_after_append(s, before))
+    s.out.copy_(out.cuda())
+    checks.assert_attention_close(s)
+    s.close()
