@@ -314,10 +314,10 @@ PSI_API int32_t psi_plan_preview(uint32_t num_q_heads, uint32_t num_kv_heads, co
                                  uint32_t* out_counts);
 
 /* The work plan of the long-query (chunk) kernels for a batch in which EVERY request carries a long run, computed on
- * the host.  equal_shares selects the plan for working sets that stay in L2 (contiguous shares of equal size) instead
- * of stream order.  out_items receives 10 u32 per item {request, kv head, flat token begin, tokens, kv_begin, kv_end,
- * partial slot or 0xFFFFFFFF, pieces of its unit, first slot of the unit, first arrival counter of the unit};
- * out_cta_item_begin num_ctas+1 entries; out_counts {items, ctas, partial slots, arrival counters, total 16-token KV
+ * the host.  equal_shares selects contiguous shares of equal size instead of stream order; the third order psi_gqa_prepare
+ * knows (whole units, longest first) and its cost per unit are not previewed.  out_items receives 10 u32 per item
+ * {request, kv head, flat token begin, tokens, kv_begin, kv_end, partial slot or 0xFFFFFFFF, pieces of its unit, first
+ * slot of the unit, first arrival counter of the unit}; out_cta_item_begin num_ctas+1 entries; out_counts {items, ctas, partial slots, arrival counters, total 16-token KV
  * tiles (saturated)}.  No reference counterpart. */
 PSI_API int32_t psi_chunk_plan_preview(uint32_t num_q_heads, uint32_t num_kv_heads, const uint32_t* token_indices,
                                        const uint32_t* cu_tokens, uint32_t num_reqs, uint32_t max_ctas,
@@ -369,7 +369,11 @@ PSI_API int32_t psi_gqa_metadata_write(psi_gqa* gqa, uint32_t which, uint64_t of
  * slots, out[3]=reduce units, out[4]=exec q tiles, out[5]=kernel (1 generic, 2 mma), out[6]=total 16-token KV tiles,
  * out[7]=rows per q tile, out[8]=CTAs of the long-query (chunk) kernel, out[9]=its work items, out[10]=launches of
  * the tcgen05 chunk kernel since the object was created, out[11]=launches of the mma.sync chunk kernel (the fallback
- * when PSI_KERNEL_MMA_SYNC asks for it or the page arena cannot be described to the TMA unit). */
+ * when PSI_KERNEL_MMA_SYNC asks for it or the page arena cannot be described to the TMA unit).
+ * A batch with adjacent one-token requests of one slot at one position (draft rows) has two plans: these figures describe
+ * the one with a row per request, which the fused append launches take; launches that read this step's K/V from their
+ * pages (psi_gqa_attend, psi_gqa_attend_partial) take the one with those rows merged.  Under a replay reservation there is
+ * the merged plan alone. */
 PSI_API int32_t psi_gqa_plan_stats(psi_gqa* gqa, uint32_t* out, uint32_t n);
 
 /* KV append: GQAKVPageWrite::invoke_bucketed (crates/inference-backend-metal/src/components/gqa_kv_page_write.rs:

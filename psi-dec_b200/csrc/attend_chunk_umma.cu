@@ -104,9 +104,6 @@ __device__ __forceinline__ void tmem_store32(uint32_t taddr, const float (&v)[32
 
 __device__ __forceinline__ void tmem_store_wait() { asm volatile("tcgen05.wait::st.sync.aligned;\n" ::: "memory"); }
 
-
-
-
 __device__ __forceinline__ void row_threads_sync() { asm volatile("bar.sync 1, 128;" ::: "memory"); }
 
 // Executed by a whole converged warp; one elected lane (always the same one for a full warp) issues.

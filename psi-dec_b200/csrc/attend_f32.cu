@@ -12,12 +12,12 @@
 //   softmax  online, in the log2 domain, on those scores; O is rescaled only when a row's maximum moved;
 //   values   lane = four (or two times four) columns of every row; the weights are read back as broadcasts.
 // The row count is rounded up to 4, 8 or 16 per item, each with code of its own.  All arithmetic is f32.
-// Measured: 16 requests of 4,096 to 12,288 tokens, 32/8 heads x 128 (1.07 GB), a whole step with append and reduce 226 us
-// = 4.75 TB/s, against 517 us with the staged kernel, whose shared-memory traffic grows with every row.
+// Measured: 16 requests of 4,096 to 12,288 tokens, 32/8 heads x 128 (1.07 GB), a whole step with append and reduce 222 us
+// = 4.8 TB/s, against 517 us with the staged kernel, whose shared-memory traffic grows with every row.
 #include <atomic>
 
-#include "device_common.cuh"
 #include "launch_util.hpp"
+#include "mma_common.cuh"
 
 namespace psi {
 
@@ -26,15 +26,6 @@ namespace {
 constexpr int kF32Warps = 8;
 constexpr int kF32Threads = kF32Warps * 32;
 constexpr uint32_t kF32Tile = 8;  // KV tokens per tile
-
-__device__ __forceinline__ void f32_cp_async_16(uint32_t dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void f32_cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void f32_cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
 
 // Shared memory: q [16][D] | weights [warp][16][8] | ring [warp][NSLOT][8][D], which the merge of the warps reuses as
 // [warp][16][D].
@@ -86,7 +77,7 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
             const uint32_t bytes = t < in_range ? 16u : 0u;  // rows beyond the item are zero
 #pragma unroll
             for (uint32_t g = 0; g < uint32_t(DG); ++g)
-                if (lane + 32 * g < c4) f32_cp_async_16(dst + t * D * 4 + g * 512, src + g * 128, bytes);
+                if (lane + 32 * g < c4) cp_async_16(dst + t * D * 4 + g * 512, src + g * 128, bytes);
         }
     };
 
@@ -102,7 +93,7 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
                 if ((h >> 1) + 2 < my_tiles) next = lookup((h >> 1) + 2);
             }
         }
-        f32_cp_async_commit();
+        cp_async_commit();
     }
 
     // lane roles: scores of tokens pair and pair + 4 over the chunks eighth, eighth + 8, ... of a row; afterwards the
@@ -124,7 +115,7 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
         for (int g = 0; g < DG; ++g) o[r][g] = make_float4(0.f, 0.f, 0.f, 0.f);
 
     for (uint32_t h = 0; h < my_halves; ++h) {
-        f32_cp_async_wait<NSLOT - 2>();
+        cp_async_wait<NSLOT - 2>();
         __syncwarp();
         const uint32_t ahead = h + NSLOT - 1;
         if (ahead < my_halves) {
@@ -134,7 +125,7 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
                 if ((ahead >> 1) + 2 < my_tiles) next = lookup((ahead >> 1) + 2);
             }
         }
-        f32_cp_async_commit();
+        cp_async_commit();
         const float* tile = my_ring + (h % NSLOT) * (kF32Tile * D);
         if ((h & 1) == 0) {
             float s[2][R];
@@ -257,7 +248,7 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
             __syncwarp();  // the weights may be overwritten
         }
     }
-    f32_cp_async_wait<0>();
+    cp_async_wait<0>();
     __syncthreads();  // every warp is done with its ring: the merge area may overwrite it
     float* mine = reinterpret_cast<float*>(ring) + warp * kMaxRows * D;
 #pragma unroll
@@ -294,11 +285,11 @@ __global__ void __launch_bounds__(kF32Threads, 1) attend_f32_kernel(AttendParams
             const uint32_t r = i / c4, c = i % c4;
             const bool present = r < v.rows;
             const float* src = static_cast<const float*>(p.q) + (present ? item_row_index(p, v, r) * D + 4 * c : 0);
-            f32_cp_async_16(q_base + i * 16, src, present ? 16u : 0u);
+            cp_async_16(q_base + i * 16, src, present ? 16u : 0u);
         }
         if (tid < kMaxRows) shared.limit[tid] = tid < v.rows ? item_row_limit(v, tid) : 0u;
-        f32_cp_async_commit();
-        f32_cp_async_wait<0>();
+        cp_async_commit();
+        cp_async_wait<0>();
         __syncthreads();
         if (v.rows <= 4) f32_item<4, DG, NSLOT>(p, v, f32_smem, shared);
         else if (v.rows <= 8) f32_item<8, DG, NSLOT>(p, v, f32_smem, shared);

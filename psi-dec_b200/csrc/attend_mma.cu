@@ -52,9 +52,9 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
     constexpr uint32_t kBlocks = D / 64;                     // 128-byte element blocks per row (TMA box layout)
     constexpr uint32_t kChunks = D / 8;                      // 16-byte chunks per row
     constexpr uint32_t kRowsPerCopy = 32 / (kChunks < 32 ? kChunks : 32);
-    // Tiles per warp fetched into the L2 before the launch's inputs are there.  Two (4 to 16 KiB a warp, at most 38 MB over
+    // Tiles per warp fetched into the L2 before the launch's inputs are there.  Two (8 to 32 KiB a warp, at most 38 MB over
     // the device): 32 requests of 1,024 to 8,192 tokens, 16/2 heads x 256, four layers, 239 us with none, 228 with one or
-    // two, 242 with four, 249 with eight; four requests of 262,144 tokens 346, 343, 339, 341 and 344 us.
+    // two, 242 with four, 249 with eight; no difference for four requests of 262,144 tokens (339 to 346 us).
     constexpr uint32_t kAheadTiles = 2;
 
     const uint32_t cta = blockIdx.x;

@@ -185,7 +185,7 @@ struct Eight {
 // steps.  Measured: 4,667 prompt tokens of 24/4 heads x 256 with gates (267 MB) 71 us = 3.8 TB/s, against 133 us with a
 // warp per row and one element per lane; a decode step of 32 tokens 5.2 us against 7.5 us.
 constexpr int kHeld = 4;
-constexpr uint64_t kRowsResidentCtas = 148 * 4;
+constexpr uint64_t kRowsResidentCtas = 148 * 4;  // of the 16-bit instantiations (three an SM in f32, whose steps are short)
 
 template <uint32_t DTYPE, int LPR>
 __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 4) norm_rope_rows_kernel(PrepParams p) {
