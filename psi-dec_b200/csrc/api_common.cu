@@ -119,6 +119,7 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
         p.new_v = nullptr;
     }
     const uint32_t num_ctas = fixed ? g->grid_cap : plan.num_ctas();
+    p.item_tiles = fixed || plan.items.empty() ? 0u : static_cast<uint32_t>(std::min<uint64_t>(plan.total_kv_tiles / plan.items.size(), kU32Max));
     if (num_ctas > 0) {
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_MAP);
         if (g->kernel == PSI_KERNEL_MMA) {
@@ -148,9 +149,9 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
         }
         cuda_check(launched, "attend (chunk) launch");
     }
-    // The mma kernel merges a unit's partials in the CTA that delivers the last one; the generic kernel needs the
-    // separate reduce pass.
-    const uint32_t num_reduces = g->kernel == PSI_KERNEL_MMA
+    // The tensor-core and the f32 kernels merge a unit's partials in the CTA that delivers the last one; the other CUDA-core
+    // kernels need the separate reduce pass.
+    const uint32_t num_reduces = g->kernel == PSI_KERNEL_MMA || attend_generic_merges(p)
                                      ? 0u
                                      : static_cast<uint32_t>(fixed ? g->cap_reduces : plan.reduces.size());
     if (num_reduces > 0) {

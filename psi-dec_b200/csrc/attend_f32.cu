@@ -2,8 +2,8 @@
 //
 // Same work items, partial slots and reduce pass as the other CUDA-core map kernels (attend_generic.cu); head_dim must be
 // a multiple of 32.  Bound by HBM: a K and a V row of 2 * 4 * D bytes feed at most 16 query rows, 2 to 8 flop/B, so f32
-// FMAs keep up as long as shared memory does.  One CTA of eight warps per SM; every warp owns every eighth 8-token tile of
-// the item and streams it through a ring of its own (K tile, V tile, K tile, ...) by 16-byte cp.async, so there is no
+// FMAs keep up as long as shared memory does.  One CTA of eight warps per SM (twelve for long items up to head_dim 128,
+// kLongItemTiles); every warp owns every eighth (twelfth) 8-token tile of the item and streams it through a ring of its own (K tile, V tile, K tile, ...) by 16-byte cp.async, so there is no
 // CTA-wide barrier between the start and the end of an item.  Per tile:
 //   scores   lane = (token pair, eighth of the row): two tokens per lane halve the reads of q, which are the larger part
 //            of the shared-memory traffic; eight lanes read 128 consecutive bytes, so no access has a bank conflict.  The
@@ -12,43 +12,47 @@
 //   softmax  online, in the log2 domain, on those scores; O is rescaled only when a row's maximum moved;
 //   values   lane = four (or two times four) columns of every row; the weights are read back as broadcasts.
 // The row count is rounded up to 4, 8 or 16 per item, each with code of its own.  All arithmetic is f32.
-// Measured: 16 requests of 4,096 to 12,288 tokens, 32/8 heads x 128 (1.07 GB), a whole step with append and reduce 222 us
-// = 4.8 TB/s, against 517 us with the staged kernel, whose shared-memory traffic grows with every row.
+// Cut units are merged by the CTA that delivers their last partial, and each warp's first two tiles are requested into the L2
+// while the append runs.  Measured: 16 requests of 4,096 to 12,288 tokens, 32/8 heads x 128 (1.07 GB), a whole step with the
+// append 190 us = 5.6 TB/s; 210 with eight warps and six ring slots each, whose issue slots were half idle with two warps a
+// scheduler (map launch 194 us; 172 with twelve and four slots, 178 with sixteen and three), 517 with the staged kernel,
+// whose shared-memory traffic grows with every row.
 #include <atomic>
 
 #include "launch_util.hpp"
 #include "mma_common.cuh"
+#include "unit_merge.cuh"
 
 namespace psi {
 
 namespace {
 
-constexpr int kF32Warps = 8;
-constexpr int kF32Threads = kF32Warps * 32;
 constexpr uint32_t kF32Tile = 8;  // KV tokens per tile
 
 // Shared memory: q [16][D] | weights [warp][16][8] | ring [warp][NSLOT][8][D], which the merge of the warps reuses as
 // [warp][16][D].
-__host__ __device__ constexpr uint32_t f32_ring_offset(uint32_t d) { return (kMaxRows * d + kF32Warps * kMaxRows * kF32Tile) * 4; }
-__host__ __device__ constexpr uint32_t f32_smem_bytes(uint32_t d, uint32_t slots) {
-    return f32_ring_offset(d) + kF32Warps * (slots * kF32Tile > kMaxRows ? slots * kF32Tile : kMaxRows) * d * 4;
+__host__ __device__ constexpr uint32_t f32_ring_offset(uint32_t d, uint32_t warps) { return (kMaxRows * d + warps * kMaxRows * kF32Tile) * 4; }
+__host__ __device__ constexpr uint32_t f32_smem_bytes(uint32_t d, uint32_t slots, uint32_t warps) {
+    return f32_ring_offset(d, warps) + warps * (slots * kF32Tile > kMaxRows ? slots * kF32Tile : kMaxRows) * d * 4;
 }
 
+template <int W>
 struct F32Shared {
-    float m[kF32Warps][kMaxRows];
-    float l[kF32Warps][kMaxRows];
+    float m[W][kMaxRows];
+    float l[W][kMaxRows];
     uint32_t limit[kMaxRows];
+    uint32_t arrival;
 };
 
 // One warp's share of an item with at most R rows; leaves the warp's (O, m, l) in the merge area and `shared`.
 // DG = float4 columns per lane (head_dim <= 128 DG).
-template <int R, int DG, int NSLOT>
-__device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& v, unsigned char* smem, F32Shared& shared) {
+template <int R, int DG, int NSLOT, int W>
+__device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& v, unsigned char* smem, F32Shared<W>& shared) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t D = p.geo.head_dim, c4 = D / 4;
     const float* q_s = reinterpret_cast<const float*>(smem);
     float* weight_s = reinterpret_cast<float*>(smem) + kMaxRows * D + warp * (kMaxRows * kF32Tile);
-    unsigned char* ring = smem + f32_ring_offset(D);
+    unsigned char* ring = smem + f32_ring_offset(D, W);
     const uint32_t tile_bytes = kF32Tile * D * 4;
     float* my_ring = reinterpret_cast<float*>(ring + warp * NSLOT * tile_bytes);
     const uint32_t my_ring_u32 = static_cast<uint32_t>(__cvta_generic_to_shared(my_ring));
@@ -58,9 +62,9 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
 
     const uint32_t first_tile = v.kv_begin / kF32Tile;
     const uint32_t item_tiles = (v.kv_end + kF32Tile - 1) / kF32Tile - first_tile;
-    const uint32_t my_tiles = item_tiles > warp ? (item_tiles - warp + kF32Warps - 1) / kF32Warps : 0;
+    const uint32_t my_tiles = item_tiles > warp ? (item_tiles - warp + W - 1) / W : 0;
     const uint32_t my_halves = 2 * my_tiles;
-    auto token_of = [&](uint32_t j) { return (first_tile + warp + j * kF32Warps) * kF32Tile; };
+    auto token_of = [&](uint32_t j) { return (first_tile + warp + j * W) * kF32Tile; };
     // element offset of the K row of token `lane & 7` of local tile j (beyond the range: the last row, which is not read)
     auto lookup = [&](uint32_t j) {
         const uint32_t at = min(token_of(j) + (lane & 7u), v.kv_end - 1);
@@ -268,20 +272,59 @@ __device__ __forceinline__ void f32_item(const AttendParams& p, const ItemView& 
     }
 }
 
-template <int DG, int NSLOT>
-__global__ void __launch_bounds__(kF32Threads, 1) attend_f32_kernel(AttendParams p) {
+template <int DG, int NSLOT, int W>
+__global__ void __launch_bounds__(W * 32, 1) attend_f32_kernel(AttendParams p) {
     const uint32_t cta = blockIdx.x;
-    await_previous_kernel();
-    if (cta >= p.scalars[kScalarNumCtas]) return;
+    // plan and page table are read before the wait for the inputs
+    const bool early = p.plan_ready != 0 && p.geo.table_settled != 0;
+    if (!early) await_previous_kernel();
+    uint32_t item_begin = 0, item_end = 0;
+    if (cta < p.scalars[kScalarNumCtas]) {
+        item_begin = p.cta_item_begin[cta];
+        item_end = p.cta_item_begin[cta + 1];
+    }
+    if (item_begin >= item_end) {
+        if (early) await_previous_kernel();
+        return;
+    }
     extern __shared__ __align__(128) unsigned char f32_smem[];
-    __shared__ F32Shared shared;
+    __shared__ F32Shared<W> shared;
     const uint32_t tid = threadIdx.x, D = p.geo.head_dim, c4 = D / 4;
     const uint32_t q_base = static_cast<uint32_t>(__cvta_generic_to_shared(f32_smem));
 
-    for (uint32_t index = p.cta_item_begin[cta]; index < p.cta_item_begin[cta + 1]; ++index) {
+    // columns [d, d + 4) of a finished row
+    auto store_row = [&](const ItemView& v, uint32_t r, uint32_t d, float4 value, float top, float sum) {
+        const uint64_t row = item_row_index(p, v, r), at = row * D + d;
+        if (p.ext_o != nullptr) {
+            *reinterpret_cast<float4*>(p.ext_o + at) = value;
+            if (d == 0) {
+                p.ext_m[row] = top * kLn2;
+                p.ext_l[row] = sum;
+            }
+            return;
+        }
+        float* out = static_cast<float*>(p.out) + at;
+        out[0] = value.x * gate_factor(p, at);
+        out[1] = value.y * gate_factor(p, at + 1);
+        out[2] = value.z * gate_factor(p, at + 2);
+        out[3] = value.w * gate_factor(p, at + 3);
+    };
+    for (uint32_t index = item_begin; index < item_end; ++index) {
         const ItemView v = view_item(p, index);
+        if (early && index == item_begin) {
+            // While the previous kernel finishes, each warp's first two tiles go into the L2: a lane takes the K or V row of one token.
+            const uint32_t lane = tid & 31u, tile = v.kv_begin / kF32Tile + (tid >> 5) + (lane >> 4) * W;
+            const uint32_t at = tile * kF32Tile + (lane & 7u);
+            if (at < v.kv_end) {
+                const uint32_t page_id = page_id_or_zero(p.geo, table_row(p.geo, v.req_slot), at / p.geo.tokens_per_page);
+                const float* row = static_cast<const float*>(p.geo.pages) +
+                                   kv_row_offset(p.geo, page_id, v.kv_head, at % p.geo.tokens_per_page) + (lane & 8u ? v_region_offset(p.geo) : 0);
+                for (uint32_t d = 0; d < D; d += 32) prefetch_l2(row + d);
+            }
+            await_previous_kernel();
+        }
         __syncthreads();  // the previous item's merge is done with the ring and the statistics
-        for (uint32_t i = tid; i < kMaxRows * c4; i += kF32Threads) {  // query rows, zero beyond the item's
+        for (uint32_t i = tid; i < kMaxRows * c4; i += W * 32) {  // query rows, zero beyond the item's
             const uint32_t r = i / c4, c = i % c4;
             const bool present = r < v.rows;
             const float* src = static_cast<const float*>(p.q) + (present ? item_row_index(p, v, r) * D + 4 * c : 0);
@@ -291,21 +334,21 @@ __global__ void __launch_bounds__(kF32Threads, 1) attend_f32_kernel(AttendParams
         cp_async_commit();
         cp_async_wait<0>();
         __syncthreads();
-        if (v.rows <= 4) f32_item<4, DG, NSLOT>(p, v, f32_smem, shared);
-        else if (v.rows <= 8) f32_item<8, DG, NSLOT>(p, v, f32_smem, shared);
-        else f32_item<16, DG, NSLOT>(p, v, f32_smem, shared);
+        if (v.rows <= 4) f32_item<4, DG, NSLOT, W>(p, v, f32_smem, shared);
+        else if (v.rows <= 8) f32_item<8, DG, NSLOT, W>(p, v, f32_smem, shared);
+        else f32_item<16, DG, NSLOT, W>(p, v, f32_smem, shared);
         __syncthreads();
 
-        const float* merge = reinterpret_cast<const float*>(f32_smem + f32_ring_offset(D));
-        for (uint32_t i = tid; i < v.rows * c4; i += kF32Threads) {
+        const float* merge = reinterpret_cast<const float*>(f32_smem + f32_ring_offset(D, W));
+        for (uint32_t i = tid; i < v.rows * c4; i += W * 32) {
             const uint32_t r = i / c4, d = 4 * (i % c4);
             float top = -INFINITY;
 #pragma unroll
-            for (int w = 0; w < kF32Warps; ++w) top = fmaxf(top, shared.m[w][r]);
+            for (int w = 0; w < W; ++w) top = fmaxf(top, shared.m[w][r]);
             float sum = 0.0f;
             float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int w = 0; w < kF32Warps; ++w) {
+            for (int w = 0; w < W; ++w) {
                 const float weight = shared.m[w][r] == -INFINITY ? 0.0f : exp2f(shared.m[w][r] - top);
                 const float4 part = *reinterpret_cast<const float4*>(merge + (w * kMaxRows + r) * D + d);
                 sum += weight * shared.l[w][r];
@@ -316,7 +359,6 @@ __global__ void __launch_bounds__(kF32Threads, 1) attend_f32_kernel(AttendParams
             }
             const float inv = sum > 0.0f ? 1.0f / sum : 0.0f;
             const float4 value = make_float4(acc.x * inv, acc.y * inv, acc.z * inv, acc.w * inv);
-            const uint64_t row = item_row_index(p, v, r);
             if (v.partial_slot != kU32Max) {
                 const uint64_t prow = static_cast<uint64_t>(v.partial_slot) * kMaxRows + r;
                 *reinterpret_cast<float4*>(p.partial_o + prow * D + d) = value;
@@ -324,32 +366,29 @@ __global__ void __launch_bounds__(kF32Threads, 1) attend_f32_kernel(AttendParams
                     p.partial_m[prow] = top;
                     p.partial_l[prow] = sum;
                 }
-            } else if (p.ext_o != nullptr) {
-                *reinterpret_cast<float4*>(p.ext_o + row * D + d) = value;
-                if (d == 0) {
-                    p.ext_m[row] = top * kLn2;
-                    p.ext_l[row] = sum;
-                }
             } else {
-                const uint64_t at = row * D + d;
-                float* out = static_cast<float*>(p.out) + at;
-                out[0] = value.x * gate_factor(p, at);
-                out[1] = value.y * gate_factor(p, at + 1);
-                out[2] = value.z * gate_factor(p, at + 2);
-                out[3] = value.w * gate_factor(p, at + 3);
+                store_row(v, r, d, value, top, sum);
             }
+        }
+        if (v.partial_slot != kU32Max && delivers_last_partial(p, v, shared.arrival)) {
+            merge_unit<W * 32>(p, v, [&](uint32_t r, uint32_t d, float4 value, float top, float sum) { store_row(v, r, d, value, top, sum); });
         }
     }
 }
 
-template <int DG, int NSLOT>
+// Two warps a scheduler leave half of the issue slots empty; short items have no tiles for more.  40 requests, 32/8 heads x 128,
+// four layers: 406 us with twelve warps and 445 with eight at 1,600 tokens each, 179 and 184 at 400, 142 both at 200, 108 and
+// 105 at 100.
+constexpr uint32_t kLongItemTiles = 20;
+
+template <int DG, int NSLOT, int W>
 cudaError_t launch_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
-    auto kernel = attend_f32_kernel<DG, NSLOT>;
+    auto kernel = attend_f32_kernel<DG, NSLOT, W>;
     static std::atomic<uint64_t> configured{0};
     // the largest head_dim sets the limit once; smaller ones fit under it
-    cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(f32_smem_bytes(128 * DG, NSLOT)), configured);
+    cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(f32_smem_bytes(128 * DG, NSLOT, W)), configured);
     if (err != cudaSuccess) return err;
-    return launch_overlapped(kernel, num_ctas, kF32Threads, f32_smem_bytes(p.geo.head_dim, NSLOT), stream, p);
+    return launch_overlapped(kernel, num_ctas, W * 32, f32_smem_bytes(p.geo.head_dim, NSLOT, W), stream, p);
 }
 
 }  // namespace
@@ -365,7 +404,8 @@ bool attend_f32_supported(const AttendParams& p) {
 
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     if (num_ctas == 0) return cudaSuccess;
-    return p.geo.head_dim <= 128 ? launch_f32<1, 6>(p, num_ctas, stream) : launch_f32<2, 3>(p, num_ctas, stream);
+    if (p.geo.head_dim > 128) return launch_f32<2, 3, 8>(p, num_ctas, stream);
+    return p.item_tiles >= kLongItemTiles ? launch_f32<1, 4, 12>(p, num_ctas, stream) : launch_f32<1, 6, 8>(p, num_ctas, stream);
 }
 
 }  // namespace psi

@@ -457,6 +457,8 @@ uint32_t attend_generic_ctas_per_sm(uint32_t head_dim, uint32_t dtype) {
     return head_dim % 4 == 0 ? attend_staged_ctas_per_sm(dtype) : 8u;
 }
 
+bool attend_generic_merges(const AttendParams& p) { return p.generic_only == 0 && (attend_mma_any_supported(p) || attend_f32_supported(p)); }
+
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     if (num_ctas == 0) return cudaSuccess;
     if (p.generic_only == 0) {

@@ -4,8 +4,8 @@
 // one (q tile, KV head) - the tokens of the tile times the heads of the GQA group, at most 16 rows - against a range
 // of KV tokens, so every KV byte of the step is read from HBM exactly once.
 //
-// Inside a CTA each of the eight warps owns every eighth 16-token KV tile of the item and streams it through its own
-// ring of shared-memory slots (K tile, V tile, K tile, ...) with 16-byte cp.async copies (a warp-wide copy covers 512
+// Inside a CTA each of the eight warps (twelve for long items at head_dim 64) owns every eighth 16-token KV tile of the item and streams it
+// through its own ring of shared-memory slots (K tile, V tile, K tile, ...) with 16-byte cp.async copies (a warp-wide copy covers 512
 // contiguous bytes of one page), so the steady state has no CTA-wide barrier: a warp waits only for its own oldest
 // slot, and two warps per scheduler hide each other's instruction latencies.  The 16 query rows are one m16 MMA
 // tile: S = Q K^T and O += P V run as mma.sync.m16n8k16 with f32 accumulators, operands fetched by ldmatrix from
@@ -26,7 +26,7 @@ namespace psi {
 
 namespace {
 
-template <int D, int NSLOT>
+template <int D, int NSLOT, int kWarps>
 struct SmemLayout {
     static constexpr uint32_t kRowBytes = D * 2;
     static constexpr uint32_t kTileBytes = kTile * kRowBytes;        // one K or V tile = one ring slot
@@ -45,10 +45,11 @@ struct SmemLayout {
 // kTma: whole K/V tiles come from their pages as TMA boxes (cp.async.bulk.tensor, one instruction per 16-token tile
 // and warp, completion on one mbarrier per ring slot) instead of 16-byte cp.async copies; the tiles then lie in the
 // box layout of tma_common.cuh.  An item's ragged last tile and this step's own rows still come by cp.async.
-template <typename T, int D, int NSLOT, bool kExchange, bool kTma>
-__global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p, const __grid_constant__ CUtensorMap kv_map,
+template <typename T, int D, int NSLOT, int kWarps, bool kExchange, bool kTma>
+__global__ void __launch_bounds__(kWarps * 32, 1) attend_mma_kernel(AttendParams p, const __grid_constant__ CUtensorMap kv_map,
                                                                 uint32_t box_rows) {
-    using L = SmemLayout<D, NSLOT>;
+    using L = SmemLayout<D, NSLOT, kWarps>;
+    constexpr int kThreads = kWarps * 32;
     constexpr uint32_t kBlocks = D / 64;                     // 128-byte element blocks per row (TMA box layout)
     constexpr uint32_t kChunks = D / 8;                      // 16-byte chunks per row
     constexpr uint32_t kRowsPerCopy = 32 / (kChunks < 32 ? kChunks : 32);
@@ -497,17 +498,25 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_kernel(AttendParams p,
     }
 }
 
+// A tile's chain of matrix fragments, softmax and copies does not shrink with head_dim, and at 64 two warps a scheduler left it
+// idle for two thirds of the time (issue slots 37 % busy, 41 us a layer for 23.5 us of bytes).  Steps of long items take twelve
+// warps there: 32 requests of 1,024 to 8,192 tokens, 16/4 heads x 64, four layers, 138 us a step, 151 with eight (141 with
+// sixteen and six slots).  Short items have no tiles for so many warps and pay for them when these meet: 40 requests of 1,600
+// tokens (32/8 heads, four layers) 144 us with twelve and 153 with eight, of 400 89 and 90, of 200 77 and 76, 52 of 25 to 139
+// under replay 114 and 106; the line is at kLongItemTiles KV tiles an item.  At 128 and 256 the accumulators leave no registers
+// for more than eight warps.
+constexpr uint32_t kLongItemTiles = 32;
 template <int D>
 constexpr int stages_for() {
     return D == 256 ? 3 : (D == 128 ? 6 : 8);  // ring slots (one K or V tile each) per warp
 }
 
-template <typename T, int D, bool kExchange, bool kTma>
+template <typename T, int D, int kWarps, bool kExchange, bool kTma>
 cudaError_t launch_one(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream, const CUtensorMap& map,
                        uint32_t box_rows) {
-    constexpr int NSLOT = stages_for<D>();
-    using L = SmemLayout<D, NSLOT>;
-    auto kernel = attend_mma_kernel<T, D, NSLOT, kExchange, kTma>;
+    constexpr int NSLOT = stages_for<D>(), kThreads = kWarps * 32;
+    using L = SmemLayout<D, NSLOT, kWarps>;
+    auto kernel = attend_mma_kernel<T, D, NSLOT, kWarps, kExchange, kTma>;
     static std::atomic<uint64_t> configured{0};  // per instantiation, one bit per device
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), static_cast<int>(L::kTotal), configured);
     if (err != cudaSuccess) return err;
@@ -526,17 +535,20 @@ cudaError_t launch_for_dim(const AttendParams& p, uint32_t num_ctas, cudaStream_
     if (tma) {
         if constexpr (!kExchange) {
             switch (p.geo.head_dim) {
-                case 64: return launch_one<T, 64, false, true>(p, num_ctas, stream, map, box_rows);
-                case 128: return launch_one<T, 128, false, true>(p, num_ctas, stream, map, box_rows);
-                case 256: return launch_one<T, 256, false, true>(p, num_ctas, stream, map, box_rows);
+                case 64: return launch_one<T, 64, 8, false, true>(p, num_ctas, stream, map, box_rows);
+                case 128: return launch_one<T, 128, 8, false, true>(p, num_ctas, stream, map, box_rows);
+                case 256: return launch_one<T, 256, 8, false, true>(p, num_ctas, stream, map, box_rows);
                 default: return cudaErrorInvalidValue;
             }
         }
     }
+    if constexpr (!kExchange) {
+        if (p.geo.head_dim == 64 && p.item_tiles >= kLongItemTiles) return launch_one<T, 64, 12, false, false>(p, num_ctas, stream, map, box_rows);
+    }
     switch (p.geo.head_dim) {
-        case 64: return launch_one<T, 64, kExchange, false>(p, num_ctas, stream, map, box_rows);
-        case 128: return launch_one<T, 128, kExchange, false>(p, num_ctas, stream, map, box_rows);
-        case 256: return launch_one<T, 256, kExchange, false>(p, num_ctas, stream, map, box_rows);
+        case 64: return launch_one<T, 64, 8, kExchange, false>(p, num_ctas, stream, map, box_rows);
+        case 128: return launch_one<T, 128, 8, kExchange, false>(p, num_ctas, stream, map, box_rows);
+        case 256: return launch_one<T, 256, 8, kExchange, false>(p, num_ctas, stream, map, box_rows);
         default: return cudaErrorInvalidValue;
     }
 }

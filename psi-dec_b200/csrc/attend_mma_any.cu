@@ -6,22 +6,26 @@
 // already and all accumulators are f32.  In bf16, which has f32's exponents, the parts add up to the weight exactly.  f16
 // ends at steps of 2^-24, so there the weights are taken 2^15 times as large (kWeightShift): exact down to 2^-16 of the
 // heaviest key of the warp, and within 2^-40 of it below that, where f32 sums over an item do not see it.  Bound by HBM; the
-// tensor pipe has room for the two extra products.  One CTA of eight warps per SM, every warp owning every eighth 16-token tile of the
-// item and a ring of its own (K tile, V tile, K tile, ...) fed by 16-byte cp.async, the next tile's page looked up one
+// tensor pipe has room for the two extra products.  One CTA of eight warps per SM (sixteen for long items up to head_dim 96,
+// kLongItemTiles), every warp owning every eighth (sixteenth) 16-token tile of the item and a ring of its own (K tile, V tile,
+// K tile, ...) fed by 16-byte cp.async, the next tile's page looked up one
 // tile ahead.  Rows are padded to DP elements plus one 16-byte chunk: an odd number of chunks per row keeps ldmatrix free
 // of bank conflicts without a swizzle, and the chunks beyond head_dim hold zeros.
-// Measured: 24 requests of 300 to 6,000 tokens, 24/8 heads x 96, pages of 12 (233 MB): 73 us = 3.2 TB/s, the
-// whole step with append and reduce 75 us where launches overlap, against 466 us on the staged kernel.
+// Cut units are merged by the CTA that delivers their last partial, and each warp's first two tiles are requested into the L2
+// while the append runs.  Measured: 24 requests of 300 to 6,000 tokens, 24/8 heads x 96, pages of 12 (233 MB): 72.7 us a
+// step with the append = 3.2 TB/s; 74.2 with eight warps and eight slots each, 79 against 75.7 with twelve and five, 75.0 with
+// the reduce as a launch of its own, 466 on the staged kernel.
 #include <atomic>
 
 #include "launch_util.hpp"
 #include "mma_common.cuh"
+#include "unit_merge.cuh"
 
 namespace psi {
 
 namespace {
 
-template <int DP, int NSLOT>
+template <int DP, int NSLOT, int kWarps>
 struct AnySmem {
     static constexpr uint32_t kStride = DP * 2 + 16;
     static constexpr uint32_t kTileBytes = kTile * kStride;
@@ -86,15 +90,27 @@ __device__ __forceinline__ void copy_16_by_elements(uint32_t dst, const void* sr
 // kAligned: the arena lies on a 16-byte boundary.  Off it, and for a q off it, elements are copied one by one: slower than
 // cp.async, but the plan is one CTA per SM for this kernel whatever the buffers of a launch, and the CUDA-core kernels
 // on such a plan took 1,037 us with an odd q for the step above (541 on a plan of their own; 85 here).
-template <typename T, int DP, int NSLOT, bool kAligned>
-__global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParams p) {
-    using L = AnySmem<DP, NSLOT>;
+template <typename T, int DP, int NSLOT, int kWarps, bool kAligned>
+__global__ void __launch_bounds__(kWarps * 32, 1) attend_mma_any_kernel(AttendParams p) {
+    using L = AnySmem<DP, NSLOT, kWarps>;
+    constexpr int kThreads = kWarps * 32;
     const uint32_t cta = blockIdx.x;
-    await_previous_kernel();
-    if (cta >= p.scalars[kScalarNumCtas]) return;
+    // plan and page table are read before the wait for the inputs
+    const bool early = p.plan_ready != 0 && p.geo.table_settled != 0;
+    if (!early) await_previous_kernel();
+    uint32_t item_begin = 0, item_end = 0;
+    if (cta < p.scalars[kScalarNumCtas]) {
+        item_begin = p.cta_item_begin[cta];
+        item_end = p.cta_item_begin[cta + 1];
+    }
+    if (item_begin >= item_end) {
+        if (early) await_previous_kernel();
+        return;
+    }
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ uint32_t limit_s[kTile];
     __shared__ float merge_m[kWarps][kTile], merge_l[kWarps][kTile];
+    __shared__ uint32_t arrival_s;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t D = p.geo.head_dim, chunks = D / 8;
@@ -119,8 +135,25 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
     // high parts alone, which have the weight's sign, and its infinities are written over what the first pass left.
     bool again = false;
     const bool wide_q = (reinterpret_cast<uintptr_t>(p.q) & 15u) == 0, wide_out = (reinterpret_cast<uintptr_t>(p.out) & 7u) == 0;
-    const uint32_t item_end = p.cta_item_begin[cta + 1];
-    for (uint32_t index = p.cta_item_begin[cta]; index < item_end;) {
+    // columns [d, d + 4) of a finished row
+    auto store_row = [&](const ItemView& v, uint32_t r, uint32_t d, float4 value, float top, float sum) {
+        const uint64_t row = item_row_index(p, v, r);
+        if (p.ext_o != nullptr) {
+            *reinterpret_cast<float4*>(p.ext_o + row * D + d) = value;
+            if (d == 0) {
+                p.ext_m[row] = top * kLn2;
+                p.ext_l[row] = sum;
+            }
+        } else if (wide_out) {
+            store_out4<T>(p, row * D + d, value);
+        } else {
+            const float x[4] = {value.x, value.y, value.z, value.w};
+#pragma unroll
+            for (uint32_t e = 0; e < 4; ++e) store_from_float(p.out, row * D + d + e, p.dtype, x[e] * gate_factor(p, row * D + d + e));
+        }
+    };
+    bool prefetched = !early;
+    for (uint32_t index = item_begin; index < item_end;) {
         const ItemView v = view_item(p, index);
         // (the previous item's merge is done with the ring, q and limit_s: the barrier at the end of this loop)
         bool not_finite = false;
@@ -150,6 +183,25 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
             }
         };
 
+        uint64_t cur = 0, next = 0;
+        if (my_tiles > 0) cur = lookup(0);
+        if (my_tiles > 1) next = lookup(1);
+        if (!prefetched) {
+            // While the previous kernel finishes, each warp's first two tiles go into the L2: a lane takes the K or V rows of a
+            // token of each.
+            prefetched = true;
+#pragma unroll
+            for (uint32_t t = 0; t < 2; ++t) {
+                const uint32_t at = token_of(t) + (lane & 15u);
+                if (t < my_tiles && at < v.kv_end) {
+                    const unsigned char* row = arena + (t == 0 ? cur : next) + (lane & 16u ? v_bytes : 0);
+                    for (uint32_t b = 0; b < D * 2; b += 128) prefetch_l2(row + b);
+                    prefetch_l2(row + D * 2 - 1);
+                }
+            }
+            await_previous_kernel();
+        }
+
         // query rows (zero beyond the item's) and the zero chunks beyond head_dim of the query tile and of this warp's ring
         // (the merge of the previous item wrote over them)
         for (uint32_t i = tid; i < kTile * (DP / 8); i += kThreads) {
@@ -167,9 +219,6 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
         if (tid < kTile) limit_s[tid] = tid < v.rows ? item_row_limit(v, tid) : v.kv_end;
         cp_async_commit();
 
-        uint64_t cur = 0, next = 0;
-        if (my_tiles > 0) cur = lookup(0);
-        if (my_tiles > 1) next = lookup(1);
 #pragma unroll
         for (uint32_t h = 0; h < NSLOT - 1; ++h) {
             if (h < my_halves) {
@@ -341,45 +390,45 @@ __global__ void __launch_bounds__(kThreads, 1) attend_mma_any_kernel(AttendParam
                 }
                 continue;
             }
-            const uint64_t row = item_row_index(p, v, r);
-            if (p.ext_o != nullptr) {
-                *reinterpret_cast<float4*>(p.ext_o + row * D + d) = value;
-                if (d == 0) {
-                    p.ext_m[row] = top * kLn2;
-                    p.ext_l[row] = sum;
-                }
-            } else if (wide_out) {
-                store_out4<T>(p, row * D + d, value);
-            } else {
-                const float x[4] = {value.x, value.y, value.z, value.w};
-#pragma unroll
-                for (uint32_t e = 0; e < 4; ++e) store_from_float(p.out, row * D + d + e, p.dtype, x[e] * gate_factor(p, row * D + d + e));
-            }
+            store_row(v, r, d, value, top, sum);
         }
         again = __syncthreads_or(not_finite && !again);
-        if (!again) ++index;
+        if (again) continue;
+        if (v.partial_slot != kU32Max && delivers_last_partial(p, v, arrival_s)) {
+            merge_unit<kThreads>(p, v, [&](uint32_t r, uint32_t d, float4 value, float top, float sum) { store_row(v, r, d, value, top, sum); });
+        }
+        ++index;
     }
 }
 
-template <typename T, int DP, int NSLOT, bool kAligned>
+template <typename T, int DP, int NSLOT, int kWarps, bool kAligned>
 cudaError_t launch_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
-    auto kernel = attend_mma_any_kernel<T, DP, NSLOT, kAligned>;
-    constexpr int kBytes = AnySmem<DP, NSLOT>::kTotal;
+    auto kernel = attend_mma_any_kernel<T, DP, NSLOT, kWarps, kAligned>;
+    constexpr int kBytes = AnySmem<DP, NSLOT, kWarps>::kTotal;
     static_assert(kBytes <= 220 * 1024, "query tile and ring share one CTA's shared memory");
     static std::atomic<uint64_t> configured{0};
     cudaError_t err = ensure_dynamic_smem(reinterpret_cast<const void*>(kernel), kBytes, configured);
     if (err != cudaSuccess) return err;
-    return launch_overlapped(kernel, num_ctas, kThreads, kBytes, stream, p);
+    return launch_overlapped(kernel, num_ctas, kWarps * 32, kBytes, stream, p);
 }
+
+// A tile is a chain of latencies, and two warps a scheduler leave 68 % of the issue slots empty; short items have no tiles for
+// more.  40 requests, 24/8 heads x 96, pages of 12, four layers: 227 us with sixteen warps and 242 with eight at 1,600 tokens each,
+// 165 both at 800, 124 and 120 at 400.  (Above 96 the accumulators leave registers for eight warps.)
+constexpr uint32_t kLongItemTiles = 64;
 
 template <typename T, bool kAligned>
 cudaError_t launch_for_dim(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     const uint32_t d = p.geo.head_dim;
-    if (d <= 64) return launch_any<T, 64, 8, kAligned>(p, num_ctas, stream);
-    if (d <= 96) return launch_any<T, 96, 8, kAligned>(p, num_ctas, stream);
-    if (d <= 128) return launch_any<T, 128, 6, kAligned>(p, num_ctas, stream);
-    if (d <= 192) return launch_any<T, 192, 4, kAligned>(p, num_ctas, stream);
-    return launch_any<T, 256, 3, kAligned>(p, num_ctas, stream);
+    if (p.item_tiles >= kLongItemTiles) {
+        if (d <= 64) return launch_any<T, 64, 5, 16, kAligned>(p, num_ctas, stream);
+        if (d <= 96) return launch_any<T, 96, 4, 16, kAligned>(p, num_ctas, stream);
+    }
+    if (d <= 64) return launch_any<T, 64, 8, 8, kAligned>(p, num_ctas, stream);
+    if (d <= 96) return launch_any<T, 96, 8, 8, kAligned>(p, num_ctas, stream);
+    if (d <= 128) return launch_any<T, 128, 6, 8, kAligned>(p, num_ctas, stream);
+    if (d <= 192) return launch_any<T, 192, 4, 8, kAligned>(p, num_ctas, stream);
+    return launch_any<T, 256, 3, 8, kAligned>(p, num_ctas, stream);
 }
 
 template <typename T>

@@ -214,12 +214,13 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         p.num_q_heads = c.num_q_heads;
         p.dtype = c.dtype;
         p.scale_log2 = c.scale * 1.4426950408889634f;
+        p.item_tiles = plan.items.empty() ? 0u : static_cast<uint32_t>(plan.total_kv_tiles / plan.items.size());
         p.generic_only = c.kernel_mode == PSI_KERNEL_GENERIC ? 1u : 0u;
         if (mma) {
             err = launch_attend_mma(p, plan.num_ctas(), stream);
         } else {
             err = launch_attend_generic(p, plan.num_ctas(), stream);
-            if (err == cudaSuccess) err = launch_attend_reduce(p, static_cast<uint32_t>(plan.reduces.size()), stream);
+            if (err == cudaSuccess && !attend_generic_merges(p)) err = launch_attend_reduce(p, static_cast<uint32_t>(plan.reduces.size()), stream);
         }
         if (err != cudaSuccess) {
             return fail(PSI_ERR_CUDA, std::string("attend launch: ") + cudaGetErrorString(err), error, error_len);

@@ -132,6 +132,7 @@ struct AttendParams {
     uint32_t plan_ready;          // the plan was in place before the stream's previous kernel started (no kernel copies it)
     uint32_t generic_only;        // generic launches: PSI_KERNEL_GENERIC asks for the staged kernels where faster ones exist
     uint32_t chunk_weights;       // ChunkWeights of a long-run launch (tcgen05 kernel)
+    uint32_t item_tiles;          // KV tiles of an item on average, 0 where that is not known (more warps for long items)
     uint32_t tma_feed;            // decode kernel: whole K/V tiles by TMA boxes instead of cp.async (PSI_KERNEL_MMA_TMA)
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none
 };
@@ -215,6 +216,9 @@ cudaError_t launch_attend_mma_any(const AttendParams& p, uint32_t num_ctas, cuda
 bool attend_f32_supported(const AttendParams& p);
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
+// Whether launch_attend_generic takes a kernel that merges cut units itself (attend_mma_any, attend_f32) instead of leaving
+// them to launch_attend_reduce.
+bool attend_generic_merges(const AttendParams& p);
 // KV tiles one item switch is worth when shares are balanced: decode kernel, attend_mma_any (24 requests of 300 to 6,000
 // tokens at head_dim 96: 91 us a step with 0, 77 with 16, 87 with 64; the f32 kernel is best with 0).
 constexpr uint32_t kMmaItemStartCost = 32, kMmaAnyItemStartCost = 16;
