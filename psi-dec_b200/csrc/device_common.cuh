@@ -162,13 +162,37 @@ __device__ __forceinline__ float gate_sigmoid(float x) {
     return x < 0.0f ? 1.0f - y : y;
 }
 
-// The same where few threads work out many gates.  The divisor lies in [1, 2], so a reciprocal of the special-function unit
-// and one Newton-Raphson step, r + r (1 - d r), take the division's place: its rounding error, without its range checks
-// (for every f32 in [1, 2] the division's own result).  Three prompts of 611 to 2,500 tokens, 24/4 heads x 256, two layers: 450 us a step, 650 with the division.
-__device__ __forceinline__ float gate_sigmoid_newton(float x) {
-    const float d = 1.0f + __expf(-fabsf(x)), r = __fdividef(1.0f, d);
-    const float y = fmaf(r, fmaf(-d, r, 1.0f), r);
-    return x < 0.0f ? 1.0f - y : y;
+// The same of N gates in place, where few threads work out many.  A divisor lies in [1, 2], so one reciprocal of the
+// special-function unit serves four of them (1 / a = b c d / (a b c d), a product of at most 16), and one Newton-Raphson
+// step each, r + r (1 - d r), takes the error of the approximation and the products away: what is left is the rounding.
+// A gate that is no number stays out of its neighbours' product and comes back in its own step.  There is no branch, so the
+// chains of latencies run side by side.
+template <int N>
+__device__ __forceinline__ void gate_sigmoids(float (&x)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+        float d[4], f[4], r[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float e;  // exp(-|x|); below the smallest normal value it is 0, which leaves d as it is
+            asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(-fabsf(x[i + k]) * 1.4426950408889634f));
+            d[k] = 1.0f + e;
+            f[k] = fminf(d[k], 2.0f);
+        }
+        const float ab = f[0] * f[1], cd = f[2] * f[3];
+        float inverse;
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inverse) : "f"(ab * cd));
+        const float inverse_ab = inverse * cd, inverse_cd = inverse * ab;
+        r[0] = inverse_ab * f[1];
+        r[1] = inverse_ab * f[0];
+        r[2] = inverse_cd * f[3];
+        r[3] = inverse_cd * f[2];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const float y = fmaf(r[k], fmaf(-d[k], r[k], 1.0f), r[k]);
+            x[i + k] = x[i + k] < 0.0f ? 1.0f - y : y;
+        }
+    }
 }
 
 __device__ __forceinline__ float warp_sum(float v) {

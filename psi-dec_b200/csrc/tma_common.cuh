@@ -17,6 +17,10 @@ constexpr uint32_t kMaxPolls = 200000;  // bound of every mbarrier wait (a try_w
 // (alignment, size, driver entry point missing).
 bool make_kv_map(const AttendParams& p, uint32_t box_rows, CUtensorMap* map);
 
+// The same memory as [8-row group of any page][K, V][element block][row in group][64 elements]: a box is the K and the V rows of
+// `box_rows / 8` consecutive groups, [group][K, V][element block]; its last coordinate is page * groups of a page + K group.
+bool make_kv_pair_map(const AttendParams& p, uint32_t box_rows, CUtensorMap* map);
+
 __device__ __forceinline__ uint32_t smem_u32(const void* ptr) { return static_cast<uint32_t>(__cvta_generic_to_shared(ptr)); }
 
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -71,6 +75,15 @@ __device__ __forceinline__ void tma_load_groups(uint32_t dst, const CUtensorMap*
         "{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
         "@e cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %4, %5}], [%2];\n\t}\n" ::"r"(dst),
         "l"(map), "r"(bar), "r"(0u), "r"(group), "r"(page)
+        : "memory");
+}
+
+// The same for make_kv_pair_map's boxes.
+__device__ __forceinline__ void tma_load_pair(uint32_t dst, const CUtensorMap* map, uint32_t bar, uint32_t group) {
+    asm volatile(
+        "{\n\t.reg .pred e;\n\telect.sync _|e, 0xFFFFFFFF;\n\t"
+        "@e cp.async.bulk.tensor.5d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %3, %3, %3, %4}], [%2];\n\t}\n" ::"r"(dst),
+        "l"(map), "r"(bar), "r"(0u), "r"(group)
         : "memory");
 }
 
