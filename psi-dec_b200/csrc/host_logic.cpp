@@ -598,32 +598,47 @@ ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, con
     if (l2_resident || order == ChunkOrder::kEqualShares) {
         // A working set that stays in L2 whatever the order: contiguous shares of equal cost, units cut where a share
         // ends (two or three pieces per cut unit instead of many), slivers below a quarter of the minimum piece folded
-        // into their neighbour.  A unit costs its KV tiles plus `unit_start_cost`, so that a share of many
-        // short units (the first tokens of a prompt) is not longer than one of a few long ones.
+        // into their neighbour.  Every item, a piece as well as a whole unit, costs its KV tiles plus `unit_start_cost`, so
+        // that a share of several short ones is not longer than a single long one.
         const uint64_t sliver = kChunkMinPieceTiles / 4;
+        // Cuts the units at the ends of `num_ctas` shares of `span`; the cost of all items.
+        auto cut = [&](uint64_t span, auto&& item) {
+            auto share_end = [&](uint64_t c) { return span * (c + 1) / num_ctas; };
+            uint64_t cursor = 0, end = share_end(0);
+            uint32_t cta = 0;
+            for (size_t k = 0; k < units.size(); ++k) {
+                const uint64_t unit_tiles = div_ceil(units[k].ctx_end, kKvTile);
+                uint64_t done = 0;
+                while (done < unit_tiles) {
+                    cursor += unit_start_cost;
+                    while (cta + 1 < num_ctas && cursor + (done == 0 ? sliver : 0) >= end) end = share_end(++cta);
+                    uint64_t take = std::min(unit_tiles - done, end > cursor ? end - cursor : 1);
+                    if (cta + 1 >= num_ctas || unit_tiles - done - take < sliver) take = unit_tiles - done;
+                    item(k, cta, done, done + take);
+                    done += take;
+                    cursor += take;
+                }
+            }
+            return cursor;
+        };
+        // How many units are cut depends on where the shares end: the smallest shares that hold all items, to within a
+        // quarter of an item's cost a share.
+        uint64_t span = total + uint64_t(unit_start_cost) * (units.size() + num_ctas);
+        if (unit_start_cost == 0) span = total;
+        for (uint64_t low = total + uint64_t(unit_start_cost) * units.size(); unit_start_cost > 0 && span - low > num_ctas * unit_start_cost / 4;) {
+            const uint64_t middle = (low + span) / 2;
+            if (cut(middle, [](size_t, uint32_t, uint64_t, uint64_t) {}) <= middle) span = middle;
+            else low = middle;
+        }
         plan.items.reserve(units.size() + num_ctas);
         std::vector<uint32_t> owner;  // CTA of every item, in item order
-        uint64_t cursor = 0;
-        uint32_t cta = 0;
-        const uint64_t span = total + uint64_t(unit_start_cost) * units.size();
-        auto share_end = [&](uint64_t c) { return span * (c + 1) / num_ctas; };
-        std::vector<std::pair<size_t, size_t>> unit_items;  // [first, last) item of every unit
-        for (const Unit& u : units) {
-            cursor += unit_start_cost;
-            const uint64_t unit_tiles = div_ceil(u.ctx_end, kKvTile);
-            const size_t first = plan.items.size();
-            uint64_t done = 0;
-            while (done < unit_tiles) {
-                while (cta + 1 < num_ctas && cursor + done + (done == 0 ? sliver : 0) >= share_end(cta)) ++cta;
-                uint64_t take = std::min(unit_tiles - done, std::max<uint64_t>(share_end(cta) - (cursor + done), 1));
-                if (cta + 1 >= num_ctas || unit_tiles - done - take < sliver) take = unit_tiles - done;
-                plan.items.push_back(make_item(u, done, done + take));
-                owner.push_back(cta);
-                done += take;
-            }
-            cursor += unit_tiles;
-            unit_items.emplace_back(first, plan.items.size());
-        }
+        std::vector<std::pair<size_t, size_t>> unit_items(units.size());  // [first, last) item of every unit
+        cut(span, [&](size_t k, uint32_t cta, uint64_t begin, uint64_t end) {
+            if (begin == 0) unit_items[k].first = plan.items.size();
+            plan.items.push_back(make_item(units[k], begin, end));
+            owner.push_back(cta);
+            unit_items[k].second = plan.items.size();
+        });
         for (const auto& range : unit_items) {
             std::vector<DeviceItem*> pieces;
             for (size_t i = range.first; i < range.second; ++i) pieces.push_back(&plan.items[i]);

@@ -216,7 +216,7 @@ constexpr uint32_t kChunkMinPieceTiles = 64;   // a KV piece of a cut unit is at
 constexpr uint32_t kChunkMaxPieces = 16;      // equal shares: a unit is cut into about this many pieces at most
 constexpr uint32_t kChunkWholeTokens = 2 * kChunkMinPieceTiles * 16;  // units of at most this many keys are not worth a cut
 constexpr uint32_t kChunkStartCostTiles = 8;   // fixed cost of a work item (query load, epilogue) in KV tiles, stream order
-constexpr uint32_t kChunkUnitCostTiles = 16;  // the same in the other orders (0 to 64 measured the same on whole units)
+constexpr uint32_t kChunkUnitCostTiles = 28;  // the same in the other orders (0 to 64 measured the same on whole units)
 
 // How the units of a chunk plan are dealt to CTAs.
 enum class ChunkOrder {
@@ -243,7 +243,7 @@ bool split_runs(const PlanGeometry& geo, const RequestRuns& runs, const ChunkRul
 // The order for the requests `split_runs` left to the chunk kernels.
 ChunkOrder chunk_order(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint64_t token_bytes);
 
-// Outside stream order a unit counts as its KV tiles plus `unit_start_cost`.
+// Outside stream order an item (a unit, or a piece of one) counts as its KV tiles plus `unit_start_cost`.
 ChunkPlan build_chunk_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, uint32_t max_ctas,
                            uint32_t slot_base, uint32_t counter_base, ChunkOrder order, uint32_t unit_start_cost = 0);
 
