@@ -108,6 +108,13 @@ __global__ void __launch_bounds__(kPrepWarps * 32) norm_rope_append_kernel(PrepP
     }
 }
 
+// 1 / sqrt(x): the device's own approximation and one Newton step, which leaves the last place of f32.  (A square root and a
+// division, each with its range checks, took a fifth of a row's instructions.)  At 0 and infinity the step has no meaning.
+__device__ __forceinline__ float inverse_root(float x) {
+    const float y = rsqrtf(x), e = fmaf(-x * y, y, 1.0f);
+    return isinf(y) || y == 0.0f ? y : fmaf(0.5f * y, e, y);
+}
+
 // Eight consecutive elements as a lane holds them.
 template <uint32_t DTYPE>
 struct Eight {
@@ -181,9 +188,11 @@ struct Eight {
 // per warp) and 16-byte aligned buffers.  A CTA works on rows of one token (blockIdx.x): the token's sines and cosines
 // are worked out once into shared memory instead of once per row, its page is looked up once, every lane moves 16 bytes
 // at a time, the 16-bit types are rounded and multiplied in pairs, and a warp has kHeld rows in flight.  blockIdx.y deals
-// the token's rows (q, k, v, gates) to CTAs.  Bound by issue slots on prompts (72 % of them) and by latency on decode
-// steps.  Measured: 4,667 prompt tokens of 24/4 heads x 256 with gates (267 MB) 71 us = 3.8 TB/s, against 133 us with a
-// warp per row and one element per lane; a decode step of 32 tokens 5.2 us against 7.5 us.
+// the token's rows (q, k, v, gates) to CTAs.  Bound by issue slots on prompts (three quarters of them) and by latency on
+// decode steps.  Measured: 4,667 prompt tokens of 24/4 heads x 256 with gates (267 MB) 63.5 us = 4.2 TB/s, 68 with a square
+// root, a division and 64-bit row offsets in every row, 133 with a warp per row and one element per lane (and 65.6 with the
+// rows' four sources chosen by selects in place of branches, 87 with a CTA for four tokens); a decode step of 32 tokens 5.2 us
+// against 7.5 us.
 constexpr int kHeld = 4;
 constexpr uint64_t kRowsResidentCtas = 148 * 4;  // of the 16-bit instantiations (three an SM in f32, whose steps are short)
 
@@ -204,12 +213,14 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
     const uint32_t first = (blockIdx.y * kPrepWarps + warp) * kRows + group;
     const uint32_t pos = p.flat_token_indices[token], slot = p.req_slots[token];
 
+    // (a token's rows lie within 2^32 elements of its first one: launch_rows looks)
+    const uint32_t q_step = static_cast<uint32_t>(p.q_head_stride);
+    const uint64_t q_row = token * p.q_token_stride + d0, kv_row = token * p.kv_token_stride + d0;
     auto fetch = [&](uint32_t row, Eight<DTYPE>& x) {
-        const uint64_t q_row = token * p.q_token_stride + d0, kv_row = token * p.kv_token_stride + d0;
-        if (row < hq) x.load(p.q_in, q_row + row * p.q_head_stride);
-        else if (row < hq + hkv) x.load(p.k_in, kv_row + static_cast<uint64_t>(row - hq) * D);
-        else if (row < hq + 2 * hkv) x.load(p.v_in, kv_row + static_cast<uint64_t>(row - hq - hkv) * D);
-        else if (row < num_rows) x.load(p.g_in, q_row + (row - hq - 2 * hkv) * p.q_head_stride);
+        if (row < hq) x.load(p.q_in, q_row + row * q_step);
+        else if (row < hq + hkv) x.load(p.k_in, kv_row + (row - hq) * D);
+        else if (row < hq + 2 * hkv) x.load(p.v_in, kv_row + (row - hq - hkv) * D);
+        else if (row < num_rows) x.load(p.g_in, q_row + (row - hq - 2 * hkv) * q_step);
     };
     // everything that needs only the plan, the table and the weights comes before the wait for the inputs
     Eight<DTYPE> q_weight, k_weight;  // the bf16 weights in T
@@ -243,6 +254,7 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
     const bool in_rope = sub < 2 * half_lanes, low = sub < half_lanes;
     const uint32_t partner = in_rope ? (low ? lane + half_lanes : lane - half_lanes) : lane;
     const float2* turns = turn_s + (low ? d0 : d0 - rope_half);
+    const uint32_t minus = !low ? 0u : (DTYPE == PSI_DTYPE_F32 ? 0x80000000u : 0x80008000u);  // x1 cos - x2 sin, x2 cos + x1 sin
 
     for (uint32_t base = first - group; base < num_rows; base += kHeld * stride) {
 #pragma unroll
@@ -259,12 +271,12 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
                 for (int j = 0; j < 8; ++j) acc += v[j] * v[j];
 #pragma unroll
                 for (int offset = LPR / 2; offset > 0; offset >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, offset);
-                const float inv_rms = 1.0f / sqrtf(acc / static_cast<float>(D) + p.eps);
+                const float inv_rms = inverse_root(acc / static_cast<float>(D) + p.eps);
                 Eight<DTYPE> n, other;
                 n.normalise(v, inv_rms, is_q ? q_weight : k_weight);
 #pragma unroll
                 for (int j = 0; j < Eight<DTYPE>::kWords; ++j)
-                    other.words()[j] = __shfl_sync(0xFFFFFFFFu, n.words()[j], partner);
+                    other.words()[j] = __shfl_sync(0xFFFFFFFFu, n.words()[j], partner) ^ minus;
                 if (in_rope) {
                     float mine[8], theirs[8];
                     n.widen(mine);
@@ -272,9 +284,12 @@ __global__ void __launch_bounds__(kPrepWarps * 32, DTYPE == PSI_DTYPE_F32 ? 3 : 
 #pragma unroll
                     for (int j = 0; j < 8; j += 2) {
                         const float4 turn = *reinterpret_cast<const float4*>(turns + j);  // two frequencies
-                        mine[j] = p.attention_factor * (low ? mine[j] * turn.x - theirs[j] * turn.y : theirs[j] * turn.y + mine[j] * turn.x);
-                        mine[j + 1] = p.attention_factor * (low ? mine[j + 1] * turn.z - theirs[j + 1] * turn.w
-                                                                : theirs[j + 1] * turn.w + mine[j + 1] * turn.z);
+                        mine[j] = theirs[j] * turn.y + mine[j] * turn.x;
+                        mine[j + 1] = theirs[j + 1] * turn.w + mine[j + 1] * turn.z;
+                    }
+                    if (p.attention_factor != 1.0f) {
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) mine[j] *= p.attention_factor;
                     }
                     n.narrow(mine);
                 }
@@ -310,7 +325,7 @@ bool launch_rows(const PrepParams& p, cudaStream_t stream, cudaError_t& status) 
     const uint64_t ctas = static_cast<uint64_t>(p.num_total_tokens) * ((rows + rows_per_cta - 1) / rows_per_cta);
     const uint32_t per_warp = static_cast<uint32_t>(ctas <= kRowsResidentCtas ? 1 : 8);
     const uint32_t split = (rows + rows_per_cta * per_warp - 1) / (rows_per_cta * per_warp);
-    if (split > 65535) return false;
+    if (split > 65535 || p.q_head_stride * p.num_q_heads > 0xFFFFFFFFull || uint64_t(p.geo.num_kv_heads) * d > 0xFFFFFFFFull) return false;
     const dim3 grid(p.num_total_tokens, split);
     auto kernel = d == 64 ? norm_rope_rows_kernel<DTYPE, 8> : (d == 128 ? norm_rope_rows_kernel<DTYPE, 16> : norm_rope_rows_kernel<DTYPE, 32>);
     status = launch_overlapped(kernel, grid, kPrepWarps * 32, 0, stream, p);
