@@ -25,8 +25,8 @@
 // gates, 3 without; 11 and 6 with one warpgroup), a cut one also the arrival (1.2 us) and for the last piece the merge (2.5
 // us; 4.6 when the eight tiles are merged one by one).  Prompts have many short items, so rows are packed (a group of six
 // fills 126 of 128 rows, not 96) and the plan deals whole units.  Three prompts of 611 to 2,500 tokens, 24/4 heads x 256,
-// gated, two layers: 404 us a step, 457 with one row warpgroup.  16 requests of 512 to 16,384 tokens, eight rows each, 40/8
-// heads x 128, two layers: 156 us, 172.
+// gated: 135 us a layer, 162 with one row warpgroup.  16 requests of 512 to 16,384 tokens, eight rows each, 40/8 heads x
+// 128: 72 us a layer, 80.
 // All hand-offs are mbarriers (TMA byte counts, tcgen05.commit, thread arrivals); every wait is bounded and reports
 // PSI_ERR_TIMEOUT through the status word instead of hanging, and the kernel frees its TMEM on every path.  The kernel
 // reads pages only: a step that appends and attends runs the append launch first.
@@ -233,8 +233,8 @@ constexpr float kRescaleThreshold = 8.0f;
 // tokens, 40/8 heads x 128: 1.6e-3 with one part, 1.3e-3 on the decode kernel, 8e-6 with two.  The high part is rounded down
 // and the low part holds the rest plus 2^-10 of the weight, so that both are positive wherever the weight is (an infinity in
 // V stays one instead of meeting 0 x Inf); every weight is then 1 + 2^-10 times itself, which the end of the item divides out.
-// Costs 5 to 12 % of such a step (16 requests of 512 to 16,384 tokens, eight rows each, 40/8 heads x 128, two layers: 164 us
-// with one part, 184 with two, 275 on the decode kernel).  Long runs keep one part, in code of their own: a branch on the
+// Costs 5 to 12 % of such a step (16 requests of 512 to 16,384 tokens, eight rows each, 40/8 heads x 128, two layers, with one
+// row warpgroup: 164 us with one part, 184 with two; 275 on the decode kernel).  Long runs keep one part, in code of their own: a branch on the
 // kind inside the MMA warp's loop alone cost them 3 %.
 constexpr float kFineScale = 1.0009765625f;
 static_assert(offsetof(DeviceItem, flat_begin) == 24 && offsetof(DeviceItem, num_tokens) == 28 && offsetof(DeviceItem, head0) == 40 &&

@@ -216,7 +216,10 @@ constexpr uint32_t kChunkMinPieceTiles = 64;   // a KV piece of a cut unit is at
 constexpr uint32_t kChunkMaxPieces = 16;      // equal shares: a unit is cut into about this many pieces at most
 constexpr uint32_t kChunkWholeTokens = 2 * kChunkMinPieceTiles * 16;  // units of at most this many keys are not worth a cut
 constexpr uint32_t kChunkStartCostTiles = 8;   // fixed cost of a work item (query load, epilogue) in KV tiles, stream order
-constexpr uint32_t kChunkUnitCostTiles = 28;  // the same in the other orders (0 to 64 measured the same on whole units)
+// The same in the other orders, for every piece of a unit: query rows, first tiles and epilogue, in the time of 16-token tiles
+// (about 7 us).  0 to 64 measured the same on whole units; with equal shares (16 requests of 512 to 16,384 tokens, eight rows
+// each, 40/8 heads x 128, pages of 8) a layer took 80.2 us with 16, 81.7 with 32, 93.7 with 48.
+constexpr uint32_t kChunkUnitCostTiles = 28;
 
 // How the units of a chunk plan are dealt to CTAs.
 enum class ChunkOrder {
