@@ -301,8 +301,8 @@ PSI_API int32_t psi_metadata_update_host(uint32_t max_tokens, const uint32_t* re
                                          uint32_t* buf_flat_token_indices, uint32_t* buf_q_token_tiles,
                                          uint32_t* buf_kv_splits, uint32_t* buf_cu_kv_splits,
                                          psi_replay_shape* out_shape);
-/* The balanced device work plan of a batch, computed on the host (what psi_gqa_prepare uploads in
- * PSI_PLAN_BALANCED).  out_items receives 6 u32 per item {q tile, head selection, kv_begin, kv_end, partial slot or
+/* The balanced device work plan of a batch, computed on the host (what psi_gqa_prepare uploads in PSI_PLAN_BALANCED
+ * unless every unit can be cut into equal pieces of one CTA each and that is cheaper).  out_items receives 6 u32 per item {q tile, head selection, kv_begin, kv_end, partial slot or
  * 0xFFFFFFFF, flat token begin of the tile}; out_cta_item_begin receives num_ctas+1 entries; out_counts receives
  * {items, ctas, partial slots, reduce units, q tiles, total 16-token KV tiles (saturated)}.  item_start_cost is the
  * number of KV tiles one additional item is charged when the shares are balanced.  No reference counterpart:

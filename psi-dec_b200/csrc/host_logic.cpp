@@ -322,7 +322,76 @@ void finish_plan(WorkPlan& plan) {
     }
 }
 
+// Lists the query tiles of `requests` and their contexts; the KV tiles of all units.
+uint64_t list_tiles(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests, WorkPlan& plan,
+                    std::vector<uint32_t>& tile_ctx) {
+    for (uint32_t r : requests) {
+        for (uint32_t begin = runs.cu_tokens[r]; begin < runs.cu_tokens[r + 1];) {
+            uint32_t end = std::min(runs.cu_tokens[r + 1], begin + geo.tokens_per_tile);
+            plan.tiles.push_back({begin, end, runs.req_slots[r], runs.position(r, begin), runs.token_indices[r],
+                                  runs.cu_tokens[r], runs.one_position(r)});
+            tile_ctx.push_back(runs.context(r, end));
+            begin = end;
+        }
+    }
+    uint64_t total = 0;
+    for (uint32_t ctx : tile_ctx) total += div_ceil(ctx, kKvTile) * geo.num_kv_heads * geo.head_tiles;
+    return plan.total_kv_tiles = total;
+}
+
 }  // namespace
+
+WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
+                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+    WorkPlan plan;
+    std::vector<uint32_t> tile_ctx;
+    const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
+    const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
+    const uint64_t units = uint64_t(plan.tiles.size()) * heads;
+    uint64_t pick = 0;
+    if (total != 0 && units <= max_ctas) {
+        // What an equal share costs, in KV tiles: whole rounds of the share itself (of as many CTAs as that plan would take) with
+        // a start for every unit, and a merge of pieces.
+        const uint64_t ctas = std::min<uint64_t>(max_ctas, std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta)));
+        const uint64_t share = (total + std::max(item_start_cost, kPieceStartTiles) * units) / ctas;
+        const uint64_t shares = div_ceil(share, kPieceRoundTiles) * kPieceRoundTiles + kPieceMergeTiles + kPieceGroupTiles;
+        const uint64_t longest = div_ceil(*std::max_element(tile_ctx.begin(), tile_ctx.end()), kKvTile);
+        uint64_t best = shares + 1;
+        // (a bound between two multiples of the round cuts the units as the smaller one does; one that is not below `best`
+        // leaves some unit a piece as long)
+        const uint64_t least = div_ceil(div_ceil(total, max_ctas), kPieceRoundTiles) * kPieceRoundTiles;
+        for (uint64_t bound = least; bound < best; bound += kPieceRoundTiles) {
+            uint64_t pieces = 0, cost = 0;
+            for (uint32_t ctx : tile_ctx) {
+                const uint64_t tiles = div_ceil(ctx, kKvTile), n = div_ceil(tiles, bound);
+                pieces += n * heads;
+                const uint64_t rounds = div_ceil(div_ceil(tiles, n), kPieceRoundTiles);
+                cost = std::max(cost, rounds * kPieceRoundTiles + (n > 1 ? kPieceMergeTiles + kPieceGroupTiles * div_ceil(n, 4) : 0));
+            }
+            if (pieces <= max_ctas && cost < best) best = cost, pick = bound;
+            if (bound >= longest) break;
+        }
+    }
+    if (pick == 0) return build_balanced_plan(geo, runs, requests, max_ctas, min_kv_tiles_per_cta, item_start_cost);
+    plan.items.reserve(max_ctas);
+    plan.cta_item_begin.assign(1, 0);
+    for (uint32_t tile = 0; tile < plan.tiles.size(); ++tile) {
+        const uint64_t tiles = div_ceil(tile_ctx[tile], kKvTile), n = div_ceil(tiles, pick);
+        for (uint32_t h = 0; h < heads; ++h) {
+            for (uint64_t k = 0; k < n; ++k) {
+                WorkItem item{};
+                item.tile = tile;
+                item.head_sel = h;
+                item.kv_begin = static_cast<uint32_t>(tiles * k / n * kKvTile);
+                item.kv_end = static_cast<uint32_t>(std::min<uint64_t>(tiles * (k + 1) / n * kKvTile, tile_ctx[tile]));
+                plan.items.push_back(item);
+                plan.cta_item_begin.push_back(static_cast<uint32_t>(plan.items.size()));
+            }
+        }
+    }
+    finish_plan(plan);
+    return plan;
+}
 
 WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
                              const uint32_t* cu_tokens, uint32_t num_reqs, uint32_t max_ctas,
@@ -337,19 +406,8 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, c
                              uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
     WorkPlan plan;
     std::vector<uint32_t> tile_ctx;
-    for (uint32_t r : requests) {
-        for (uint32_t begin = runs.cu_tokens[r]; begin < runs.cu_tokens[r + 1];) {
-            uint32_t end = std::min(runs.cu_tokens[r + 1], begin + geo.tokens_per_tile);
-            plan.tiles.push_back({begin, end, runs.req_slots[r], runs.position(r, begin), runs.token_indices[r],
-                                  runs.cu_tokens[r], runs.one_position(r)});
-            tile_ctx.push_back(runs.context(r, end));
-            begin = end;
-        }
-    }
+    const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
     const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
-    uint64_t total = 0;
-    for (uint32_t ctx : tile_ctx) total += div_ceil(ctx, kKvTile) * heads;
-    plan.total_kv_tiles = total;
     if (total == 0) return plan;
 
     uint64_t wanted = std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta));

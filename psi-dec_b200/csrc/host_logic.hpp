@@ -190,6 +190,23 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots,
 WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
                              uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost = 0);
 
+// The plan of the kernels that run one CTA of eight warps or more an SM.  Where every unit can be cut into equal pieces of one
+// CTA each, no CTA opens a second item, and pieces are whole rounds of a tile a warp: a step that does not fill the device is
+// then bounded by its longest piece and the merge, where an equal share may hold the ends of two units or many short ones.
+// The bound on a piece is the one with the smallest modelled cost, and the equal shares stay where theirs is smaller.  In KV
+// tiles (eight, a round of all warps: 1.08 us at head_dim 128): a cut unit pays 14 for arrival and merge and 4 for every four
+// pieces, which are merged at a time (fitted on one request of 100 to 8,000 tokens cut in every way: 2.5 us a merge, 0.6 us
+// four pieces).  Replayed steps, equal shares and pieces:
+//   one request of 777 tokens, 40/8 heads x 128, six layers: 75.9 and 64.6 us; of 100: 87.4 and 45.6; of 2,500: 82.2 and 77.1;
+//   four layers: 16 of 700 tokens 87.7 and 66.1; 8 of 1,000, 16/2 x 256, 76.7 and 64.0; 64 of 300 90.9 and 71.1; 16 of 1,000,
+//   32/8 x 64, 77.1 and 58.0; 24/8 x 96 102.9 and 84.3; f32 16/2 x 256 148.4 and 121.3; 16 of 4,000, 16/2 x 256, 126.4 and 125.5.
+//   (A start counts 16 tiles where the shares count less: f32.)
+// Unequal steps the model leaves to the shares: 32 of 1,000 to 8,000 tokens, 16/2 x 256, 175.2 and 186.6 us; 16 of 500 to
+// 4,000 87.1 and 88.8; f32, 16 of 300 to 2,000, 32/8 x 128, 164.1 and 194.2.
+constexpr uint32_t kPieceRoundTiles = 8, kPieceMergeTiles = 14, kPieceGroupTiles = 4, kPieceStartTiles = 16;
+WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
+                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost);
+
 // One CTA per (reference KV split, head_sel); reference q tiles wider than tokens_per_tile are cut into sub-tiles
 // that share the split boundaries.
 WorkPlan build_reference_plan(const PlanGeometry& geo, const ReferenceMetadata& md, const psi_replay_shape& shape,
