@@ -339,77 +339,10 @@ uint64_t list_tiles(const PlanGeometry& geo, const RequestRuns& runs, const std:
     return plan.total_kv_tiles = total;
 }
 
-}  // namespace
-
-WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
-                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
-    WorkPlan plan;
-    std::vector<uint32_t> tile_ctx;
-    const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
-    const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
-    const uint64_t units = uint64_t(plan.tiles.size()) * heads;
-    uint64_t pick = 0;
-    if (total != 0 && units <= max_ctas) {
-        // What an equal share costs, in KV tiles: whole rounds of the share itself (of as many CTAs as that plan would take) with
-        // a start for every unit, and a merge of pieces.
-        const uint64_t ctas = std::min<uint64_t>(max_ctas, std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta)));
-        const uint64_t share = (total + std::max(item_start_cost, kPieceStartTiles) * units) / ctas;
-        const uint64_t shares = div_ceil(share, kPieceRoundTiles) * kPieceRoundTiles + kPieceMergeTiles + kPieceGroupTiles;
-        const uint64_t longest = div_ceil(*std::max_element(tile_ctx.begin(), tile_ctx.end()), kKvTile);
-        uint64_t best = shares + 1;
-        // (a bound between two multiples of the round cuts the units as the smaller one does; one that is not below `best`
-        // leaves some unit a piece as long)
-        const uint64_t least = div_ceil(div_ceil(total, max_ctas), kPieceRoundTiles) * kPieceRoundTiles;
-        for (uint64_t bound = least; bound < best; bound += kPieceRoundTiles) {
-            uint64_t pieces = 0, cost = 0;
-            for (uint32_t ctx : tile_ctx) {
-                const uint64_t tiles = div_ceil(ctx, kKvTile), n = div_ceil(tiles, bound);
-                pieces += n * heads;
-                const uint64_t rounds = div_ceil(div_ceil(tiles, n), kPieceRoundTiles);
-                cost = std::max(cost, rounds * kPieceRoundTiles + (n > 1 ? kPieceMergeTiles + kPieceGroupTiles * div_ceil(n, 4) : 0));
-            }
-            if (pieces <= max_ctas && cost < best) best = cost, pick = bound;
-            if (bound >= longest) break;
-        }
-    }
-    if (pick == 0) return build_balanced_plan(geo, runs, requests, max_ctas, min_kv_tiles_per_cta, item_start_cost);
-    plan.items.reserve(max_ctas);
-    plan.cta_item_begin.assign(1, 0);
-    for (uint32_t tile = 0; tile < plan.tiles.size(); ++tile) {
-        const uint64_t tiles = div_ceil(tile_ctx[tile], kKvTile), n = div_ceil(tiles, pick);
-        for (uint32_t h = 0; h < heads; ++h) {
-            for (uint64_t k = 0; k < n; ++k) {
-                WorkItem item{};
-                item.tile = tile;
-                item.head_sel = h;
-                item.kv_begin = static_cast<uint32_t>(tiles * k / n * kKvTile);
-                item.kv_end = static_cast<uint32_t>(std::min<uint64_t>(tiles * (k + 1) / n * kKvTile, tile_ctx[tile]));
-                plan.items.push_back(item);
-                plan.cta_item_begin.push_back(static_cast<uint32_t>(plan.items.size()));
-            }
-        }
-    }
-    finish_plan(plan);
-    return plan;
-}
-
-WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
-                             const uint32_t* cu_tokens, uint32_t num_reqs, uint32_t max_ctas,
-                             uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
-    std::vector<uint32_t> all(num_reqs);
-    for (uint32_t r = 0; r < num_reqs; ++r) all[r] = r;
-    return build_balanced_plan(geo, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), all, max_ctas,
-                               min_kv_tiles_per_cta, item_start_cost);
-}
-
-WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
-                             uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
-    WorkPlan plan;
-    std::vector<uint32_t> tile_ctx;
-    const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
-    const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
-    if (total == 0) return plan;
-
+// Cuts the units of the plan's query tiles into equal shares (build_balanced_plan).
+void share_out(WorkPlan& plan, const std::vector<uint32_t>& tile_ctx, uint32_t heads, uint32_t max_ctas,
+               uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+    const uint64_t total = plan.total_kv_tiles;
     uint64_t wanted = std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta));
     const uint64_t num_ctas = std::min<uint64_t>(std::max(1u, max_ctas), wanted);
     // Every unit is laid out as `start_cost` virtual tiles (what opening a new item costs a CTA: pipeline drain,
@@ -449,6 +382,86 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, c
     }
     while (plan.cta_item_begin.size() < num_ctas + 1) plan.cta_item_begin.push_back(static_cast<uint32_t>(plan.items.size()));
     finish_plan(plan);
+}
+
+}  // namespace
+
+WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
+                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+    WorkPlan plan;
+    std::vector<uint32_t> tile_ctx;
+    const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
+    const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
+    const uint64_t units = uint64_t(plan.tiles.size()) * heads;
+    uint64_t pick = 0;
+    if (total != 0 && units <= max_ctas) {
+        // What an equal share costs, in KV tiles: whole rounds of the share itself (of as many CTAs as that plan would take) with
+        // a start for every unit, and a merge of pieces.
+        const uint64_t ctas = std::min<uint64_t>(max_ctas, std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta)));
+        const uint64_t share = (total + std::max(item_start_cost, kPieceStartTiles) * units) / ctas;
+        const uint64_t shares = div_ceil(share, kPieceRoundTiles) * kPieceRoundTiles + kPieceMergeTiles + kPieceGroupTiles;
+        const uint64_t longest = div_ceil(*std::max_element(tile_ctx.begin(), tile_ctx.end()), kKvTile);
+        uint64_t best = shares + 1;
+        // (a bound between two multiples of the round cuts the units as the smaller one does; one that is not below `best`
+        // leaves some unit a piece as long)
+        const uint64_t least = div_ceil(div_ceil(total, max_ctas), kPieceRoundTiles) * kPieceRoundTiles;
+        for (uint64_t bound = least; bound < best; bound += kPieceRoundTiles) {
+            // (most bounds fail by the number of pieces: one 32-bit division a query tile, and no more than that)
+            const uint32_t cap = static_cast<uint32_t>(bound), room = max_ctas / heads;
+            uint32_t pieces = 0;
+            for (size_t t = 0; t < tile_ctx.size() && pieces <= room; ++t) pieces += ((tile_ctx[t] - 1) / kKvTile + cap) / cap;
+            if (pieces <= room) {
+                uint64_t cost = 0;
+                for (uint32_t ctx : tile_ctx) {
+                    const uint32_t tiles = (ctx - 1) / kKvTile + 1, n = (tiles + cap - 1) / cap;
+                    const uint32_t rounds = ((tiles + n - 1) / n + kPieceRoundTiles - 1) / kPieceRoundTiles;
+                    cost = std::max<uint64_t>(cost, rounds * kPieceRoundTiles + (n > 1 ? kPieceMergeTiles + kPieceGroupTiles * ((n + 3) / 4) : 0));
+                }
+                if (cost < best) best = cost, pick = bound;
+            }
+            if (bound >= longest) break;
+        }
+    }
+    if (pick == 0) {
+        if (total != 0) share_out(plan, tile_ctx, heads, max_ctas, min_kv_tiles_per_cta, item_start_cost);
+        return plan;
+    }
+    plan.items.reserve(max_ctas);
+    plan.cta_item_begin.assign(1, 0);
+    for (uint32_t tile = 0; tile < plan.tiles.size(); ++tile) {
+        const uint64_t tiles = div_ceil(tile_ctx[tile], kKvTile), n = div_ceil(tiles, pick);
+        for (uint32_t h = 0; h < heads; ++h) {
+            for (uint64_t k = 0; k < n; ++k) {
+                WorkItem item{};
+                item.tile = tile;
+                item.head_sel = h;
+                item.kv_begin = static_cast<uint32_t>(tiles * k / n * kKvTile);
+                item.kv_end = static_cast<uint32_t>(std::min<uint64_t>(tiles * (k + 1) / n * kKvTile, tile_ctx[tile]));
+                plan.items.push_back(item);
+                plan.cta_item_begin.push_back(static_cast<uint32_t>(plan.items.size()));
+            }
+        }
+    }
+    finish_plan(plan);
+    return plan;
+}
+
+WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
+                             const uint32_t* cu_tokens, uint32_t num_reqs, uint32_t max_ctas,
+                             uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+    std::vector<uint32_t> all(num_reqs);
+    for (uint32_t r = 0; r < num_reqs; ++r) all[r] = r;
+    return build_balanced_plan(geo, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), all, max_ctas,
+                               min_kv_tiles_per_cta, item_start_cost);
+}
+
+WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
+                             uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+    WorkPlan plan;
+    std::vector<uint32_t> tile_ctx;
+    const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
+    const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
+    if (total != 0) share_out(plan, tile_ctx, heads, max_ctas, min_kv_tiles_per_cta, item_start_cost);
     return plan;
 }
 
