@@ -990,11 +990,11 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                 }
                 __syncwarp();  // the TMEM load of the next pass is warp-collective
             }
-            // The next item's first P V overwrites an accumulator as soon as its own stream's warps have delivered P.
-            if constexpr (kStreams == 2) {
-                tc_fence_before();
-                row_pair_sync(rows_warp);
-            }
+            // Both warps have read these rows' accumulators before either goes on.  The next item's first P V overwrites an
+            // accumulator as soon as four of the eight row warps have delivered its P (at head_dim 256 always the first four,
+            // and the others read half of that one O), and its Q K^T may be complete already.
+            tc_fence_before();
+            row_pair_sync(rows_warp);
             if (row_valid && half == 0) {
                 if (is_partial) {
                     p.partial_m[prow] = whole_max;
