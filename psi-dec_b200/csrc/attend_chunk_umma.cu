@@ -718,12 +718,12 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                 *reinterpret_cast<volatile uint32_t*>(&shared.cleaned[index & 1]) = index + 1;
             };
             uint32_t next_row = 0, next_rows = 0;  // this thread's row of the next item
-                if (index + 1 < item_end) {  // the next item's query rows travel under this item's tiles
-                    next_rows = next_rows_of.w * next_heads_of.w;
-                    const uint32_t r = row_id < next_rows ? row_id : 0;
-                    next_row = (next_rows_of.z + r / next_heads_of.w) * p.num_q_heads + next_heads_of.z + r % next_heads_of.w;
-                    stage_in(p.q, next_row, next_rows, column0, true);
-                }
+            if (index + 1 < item_end) {  // the next item's query rows travel under this item's tiles
+                next_rows = next_rows_of.w * next_heads_of.w;
+                const uint32_t r = row_id < next_rows ? row_id : 0;
+                next_row = (next_rows_of.z + r / next_heads_of.w) * p.num_q_heads + next_heads_of.z + r % next_heads_of.w;
+                stage_in(p.q, next_row, next_rows, column0, true);
+            }
             const bool more = index + 1 < item_end;
             const uint32_t end_tile = kStreams == 2 || half == 0 ? num_tiles : 0;
             for (uint32_t i = kStreams == 2 ? (tile_base ^ half) & 1u : 0u; i < end_tile; i += kStreams) {
@@ -866,13 +866,18 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                 __syncwarp();
             }
             // Both threads of a row finish it, back at the true max as the reference: l' = l * 2^(ref - max); O / l is unchanged
-            // by the shift.  With two streams O is the sum of their O_i * 2^(ref_i - max); one that saw no key takes no part.
+            // by the shift.  With two streams O is the sum of their O_i * 2^(ref_i - max).  A stream takes no part where it saw no
+            // key of the row, and only there: a weight that is no number (a score of +Inf) and the 0 x Inf of an infinity in V
+            // under a weight that underflows go into the row as they do with one stream.
             // (The exchange also says that the other warp's last P V is complete.)
-            float sum_at_max, weights[2] = {1.0f, 0.0f};  // of the stream of the item's first tile, and of the other
+            constexpr float kNoKey = -1.0f;
+            float sum_at_max, weights[2] = {1.0f, kNoKey};  // of the stream of the item's first tile, and of the other
             if constexpr (kStreams == 2) {
-                const float weight = row_max == -INFINITY ? (row_sum == 0.0f ? 0.0f : 1.0f) : fast_exp2(row_ref - whole_max);
+                const bool no_key = row_max == -INFINITY && row_sum == 0.0f;
+                // (scores that are no numbers alone leave the maximum at -Inf)
+                const float weight = no_key ? kNoKey : (row_max == -INFINITY ? 1.0f : fast_exp2(row_ref - whole_max));
                 const float other = exchange(weight);
-                row_sum *= weight;
+                if (!no_key) row_sum *= weight;
                 row_sum += exchange(row_sum);
                 sum_at_max = row_sum;
                 const bool first = ((tile_base ^ half) & 1u) == 0;
@@ -897,12 +902,12 @@ __device__ __forceinline__ void attend_chunk_umma(const AttendParams& p, const C
                     tmem_load16(tmem + kColO + first_stream * D + lane_base + c, o);
                     if constexpr (kStreams == 2) {
 #pragma unroll
-                        for (int e = 0; e < 16; ++e) o[e] = weights[0] > 0.0f ? o[e] * weights[0] : 0.0f;
+                        for (int e = 0; e < 16; ++e) o[e] = weights[0] == kNoKey ? 0.0f : o[e] * weights[0];
                         if (num_tiles > 1) {
                             float other[16];
                             tmem_load16(tmem + kColO + (first_stream ^ 1u) * D + lane_base + c, other);
 #pragma unroll
-                            for (int e = 0; e < 16; ++e) o[e] = weights[1] > 0.0f ? fmaf(other[e], weights[1], o[e]) : o[e];
+                            for (int e = 0; e < 16; ++e) o[e] = weights[1] == kNoKey ? o[e] : fmaf(other[e], weights[1], o[e]);
                         }
                     }
                 } else {
