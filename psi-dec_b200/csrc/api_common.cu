@@ -233,10 +233,7 @@ static void plan_runs(const psi_gqa* g, const RequestRuns& runs, uint64_t handic
     std::vector<uint32_t> decode_reqs, chunk_reqs;
     const ChunkRule rule = chunk_rule(g, handicap);
     const bool fine = split_requests(g, runs, rule, decode_reqs, chunk_reqs);
-    const uint32_t min_tiles = g->kernel == PSI_KERNEL_MMA ? 16u : 4u;
-    // (the CUDA-core kernels behind PSI_KERNEL_GENERIC keep the equal shares)
-    plan = g->cfg.kernel_mode == PSI_KERNEL_GENERIC ? build_balanced_plan(g->geo, runs, decode_reqs, g->grid_cap, min_tiles, g->item_start_cost)
-                                                    : build_decode_plan(g->geo, runs, decode_reqs, g->grid_cap, min_tiles, g->item_start_cost);
+    plan = build_decode_plan(g->geo, runs, decode_reqs, g->grid_cap, g->decode.min_tiles, g->decode.item_start_cost, g->decode.kernel);
     chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots, static_cast<uint32_t>(plan.reduces.size()),
                              chunk_order(g->geo, runs, chunk_reqs, rule.token_bytes), kChunkUnitCostTiles);
     chunk.fine = fine;

@@ -34,14 +34,9 @@ int32_t psi_gqa_create(psi_ctx* ctx, const psi_gqa_config* config, psi_gqa** out
         g->geo = plan_geometry(c.num_q_heads, c.num_kv_heads);
         const bool mma_ok = attend_mma_supported(c.dtype, c.head_dim, g->tokens_per_page);
         if (c.kernel_mode >= PSI_KERNEL_MMA) require(mma_ok, "the mma kernel does not support this profile");
-        g->kernel = (c.kernel_mode == PSI_KERNEL_GENERIC || !mma_ok) ? PSI_KERNEL_GENERIC : PSI_KERNEL_MMA;
-        g->any_mma = g->kernel == PSI_KERNEL_GENERIC && c.kernel_mode != PSI_KERNEL_GENERIC &&
-                     attend_mma_any_profile(c.dtype, c.head_dim);
-        const uint32_t per_sm =
-            g->kernel == PSI_KERNEL_MMA ? attend_mma_ctas_per_sm(c.head_dim)
-                                        : (g->any_mma ? 1u : attend_generic_ctas_per_sm(c.head_dim, c.dtype));
-        g->grid_cap = c.max_ctas > 0 ? c.max_ctas : static_cast<uint32_t>(ctx->sm_count) * per_sm;
-        g->item_start_cost = g->kernel == PSI_KERNEL_MMA ? kMmaItemStartCost : (g->any_mma ? kMmaAnyItemStartCost : 0u);
+        g->decode = decode_profile(c.kernel_mode, c.dtype, c.head_dim, g->tokens_per_page);
+        g->kernel = g->decode.kernel == DecodeKernel::kMma ? PSI_KERNEL_MMA : PSI_KERNEL_GENERIC;
+        g->grid_cap = c.max_ctas > 0 ? c.max_ctas : static_cast<uint32_t>(ctx->sm_count) * g->decode.ctas_per_sm;
         // (a component whose batches cannot hold a run of two query tiles never launches the long-run kernel, which under a
         // replay reservation would otherwise be part of every step)
         g->chunk_supported = g->kernel == PSI_KERNEL_MMA && c.plan_mode == PSI_PLAN_BALANCED && c.max_tokens > g->geo.tokens_per_tile &&

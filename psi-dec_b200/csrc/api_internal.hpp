@@ -187,10 +187,9 @@ struct psi_gqa {
     psi_gqa_config cfg{};
     uint32_t tokens_per_page = 0;
     uint32_t kernel = PSI_KERNEL_GENERIC;  // resolved kernel
-    bool any_mma = false;                  // the generic path runs on the tensor cores (attend_mma_any.cu)
+    psi::DecodeProfile decode{};           // and what its plans are made for
     uint32_t grid_cap = 1;
     bool exchanges = false;      // attend_exchange has been called: short runs leave its single launch only where that pays more
-    uint32_t item_start_cost = 0;  // KV tiles one item switch is worth when shares are balanced
     psi::PlanGeometry geo{};
     std::unique_ptr<psi::SplitKvSelector> selector;  // null when the profile is outside the reference selector's domain
     std::unique_ptr<psi::ReferenceMetadata> md;

@@ -395,11 +395,13 @@ cudaError_t launch_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
 
 // f32, head_dim a multiple of 32 up to 256 (a row is a whole number of 128-byte pieces), and arena, q and partial buffers
 // on 16-byte boundaries.  Other head dims and buffers stay on the staged kernel.
+bool attend_f32_profile(uint32_t dtype, uint32_t head_dim) {
+    return dtype == PSI_DTYPE_F32 && head_dim >= 32 && head_dim <= 256 && head_dim % 32 == 0;
+}
+
 bool attend_f32_supported(const AttendParams& p) {
     auto aligned = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; };
-    const uint32_t d = p.geo.head_dim;
-    return p.dtype == PSI_DTYPE_F32 && d >= 32 && d <= 256 && d % 32 == 0 && aligned(p.geo.pages) && aligned(p.q) &&
-           aligned(p.partial_o) && aligned(p.ext_o);
+    return attend_f32_profile(p.dtype, p.geo.head_dim) && aligned(p.geo.pages) && aligned(p.q) && aligned(p.partial_o) && aligned(p.ext_o);
 }
 
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {

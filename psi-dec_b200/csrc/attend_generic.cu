@@ -457,6 +457,15 @@ uint32_t attend_generic_ctas_per_sm(uint32_t head_dim, uint32_t dtype) {
     return head_dim % 4 == 0 ? attend_staged_ctas_per_sm(dtype) : 8u;
 }
 
+DecodeProfile decode_profile(uint32_t kernel_mode, uint32_t dtype, uint32_t head_dim, uint32_t tokens_per_page) {
+    const bool generic = kernel_mode == PSI_KERNEL_GENERIC;
+    if (!generic && attend_mma_supported(dtype, head_dim, tokens_per_page))
+        return {DecodeKernel::kMma, attend_mma_ctas_per_sm(head_dim), 16, kMmaItemStartCost};
+    if (!generic && attend_mma_any_profile(dtype, head_dim)) return {DecodeKernel::kMmaAny, 1, 4, kMmaAnyItemStartCost};
+    const bool f32 = !generic && attend_f32_profile(dtype, head_dim);
+    return {f32 ? DecodeKernel::kF32 : DecodeKernel::kCudaCore, attend_generic_ctas_per_sm(head_dim, dtype), 4, 0};
+}
+
 bool attend_generic_merges(const AttendParams& p) { return p.generic_only == 0 && (attend_mma_any_supported(p) || attend_f32_supported(p)); }
 
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {

@@ -387,14 +387,14 @@ void share_out(WorkPlan& plan, const std::vector<uint32_t>& tile_ctx, uint32_t h
 }  // namespace
 
 WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
-                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {
+                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost, DecodeKernel kernel) {
     WorkPlan plan;
     std::vector<uint32_t> tile_ctx;
     const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
     const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
     const uint64_t units = uint64_t(plan.tiles.size()) * heads;
     uint64_t pick = 0;
-    if (total != 0 && units <= max_ctas) {
+    if (kernel != DecodeKernel::kCudaCore && total != 0 && units <= max_ctas) {
         // What an equal share costs, in KV tiles: whole rounds of the share itself (of as many CTAs as that plan would take) with
         // a start for every unit, and a merge of pieces.
         const uint64_t ctas = std::min<uint64_t>(max_ctas, std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta)));

@@ -190,7 +190,11 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots,
 WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
                              uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost = 0);
 
-// The plan of the kernels that run one CTA of eight warps or more an SM.  Where every unit can be cut into equal pieces of one
+// The kernels that take decode rows: the tensor-core kernels of head_dim 64, 128 and 256 and of the odd 16-bit profiles, the f32
+// kernel, and the CUDA-core kernels of every other profile and of PSI_KERNEL_GENERIC (staged, or one warp an item).
+enum class DecodeKernel : uint32_t { kMma, kMmaAny, kF32, kCudaCore };
+
+// The plan of the kernels that run one CTA of eight warps or more an SM (all but kCudaCore).  Where every unit can be cut into equal pieces of one
 // CTA each, no CTA opens a second item, and pieces are whole rounds of a tile a warp: a step that does not fill the device is
 // then bounded by its longest piece and the merge, where an equal share may hold the ends of two units or many short ones.
 // The bound on a piece is the one with the smallest modelled cost, and the equal shares stay where theirs is smaller.  In KV
@@ -203,9 +207,13 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, c
 //   (A start counts 16 tiles where the shares count less: f32.)
 // Unequal steps the model leaves to the shares: 32 of 1,000 to 8,000 tokens, 16/2 x 256, 175.2 and 186.6 us; 16 of 500 to
 // 4,000 87.1 and 88.8; f32, 16 of 300 to 2,000, 32/8 x 128, 164.1 and 194.2.
+// The CUDA-core kernels always keep the shares: they have no warps that take a tile each, and run several CTAs an SM.  Four layers,
+// shares and these pieces: one request of 300 tokens, 40/8 heads, f32 x 80 76 and 112 us, bf16 x 84 112 and 210, x 66 389 and
+// 1,553; 8 of 370, 16/2 heads, 71 and 147, 90 and 260, 504 and 2,554.
 constexpr uint32_t kPieceRoundTiles = 8, kPieceMergeTiles = 14, kPieceGroupTiles = 4, kPieceStartTiles = 16;
 WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
-                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost);
+                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost,
+                           DecodeKernel kernel = DecodeKernel::kMma);
 
 // One CTA per (reference KV split, head_sel); reference q tiles wider than tokens_per_tile are cut into sub-tiles
 // that share the split boundaries.

@@ -213,12 +213,20 @@ bool attend_mma_any_profile(uint32_t dtype, uint32_t head_dim);
 bool attend_mma_any_supported(const AttendParams& p);
 cudaError_t launch_attend_mma_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 // The ring-fed f32 map kernel (attend_f32.cu): taken before the staged one when the launch qualifies.
+bool attend_f32_profile(uint32_t dtype, uint32_t head_dim);
 bool attend_f32_supported(const AttendParams& p);
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 // Whether launch_attend_generic takes a kernel that merges cut units itself (attend_mma_any, attend_f32) instead of leaving
 // them to launch_attend_reduce.
 bool attend_generic_merges(const AttendParams& p);
+// What a component plans its decode rows for: the kernel its profile takes on buffers that qualify, CTAs per SM, the fewest KV
+// tiles worth a CTA, and the cost of an item's start in the shares.
+struct DecodeProfile {
+    DecodeKernel kernel;
+    uint32_t ctas_per_sm, min_tiles, item_start_cost;
+};
+DecodeProfile decode_profile(uint32_t kernel_mode, uint32_t dtype, uint32_t head_dim, uint32_t tokens_per_page);
 // KV tiles one item switch is worth when shares are balanced: decode kernel, attend_mma_any (24 requests of 300 to 6,000
 // tokens at head_dim 96: 91 us a step with 0, 77 with 16, 87 with 64; the f32 kernel is best with 0).
 constexpr uint32_t kMmaItemStartCost = 32, kMmaAnyItemStartCost = 16;
