@@ -119,6 +119,7 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
         p.new_v = nullptr;
     }
     const uint32_t num_ctas = fixed ? g->grid_cap : plan.num_ctas();
+    p.merges = (fixed ? merges_in_launch(g->geo, g->grid_cap, g->cfg.head_dim) : plan.merges) ? 1u : 0u;
     p.item_tiles = fixed || plan.items.empty() ? 0u : static_cast<uint32_t>(std::min<uint64_t>(plan.total_kv_tiles / plan.items.size(), kU32Max));
     if (num_ctas > 0) {
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_MAP);
@@ -149,8 +150,8 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
         }
         cuda_check(launched, "attend (chunk) launch");
     }
-    // The tensor-core and the f32 kernels merge a unit's partials in the CTA that delivers the last one; the other CUDA-core
-    // kernels need the separate reduce pass.
+    // The mma kernel merges a unit's partials in the CTA that delivers the last one, the odd-profile and the f32 kernel do where
+    // that is short; what is left, and the units of the other CUDA-core kernels, takes the separate reduce pass.
     const uint32_t num_reduces = g->kernel == PSI_KERNEL_MMA || attend_generic_merges(p)
                                      ? 0u
                                      : static_cast<uint32_t>(fixed ? g->cap_reduces : plan.reduces.size());
@@ -234,6 +235,7 @@ static void plan_runs(const psi_gqa* g, const RequestRuns& runs, uint64_t handic
     const ChunkRule rule = chunk_rule(g, handicap);
     const bool fine = split_requests(g, runs, rule, decode_reqs, chunk_reqs);
     plan = build_decode_plan(g->geo, runs, decode_reqs, g->grid_cap, g->decode.min_tiles, g->decode.item_start_cost, g->decode.kernel);
+    plan.merges = merges_in_launch(g->geo, plan, g->cfg.head_dim);
     chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots, static_cast<uint32_t>(plan.reduces.size()),
                              chunk_order(g->geo, runs, chunk_reqs, rule.token_bytes), kChunkUnitCostTiles);
     chunk.fine = fine;
@@ -333,6 +335,7 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
         if (g->cfg.plan_mode == PSI_PLAN_REFERENCE) {
             g->plan = build_reference_plan(g->geo, *g->md, shape, variant.tiled_q != 0, token_indices, cu_tokens,
                                            num_reqs);
+            g->plan.merges = merges_in_launch(g->geo, g->plan, g->cfg.head_dim);
             g->chunk = ChunkPlan{};
             g->has_merged = false;
         } else {

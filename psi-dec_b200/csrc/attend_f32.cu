@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(W * 32, 1) attend_f32_kernel(AttendParams p) {
                 store_row(v, r, d, value, top, sum);
             }
         }
-        if (v.partial_slot != kU32Max && delivers_last_partial(p, v, shared.arrival)) {
+        if (p.merges != 0 && v.partial_slot != kU32Max && delivers_last_partial(p, v, shared.arrival)) {
             merge_unit<W * 32>(p, v, [&](uint32_t r, uint32_t d, float4 value, float top, float sum) { store_row(v, r, d, value, top, sum); });
         }
     }

@@ -466,7 +466,7 @@ DecodeProfile decode_profile(uint32_t kernel_mode, uint32_t dtype, uint32_t head
     return {f32 ? DecodeKernel::kF32 : DecodeKernel::kCudaCore, attend_generic_ctas_per_sm(head_dim, dtype), 4, 0};
 }
 
-bool attend_generic_merges(const AttendParams& p) { return p.generic_only == 0 && (attend_mma_any_supported(p) || attend_f32_supported(p)); }
+bool attend_generic_merges(const AttendParams& p) { return p.merges != 0 && p.generic_only == 0 && (attend_mma_any_supported(p) || attend_f32_supported(p)); }
 
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     if (num_ctas == 0) return cudaSuccess;

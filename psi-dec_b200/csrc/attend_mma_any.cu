@@ -394,7 +394,7 @@ __global__ void __launch_bounds__(kWarps * 32, 1) attend_mma_any_kernel(AttendPa
         }
         again = __syncthreads_or(not_finite && !again);
         if (again) continue;
-        if (v.partial_slot != kU32Max && delivers_last_partial(p, v, arrival_s)) {
+        if (p.merges != 0 && v.partial_slot != kU32Max && delivers_last_partial(p, v, arrival_s)) {
             merge_unit<kThreads>(p, v, [&](uint32_t r, uint32_t d, float4 value, float top, float sum) { store_row(v, r, d, value, top, sum); });
         }
         ++index;

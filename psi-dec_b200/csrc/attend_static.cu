@@ -214,6 +214,7 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         p.num_q_heads = c.num_q_heads;
         p.dtype = c.dtype;
         p.scale_log2 = c.scale * 1.4426950408889634f;
+        p.merges = merges_in_launch(geo, plan, c.head_dim) ? 1u : 0u;
         p.item_tiles = plan.items.empty() ? 0u : static_cast<uint32_t>(plan.total_kv_tiles / plan.items.size());
         p.generic_only = c.kernel_mode == PSI_KERNEL_GENERIC ? 1u : 0u;
         if (mma) {

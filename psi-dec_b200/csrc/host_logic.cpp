@@ -446,6 +446,18 @@ WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, con
     return plan;
 }
 
+bool merges_in_launch(const PlanGeometry& geo, const WorkPlan& plan, uint32_t head_dim) {
+    for (const ReduceUnit& unit : plan.reduces) {
+        const ExecTile& tile = plan.tiles[plan.items[unit.first_item].tile];
+        if (merge_shape(unit.num_items, (tile.flat_end - tile.flat_begin) * geo.heads_per_tile, head_dim, 256).trips > 2) return false;
+    }
+    return true;
+}
+
+bool merges_in_launch(const PlanGeometry& geo, uint32_t max_ctas, uint32_t head_dim) {
+    return merge_shape(max_ctas / (geo.num_kv_heads * geo.head_tiles) + 2, geo.heads_per_tile, head_dim, 256).trips <= 2;
+}
+
 WorkPlan build_balanced_plan(const PlanGeometry& geo, const uint32_t* req_slots, const uint32_t* token_indices,
                              const uint32_t* cu_tokens, uint32_t num_reqs, uint32_t max_ctas,
                              uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost) {

@@ -10,6 +10,12 @@
 
 #include "psi_cuda.h"
 
+#ifdef __CUDACC__
+#define PSI_HOST_DEVICE __host__ __device__
+#else
+#define PSI_HOST_DEVICE
+#endif
+
 namespace psi {
 
 // A violated caller contract (the reference panics); mapped to PSI_ERR_INVALID_ARGUMENT at the C ABI.
@@ -177,6 +183,7 @@ struct WorkPlan {
     std::vector<ReduceUnit> reduces;
     uint32_t num_partial_slots = 0;
     uint64_t total_kv_tiles = 0;
+    bool merges = false;  // merges_in_launch of this plan (prepare fills it in)
     uint32_t num_ctas() const { return cta_item_begin.empty() ? 0u : static_cast<uint32_t>(cta_item_begin.size() - 1); }
 };
 
@@ -214,6 +221,29 @@ constexpr uint32_t kPieceRoundTiles = 8, kPieceMergeTiles = 14, kPieceGroupTiles
 WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
                            uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost,
                            DecodeKernel kernel = DecodeKernel::kMma);
+
+// How a CTA of `threads` threads merges `pieces` partials of `rows` x head_dim outputs (unit_merge.cuh): `at_once` pieces are loaded
+// at a time, `ways` threads share the pieces of four columns, and `trips` is the number of round trips to the L2, one after
+// another.  Eight at a time only for more than eight pieces: replayed bf16 steps of 24/8 heads x 96, 8 requests of 100 to 4,000
+// tokens, 78.0 us with four and 80.2 with eight; f32 steps of one request of 2,500, 32/8 x 128 (19 pieces), 90 and 84.
+struct MergeShape {
+    uint32_t at_once, ways, trips;
+};
+PSI_HOST_DEVICE constexpr MergeShape merge_shape(uint32_t pieces, uint32_t rows, uint32_t head_dim, uint32_t threads) {
+    const uint32_t outputs = rows * head_dim / 4, at_once = pieces <= 8 ? 4 : 8;
+    uint32_t ways = 1;
+    while (pieces > 8 * ways && ways < 4 && 2 * ways * outputs <= threads) ways *= 2;
+    return {at_once, ways, (pieces + at_once * ways - 1) / (at_once * ways) * ((outputs * ways + threads - 1) / threads)};
+}
+// Whether the f32 and the odd-profile kernel merge a plan's cut units in the launch: only where no unit takes more than two round
+// trips, since one CTA merges a unit while the reduce launch has one for every row.  Four layers, replayed, in the launch (four
+// pieces at a time) and by the reduce launch: f32, 32/8 heads x 128, 16 requests of 100 tokens (one or two pieces) 42 and 53 us,
+// of 500 94 and 102, 4 of 2,500 (five pieces) 116 and 122; 16/2 x 256, 4 of 2,500 (19 pieces, two outputs a thread) 154 and 120;
+// 16/1 x 128, one of 5,000 (148 pieces) 236 and 112; bf16, 24/8 x 96, 8 of 370 52 and 59; 16/1 x 160, one of 5,000 256 and 98.
+bool merges_in_launch(const PlanGeometry& geo, const WorkPlan& plan, uint32_t head_dim);
+// The same for every plan of up to max_ctas CTAs (a replay reservation, whose launches are the same for all of them): a unit has
+// at most max_ctas / (units of a query tile) + 2 pieces.  Rows count as one token's.
+bool merges_in_launch(const PlanGeometry& geo, uint32_t max_ctas, uint32_t head_dim);
 
 // One CTA per (reference KV split, head_sel); reference q tiles wider than tokens_per_tile are cut into sub-tiles
 // that share the split boundaries.

@@ -123,7 +123,7 @@ struct AttendParams {
     float* partial_o;             // [slots][16][D] normalised
     float* partial_m;             // [slots][16] log2-domain max
     float* partial_l;             // [slots][16]
-    uint32_t* unit_counters;      // [reduce units], zero between launches: arrivals of a unit's items (mma kernel)
+    uint32_t* unit_counters;      // [reduce units], zero between launches: arrivals of a unit's items, in the kernels that merge cut units
     const uint32_t* scalars;
     uint32_t num_q_heads;
     uint32_t dtype;
@@ -132,6 +132,7 @@ struct AttendParams {
     uint32_t plan_ready;          // the plan was in place before the stream's previous kernel started (no kernel copies it)
     uint32_t generic_only;        // generic launches: PSI_KERNEL_GENERIC asks for the staged kernels where faster ones exist
     uint32_t chunk_weights;       // ChunkWeights of a long-run launch (tcgen05 kernel)
+    uint32_t merges;              // f32 and odd-profile kernels: cut units are merged in the launch (merges_in_launch)
     uint32_t item_tiles;          // KV tiles of an item on average, 0 where that is not known (more warps for long items)
     uint32_t tma_feed;            // decode kernel: whole K/V tiles by TMA boxes instead of cp.async (PSI_KERNEL_MMA_TMA)
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none
@@ -217,8 +218,8 @@ bool attend_f32_profile(uint32_t dtype, uint32_t head_dim);
 bool attend_f32_supported(const AttendParams& p);
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
 cudaError_t launch_attend_generic(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream);
-// Whether launch_attend_generic takes a kernel that merges cut units itself (attend_mma_any, attend_f32) instead of leaving
-// them to launch_attend_reduce.
+// Whether launch_attend_generic takes a kernel that can merge cut units itself (attend_mma_any, attend_f32) and p.merges tells
+// it to, instead of leaving them to launch_attend_reduce.
 bool attend_generic_merges(const AttendParams& p);
 // What a component plans its decode rows for: the kernel its profile takes on buffers that qualify, CTAs per SM, the fewest KV
 // tiles worth a CTA, and the cost of an item's start in the shares.
