@@ -234,7 +234,8 @@ static void plan_runs(const psi_gqa* g, const RequestRuns& runs, uint64_t handic
     std::vector<uint32_t> decode_reqs, chunk_reqs;
     const ChunkRule rule = chunk_rule(g, handicap);
     const bool fine = split_requests(g, runs, rule, decode_reqs, chunk_reqs);
-    plan = build_decode_plan(g->geo, runs, decode_reqs, g->grid_cap, g->decode.min_tiles, g->decode.item_start_cost, g->decode.kernel);
+    plan = build_decode_plan(g->geo, runs, decode_reqs, g->grid_cap, g->decode.min_tiles, g->decode.item_start_cost,
+                             piece_model(g->decode.kernel, g->cfg.head_dim));
     plan.merges = merges_in_launch(g->geo, plan, g->cfg.head_dim);
     chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots, static_cast<uint32_t>(plan.reduces.size()),
                              chunk_order(g->geo, runs, chunk_reqs, rule.token_bytes), kChunkUnitCostTiles);

@@ -387,25 +387,26 @@ void share_out(WorkPlan& plan, const std::vector<uint32_t>& tile_ctx, uint32_t h
 }  // namespace
 
 WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
-                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost, DecodeKernel kernel) {
+                           uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost, const PieceModel& model) {
     WorkPlan plan;
     std::vector<uint32_t> tile_ctx;
     const uint64_t total = list_tiles(geo, runs, requests, plan, tile_ctx);
     const uint32_t heads = geo.num_kv_heads * geo.head_tiles;
     const uint64_t units = uint64_t(plan.tiles.size()) * heads;
+    const uint32_t round = model.round_tiles;
     uint64_t pick = 0;
-    if (kernel != DecodeKernel::kCudaCore && total != 0 && units <= max_ctas) {
+    if (model.round_tiles != 0 && total != 0 && units <= max_ctas) {
         // What an equal share costs, in KV tiles: whole rounds of the share itself (of as many CTAs as that plan would take) with
         // a start for every unit, and a merge of pieces.
         const uint64_t ctas = std::min<uint64_t>(max_ctas, std::max<uint64_t>(1, total / std::max(1u, min_kv_tiles_per_cta)));
         const uint64_t share = (total + std::max(item_start_cost, kPieceStartTiles) * units) / ctas;
-        const uint64_t shares = div_ceil(share, kPieceRoundTiles) * kPieceRoundTiles + kPieceMergeTiles + kPieceGroupTiles;
+        const uint64_t shares = div_ceil(share, round) * round + model.merge_tiles + model.group_tiles;
         const uint64_t longest = div_ceil(*std::max_element(tile_ctx.begin(), tile_ctx.end()), kKvTile);
         uint64_t best = shares + 1;
         // (a bound between two multiples of the round cuts the units as the smaller one does; one that is not below `best`
         // leaves some unit a piece as long)
-        const uint64_t least = div_ceil(div_ceil(total, max_ctas), kPieceRoundTiles) * kPieceRoundTiles;
-        for (uint64_t bound = least; bound < best; bound += kPieceRoundTiles) {
+        const uint64_t least = div_ceil(div_ceil(total, max_ctas), round) * round;
+        for (uint64_t bound = least; bound < best; bound += round) {
             // (most bounds fail by the number of pieces: one 32-bit division a query tile, and no more than that)
             const uint32_t cap = static_cast<uint32_t>(bound), room = max_ctas / heads;
             uint32_t pieces = 0;
@@ -414,8 +415,8 @@ WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, con
                 uint64_t cost = 0;
                 for (uint32_t ctx : tile_ctx) {
                     const uint32_t tiles = (ctx - 1) / kKvTile + 1, n = (tiles + cap - 1) / cap;
-                    const uint32_t rounds = ((tiles + n - 1) / n + kPieceRoundTiles - 1) / kPieceRoundTiles;
-                    cost = std::max<uint64_t>(cost, rounds * kPieceRoundTiles + (n > 1 ? kPieceMergeTiles + kPieceGroupTiles * ((n + 3) / 4) : 0));
+                    const uint32_t rounds = ((tiles + n - 1) / n + round - 1) / round;
+                    cost = std::max<uint64_t>(cost, rounds * round + (n > 1 ? model.merge_tiles + model.group_tiles * ((n + 3) / 4) : 0));
                 }
                 if (cost < best) best = cost, pick = bound;
             }

@@ -201,26 +201,42 @@ WorkPlan build_balanced_plan(const PlanGeometry& geo, const RequestRuns& runs, c
 // kernel, and the CUDA-core kernels of every other profile and of PSI_KERNEL_GENERIC (staged, or one warp an item).
 enum class DecodeKernel : uint32_t { kMma, kMmaAny, kF32, kCudaCore };
 
-// The plan of the kernels that run one CTA of eight warps or more an SM (all but kCudaCore).  Where every unit can be cut into equal pieces of one
-// CTA each, no CTA opens a second item, and pieces are whole rounds of a tile a warp: a step that does not fill the device is
-// then bounded by its longest piece and the merge, where an equal share may hold the ends of two units or many short ones.
-// The bound on a piece is the one with the smallest modelled cost, and the equal shares stay where theirs is smaller.  In KV
-// tiles (eight, a round of all warps: 1.08 us at head_dim 128): a cut unit pays 14 for arrival and merge and 4 for every four
-// pieces, which are merged at a time (fitted on one request of 100 to 8,000 tokens cut in every way: 2.5 us a merge, 0.6 us
-// four pieces).  Replayed steps, equal shares and pieces:
+// The plan of the kernels that run one CTA of eight warps or more an SM (all but kCudaCore).  Where every unit can be cut into
+// equal pieces of one CTA each, no CTA opens a second item, and pieces are whole rounds of a tile a warp: a step that does not
+// fill the device is then bounded by its longest piece and the merge, where an equal share may hold the ends of two units or many
+// short ones.  The bound on a piece is the one with the smallest modelled cost, and the equal shares stay where theirs is smaller.
+// In KV tiles: a piece costs its rounds, a cut unit pays `merge_tiles` for arrival and merge and `group_tiles` for every four
+// pieces, and a start counts 16 in the shares where they count less (f32).
+struct PieceModel {
+    uint32_t round_tiles;  // 0: always the shares
+    uint32_t merge_tiles, group_tiles;
+};
+constexpr uint32_t kPieceStartTiles = 16;
+// The tensor-core kernel of the even profiles (eight tiles, a round of all warps, take 1.08 us at head_dim 128), fitted on one
+// request of 100 to 8,000 tokens cut in every way: 2.5 us a merge, 0.6 us four pieces.  Replayed steps, equal shares and pieces:
 //   one request of 777 tokens, 40/8 heads x 128, six layers: 75.9 and 64.6 us; of 100: 87.4 and 45.6; of 2,500: 82.2 and 77.1;
 //   four layers: 16 of 700 tokens 87.7 and 66.1; 8 of 1,000, 16/2 x 256, 76.7 and 64.0; 64 of 300 90.9 and 71.1; 16 of 1,000,
-//   32/8 x 64, 77.1 and 58.0; 24/8 x 96 102.9 and 84.3; f32 16/2 x 256 148.4 and 121.3; 16 of 4,000, 16/2 x 256, 126.4 and 125.5.
-//   (A start counts 16 tiles where the shares count less: f32.)
-// Unequal steps the model leaves to the shares: 32 of 1,000 to 8,000 tokens, 16/2 x 256, 175.2 and 186.6 us; 16 of 500 to
-// 4,000 87.1 and 88.8; f32, 16 of 300 to 2,000, 32/8 x 128, 164.1 and 194.2.
-// The CUDA-core kernels always keep the shares: they have no warps that take a tile each, and run several CTAs an SM.  Four layers,
-// shares and these pieces: one request of 300 tokens, 40/8 heads, f32 x 80 76 and 112 us, bf16 x 84 112 and 210, x 66 389 and
-// 1,553; 8 of 370, 16/2 heads, 71 and 147, 90 and 260, 504 and 2,554.
-constexpr uint32_t kPieceRoundTiles = 8, kPieceMergeTiles = 14, kPieceGroupTiles = 4, kPieceStartTiles = 16;
+//   32/8 x 64, 77.1 and 58.0; 24/8 x 96 102.9 and 84.3; 16 of 4,000, 16/2 x 256, 126.4 and 125.5.
+// Unequal steps it leaves to the shares: 32 of 1,000 to 8,000 tokens, 16/2 x 256, 175.2 and 186.6 us; 16 of 500 to 4,000 87.1 and
+// 88.8; f32, 16 of 300 to 2,000, 32/8 x 128, 164.1 and 194.2.
+constexpr PieceModel kMmaPieces{8, 14, 4};
+// An f32 round is eight tokens a warp, four tiles, and takes longer than a round above, so that a merge is worth fewer tiles; so
+// it is in the odd-profile kernel above head_dim 96, where half a round more of warps still saves time.  Replayed, four layers,
+// shares, the model above and this one: f32, 16/2 heads x 256, one request of 300 tokens 84, 107 and 63 us; 8 of 370 65, 120 and
+// 65; 4 of 600 87, 87 and 71; 16 of 1,000 136, 116 and 117; 32/8 x 128, one of 300 66, 61 and 51; 8 of 370 87, 72 and 65; 16/1 x
+// 128, 4 of 300 88, 108 and 71; bf16, 16/2 x 200, 8 of 370 63, 75 and 60; 24/8 x 120, 4 of 700 59, 60 and 54; 24/8 x 96, 8 of 370
+// 60, 52 and 53; 16/2 x 48, one of 300 49, 46 and 49.
+constexpr PieceModel kSlowRoundPieces{4, 6, 2};
+// The CUDA-core kernels have no warps that take a tile each, and run several CTAs an SM.  Four layers, shares and the first model:
+// one request of 300 tokens, 40/8 heads, f32 x 80 76 and 112 us, bf16 x 84 112 and 210, x 66 389 and 1,553; 8 of 370, 16/2 heads,
+// 71 and 147, 90 and 260, 504 and 2,554.
+constexpr PieceModel piece_model(DecodeKernel kernel, uint32_t head_dim) {
+    return kernel == DecodeKernel::kCudaCore ? PieceModel{0, 0, 0}
+           : kernel == DecodeKernel::kMma || (kernel == DecodeKernel::kMmaAny && head_dim <= 96) ? kMmaPieces : kSlowRoundPieces;
+}
 WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, const std::vector<uint32_t>& requests,
                            uint32_t max_ctas, uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost,
-                           DecodeKernel kernel = DecodeKernel::kMma);
+                           const PieceModel& model = kMmaPieces);
 
 // How a CTA of `threads` threads merges `pieces` partials of `rows` x head_dim outputs (unit_merge.cuh): `at_once` pieces are loaded
 // at a time, `ways` threads share the pieces of four columns, and `trips` is the number of round trips to the L2, one after

@@ -1,5 +1,7 @@
 // Where the f32 and the odd-profile kernel merge cut units: the bound on a unit's pieces that a replay reservation relies on, over
-// random steps, and that a reservation which merges in the launch does so for every plan of one-token requests.
+// random steps, and that a reservation which merges in the launch does so for every plan of one-token requests.  And how long the
+// pieces of a step are for each kernel.
+#include <algorithm>
 #include <cstdio>
 #include <random>
 
@@ -27,7 +29,7 @@ int main() {
         }
         const RequestRuns runs = plain_runs(slots.data(), positions.data(), cu.data(), n);
         for (DecodeKernel kernel : {DecodeKernel::kMmaAny, DecodeKernel::kF32}) {
-            const WorkPlan plan = build_decode_plan(geo, runs, all, max_ctas, 4, kernel == DecodeKernel::kF32 ? 0 : 16, kernel);
+            const WorkPlan plan = build_decode_plan(geo, runs, all, max_ctas, 4, kernel == DecodeKernel::kF32 ? 0 : 16, piece_model(kernel, trial % 4 ? 128 : 64));
             const uint32_t bound = max_ctas / (geo.num_kv_heads * geo.head_tiles) + 2;
             for (const ReduceUnit& unit : plan.reduces) {
                 CHECK(unit.num_items <= bound);
@@ -52,6 +54,33 @@ int main() {
         }
     }
     CHECK(many > 500 && merging > 500);
+
+    // The longest piece, in KV tiles, of steps timed with either model (0: equal shares).
+    struct Timed { uint32_t hq, hkv, requests, tokens; DecodeKernel kernel; uint32_t head_dim, longest; };
+    const Timed timed[] = {{16, 2, 1, 300, DecodeKernel::kF32, 256, 4}, {16, 2, 8, 370, DecodeKernel::kF32, 256, 0}, {16, 2, 4, 600, DecodeKernel::kF32, 256, 4},
+                           {32, 8, 1, 300, DecodeKernel::kF32, 128, 4}, {32, 8, 8, 370, DecodeKernel::kF32, 128, 12}, {16, 1, 4, 300, DecodeKernel::kF32, 128, 4},
+                           {16, 2, 16, 600, DecodeKernel::kMmaAny, 200, 10}, {24, 8, 4, 700, DecodeKernel::kMmaAny, 120, 11}, {24, 8, 8, 370, DecodeKernel::kMmaAny, 96, 24},
+                           {16, 2, 1, 300, DecodeKernel::kMmaAny, 48, 19}, {40, 8, 1, 300, DecodeKernel::kCudaCore, 80, 0}, {16, 2, 8, 370, DecodeKernel::kCudaCore, 66, 0}};
+    for (const Timed& t : timed) {
+        std::vector<uint32_t> slots, positions(t.requests, t.tokens), cu{0}, all;
+        for (uint32_t r = 0; r < t.requests; ++r) {
+            slots.push_back(r);
+            all.push_back(r);
+            cu.push_back(r + 1);
+        }
+        const WorkPlan plan = build_decode_plan(plan_geometry(t.hq, t.hkv), plain_runs(slots.data(), positions.data(), cu.data(), t.requests), all, 148, 4,
+                                                t.kernel == DecodeKernel::kMmaAny ? 16 : 0, piece_model(t.kernel, t.head_dim));
+        const WorkPlan shares = build_balanced_plan(plan_geometry(t.hq, t.hkv), plain_runs(slots.data(), positions.data(), cu.data(), t.requests), all, 148, 4,
+                                                    t.kernel == DecodeKernel::kMmaAny ? 16 : 0);
+        uint32_t longest = 0;
+        for (const WorkItem& item : plan.items) longest = std::max(longest, (item.kv_end - item.kv_begin + kKvTile - 1) / kKvTile);
+        if (plan.cta_item_begin == shares.cta_item_begin &&
+            std::equal(plan.items.begin(), plan.items.end(), shares.items.begin(), shares.items.end(),
+                       [](const WorkItem& a, const WorkItem& b) { return a.tile == b.tile && a.kv_begin == b.kv_begin && a.kv_end == b.kv_end; }))
+            longest = 0;
+        if (longest != t.longest) std::printf("%u x %u, %u/%u heads: %u\n", t.requests, t.tokens, t.hq, t.hkv, longest);
+        CHECK(longest == t.longest);
+    }
     std::printf("merges ok\n");
     return 0;
 }
