@@ -120,7 +120,8 @@ void run_attend(psi_gqa* g, const AttendParams& params) {
     }
     const uint32_t num_ctas = fixed ? g->grid_cap : plan.num_ctas();
     p.merges = (fixed ? merges_in_launch(g->geo, g->grid_cap, g->cfg.head_dim) : plan.merges) ? 1u : 0u;
-    p.item_tiles = fixed || plan.items.empty() ? 0u : static_cast<uint32_t>(std::min<uint64_t>(plan.total_kv_tiles / plan.items.size(), kU32Max));
+    p.item_tiles = fixed ? 0u : plan.item_tiles;
+    p.least_item_tiles = fixed ? 0u : plan.least_item_tiles;
     if (num_ctas > 0) {
         LaunchScope scope(ctx, PSI_KERNEL_CLASS_ATTEND_MAP);
         if (g->kernel == PSI_KERNEL_MMA) {
@@ -228,6 +229,14 @@ void run_staged_host_step(psi_gqa* g, psi_pages* pages, psi_table* table, uint32
 }
 
 
+// What launches of the plan look at.
+static void describe_plan(const psi_gqa* g, WorkPlan& plan) {
+    const ItemLengths lengths = item_lengths(plan);
+    plan.item_tiles = lengths.mean;
+    plan.least_item_tiles = lengths.least;
+    plan.merges = g->kernel != PSI_KERNEL_MMA && merges_in_launch(g->geo, plan, g->cfg.head_dim);
+}
+
 // This library's plan of a step: requests with a long run of query tokens go to the chunk kernel (one pass over their KV
 // for eight query tiles at a time); the rest are decode rows.
 static void plan_runs(const psi_gqa* g, const RequestRuns& runs, uint64_t handicap, WorkPlan& plan, ChunkPlan& chunk) {
@@ -236,7 +245,7 @@ static void plan_runs(const psi_gqa* g, const RequestRuns& runs, uint64_t handic
     const bool fine = split_requests(g, runs, rule, decode_reqs, chunk_reqs);
     plan = build_decode_plan(g->geo, runs, decode_reqs, g->grid_cap, g->decode.min_tiles, g->decode.item_start_cost,
                              piece_model(g->decode.kernel, g->cfg.head_dim));
-    plan.merges = merges_in_launch(g->geo, plan, g->cfg.head_dim);
+    describe_plan(g, plan);
     chunk = build_chunk_plan(g->geo, runs, chunk_reqs, g->grid_cap, plan.num_partial_slots, static_cast<uint32_t>(plan.reduces.size()),
                              chunk_order(g->geo, runs, chunk_reqs, rule.token_bytes), kChunkUnitCostTiles);
     chunk.fine = fine;
@@ -336,7 +345,7 @@ void prepare_impl(psi_gqa* g, const uint32_t* req_slots, const uint32_t* token_i
         if (g->cfg.plan_mode == PSI_PLAN_REFERENCE) {
             g->plan = build_reference_plan(g->geo, *g->md, shape, variant.tiled_q != 0, token_indices, cu_tokens,
                                            num_reqs);
-            g->plan.merges = merges_in_launch(g->geo, g->plan, g->cfg.head_dim);
+            describe_plan(g, g->plan);
             g->chunk = ChunkPlan{};
             g->has_merged = false;
         } else {

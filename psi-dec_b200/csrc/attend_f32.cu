@@ -379,7 +379,10 @@ __global__ void __launch_bounds__(W * 32, 1) attend_f32_kernel(AttendParams p) {
 // Two warps a scheduler leave half of the issue slots empty; short items have no tiles for more.  40 requests, 32/8 heads x 128,
 // four layers: 406 us with twelve warps and 445 with eight at 1,600 tokens each, 179 and 184 at 400, 142 both at 200, 108 and
 // 105 at 100.
-constexpr uint32_t kLongItemTiles = 20;
+// Where a CTA of many short items stands beside those of long ones it ends later still: 64 requests of 20 to 4,000 tokens, mostly
+// short, 655 us with twelve and 605 with eight (its items have 3 tiles on average); 32 of 50 to 20,000 791 and 782 (13 to 16); 60
+// of 200 to 8,000, 16/4 heads, 456 and 473 (18); 40 of 300 to 3,000 470 and 485 (22).
+constexpr uint32_t kLongItemTiles = 20, kLeastItemTiles = 16;
 
 template <int DG, int NSLOT, int W>
 cudaError_t launch_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
@@ -407,7 +410,8 @@ bool attend_f32_supported(const AttendParams& p) {
 cudaError_t launch_attend_f32(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     if (num_ctas == 0) return cudaSuccess;
     if (p.geo.head_dim > 128) return launch_f32<2, 3, 8>(p, num_ctas, stream);
-    return p.item_tiles >= kLongItemTiles ? launch_f32<1, 4, 12>(p, num_ctas, stream) : launch_f32<1, 6, 8>(p, num_ctas, stream);
+    const bool long_items = p.item_tiles >= kLongItemTiles && p.least_item_tiles >= kLeastItemTiles;
+    return long_items ? launch_f32<1, 4, 12>(p, num_ctas, stream) : launch_f32<1, 6, 8>(p, num_ctas, stream);
 }
 
 }  // namespace psi

@@ -415,12 +415,15 @@ cudaError_t launch_any(const AttendParams& p, uint32_t num_ctas, cudaStream_t st
 // A tile is a chain of latencies, and two warps a scheduler leave 68 % of the issue slots empty; short items have no tiles for
 // more.  40 requests, 24/8 heads x 96, pages of 12, four layers: 227 us with sixteen warps and 242 with eight at 1,600 tokens each,
 // 165 both at 800, 124 and 120 at 400.  (Above 96 the accumulators leave registers for eight warps.)
-constexpr uint32_t kLongItemTiles = 64;
+// A CTA of many short items beside long ones ends last: 24 requests of 300 to 6,000 tokens, more short than long ones, 194 us with
+// sixteen and 189 with eight (16 to 20 tiles an item in that CTA); 40 of 100 to 10,000 301 and 295 (10); as many short as long
+// ones, 251 and 256 (24); 80-wide heads, 24 of 400 to 12,000, 270 and 285 (27).
+constexpr uint32_t kLongItemTiles = 64, kLeastItemTiles = 20;
 
 template <typename T, bool kAligned>
 cudaError_t launch_for_dim(const AttendParams& p, uint32_t num_ctas, cudaStream_t stream) {
     const uint32_t d = p.geo.head_dim;
-    if (p.item_tiles >= kLongItemTiles) {
+    if (p.item_tiles >= kLongItemTiles && p.least_item_tiles >= kLeastItemTiles) {
         if (d <= 64) return launch_any<T, 64, 5, 16, kAligned>(p, num_ctas, stream);
         if (d <= 96) return launch_any<T, 96, 4, 16, kAligned>(p, num_ctas, stream);
     }

@@ -215,7 +215,9 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         p.dtype = c.dtype;
         p.scale_log2 = c.scale * 1.4426950408889634f;
         p.merges = merges_in_launch(geo, plan, c.head_dim) ? 1u : 0u;
-        p.item_tiles = plan.items.empty() ? 0u : static_cast<uint32_t>(plan.total_kv_tiles / plan.items.size());
+        const ItemLengths lengths = item_lengths(plan);
+        p.item_tiles = lengths.mean;
+        p.least_item_tiles = lengths.least;
         p.generic_only = c.kernel_mode == PSI_KERNEL_GENERIC ? 1u : 0u;
         if (mma) {
             err = launch_attend_mma(p, plan.num_ctas(), stream);

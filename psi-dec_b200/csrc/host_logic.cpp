@@ -447,6 +447,20 @@ WorkPlan build_decode_plan(const PlanGeometry& geo, const RequestRuns& runs, con
     return plan;
 }
 
+ItemLengths item_lengths(const WorkPlan& plan) {
+    ItemLengths lengths{0, kU32Max};
+    if (plan.items.empty()) return lengths;
+    lengths.mean = static_cast<uint32_t>(std::min<uint64_t>(plan.total_kv_tiles / plan.items.size(), kU32Max));
+    for (uint32_t c = 0; c < plan.num_ctas(); ++c) {
+        const uint32_t begin = plan.cta_item_begin[c], end = plan.cta_item_begin[c + 1];
+        if (end - begin < 2) continue;
+        uint64_t tiles = 0;
+        for (uint32_t i = begin; i < end; ++i) tiles += div_ceil(plan.items[i].kv_end - plan.items[i].kv_begin, kKvTile);
+        lengths.least = static_cast<uint32_t>(std::min<uint64_t>(tiles / (end - begin), lengths.least));
+    }
+    return lengths;
+}
+
 bool merges_in_launch(const PlanGeometry& geo, const WorkPlan& plan, uint32_t head_dim) {
     for (const ReduceUnit& unit : plan.reduces) {
         const ExecTile& tile = plan.tiles[plan.items[unit.first_item].tile];

@@ -183,7 +183,9 @@ struct WorkPlan {
     std::vector<ReduceUnit> reduces;
     uint32_t num_partial_slots = 0;
     uint64_t total_kv_tiles = 0;
-    bool merges = false;  // merges_in_launch of this plan (prepare fills it in)
+    // what a launch of the plan looks at, where its kernel does: merges_in_launch and item_lengths
+    bool merges = false;
+    uint32_t item_tiles = 0, least_item_tiles = 0;
     uint32_t num_ctas() const { return cta_item_begin.empty() ? 0u : static_cast<uint32_t>(cta_item_begin.size() - 1); }
 };
 
@@ -260,6 +262,13 @@ bool merges_in_launch(const PlanGeometry& geo, const WorkPlan& plan, uint32_t he
 // The same for every plan of up to max_ctas CTAs (a replay reservation, whose launches are the same for all of them): a unit has
 // at most max_ctas / (units of a query tile) + 2 pieces.  Rows count as one token's.
 bool merges_in_launch(const PlanGeometry& geo, uint32_t max_ctas, uint32_t head_dim);
+
+// KV tiles of an item: over the plan, and in the CTA of several items whose are the shortest (kU32Max: every CTA has one).  More
+// warps an item pay where items are long, and the CTA of many short ones ends last with them.
+struct ItemLengths {
+    uint32_t mean, least;
+};
+ItemLengths item_lengths(const WorkPlan& plan);
 
 // One CTA per (reference KV split, head_sel); reference q tiles wider than tokens_per_tile are cut into sub-tiles
 // that share the split boundaries.

@@ -133,7 +133,9 @@ struct AttendParams {
     uint32_t generic_only;        // generic launches: PSI_KERNEL_GENERIC asks for the staged kernels where faster ones exist
     uint32_t chunk_weights;       // ChunkWeights of a long-run launch (tcgen05 kernel)
     uint32_t merges;              // f32 and odd-profile kernels: cut units are merged in the launch (merges_in_launch)
-    uint32_t item_tiles;          // KV tiles of an item on average, 0 where that is not known (more warps for long items)
+    // KV tiles of an item on average and in the CTA of the shortest ones (ItemLengths), 0 where they are not known: more warps
+    // for long items
+    uint32_t item_tiles, least_item_tiles;
     uint32_t tma_feed;            // decode kernel: whole K/V tiles by TMA boxes instead of cp.async (PSI_KERNEL_MMA_TMA)
     ExchangeParams xchg;          // KV-range exchange in the same launch (mma kernel); xchg.flag == nullptr: none
 };

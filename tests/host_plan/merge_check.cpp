@@ -81,6 +81,23 @@ int main() {
         if (longest != t.longest) std::printf("%u x %u, %u/%u heads: %u\n", t.requests, t.tokens, t.hq, t.hkv, longest);
         CHECK(longest == t.longest);
     }
+    // Item lengths: a step of equal pieces has no CTA of several items; one long request among short ones has a long mean and a
+    // CTA of short items, which is what the kernels with more warps look at.
+    for (const bool unequal : {false, true}) {
+        std::vector<uint32_t> slots, positions, cu{0}, all;
+        for (uint32_t r = 0; r < (unequal ? 40u : 4u); ++r) {
+            slots.push_back(r);
+            all.push_back(r);
+            positions.push_back(!unequal ? 1000 : r < 4 ? 60000 : 60);
+            cu.push_back(r + 1);
+        }
+        const WorkPlan plan = build_decode_plan(plan_geometry(32, 8), plain_runs(slots.data(), positions.data(), cu.data(), cu.back()), all, 148, 4, 0, kSlowRoundPieces);
+        const ItemLengths lengths = item_lengths(plan);
+        CHECK(lengths.mean == plan.total_kv_tiles / plan.items.size());
+        if (unequal) CHECK(lengths.mean >= 64 && lengths.least < 16);
+        else CHECK(lengths.least == kU32Max);
+    }
+    CHECK(item_lengths(WorkPlan{}).mean == 0);
     std::printf("merges ok\n");
     return 0;
 }
