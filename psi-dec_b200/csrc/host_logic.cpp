@@ -464,7 +464,8 @@ ItemLengths item_lengths(const WorkPlan& plan) {
 bool merges_in_launch(const PlanGeometry& geo, const WorkPlan& plan, uint32_t head_dim) {
     for (const ReduceUnit& unit : plan.reduces) {
         const ExecTile& tile = plan.tiles[plan.items[unit.first_item].tile];
-        if (merge_shape(unit.num_items, (tile.flat_end - tile.flat_begin) * geo.heads_per_tile, head_dim, 256).trips > 2) return false;
+        if (unit.num_items > 8 || merge_shape(unit.num_items, (tile.flat_end - tile.flat_begin) * geo.heads_per_tile, head_dim, 256).trips > 2)
+            return false;
     }
     return true;
 }

@@ -253,14 +253,17 @@ PSI_HOST_DEVICE constexpr MergeShape merge_shape(uint32_t pieces, uint32_t rows,
     while (pieces > 8 * ways && ways < 4 && 2 * ways * outputs <= threads) ways *= 2;
     return {at_once, ways, (pieces + at_once * ways - 1) / (at_once * ways) * ((outputs * ways + threads - 1) / threads)};
 }
-// Whether the f32 and the odd-profile kernel merge a plan's cut units in the launch: only where no unit takes more than two round
-// trips, since one CTA merges a unit while the reduce launch has one for every row.  Four layers, replayed, in the launch (four
-// pieces at a time) and by the reduce launch: f32, 32/8 heads x 128, 16 requests of 100 tokens (one or two pieces) 42 and 53 us,
-// of 500 94 and 102, 4 of 2,500 (five pieces) 116 and 122; 16/2 x 256, 4 of 2,500 (19 pieces, two outputs a thread) 154 and 120;
-// 16/1 x 128, one of 5,000 (148 pieces) 236 and 112; bf16, 24/8 x 96, 8 of 370 52 and 59; 16/1 x 160, one of 5,000 256 and 98.
+// Whether the f32 and the odd-profile kernel merge a plan's cut units in the launch: only where no unit has more than eight pieces
+// or takes more than two round trips, since one CTA merges a unit while the reduce launch has one for every row.  Four layers, in
+// the launch (four pieces at a time) and by the reduce launch: f32, 32/8 heads x 128, 16 requests of 100 tokens (one or two
+// pieces) 42 and 53 us, of 500 94 and 102, 4 of 2,500 (five pieces) 116 and 122, 2 of 8,000 (ten) 168 and 163, one of 20,000 (19)
+// 205 and 187; 16/2 x 256, 4 of 2,500 (19 pieces, two outputs a thread) 154 and 120; 16/1 x 128, one of 5,000 (148 pieces) 236 and
+// 112; bf16, 24/8 x 96, 8 of 370 52 and 59; 16/1 x 160, one of 5,000 256 and 98.
 bool merges_in_launch(const PlanGeometry& geo, const WorkPlan& plan, uint32_t head_dim);
 // The same for every plan of up to max_ctas CTAs (a replay reservation, whose launches are the same for all of them): a unit has
-// at most max_ctas / (units of a query tile) + 2 pieces.  Rows count as one token's.
+// at most max_ctas / (units of a query tile) + 2 pieces, which may be more than eight here, as most steps' units have fewer: 32/8
+// heads x 128 as above, replayed, 16 of 500 92 us in the launch and 102 with the reduce launch, one of 2,500 86 and 79.  Rows
+// count as one token's.
 bool merges_in_launch(const PlanGeometry& geo, uint32_t max_ctas, uint32_t head_dim);
 
 // KV tiles of an item: over the plan, and in the CTA of several items whose are the shortest (kU32Max: every CTA has one).  More

@@ -36,18 +36,19 @@ int main() {
                 many += unit.num_items > 8;
             }
             for (uint32_t head_dim : {32u, 96u, 128u, 256u}) {
-                bool few = true;
+                bool few = true, short_merges = true;
                 for (const ReduceUnit& unit : plan.reduces) {
                     const ExecTile& tile = plan.tiles[plan.items[unit.first_item].tile];
                     const uint32_t rows = (tile.flat_end - tile.flat_begin) * geo.heads_per_tile;
                     const MergeShape shape = merge_shape(unit.num_items, rows, head_dim, 256);
                     CHECK(shape.ways == 1 || shape.ways == 2 || shape.ways == 4);
                     CHECK(uint64_t(shape.trips) * shape.at_once * 256 >= uint64_t(unit.num_items) * rows * head_dim / 4);
-                    few = few && shape.trips <= 2;
+                    short_merges = short_merges && shape.trips <= 2;
+                    few = few && shape.trips <= 2 && unit.num_items <= 8;
                 }
                 CHECK(merges_in_launch(geo, plan, head_dim) == few);
                 if (one_token && merges_in_launch(geo, max_ctas, head_dim)) {
-                    CHECK(few);
+                    CHECK(short_merges);
                     merging += !plan.reduces.empty();
                 }
             }
