@@ -29,7 +29,7 @@ namespace {
 // Capacity of the fixed scratch.  A step that needs more is rejected before anything is enqueued.
 constexpr uint32_t kStaticMaxCtas = PSI_STATIC_MAX_CTAS;
 constexpr uint32_t kStaticMaxItems = PSI_STATIC_MAX_ITEMS;
-constexpr uint32_t kStaticMaxSlots = 2 * kStaticMaxCtas;  // a CTA share cuts at most two units
+constexpr uint32_t kStaticMaxSlots = 2 * kStaticMaxCtas;  // a CTA share cuts at most two units, a piece is one of a CTA
 constexpr uint32_t kStaticMaxHeadDim = 256;
 
 constexpr uint64_t align_up(uint64_t v, uint64_t a) { return (v + a - 1) / a * a; }
@@ -146,18 +146,18 @@ extern "C" int32_t psi_gqa_attend_static(int32_t device, void* cuda_stream, cons
         err = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
         if (err != cudaSuccess) return fail(PSI_ERR_CUDA, cudaGetErrorString(err), error, error_len);
 
-        // Plan on the host as psi_gqa_prepare does in PSI_PLAN_BALANCED (same kernel choice, same balance costs), with
+        // Plan on the host as psi_gqa_prepare does in PSI_PLAN_BALANCED (same kernel choice, same costs, pieces or shares), with
         // the CTA count capped by the scratch.  Long query runs stay on this kernel: the chunk kernels are not used.
         const PlanGeometry geo = plan_geometry(c.num_q_heads, c.num_kv_heads);
-        const bool mma = c.kernel_mode != PSI_KERNEL_GENERIC && attend_mma_supported(c.dtype, c.head_dim, tokens_per_page);
+        const DecodeProfile profile = decode_profile(c.kernel_mode, c.dtype, c.head_dim, tokens_per_page);
+        const bool mma = profile.kernel == DecodeKernel::kMma;
         require(mma || c.kernel_mode < PSI_KERNEL_MMA, "the mma kernel does not support this profile");
-        const bool any_mma = !mma && c.kernel_mode != PSI_KERNEL_GENERIC && attend_mma_any_profile(c.dtype, c.head_dim);
-        const uint32_t per_sm = mma ? attend_mma_ctas_per_sm(c.head_dim)
-                                    : (any_mma ? 1u : attend_generic_ctas_per_sm(c.head_dim, c.dtype));
-        uint32_t max_ctas = std::min<uint32_t>(kStaticMaxCtas, static_cast<uint32_t>(sm_count) * per_sm);
+        uint32_t max_ctas = std::min<uint32_t>(kStaticMaxCtas, static_cast<uint32_t>(sm_count) * profile.ctas_per_sm);
         if (c.max_ctas > 0) max_ctas = std::min(max_ctas, c.max_ctas);
-        const WorkPlan plan = build_balanced_plan(geo, req_slots, token_indices, cu_tokens, num_reqs, max_ctas,
-                                                  mma ? 16u : 4u, mma ? kMmaItemStartCost : (any_mma ? kMmaAnyItemStartCost : 0u));
+        std::vector<uint32_t> requests(num_reqs);
+        for (uint32_t r = 0; r < num_reqs; ++r) requests[r] = r;
+        const WorkPlan plan = build_decode_plan(geo, plain_runs(req_slots, token_indices, cu_tokens, num_reqs), requests, max_ctas, profile.min_tiles,
+                                                profile.item_start_cost, piece_model(profile.kernel, c.head_dim));
         if (plan.items.size() > kStaticMaxItems) {
             return fail(PSI_ERR_INVALID_ARGUMENT,
                         "the step needs " + std::to_string(plan.items.size()) + " work items; the static scratch holds " +
