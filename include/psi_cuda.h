@@ -301,8 +301,9 @@ PSI_API int32_t psi_metadata_update_host(uint32_t max_tokens, const uint32_t* re
                                          uint32_t* buf_flat_token_indices, uint32_t* buf_q_token_tiles,
                                          uint32_t* buf_kv_splits, uint32_t* buf_cu_kv_splits,
                                          psi_replay_shape* out_shape);
-/* The balanced device work plan of a batch, computed on the host (what psi_gqa_prepare uploads in PSI_PLAN_BALANCED
- * unless every unit can be cut into equal pieces of one CTA each and that is cheaper).  out_items receives 6 u32 per item {q tile, head selection, kv_begin, kv_end, partial slot or
+/* Equal shares of a batch's decode work, computed on the host: what psi_gqa_prepare uploads in PSI_PLAN_BALANCED, with the
+ * CTAs, fewest tiles a CTA and start cost of the profile's kernel, where it does not take equal pieces
+ * (psi_decode_plan_preview).  out_items receives 6 u32 per item {q tile, head selection, kv_begin, kv_end, partial slot or
  * 0xFFFFFFFF, flat token begin of the tile}; out_cta_item_begin receives num_ctas+1 entries; out_counts receives
  * {items, ctas, partial slots, reduce units, q tiles, total 16-token KV tiles (saturated)}.  item_start_cost is the
  * number of KV tiles one additional item is charged when the shares are balanced.  No reference counterpart:
@@ -312,6 +313,14 @@ PSI_API int32_t psi_plan_preview(uint32_t num_q_heads, uint32_t num_kv_heads, co
                                  uint32_t min_kv_tiles_per_cta, uint32_t item_start_cost, uint32_t* out_items,
                                  uint64_t items_cap, uint32_t* out_cta_item_begin, uint64_t cta_cap,
                                  uint32_t* out_counts);
+
+/* The decode plan that psi_gqa_prepare uploads in PSI_PLAN_BALANCED for a batch of a component with this configuration and
+ * `max_ctas` CTAs, where no request goes to the long-query kernels: the equal shares above, or every unit in equal pieces of
+ * one CTA each where the profile's kernel takes them and that is cheaper.  Of the configuration the head counts, head_dim,
+ * dtype, page_bytes and kernel_mode are read.  Outputs as above.  No reference counterpart. */
+PSI_API int32_t psi_decode_plan_preview(const psi_gqa_config* config, const uint32_t* token_indices, const uint32_t* cu_tokens,
+                                        uint32_t num_reqs, uint32_t max_ctas, uint32_t* out_items, uint64_t items_cap,
+                                        uint32_t* out_cta_item_begin, uint64_t cta_cap, uint32_t* out_counts);
 
 /* The work plan of the long-query (chunk) kernels for a batch in which EVERY request carries a long run, computed on
  * the host.  equal_shares selects contiguous shares of equal size instead of stream order; the third order psi_gqa_prepare

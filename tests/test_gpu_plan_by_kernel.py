@@ -3,6 +3,7 @@ each; the CUDA-core kernels keep the equal shares that psi_plan_preview lays out
 import numpy as np
 import pytest
 
+import decode_preview as P
 import gpuharness as G
 import hostapi as H
 import workloads as W
@@ -39,3 +40,14 @@ def test_the_other_kernels_take_pieces(dtype, head_dim, min_tiles, start_cost):
     stats = s.gqa.plan_stats()
     s.close()
     assert stats["items"] == stats["ctas"] >= 64
+
+
+@pytest.mark.parametrize("dtype,heads,head_dim,page", [(pkg.BF16, (40, 8), 128, 8), (pkg.F16, (16, 4), 64, 16), (pkg.BF16, (24, 8), 96, 12), (pkg.BF16, (16, 2), 200, 16),
+                                                       (pkg.F32, (16, 2), 256, 16), (pkg.F32, (8, 2), 80, 16), (pkg.BF16, (4, 2), 66, 16)])
+@pytest.mark.parametrize("contexts", [[300], [777, 3], [370] * 8, [1000, 40, 9000]])
+def test_the_preview_is_what_prepare_uploads(dtype, heads, head_dim, page, contexts):
+    s = W.Session(W.Spec("plan", dtype, *heads, head_dim, page, contexts, [1] * len(contexts), seed=95), max_ctas=100)
+    stats = s.gqa.plan_stats()
+    s.close()
+    counts = P.preview(P.config(dtype, heads, head_dim, page, pkg.KERNEL_AUTO), contexts, np.arange(len(contexts) + 1), 100)[2]
+    assert tuple(int(x) for x in counts) == tuple(stats[k] for k in ("items", "ctas", "partial_slots", "reduce_units", "q_tiles", "kv_tiles"))
