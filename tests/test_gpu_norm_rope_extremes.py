@@ -1,6 +1,6 @@
 """The vectorised front-stage kernel at the ends of its arithmetic, against the general one on the same inputs: rows of zeros
-(also with eps 0: 0 / 0), rows whose squares overflow f32 (1 / rms is 0) or underflow, rows with an infinity or a NaN, and a
-rotation with an attention factor.  A projection that starts off a 16-byte boundary takes the general kernel."""
+(also with eps 0: 0 / 0), rows at the ends of their type (in f32 and bf16 with squares that overflow f32, where 1 / rms is 0, or
+underflow), rows with an infinity or a NaN, and a rotation with an attention factor.  A projection that starts off a 16-byte boundary takes the general kernel."""
 import numpy as np
 import pytest
 
@@ -22,7 +22,8 @@ def test_extreme_rows_equal_the_general_kernel(dtype, eps, yarn, runs):
     spec = W.Spec("ends", dtype, 6, 2, 128, 16, [300, 4], runs, seed=29)
     weights = [O.encode(np.linspace(0.5, 1.5, 128).astype(np.float32), O.BF16).tolist() for _ in range(2)]
     width = 2 * (6 + 2) * 128
-    big, small = (3e38, 1e-30) if dtype != pkg.F16 else (6e4, 6e-8)  # (their squares: beyond f32, or beyond it downwards)
+    # (their squares lie beyond f32, or beyond it downwards; f16 ends long before: its squares are ordinary f32 values)
+    big, small = (3e38, 1e-30) if dtype != pkg.F16 else (6e4, 6e-8)
     got = []
     for shift in (0, 1):
         s = W.Session(spec)
@@ -44,14 +45,22 @@ def test_extreme_rows_equal_the_general_kernel(dtype, eps, yarn, runs):
         got.append([O.decode(checks.to_numpy_bits(x).reshape(-1), dtype).astype(np.float64) for x in (q, gates, s.arena)])
         s.close()
     # As beside the ordinary rows: the two kernels' 1 / rms differ by an ulp or two of f32 (2^-22 with the sum's order), which
-    # may turn over either rounding of a normalised element to 16 bits; a rotated output adds two of them and rounds again.
+    # may turn over either rounding of a normalised element to 16 bits, an ulp of it each.  A rotated output adds two of them,
+    # x1 cos - x2 sin, so that two ulps of (x1, x2)'s length bound what they bring in (the rotation keeps the length, and the
+    # factor is part of the outputs'), and rounds again.  Other elements have their own size for it.
     ulp = {pkg.F32: 2.0 ** -21, pkg.BF16: 2.0 ** -7, pkg.F16: 2.0 ** -10}[dtype]
     for a, b in zip(*got):
         assert np.array_equal(np.isnan(a), np.isnan(b))
         assert np.array_equal(np.isposinf(a), np.isposinf(b)) and np.array_equal(np.isneginf(a), np.isneginf(b))
+        rows = b.reshape(-1, 128)
+        with np.errstate(all="ignore"):
+            length = np.abs(rows)
+            pair = np.tile(np.hypot(rows[:, :32], rows[:, 32:64]), 2)
+        length[:, :64] = np.where(np.isfinite(pair), pair, length[:, :64])  # (a value's neighbour may be no number)
+        length = length.reshape(-1)
         fine = np.isfinite(a) & np.isfinite(b)
-        a, b = a[fine], b[fine]
+        a, b, length = a[fine], b[fine], length[fine]
         near = np.abs(b) < 1e4  # (gates and values pass through with the inputs' size: those are equal)
         assert np.array_equal(a[~near], b[~near])
-        a, b = a[near], b[near]
-        assert np.all(np.abs(a - b) <= 2 * ulp * 2 ** 0.5 * max(np.abs(b).max(), 1.0) * 1.25 + ulp * np.abs(b))
+        a, b, length = a[near], b[near], length[near]
+        assert np.all(np.abs(a - b) <= 2 * ulp * length + ulp * np.abs(b))
