@@ -1,10 +1,10 @@
 // Split-KV flash-decode map kernel for f32 pages: CUDA cores fed from per-warp shared-memory rings.
 //
-// Same work items, partial slots and reduce pass as the other CUDA-core map kernels (attend_generic.cu); head_dim must be
-// a multiple of 32.  Bound by HBM: a K and a V row of 2 * 4 * D bytes feed at most 16 query rows, 2 to 8 flop/B, so f32
-// FMAs keep up as long as shared memory does.  One CTA of eight warps per SM (twelve for long items up to head_dim 128,
-// kLongItemTiles); every warp owns every eighth (twelfth) 8-token tile of the item and streams it through a ring of its own (K tile, V tile, K tile, ...) by 16-byte cp.async, so there is no
-// CTA-wide barrier between the start and the end of an item.  Per tile:
+// Same work items and partial slots as the other CUDA-core map kernels (attend_generic.cu); head_dim must be a multiple of 32.
+// Bound by HBM: a K and a V row of 2 * 4 * D bytes feed at most 16 query rows, 2 to 8 flop/B, so f32 FMAs keep up as long as
+// shared memory does.  One CTA of eight warps per SM (twelve for long items up to head_dim 128, kLongItemTiles); every warp owns
+// every eighth (twelfth) 8-token tile of the item and streams it through a ring of its own (K tile, V tile, K tile, ...) by
+// 16-byte cp.async, so there is no CTA-wide barrier between the start and the end of an item.  Per tile:
 //   scores   lane = (token pair, eighth of the row): two tokens per lane halve the reads of q, which are the larger part
 //            of the shared-memory traffic; eight lanes read 128 consecutive bytes, so no access has a bank conflict.  The
 //            2 R partial sums are reduced and scattered over the eight lanes in one butterfly, which leaves R / 4 of the
@@ -12,11 +12,11 @@
 //   softmax  online, in the log2 domain, on those scores; O is rescaled only when a row's maximum moved;
 //   values   lane = four (or two times four) columns of every row; the weights are read back as broadcasts.
 // The row count is rounded up to 4, 8 or 16 per item, each with code of its own.  All arithmetic is f32.
-// Cut units are merged by the CTA that delivers their last partial, and each warp's first two tiles are requested into the L2
-// while the append runs.  Measured: 16 requests of 4,096 to 12,288 tokens, 32/8 heads x 128 (1.07 GB), a whole step with the
-// append 190 us = 5.6 TB/s; 210 with eight warps and six ring slots each, whose issue slots were half idle with two warps a
-// scheduler (map launch 194 us; 172 with twelve and four slots, 178 with sixteen and three), 517 with the staged kernel,
-// whose shared-memory traffic grows with every row.
+// Units cut into a few pieces are merged by the CTA that delivers the last partial, the others by the reduce launch
+// (merges_in_launch), and each warp's first two tiles are requested into the L2 while the append runs.  Measured: 16 requests of
+// 4,096 to 12,288 tokens, 32/8 heads x 128 (1.07 GB), a whole step with the append 203 us = 5.3 TB/s; 224 with eight warps
+// and six ring slots each and a reduce launch (map launch alone, with two warps a scheduler, 194 us; 172 with twelve and four
+// slots, 178 with sixteen and three), 517 with the staged kernel, whose shared-memory traffic grows with every row.
 #include <atomic>
 
 #include "launch_util.hpp"

@@ -1,18 +1,16 @@
 // Split-KV flash-decode map kernel on the tensor cores for the 16-bit profiles attend_mma.cu does not take: head dims
 // that are no multiple of 64 (any multiple of eight up to 256) and any page size.
 //
-// Same work items, partial slots and reduce pass as the CUDA-core kernels (attend_generic.cu), whose arithmetic it keeps:
-// the weights stay f32.  Each is split into three 16-bit parts, and O += P V runs once per part; K, V and q are 16-bit values
+// Same work items and partial slots as the CUDA-core kernels (attend_generic.cu), whose arithmetic it keeps: the weights stay f32.  Each is split into three 16-bit parts, and O += P V runs once per part; K, V and q are 16-bit values
 // already and all accumulators are f32.  In bf16, which has f32's exponents, the parts add up to the weight exactly.  f16
 // ends at steps of 2^-24, so there the weights are taken 2^15 times as large (kWeightShift): exact down to 2^-16 of the
 // heaviest key of the warp, and within 2^-40 of it below that, where f32 sums over an item do not see it.  Bound by HBM; the
 // tensor pipe has room for the two extra products.  One CTA of eight warps per SM (sixteen for long items up to head_dim 96,
 // kLongItemTiles), every warp owning every eighth (sixteenth) 16-token tile of the item and a ring of its own (K tile, V tile,
-// K tile, ...) fed by 16-byte cp.async, the next tile's page looked up one
-// tile ahead.  Rows are padded to DP elements plus one 16-byte chunk: an odd number of chunks per row keeps ldmatrix free
+// K tile, ...) fed by 16-byte cp.async, the next tile's page looked up one tile ahead.  Rows are padded to DP elements plus one 16-byte chunk: an odd number of chunks per row keeps ldmatrix free
 // of bank conflicts without a swizzle, and the chunks beyond head_dim hold zeros.
-// Cut units are merged by the CTA that delivers their last partial, and each warp's first two tiles are requested into the L2
-// while the append runs.  Measured: 24 requests of 300 to 6,000 tokens, 24/8 heads x 96, pages of 12 (233 MB): 72.7 us a
+// Units cut into a few pieces are merged by the CTA that delivers the last partial, the others by the reduce launch
+// (merges_in_launch), and each warp's first two tiles are requested into the L2 while the append runs.  Measured: 24 requests of 300 to 6,000 tokens, 24/8 heads x 96, pages of 12 (233 MB): 72.7 us a
 // step with the append = 3.2 TB/s; 74.2 with eight warps and eight slots each, 79 against 75.7 with twelve and five, 75.0 with
 // the reduce as a launch of its own, 466 on the staged kernel.
 #include <atomic>

@@ -300,8 +300,10 @@ constexpr uint32_t kChunkMaxPieces = 16;      // equal shares: a unit is cut int
 constexpr uint32_t kChunkWholeTokens = 2 * kChunkMinPieceTiles * 16;  // units of at most this many keys are not worth a cut
 constexpr uint32_t kChunkStartCostTiles = 8;   // fixed cost of a work item (query load, epilogue) in KV tiles, stream order
 // The same in the other orders, for every piece of a unit: query rows, first tiles and epilogue, in the time of 16-token tiles
-// (about 7 us).  0 to 64 measured the same on whole units; with equal shares (16 requests of 512 to 16,384 tokens, eight rows
-// each, 40/8 heads x 128, pages of 8) a layer took 80.2 us with 16, 81.7 with 32, 93.7 with 48.
+// (about 7 us).  0 to 64 measured the same on whole units.  Equal shares, two layers, with 12, 16, 20, 24, 28, 32 and 40: 16 requests
+// of 512 to 16,384 tokens, eight rows each, 40/8 heads x 128 169, 164, 164, 161, 163, 160 and 162 us; 64 of 100 to 4,000, four rows
+// each, 199, 192, 180, 177, 177, 175 and 177; 24 of 300 to 12,000, eight rows, 32/8 x 128 174, 169, 166, 164, 163, 163 and 166; at
+// head_dim 256 a little less is better: 24 of 2,500, eight rows, 16/2 heads 102, 102, 100, 105, 108, 107 and 106.
 constexpr uint32_t kChunkUnitCostTiles = 28;
 
 // How the units of a chunk plan are dealt to CTAs.
