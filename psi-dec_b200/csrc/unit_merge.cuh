@@ -21,7 +21,7 @@ __device__ __forceinline__ bool delivers_last_partial(const AttendParams& p, con
 }
 
 // Merges the unit's partials: M = max m_i, w_i = 2^(m_i - M) * l_i (0 when m_i is not finite), out = sum w_i o_i / sum w_i
-// (0 when empty), crates/inference-backend-metal/src/components/metal/gqa_split_kv_single_q_reduce.metal:27-48.  A thread owns
+// (0 when empty), as the reduce launch has it (crates/inference-backend-metal/src/components/metal/gqa_split_kv_single_q_reduce.metal:27-48).  A thread owns
 // four columns of a row; the pieces' statistics and values go out four pieces at a time.  `store(r, d, value, m, l)` takes
 // columns [d, d + 4) of row r.
 template <int kThreadCount, typename Store>
